@@ -4,8 +4,19 @@
 //          7 NormSiTU; the Norm codes first divide the gate row by rms = sqrt(mean(g^2) + 1e-6).
 //   codes 3 (Identity) and 4 (Zero) are expert KINDS without weights: their rows are copied / zeroed.
 // Semantics follow kernels/sm75/moe.py:163-232 (_glu_fwd_row_kernel, _glu_bwd_row_kernel) and
-// :859-881 (_act_eager) of the reference; math in fp32, bf16 in and out.  One CTA per padded row.
+// :859-881 (_act_eager) of the reference; math in fp32, bf16 in and out.
+//
+// Bound: HBM (forward 3 I, backward 5 I bf16 values a row) and, close behind it, the exponentials.  The kernels that
+// carry the path (`glu_*_vec_kernel`) hold a row in registers: TPR threads share a row, each with VPT 16-byte vectors of
+// every operand, all loaded before the first use, so a row is read once however many reductions its activation needs.
+// Rows of one CTA lie inside one 256-row tile and share its expert, so the activation code is uniform over the CTA and
+// the element loops are compiled per code.  The one-value-per-thread kernels below them read each value with a
+// 2-byte access, once per reduction; they remain for d_ff that is no multiple of 8 or above 8192 and for unaligned
+// buffers.  32 768 rows, d_ff 768, codes 0 1 2 5 6 7 in turn: forward 86 -> 40 us,
+// backward 194 -> 78 us (56 us of it at copy rate for both).
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -41,6 +52,238 @@ __device__ __forceinline__ float act_value(int code, float gate, float gn, float
   return gn * sig;   // codes 0 and 2
 }
 
+// ---------------------------------------------------------------------------- a row held in registers
+constexpr int kRowThreads = 256;
+
+// sum over the TPR threads of a row; every thread of the CTA calls it (uniformly)
+template <int TPR>
+__device__ __forceinline__ float row_sum(float v, float* red) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if constexpr (TPR > 32) {
+    const int warp = threadIdx.x >> 5;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[warp] = v;
+    __syncthreads();
+    const int w0 = warp & ~(TPR / 32 - 1);
+    v = 0.0f;
+#pragma unroll
+    for (int i = 0; i < TPR / 32; ++i) v += red[w0 + i];
+  }
+  return v;
+}
+
+// activation value and its derivative with respect to gn (gn = gate, or gate / rms for the Norm codes).  Code 5:
+// dal = d(act)/d(alpha), t5s = act / gamma
+template <int CODE>
+__device__ __forceinline__ void act_eval(float gn, float alpha, float gamma, float& act, float& d, float& dal, float& t5s) {
+  if constexpr (CODE == 1 || CODE == 6) {
+    const float r = fmaxf(gn, 0.0f);
+    act = r * r;
+    d = 2.0f * r;
+  } else {
+    const float sig = sigmoidf_(gn);
+    if constexpr (CODE == 5) {
+      const float t5 = tanh_via_sigmoid(alpha * gn);
+      t5s = t5 * sig;
+      act = gamma * t5s;
+      d = gamma * (alpha * (1.0f - t5 * t5) * sig + t5s * (1.0f - sig));
+      dal = gamma * gn * (1.0f - t5 * t5) * sig;
+    } else if constexpr (CODE == 7) {
+      const float tg = tanh_via_sigmoid(gn);
+      act = tg * sig;
+      d = (1.0f - tg * tg) * sig + tg * sig * (1.0f - sig);
+    } else {
+      act = gn * sig;
+      d = sig * (1.0f + gn * (1.0f - sig));
+    }
+  }
+}
+
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
+template <int TPR, int VPT>
+__device__ __forceinline__ float row_rms_inv(const uint4 (&g)[VPT], int I, float* red) {
+  float ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    float f[8];
+    unpack8(g[i], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+  }
+  ss = row_sum<TPR>(ss, red);
+  return 1.0f / sqrtf(ss / static_cast<float>(I) + kRmsEps);
+}
+
+template <int CODE, int TPR, int VPT>
+__device__ __forceinline__ void glu_fwd_row(const uint4 (&g)[VPT], const uint4 (&u)[VPT], uint4* dst, int t, int nvec,
+                                            float alpha, float gamma, float* red) {
+  constexpr bool NORM = CODE == 2 || CODE == 6 || CODE == 7;
+  float inv_r = 1.0f;
+  if constexpr (NORM) inv_r = row_rms_inv<TPR, VPT>(g, nvec * 8, red);
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = t + TPR * i;
+    if (c >= nvec) continue;
+    float gf[8], uf[8];
+    unpack8(g[i], gf);
+    unpack8(u[i], uf);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float act, d, dal, t5s;
+      act_eval<CODE>(NORM ? gf[j] * inv_r : gf[j], alpha, gamma, act, d, dal, t5s);
+      gf[j] = act * uf[j];
+    }
+    dst[c] = pack8(gf);
+  }
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+glu_fwd_vec_kernel(const uint4* __restrict__ gate_up, const int* __restrict__ tile_expert, const int* __restrict__ codes,
+                   const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
+                   uint4* __restrict__ inter) {
+  constexpr int RPB = kRowThreads / TPR;   // rows a CTA works on at a time; divides the 256-row tile
+  __shared__ float red[kRowThreads / 32];
+  const int total = *total_rows;
+  const int t = threadIdx.x % TPR;
+  for (long long r0 = static_cast<long long>(blockIdx.x) * RPB; r0 < total; r0 += static_cast<long long>(gridDim.x) * RPB) {
+    const long long r = r0 + threadIdx.x / TPR;
+    const bool live = r < total;
+    const int n = live ? nvec : 0;         // a row past the end takes part in the reductions with zeros
+    uint4 g[VPT], u[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c = t + TPR * i;
+      g[i] = c < n ? gate_up[r * (2LL * nvec) + c] : make_uint4(0u, 0u, 0u, 0u);
+      u[i] = c < n ? gate_up[r * (2LL * nvec) + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const int e = tile_expert[r0 / B200MOE_TILE_M];
+    const int code = codes[e];
+    const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
+    const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
+    uint4* dst = inter + r * nvec;
+    switch (code) {                        // uniform over the CTA
+      case 1: glu_fwd_row<1, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+      case 2: glu_fwd_row<2, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+      case 5: glu_fwd_row<5, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+      case 6: glu_fwd_row<6, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+      case 7: glu_fwd_row<7, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+      default: glu_fwd_row<0, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
+    }
+  }
+}
+
+// da / dg: this thread's share of the row's alpha / gamma gradient (code 5 only)
+template <int CODE, int TPR, int VPT>
+__device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (&u)[VPT], const uint4 (&go)[VPT],
+                                            uint4* gg, uint4* gu, int t, int nvec, float alpha, float gamma, float* red,
+                                            float& da, float& dg) {
+  constexpr bool NORM = CODE == 2 || CODE == 6 || CODE == 7;
+  float inv_r = 1.0f, S = 0.0f;
+  float act[NORM ? 8 * VPT : 8], d[NORM ? 8 * VPT : 8];
+  float dal = 0.0f, t5s = 0.0f;
+  if constexpr (NORM) {   // RMS coupling term: mean of go * up * f'(gn) * gn
+    inv_r = row_rms_inv<TPR, VPT>(g, nvec * 8, red);
+    float part = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      float gf[8], uf[8], of[8];
+      unpack8(g[i], gf);
+      unpack8(u[i], uf);
+      unpack8(go[i], of);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float gn = gf[j] * inv_r;
+        act_eval<CODE>(gn, alpha, gamma, act[8 * i + j], d[8 * i + j], dal, t5s);
+        part += of[j] * uf[j] * d[8 * i + j] * gn;
+      }
+    }
+    S = row_sum<TPR>(part, red) / static_cast<float>(nvec * 8);
+  }
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = t + TPR * i;
+    if (c >= nvec) continue;
+    float gf[8], uf[8], of[8];
+    unpack8(g[i], gf);
+    unpack8(u[i], uf);
+    unpack8(go[i], of);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int q = NORM ? 8 * i + j : j;
+      if constexpr (!NORM) act_eval<CODE>(gf[j], alpha, gamma, act[q], d[q], dal, t5s);
+      const float gi = of[j], w = gi * uf[j];
+      if constexpr (CODE == 5) {
+        da += w * dal;
+        dg += w * t5s;
+      }
+      gf[j] = NORM ? (w * d[q] - S * (gf[j] * inv_r)) * inv_r : w * d[q];
+      uf[j] = gi * act[q];
+    }
+    gg[c] = pack8(gf);
+    gu[c] = pack8(uf);
+  }
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+glu_bwd_vec_kernel(const uint4* __restrict__ grad_inter, const uint4* __restrict__ gate_up,
+                   const int* __restrict__ tile_expert, const int* __restrict__ codes,
+                   const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
+                   uint4* __restrict__ grad_gate_up, float* __restrict__ row_da, float* __restrict__ row_dg) {
+  constexpr int RPB = kRowThreads / TPR;
+  __shared__ float red[kRowThreads / 32];
+  const int total = *total_rows;
+  const int t = threadIdx.x % TPR;
+  for (long long r0 = static_cast<long long>(blockIdx.x) * RPB; r0 < total; r0 += static_cast<long long>(gridDim.x) * RPB) {
+    const long long r = r0 + threadIdx.x / TPR;
+    const bool live = r < total;
+    const int n = live ? nvec : 0;
+    uint4 g[VPT], u[VPT], go[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c = t + TPR * i;
+      g[i] = c < n ? gate_up[r * (2LL * nvec) + c] : make_uint4(0u, 0u, 0u, 0u);
+      u[i] = c < n ? gate_up[r * (2LL * nvec) + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+      go[i] = c < n ? grad_inter[r * nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const int e = tile_expert[r0 / B200MOE_TILE_M];
+    const int code = codes[e];
+    const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
+    const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
+    uint4* gg = grad_gate_up + r * (2LL * nvec);
+    uint4* gu = gg + nvec;
+    float da = 0.0f, dg = 0.0f;
+    switch (code) {                        // uniform over the CTA
+      case 1: glu_bwd_row<1, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+      case 2: glu_bwd_row<2, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+      case 5: glu_bwd_row<5, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+      case 6: glu_bwd_row<6, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+      case 7: glu_bwd_row<7, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+      default: glu_bwd_row<0, TPR, VPT>(g, u, go, gg, gu, t, n, alpha, gamma, red, da, dg); break;
+    }
+    if (row_da != nullptr) {
+      if (code == 5) {
+        da = row_sum<TPR>(da, red);
+        dg = row_sum<TPR>(dg, red);
+      }
+      if (live && t == 0) {
+        row_da[r] = da;
+        row_dg[r] = dg;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------- one value per thread
 __global__ void __launch_bounds__(256)
 glu_fwd_rows_kernel(const __nv_bfloat16* __restrict__ gate_up, const int* __restrict__ tile_expert,
                     const int* __restrict__ codes, const float* __restrict__ params, const int* __restrict__ total_rows,
@@ -162,11 +405,13 @@ glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ grad_inter, const __nv_bfl
   }
 }
 
-// out[e] = (sum of row_da over the rows of e, sum of row_dg): deterministic, one CTA per expert
-__global__ void __launch_bounds__(256)
+// out[e] = (sum of row_da over the rows of e, sum of row_dg): deterministic, one CTA per expert.  Bound by the latency
+// of its loads: 1024 threads keep a segment's rows in flight in a few rounds (3000 rows an expert: 8.7 -> 4.1 us with 256 -> 1024).
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads)
 expert_row_sums_kernel(const float* __restrict__ row_da, const float* __restrict__ row_dg, const int* __restrict__ poffs,
                        float* __restrict__ out) {
-  __shared__ float red[8];
+  __shared__ float red[kSumThreads / 32];
   const int e = blockIdx.x;
   float a = 0.0f, b = 0.0f;
   for (int r = poffs[e] + threadIdx.x; r < poffs[e + 1]; r += blockDim.x) {
@@ -195,11 +440,28 @@ special_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ tile_
   }
 }
 
+static long long ceil_div64(long long a, long long b) { return (a + b - 1) / b; }
 static int rows_grid(long long rows_cap) {
   long long g = rows_cap;
   const long long cap = static_cast<long long>(num_sms()) * 16;
   if (g > cap) g = cap;
   return static_cast<int>(g < 1 ? 1 : g);
+}
+
+// The register-resident kernels take 16-byte-aligned rows of at most 8192 values
+constexpr int64_t kMaxVecWidth = 8192;
+static bool rows_in_registers(int64_t I, const void* a, const void* b, const void* c) {
+  return I % 8 == 0 && I <= kMaxVecWidth && aligned16(a) && aligned16(b) && aligned16(c);
+}
+// f(TPR, VPT): the narrowest row group that holds nvec vectors; two vectors of each operand a thread keep the backward
+// near 100 registers, so a wider row takes more threads first
+template <class F>
+static void by_row_width(int nvec, F f) {
+  if (nvec <= 64) f(std::integral_constant<int, 32>(), std::integral_constant<int, 2>());
+  else if (nvec <= 128) f(std::integral_constant<int, 64>(), std::integral_constant<int, 2>());
+  else if (nvec <= 256) f(std::integral_constant<int, 128>(), std::integral_constant<int, 2>());
+  else if (nvec <= 512) f(std::integral_constant<int, 256>(), std::integral_constant<int, 2>());
+  else f(std::integral_constant<int, 256>(), std::integral_constant<int, 4>());
 }
 
 }  // namespace b200moe
@@ -214,6 +476,16 @@ int b200moe_glu_fwd_rows(const void* gate_up, const int32_t* tile_expert, const 
   B200_CHECK_ARG(gate_up && tile_expert && act_codes && total_rows && inter, B200MOE_E_NULL, "glu_fwd_rows: null pointer");
   B200_CHECK_ARG(I > 0, B200MOE_E_BAD_SHAPE, "glu_fwd_rows: I = %lld", (long long)I);
   if (rows_cap <= 0) return 0;
+  if (rows_in_registers(I, gate_up, inter, inter)) {
+    const int nvec = static_cast<int>(I / 8);
+    by_row_width(nvec, [&](auto tpr, auto vpt) {
+      glu_fwd_vec_kernel<tpr.value, vpt.value><<<rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)), kRowThreads, 0, (cudaStream_t)stream>>>(
+          reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes, act_params, total_rows, nvec,
+          reinterpret_cast<uint4*>(inter));
+    });
+    B200_CUDA(cudaGetLastError());
+    return 0;
+  }
   glu_fwd_rows_kernel<<<rows_grid(rows_cap), 256, 0, (cudaStream_t)stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert, act_codes, act_params, total_rows, static_cast<int>(I),
       reinterpret_cast<__nv_bfloat16*>(inter));
@@ -229,6 +501,16 @@ int b200moe_glu_bwd_rows(const void* grad_inter, const void* gate_up, const int3
   B200_CHECK_ARG((row_da == nullptr) == (row_dg == nullptr), B200MOE_E_NULL, "glu_bwd_rows: row_da and row_dg go together");
   B200_CHECK_ARG(I > 0, B200MOE_E_BAD_SHAPE, "glu_bwd_rows: I = %lld", (long long)I);
   if (rows_cap <= 0) return 0;
+  if (rows_in_registers(I, grad_inter, gate_up, grad_gate_up)) {
+    const int nvec = static_cast<int>(I / 8);
+    by_row_width(nvec, [&](auto tpr, auto vpt) {
+      glu_bwd_vec_kernel<tpr.value, vpt.value><<<rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)), kRowThreads, 0, (cudaStream_t)stream>>>(
+          reinterpret_cast<const uint4*>(grad_inter), reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes,
+          act_params, total_rows, nvec, reinterpret_cast<uint4*>(grad_gate_up), row_da, row_dg);
+    });
+    B200_CUDA(cudaGetLastError());
+    return 0;
+  }
   glu_bwd_rows_kernel<<<rows_grid(rows_cap), 256, 0, (cudaStream_t)stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(grad_inter), reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert,
       act_codes, act_params, total_rows, static_cast<int>(I), reinterpret_cast<__nv_bfloat16*>(grad_gate_up), row_da, row_dg);
@@ -240,7 +522,7 @@ int b200moe_expert_row_sums(const float* row_da, const float* row_dg, const int3
                             b200moe_stream_t stream) {
   B200_CHECK_ARG(row_da && row_dg && poffs && out, B200MOE_E_NULL, "expert_row_sums: null pointer");
   B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_row_sums: E = %d", E);
-  expert_row_sums_kernel<<<E, 256, 0, (cudaStream_t)stream>>>(row_da, row_dg, poffs, out);
+  expert_row_sums_kernel<<<E, kSumThreads, 0, (cudaStream_t)stream>>>(row_da, row_dg, poffs, out);
   B200_CUDA(cudaGetLastError());
   return 0;
 }
