@@ -173,6 +173,16 @@ int b200moe_expert_gate_up_act(const void* x_s, const void* gate_up_proj, const 
                                const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo,
                                int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
                                int32_t* status, b200moe_stream_t stream);
+/* The forward products for few rows per expert, over rows in COMPACT expert order (b200moe_permute_build's `order`):
+ * rows [offs[e], offs[e] + counts[e]) belong to expert e, rows_cap (>= offs[E]) bounds the buffers, E <= 256.  The
+ * weights are the MMA's M operand, so the work follows the live rows in steps of 16 instead of 256-row tiles.
+ * gate_up_few: inter (rows,I) = act(gate) * up without storing gate_up (act_codes as above, NULL = SiLU);
+ * linear_few: out (rows,N) = x (rows,K) * W[e]^T, W (E,N,K).  Same rounding points as the row-tile kernels. */
+int b200moe_expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
+                               const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, void* inter,
+                               int32_t* status, b200moe_stream_t stream);
+int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap,
+                              int E, int64_t N, int64_t K, void* out, int32_t* status, b200moe_stream_t stream);
 /* Generic grouped products over the padded rows (the two entry points after them are special cases):
  * linear:   out (rows,N) = a (rows,K) * W[e]^T, W (E,N,K)   -- kernels/sm75/moe.py:765,770 (x @ W[e].t())
  * linear_t: out (rows,N) = a (rows,K) * W[e],   W (E,K,N)   -- kernels/sm75/moe.py:807,822 (g @ W[e]) */

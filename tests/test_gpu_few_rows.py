@@ -1,0 +1,69 @@
+"""GPU: the grouped products for few rows per expert against the row-tile kernels and an fp32 reference."""
+import importlib
+
+import pytest
+import torch
+
+from oracle import moe_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# one bf16 rounding of the result (2^-9 of each value) on fp32 sums
+TOL = 2.1e-3
+
+
+# rows an expert gets: none, one, both sides of the 16-row step and of the 64 / 128 / 192-row tiles, several tiles;
+# widths that fill no tile, one k-block and a remainder, the smallest
+@pytest.mark.parametrize("counts,H,I", [([1], 8, 8), ([0, 1, 0, 15, 16, 17, 0], 72, 136), ([63, 64, 65, 0], 256, 128),
+                                        ([129, 100, 0, 128], 1032, 680), ([193, 150, 192, 0, 385], 264, 200),
+                                        ([700, 0, 0, 0, 0, 0, 0, 0], 512, 264), ([2] * 256, 64, 128)])
+@pytest.mark.parametrize("codes", [False, True])
+def test_few_rows_products(pkg, counts, H, I, codes):
+    E, M = len(counts), sum(counts)
+    g = torch.Generator().manual_seed(M + H)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(M, generator=g)].view(M, 1).to(DEV)
+    x = torch.randn(M, H, generator=g).to(torch.bfloat16).to(DEV)
+    gu = (torch.randn(E, 2 * I, H, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    dn = (torch.randn(E, H, I, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    act = torch.tensor([(0, 1, 5)[e % 3] for e in range(E)], dtype=torch.int32, device=DEV) if codes else None
+    ops = pkg.ops
+    perm = ops.permute_build(idx, E, want_order=True)
+    inter = ops.expert_gate_up_few(ops.gather_compact(x, perm), gu, perm, act)
+    out = ops.expert_linear_few(inter, dn, perm)
+    pkg.check_status()
+    # the same rounding points and k order as the row-tile kernels: bit-identical
+    _, ref_inter = ops.expert_gate_up_swiglu(ops.gather_rows(x, perm), gu, perm, act)
+    ref_out = ops.expert_down(ref_inter, dn, perm)
+    r, c = perm.slot_row.long(), perm.slot_pos.long()
+    assert torch.equal(inter[c], ref_inter[r]) and torch.equal(out[c], ref_out[r])
+    e = idx[:, 0].cpu()
+    ref = torch.einsum("mi,mhi->mh", inter[c].cpu().float(), dn.cpu().float()[e])
+    assert O.rel_l2(out[c].cpu().float(), ref) < TOL
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 8, 2), (40, 16, 4), (1279, 16, 2), (1281, 16, 2)])   # both sides of the limit
+def test_forward_without_gradient_equals_the_training_forward(pkg, T, E, k):
+    torch.manual_seed(T)
+    layer = pkg.MoELayer(264, 136, E, top_k=k).to(DEV).to(torch.bfloat16)
+    x = torch.randn(T, 264, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        quiet = layer(x)
+    assert torch.equal(quiet, layer(x))
+    moe_mod = importlib.import_module(pkg.__name__ + ".moe")
+    assert moe_mod.FEW_ROWS * 16 == 2560
+    pkg.check_status()
+
+
+def test_bad_expert_index_without_gradient(pkg):
+    """A slot whose expert index is out of range adds nothing and raises the status word."""
+    x = torch.randn(3, 64, device=DEV).to(torch.bfloat16)
+    gu, dn = (torch.randn(4, *s, device=DEV).to(torch.bfloat16) for s in ((128, 64), (64, 64)))
+    idx = torch.tensor([[0, 9], [1, 2], [-1, 3]], device=DEV)
+    w = torch.rand(3, 2, device=DEV)
+    out = pkg.moe(x, idx, w, gu, dn, torch.zeros(4, dtype=torch.int32, device=DEV))
+    with pytest.raises(RuntimeError, match="expert index"):
+        pkg.check_status()
+    ok = pkg.moe(x, idx.clamp(0, 3), w * torch.tensor([[1, 0], [1, 1], [0, 1]], device=DEV), gu, dn,
+                 torch.zeros(4, dtype=torch.int32, device=DEV))
+    pkg.check_status()
+    assert torch.equal(out, ok)

@@ -1,0 +1,361 @@
+// Grouped GEMMs for few rows per expert (decoding and prompts, forward only): the WEIGHTS are the M operand of
+// tcgen05.mma and the expert's rows the N operand, so the cost of a tile follows the rows an expert really has, in steps
+// of 16, instead of whole 256-row tiles.
+//
+//   D(rows of e, N) = X(rows of e, K) * W[e](N, K)^T        computed as W[e] (128 rows of it per MMA) * X^T
+//
+// Bound: HBM, by the one read of the weights of the experts that have rows.  The row-tile kernels (gemm.cu) give every
+// such expert a 256-row tile of MMAs, operand loads, activations and stores.  Here X lies in compact expert order
+// (no pad rows), 16-row boxes of it are loaded up to the last live row, and the accumulator holds output columns in
+// its lanes and rows in its columns.  A box may reach past the expert's rows: they only feed accumulator columns that
+// are not stored.
+// H 2048, I 1408, 64 experts, 288 rows (4.5 an expert; 111 + 56 us at copy rate): gate/up 158 -> 111 us, down 79 -> 59 us;
+// 9000 rows (141 an expert): 159 -> 138 and 79 -> 75 us; 6 rows of one token: 21 -> 19 and 15 -> 12 us.  Loading the weights
+// in 16-row boxes (64 gate and 64 up rows a tile) costs 132 us in place of 111: TMA instructions bound it then.
+//
+// Warp roles as in gemm.cu: warp 0 TMA producer (a lane per box), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.
+#include <cuda.h>
+
+#include <algorithm>
+#include <mutex>
+#include <type_traits>
+
+#include "gemm_common.cuh"
+
+namespace b200moe {
+
+struct FewParams {
+  int E;
+  int N;                  // output columns (SwiGLU: I)
+  int K;
+  const int* counts;      // rows of each expert
+  const int* offs;        // first row of each expert
+  void* D;                // (rows, N) bf16
+  const int* act_codes;   // SwiGLU: activation code of each expert, nullptr = SiLU
+  int* status;
+};
+
+constexpr int kFewBK = 64;      // k-block: one 128-byte swizzle row
+constexpr int kFewBox = 16;     // rows of X per TMA box = granularity of the MMA's N
+
+// NT: most rows of one tile.  HALVES: 128-row weight blocks per stage, each with an accumulator of its own (SwiGLU:
+// gate and up).  A CTA streams HALVES * 16 KB of weights for every live * 128 bytes of X a k-block.
+template <int NT, int HALVES>
+struct FewCfg {
+  static constexpr int W_BYTES = HALVES * 128 * kFewBK * 2;
+  static constexpr int X_BYTES = NT * kFewBK * 2;
+  static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
+  static constexpr int kFit = (232448 - 1024 - 2048) / STAGE_BYTES;
+  static constexpr int NSTAGE = kFit > 8 ? 8 : kFit;
+  static constexpr int ACC_COLS = HALVES * NT;                  // one tile's accumulators
+  static constexpr int NBUF = 2 * ACC_COLS <= 512 ? 2 : 1;
+  static constexpr int TMEM_COLS = NBUF * ACC_COLS > 256 ? 512 : NBUF * ACC_COLS > 128 ? 256 : 128;
+  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + (2 * NSTAGE + 2 * NBUF) * 8 + 16 + 1024;
+};
+
+struct FewTile { int e, m0, row0, live; };
+
+// tile -> (expert, chunk of its rows, block of output columns); pre[] = exclusive prefix of the experts' chunk counts
+template <int NT, int TM>
+__device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, int tile) {
+  const int mt = (p.N + TM - 1) / TM;
+  const int c = tile / mt;
+  int lo = 0, hi = p.E;                       // the last expert with pre[e] <= c
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (pre[mid] <= c) lo = mid;
+    else hi = mid;
+  }
+  FewTile t;
+  t.e = lo;
+  t.m0 = (tile - c * mt) * TM;
+  const int first = (c - pre[lo]) * NT;
+  t.row0 = p.offs[lo] + first;
+  t.live = min(NT, p.counts[lo] - first);
+  return t;
+}
+
+template <int EPI, int NT, int HALVES>
+__global__ void __launch_bounds__(kThreads, 1)
+few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const FewParams p) {
+  using C = FewCfg<NT, HALVES>;
+  constexpr int NSTAGE = C::NSTAGE, NBUF = C::NBUF;
+  constexpr int TM = (EPI == EPI_SWIGLU) ? 128 : 128 * HALVES;   // output columns of a tile
+  static_assert(EPI != EPI_SWIGLU || HALVES == 2, "SwiGLU needs the gate and the up accumulator");
+  static_assert(HALVES + NT / kFewBox <= 32, "a lane per box");
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * C::STAGE_BYTES);
+  const uint32_t bar_full = smem_u32(bars);
+  const uint32_t bar_empty = smem_u32(bars + NSTAGE);
+  const uint32_t bar_tfull = smem_u32(bars + 2 * NSTAGE);
+  const uint32_t bar_tempty = smem_u32(bars + 2 * NSTAGE + NBUF);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 2 * NBUF);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  __shared__ int pre[B200MOE_MAX_EXPERTS + 1];
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(bar_full + 8 * s, 1);
+      mbar_init(bar_empty + 8 * s, 1);
+    }
+    for (int b = 0; b < NBUF; ++b) {
+      mbar_init(bar_tfull + 8 * b, 1);
+      mbar_init(bar_tempty + 8 * b, kEpiWarps);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  if (warp == 2) {                       // prefix of the chunk counts: a lane takes 8 neighbouring experts
+    constexpr int V = B200MOE_MAX_EXPERTS / 32;
+    int c[V], sum = 0;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int e = lane * V + i;
+      c[i] = e < p.E ? (p.counts[e] + NT - 1) / NT : 0;
+      sum += c[i];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    int run = incl - sum;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      pre[lane * V + i] = run;
+      run += c[i];
+    }
+    if (lane == 31) pre[B200MOE_MAX_EXPERTS] = run;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int mt = (p.N + TM - 1) / TM;
+  const int total = pre[p.E] * mt;
+  const int nkb = (p.K + kFewBK - 1) / kFewBK;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer: lanes 0.. weights, then X boxes
+    const bool isW = lane < HALVES;
+    const int j = isW ? lane : lane - HALVES;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+      const FewTile t = few_tile<NT, TM>(p, pre, tile);
+      const int nb = (t.live + kFewBox - 1) / kFewBox;
+      const bool active = isW || j < nb;
+      int c1, c2 = 0;
+      if (isW) {
+        c1 = (EPI == EPI_SWIGLU) ? t.m0 : t.m0 + 128 * j;
+        c2 = (EPI == EPI_SWIGLU) ? 2 * t.e + j : t.e;
+      } else {
+        c1 = t.row0 + kFewBox * j;
+      }
+      const CUtensorMap* tm = isW ? &tmW : &tmX;
+      const uint32_t dst = isW ? j * (128 * kFewBK * 2) : C::W_BYTES + j * (kFewBox * kFewBK * 2);
+      const uint32_t bytes = C::W_BYTES + nb * (kFewBox * kFewBK * 2);
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
+          ok = false;
+          break;
+        }
+        if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
+        if (active) tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, c2);
+        if (++s == NSTAGE) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      int s = 0, it = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++it) {
+        const FewTile t = few_tile<NT, TM>(p, pre, tile);
+        const uint32_t idesc = umma_idesc_bf16((t.live + kFewBox - 1) / kFewBox * kFewBox, 0, 0, 128);
+        const int buf = it % NBUF;
+        if (!mbar_wait(bar_tempty + 8 * buf, ((it / NBUF) & 1) ^ 1, abort_flag, ST_WAIT_MMA_TMEM)) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * C::ACC_COLS;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sw = smem_u32(smem + s * C::STAGE_BYTES);
+          const uint32_t sx = sw + C::W_BYTES;
+#pragma unroll
+          for (int k = 0; k < kFewBK / 16; ++k) {
+            const uint64_t dx = umma_desc_sw128(sx + 32 * k, 0, 1024);
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h)
+              umma_bf16(d_tmem + h * NT, umma_desc_sw128(sw + h * (128 * kFewBK * 2) + 32 * k, 0, 1024), dx, idesc,
+                        (kb | k) != 0);
+          }
+          umma_commit(bar_empty + 8 * s);
+          if (++s == NSTAGE) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (!ok) break;
+        umma_commit(bar_tfull + 8 * buf);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue: lane = output column, register = row
+    const int q = warp & 3;              // TMEM lane quarter this warp may read
+    const int half = (warp - 2) >> 2;    // even or odd 16-row groups
+    int it = 0;
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
+      const FewTile t = few_tile<NT, TM>(p, pre, tile);
+      const int buf = it % NBUF;
+      int code = 0;
+      if (EPI == EPI_SWIGLU && p.act_codes != nullptr) code = p.act_codes[t.e];
+      if (!mbar_wait(bar_tfull + 8 * buf, (it / NBUF) & 1, abort_flag, ST_WAIT_EPILOGUE)) break;
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::ACC_COLS;
+      for (int c = 16 * half; c < t.live; c += 32) {
+        uint32_t a[HALVES][16];
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h) tmem_ld16(taddr + h * NT + c, a[h]);
+        tmem_ld_wait();
+        const int nr = min(16, t.live - c);                  // live rows of this group
+        __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(t.row0 + c) * p.N;
+        if constexpr (EPI == EPI_SWIGLU) {
+          const int col = t.m0 + 32 * q + lane;
+          auto rows = [&](auto tag) {
+            constexpr int CODE = decltype(tag)::value;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              // gate and up are rounded to bf16 before the activation, as where they are stored
+              const float g = bf16_round(__uint_as_float(a[0][i])), u = bf16_round(__uint_as_float(a[HALVES - 1][i]));
+              if (i < nr && col < p.N) d[static_cast<long long>(i) * p.N + col] = __float2bfloat16_rn(glu_fwd_val<CODE>(g, u));
+            }
+          };
+          if (code == 1) rows(std::integral_constant<int, 1>());
+          else if (code == 5) rows(std::integral_constant<int, 5>());
+          else rows(std::integral_constant<int, 0>());
+        } else {
+#pragma unroll
+          for (int h = 0; h < HALVES; ++h) {
+            const int col = t.m0 + 128 * h + 32 * q + lane;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (i < nr && col < p.N)
+                d[static_cast<long long>(i) * p.N + col] = __float2bfloat16_rn(__uint_as_float(a[h][i]));
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+    }
+  }
+
+  // ------------------------------------------------------------------ tear-down
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_flag);
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------- host side
+template <int EPI, int NT, int HALVES>
+static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows, int wgroups, const FewParams& p,
+                      cudaStream_t stream) {
+  using C = FewCfg<NT, HALVES>;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(few_rows_kernel<EPI, NT, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    C::SMEM_BYTES);
+  });
+  if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
+  CUtensorMap tmW, tmX;
+  int rc = make_map(&tmW, w, p.K, wrows, wgroups, p.K, static_cast<uint64_t>(wrows) * p.K, kFewBK, 128);
+  if (rc) return rc;
+  rc = make_map(&tmX, x, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, kFewBK, kFewBox);
+  if (rc) return rc;
+  constexpr int TM = (EPI == EPI_SWIGLU) ? 128 : 128 * HALVES;
+  const long long chunks = std::min<long long>(rows_cap, p.E + rows_cap / NT);   // at most
+  const long long tiles = chunks * ceil_div(p.N, TM);
+  const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(gemm_cta_budget(), tiles)));
+  few_rows_kernel<EPI, NT, HALVES><<<grid, kThreads, C::SMEM_BYTES, stream>>>(tmW, tmX, p);
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// Tile by the mean rows per expert.  A larger NT keeps an expert's rows in one tile, so its weights pass through shared
+// memory once; a smaller one leaves room for more k-blocks in flight and double-buffered accumulators.  Gate/up, us, at
+// H 2048, I 1408, 64 experts: 28 rows an expert NT 64 / 128 / 192: 115 / 116 / 117; 66 rows 134 / 119 / 125; 94 rows 153 /
+// 122 / 131; 141 rows 210 / 155 / 138.  Down (one / one / two 128-row weight blocks a tile): 61 / 61 / 63, 87 / 64 / 66,
+// 107 / 70 / 69, 150 / 123 / 75.
+constexpr int64_t kFewRows64 = 40, kFewRows128 = 110;
+
+static int check_few(const char* who, const void* x, const void* w, const void* d, const int32_t* counts,
+                     const int32_t* offs, int64_t rows_cap, int E, int64_t N, int64_t K) {
+  B200_CHECK_ARG(x && w && d && counts && offs, B200MOE_E_NULL, "%s: null pointer", who);
+  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED, "%s: E = %d, supported 1..%d", who, E,
+                 B200MOE_MAX_EXPERTS);
+  B200_CHECK_ARG(rows_cap > 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE, "%s: rows_cap = %lld", who, (long long)rows_cap);
+  B200_CHECK_ARG(N > 0 && N % 8 == 0 && K > 0 && K % 8 == 0, B200MOE_E_BAD_SHAPE,
+                 "%s: N = %lld and K = %lld must be positive multiples of 8", who, (long long)N, (long long)K);
+  B200_CHECK_ARG(N < (1LL << 31) && K < (1LL << 31), B200MOE_E_BAD_SHAPE, "%s: extent beyond 2^31", who);
+  return 0;
+}
+
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" {
+
+int b200moe_expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
+                               const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, void* inter,
+                               int32_t* status, b200moe_stream_t stream) {
+  int rc = check_few("expert_gate_up_few", x, gate_up_proj, inter, counts, offs, rows_cap, E, I, H);
+  if (rc) return rc;
+  FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status};
+  cudaStream_t st = (cudaStream_t)stream;
+  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
+  if (rows_cap <= kFewRows64 * E) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  if (rows_cap <= kFewRows128 * E) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+}
+
+int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap,
+                              int E, int64_t N, int64_t K, void* out, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_few("expert_linear_few", x, w, out, counts, offs, rows_cap, E, N, K);
+  if (rc) return rc;
+  FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status};
+  cudaStream_t st = (cudaStream_t)stream;
+  if (rows_cap <= kFewRows64 * E) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
+  if (rows_cap <= kFewRows128 * E) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
+  return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
+}
+
+}  // extern "C"

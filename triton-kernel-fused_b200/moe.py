@@ -17,6 +17,12 @@ __all__ = ["moe", "moe_grouped", "moe_per_expert", "GROUPED_MIN_TOKENS"]
 GROUPED_MIN_TOKENS = 4096   # kept for API compatibility (kernels/sm75/moe.py:78); one path here
 
 
+# Most rows per expert, on average, for which a forward without a backward runs over compact rows with the weights as
+# the MMA's M operand (csrc/gemm_few.cu).  Gate/up + down, us, row tiles against compact rows, at H 2048, I 1408, 64
+# experts: 4.5 rows an expert 237 / 170, 141 rows 238 / 213, 206 rows 240 / 328 (an expert then takes two tiles).
+FEW_ROWS = 160
+
+
 def _amp_cast(*ts):
     """Under CUDA autocast cast float tensors to the autocast dtype (kernels/sm75/moe.py:97-104)."""
     if torch.is_autocast_enabled("cuda"):
@@ -30,7 +36,8 @@ class _GroupedMoE(torch.autograd.Function):
     Function does (kernels/sm75/moe.py:576-599); backward follows :602-618."""
 
     @staticmethod
-    def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes):
+    def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes, keep=True):
+        """keep=False: no backward will follow (the caller knows the grad mode, which is off in here)."""
         hidden, gate_up_proj, down_proj = _amp_cast(hidden, gate_up_proj, down_proj)
         L.require(hidden.dim() == 2, "hidden must be (N,H)")
         for name, t in (("hidden", hidden), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
@@ -54,6 +61,11 @@ class _GroupedMoE(torch.autograd.Function):
         if any(c != 0 for c in codes):
             codes_dev = act_codes.to(device=hidden.device, dtype=torch.int32).contiguous()
 
+        if not keep and idx.numel() <= FEW_ROWS * E:
+            perm = ops.permute_build(idx, E, want_order=True)
+            inter = ops.expert_gate_up_few(ops.gather_compact(hidden, perm), gate_up_proj, perm, codes_dev)
+            return ops.combine_raw(ops.expert_linear_few(inter, down_proj, perm), w32, perm.slot_pos, N, perm.k)
+
         perm = ops.permute_build(idx, E)
         x_s = ops.gather_rows(hidden, perm)
         gate_up, inter = ops.expert_gate_up_swiglu(x_s, gate_up_proj, perm, codes_dev)
@@ -70,7 +82,7 @@ class _GroupedMoE(torch.autograd.Function):
     def backward(ctx, grad_out):
         x_s, gate_up, inter, eo, w32, gate_up_proj, down_proj = ctx.saved_tensors
         perm = ctx.perm
-        need_x, _, need_w, need_gu, need_dn, _ = ctx.needs_input_grad
+        need_x, _, need_w, need_gu, need_dn = ctx.needs_input_grad[:5]
         grad_out = grad_out.contiguous()
         if grad_out.dtype != torch.bfloat16:
             grad_out = grad_out.to(torch.bfloat16)
@@ -86,7 +98,8 @@ class _GroupedMoE(torch.autograd.Function):
         if need_dn:
             grad_down_proj = ops.expert_wgrad(grad_eo, inter, perm)
         grad_wt = grad_w.to(ctx.wt_dtype) if need_w else None
-        return grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None
+        grads = (grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None, None)
+        return grads[:len(ctx.needs_input_grad)]
 
 
 GLU_CODES = (0, 1, 2, 5, 6, 7)     # weight-carrying experts (kernels/sm75/moe.py:1-31)
@@ -236,7 +249,8 @@ def moe(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes
                   act_codes, act_params)
         return out.to(hidden.dtype)
     if act_params is None and n_glu == len(codes) and all(c in FUSED_CODES for c in codes):
-        return _GroupedMoE.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes)
+        keep = torch.is_grad_enabled() and any(t.requires_grad for t in (hidden, top_k_weights, gate_up_proj, down_proj))
+        return _GroupedMoE.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, keep)
     return _PolyGLUMoE.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, act_params)
 
 

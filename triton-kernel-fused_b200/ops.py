@@ -213,6 +213,27 @@ def expert_gate_up_swiglu(x_s, gate_up_proj, perm: Permutation, act_codes=None, 
     return gate_up, inter
 
 
+@_op("expert_gate_up_few", 1)
+def expert_gate_up_few(x_c, gate_up_proj, perm: Permutation, act_codes=None):
+    """inter (T*k, I) of rows in compact expert order (gather_compact), without the gate_up buffer a backward needs."""
+    E, twoI, H = gate_up_proj.shape
+    inter = torch.empty(x_c.shape[0], twoI // 2, dtype=torch.bfloat16, device=x_c.device)
+    L.check(L.lib().b200moe_expert_gate_up_few(L.ptr(x_c), L.ptr(gate_up_proj), L.ptr(act_codes), L.ptr(perm.counts),
+                                               L.ptr(perm.offs), x_c.shape[0], E, H, twoI // 2, L.ptr(inter),
+                                               L.ptr(L.status_word(x_c.device)), L.stream_of(x_c)))
+    return inter
+
+
+@_op("expert_linear_few", 1)
+def expert_linear_few(a, w, perm: Permutation):
+    """out (rows,N) = a (rows,K) @ W[e]^T, W (E,N,K), rows in compact expert order."""
+    E, N, K = w.shape
+    out = torch.empty(a.shape[0], N, dtype=torch.bfloat16, device=a.device)
+    L.check(L.lib().b200moe_expert_linear_few(L.ptr(a), L.ptr(w), L.ptr(perm.counts), L.ptr(perm.offs), a.shape[0], E, N,
+                                              K, L.ptr(out), L.ptr(L.status_word(a.device)), L.stream_of(a)))
+    return out
+
+
 @_op("expert_down", 1)
 def expert_down(inter, down_proj, perm: Permutation, out=None):
     E, H, I = down_proj.shape
