@@ -8,8 +8,8 @@ from oracle import moe_oracle as O
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-# one bf16 rounding of the result (2^-9 of each value) on fp32 sums
-TOL = 2.1e-3
+# one bf16 rounding of the result (8 significant bits: at most 2^-8 = 3.9e-3 of each value) on fp32 sums
+TOL = 3.95e-3
 
 
 # rows an expert gets: none, one, both sides of the 16-row step and of the 64 / 128 / 192-row tiles, several tiles;

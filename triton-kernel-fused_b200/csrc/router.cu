@@ -35,6 +35,51 @@ constexpr uint32_t kKnockOut = ~0xf149f2cau;   // select_key(-1e30f)
 // k = 8: 80 -> 26 us).  A pick is one
 // redux.max over the lanes' best keys and one redux.min over the ids that hold it (ties to the lowest expert id, as a
 // stable sort gives), instead of five shuffle rounds of (value, id) pairs.
+// The k picks of the token whose scores and selection keys a warp holds: lane j < k gets pick j and its weight.
+template <int VPL>
+__device__ __forceinline__ void topk_of_token(const float (&sc)[VPL], uint32_t (&key)[VPL], int k, int norm, float scale,
+                                              int* hist, bool count, int& my_idx, float& my_w) {
+  const int lane = threadIdx.x & 31;
+  my_idx = 0;
+  my_w = 0.0f;
+  for (int j = 0; j < k; ++j) {
+    // lane-local best: ascending i = ascending expert id, strict '>' keeps the lowest id
+    uint32_t bk = key[0];
+    int bi = lane;
+#pragma unroll
+    for (int i = 1; i < VPL; ++i) {
+      if (key[i] > bk) {
+        bk = key[i];
+        bi = lane + 32 * i;
+      }
+    }
+    const uint32_t best = __reduce_max_sync(0xffffffffu, bk);
+    bi = static_cast<int>(__reduce_min_sync(0xffffffffu, bk == best ? static_cast<unsigned>(bi) : 0xffffffffu));
+    // owner lane hands out the unbiased score and knocks the pick out
+    float wv = 0.0f;
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      if (bi == lane + 32 * i) {
+        wv = sc[i];
+        key[i] = kKnockOut;
+      }
+    }
+    wv = __shfl_sync(0xffffffffu, wv, bi & 31);
+    if (lane == j) {
+      my_idx = bi;
+      my_w = wv;
+    }
+  }
+  if (count && lane < k) atomicAdd(&hist[my_idx], 1);
+  if (norm && k > 1) {
+    float tsum = 0.0f;
+    for (int j = 0; j < k; ++j) tsum += __shfl_sync(0xffffffffu, my_w, j);  // fixed order
+    tsum += 1e-20f;
+    my_w = my_w / tsum;
+  }
+  my_w = my_w * scale;
+}
+
 template <int KIND, int VPL>
 __global__ void __launch_bounds__(256)
 router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__ bias, long long T, int E,
@@ -69,44 +114,107 @@ router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__
         key[i] = select_key(sc[i] + b[i]);
       }
     }
-    int my_idx = 0;
-    float my_w = 0.0f;
-    for (int j = 0; j < k; ++j) {
-      // lane-local best: ascending i = ascending expert id, strict '>' keeps the lowest id
-      uint32_t bk = key[0];
-      int bi = lane;
+    int my_idx;
+    float my_w;
+    topk_of_token<VPL>(sc, key, k, norm, scale, hist, counts != nullptr, my_idx, my_w);
+    if (lane < k) {
+      idx_out[t * k + lane] = my_idx;
+      w_out[t * k + lane] = my_w;
+    }
+  }
+  if (counts != nullptr) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+      const int c = hist[e];
+      if (c != 0) atomicAdd(&counts[e], c);
+    }
+  }
+}
+
+// Logits and top-k of a small batch in one launch: a CTA takes TPB tokens, its warps split the experts in groups of 8
+// and, where that leaves warps over, the reduction, and a lane keeps 8 weight vectors and more in flight (each used for
+// all TPB tokens).  Bound by the latency of the weights' way from L2 (every CTA reads all E * H of them) and, with
+// more tokens, by the FMAs.  The GEMM it stands in for has one CTA per 128 tokens walk the whole reduction (32 dependent
+// k-blocks at H = 2048).  Sums are fp32 per lane, then across lanes and warps; the logits are rounded to bf16
+// before the picks, as the GEMM stores them.  48 tokens, H 2048, 64 experts, top-6: 15.6 us for GEMM and top-k, 7.5 us here.
+constexpr int kSmallWarps = 16;
+template <int VPL, int TPB>
+__global__ void __launch_bounds__(32 * kSmallWarps)
+router_small_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ weight, const float* __restrict__ bias,
+                        int T, int nvec, int E, int k, int norm, float scale, __nv_bfloat16* __restrict__ logits,
+                        long long* __restrict__ idx_out, float* __restrict__ w_out, int* __restrict__ counts) {
+  constexpr int kPart = B200MOE_MAX_EXPERTS;        // partial sums a token needs: parts * E <= 8 * 16, or E
+  __shared__ float s_part[TPB][kPart];
+  __shared__ int hist[B200MOE_MAX_EXPERTS];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int t0 = blockIdx.x * TPB;
+  const int groups = E / 8;                         // E is a multiple of 8
+  const int parts = groups < kSmallWarps ? kSmallWarps / groups : 1;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
+  for (int u = warp; u < groups * parts; u += kSmallWarps) {
+    const int g = u % groups, part = u / groups;
+    const uint4* wrow = weight + static_cast<long long>(8 * g) * nvec;
+    float acc[8][TPB];
 #pragma unroll
-      for (int i = 1; i < VPL; ++i) {
-        if (key[i] > bk) {
-          bk = key[i];
-          bi = lane + 32 * i;
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int t = 0; t < TPB; ++t) acc[i][t] = 0.0f;
+#pragma unroll 2
+    for (int c = lane + 32 * part; c < nvec; c += 32 * parts) {
+      uint4 wv[8], xv[TPB];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) wv[i] = wrow[static_cast<long long>(i) * nvec + c];
+#pragma unroll
+      for (int t = 0; t < TPB; ++t)
+        xv[t] = t0 + t < T ? x[static_cast<long long>(t0 + t) * nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const float2 wf = unpack_bf16x2(ww[h]);
+#pragma unroll
+          for (int t = 0; t < TPB; ++t) {
+            const float2 xf = unpack_bf16x2(h == 0 ? xv[t].x : h == 1 ? xv[t].y : h == 2 ? xv[t].z : xv[t].w);
+            acc[i][t] = fmaf(wf.x, xf.x, acc[i][t]);
+            acc[i][t] = fmaf(wf.y, xf.y, acc[i][t]);
+          }
         }
       }
-      const uint32_t best = __reduce_max_sync(0xffffffffu, bk);
-      bi = static_cast<int>(__reduce_min_sync(0xffffffffu, bk == best ? static_cast<unsigned>(bi) : 0xffffffffu));
-      // owner lane hands out the unbiased score and knocks the pick out
-      float wv = 0.0f;
+    }
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        if (bi == lane + 32 * i) {
-          wv = sc[i];
-          key[i] = kKnockOut;
-        }
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int t = 0; t < TPB; ++t) {
+        float v = acc[i][t];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        if (lane == 0) s_part[t][part * E + 8 * g + i] = v;
       }
-      wv = __shfl_sync(0xffffffffu, wv, bi & 31);
-      if (lane == j) {
-        my_idx = bi;
-        my_w = wv;
+  }
+  __syncthreads();
+  if (warp < TPB && t0 + warp < T) {
+    const long long t = t0 + warp;
+    float sc[VPL];
+    uint32_t key[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int e = lane + 32 * i;
+      sc[i] = 0.0f;
+      key[i] = 0u;
+      if (e < E) {
+        float v = s_part[warp][e];
+        for (int q = 1; q < parts; ++q) v += s_part[warp][q * E + e];
+        v = bf16_round(v);
+        logits[t * E + e] = __float2bfloat16_rn(v);
+        sc[i] = sigmoid_f(v);
+        key[i] = select_key(sc[i] + (bias != nullptr ? bias[e] : 0.0f));
       }
     }
-    if (counts != nullptr && lane < k) atomicAdd(&hist[my_idx], 1);
-    if (norm && k > 1) {
-      float tsum = 0.0f;
-      for (int j = 0; j < k; ++j) tsum += __shfl_sync(0xffffffffu, my_w, j);  // fixed order
-      tsum += 1e-20f;
-      my_w = my_w / tsum;
-    }
-    my_w = my_w * scale;
+    int my_idx;
+    float my_w;
+    topk_of_token<VPL>(sc, key, k, norm, scale, hist, counts != nullptr, my_idx, my_w);
     if (lane < k) {
       idx_out[t * k + lane] = my_idx;
       w_out[t * k + lane] = my_w;
@@ -259,6 +367,37 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
       set_error("router_topk_fwd: unknown input_kind %d", input_kind);
       return B200MOE_E_UNSUPPORTED;
   }
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int b200moe_router_small_fwd(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
+                             int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
+                             b200moe_stream_t stream) {
+  B200_CHECK_ARG(x && weight && logits && idx && w, B200MOE_E_NULL, "router_small_fwd: null pointer");
+  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
+                 "router_small_fwd: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
+  B200_CHECK_ARG(E % 8 == 0 && H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE,
+                 "router_small_fwd: E = %d and H = %lld must be positive multiples of 8", E, (long long)H);
+  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE,
+                 "router_small_fwd: top_k = %d must be in 1..min(E=%d, %d)", k, E, B200MOE_MAX_TOPK);
+  B200_CHECK_ARG(T >= 0 && T < (1LL << 31) && H < (1LL << 31), B200MOE_E_BAD_SHAPE, "router_small_fwd: T = %lld", (long long)T);
+  B200_CHECK_ARG(aligned16(x) && aligned16(weight), B200MOE_E_ALIGN, "router_small_fwd: x and weight must be 16-byte aligned");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (counts != nullptr) B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * E, st));
+  if (T == 0) return 0;
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  const uint4* wv = reinterpret_cast<const uint4*>(weight);
+  __nv_bfloat16* lg = reinterpret_cast<__nv_bfloat16*>(logits);
+  long long* idx_ll = reinterpret_cast<long long*>(idx);
+  const int Ti = static_cast<int>(T), nvec = static_cast<int>(H / 8);
+  // one token a CTA while that fills no more than the SMs; four share the reads of the weights beyond
+  by_experts(E, [&](auto v) {
+    if (T <= num_sms())
+      router_small_fwd_kernel<v.value, 1><<<Ti, 32 * kSmallWarps, 0, st>>>(xv, wv, bias, Ti, nvec, E, k, norm_topk, scale, lg, idx_ll, w, counts);
+    else
+      router_small_fwd_kernel<v.value, 4><<<(Ti + 3) / 4, 32 * kSmallWarps, 0, st>>>(xv, wv, bias, Ti, nvec, E, k, norm_topk, scale, lg, idx_ll, w, counts);
+  });
   B200_CUDA(cudaGetLastError());
   return 0;
 }

@@ -67,6 +67,25 @@ def router_topk_fwd(logits, bias, top_k, norm_topk=True, scale=1.0, want_counts=
     return idx, w, counts
 
 
+@_op("router_small_fwd", 1)
+def router_small_fwd(x, weight, bias, top_k, norm_topk=True, scale=1.0):
+    """Logits and picks of a small batch in one launch: (logits bf16 (T,E), idx, w, counts)."""
+    L.require_cuda_bf16("x", x); L.require_cuda_bf16("gate_weight", weight)
+    L.require(x.is_contiguous() and weight.is_contiguous() and x.shape[1] == weight.shape[1], "router_small_fwd: need contiguous (T,H),(E,H)")
+    if bias is not None:
+        L.require(bias.is_cuda and bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == weight.shape[0],
+                  "bias must be a contiguous float32 CUDA tensor of E entries")
+    (T, H), E, dev = x.shape, weight.shape[0], x.device
+    logits = torch.empty(T, E, dtype=torch.bfloat16, device=dev)
+    idx = torch.empty(T, top_k, dtype=torch.int64, device=dev)
+    w = torch.empty(T, top_k, dtype=torch.float32, device=dev)
+    counts = torch.empty(E, dtype=torch.int32, device=dev)
+    L.check(L.lib().b200moe_router_small_fwd(L.ptr(x), L.ptr(weight), L.ptr(bias), T, H, E, int(top_k),
+                                             int(bool(norm_topk)), float(scale), L.ptr(logits), L.ptr(idx), L.ptr(w),
+                                             L.ptr(counts), L.stream_of(x)))
+    return logits, idx, w, counts
+
+
 @_op("router_topk_bwd", 1)
 def router_topk_bwd(logits, idx, grad_w, norm_topk=True, scale=1.0):
     N, E = logits.shape

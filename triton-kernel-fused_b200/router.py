@@ -2,7 +2,7 @@
 
 `fused_mlp_router` (:277-289), `FusedMLPRouter` (:221-260) and `router_bias_update` (:292-301) keep
 their signatures.  Logits are a tcgen05 GEMM (fp32 accumulate, stored in x's dtype as the reference
-does), followed by the warp-level top-k epilogue kernel; backward is the epilogue Jacobian kernel
+does), followed by the warp-level top-k epilogue kernel (a small batch: both in one launch); backward is the epilogue Jacobian kernel
 plus two tcgen05 GEMMs (dX, and dW as a split-K reduction over the tokens).
 """
 from __future__ import annotations
@@ -13,6 +13,13 @@ from . import _lib as L
 from . import ops
 
 __all__ = ["fused_mlp_router", "FusedMLPRouter", "fused_router", "FusedConvRouter", "router_bias_update"]
+
+
+# Up to this many tokens (four for each of 148 SMs; with more than 64 experts correspondingly fewer) logits and picks are
+# one launch of CUDA-core dot products.  GEMM + top-k against it, us, top-6 of 64 experts at H 2048: 48 tokens 15.6 / 7.5,
+# 512 tokens 16.1 / 11.7, 1024 tokens 16.1 / 20.9; 128 experts: 128 tokens 17.6 / 10.0, 256 tokens 17.6 / 16.2; 256 experts:
+# 100 tokens at H 4096 29.1 / 27.3, 256 tokens at H 1024 15.5 / 19.0.
+SMALL_TOKENS = 592
 
 
 class FusedMLPRouter(torch.autograd.Function):
@@ -30,11 +37,15 @@ class FusedMLPRouter(torch.autograd.Function):
         L.require(num_experts is None or int(num_experts) == weight.shape[0], "num_experts must equal gate_weight.shape[0]")
         xf = x.reshape(-1, x.shape[-1]).contiguous()
         weight = weight.contiguous()
-        logits = ops.gemm_nt(xf, weight)
         bias32 = None
         if bias is not None:
             bias32 = bias.detach().float().contiguous()
-        idx, w, counts = ops.router_topk_fwd(logits, bias32, top_k, norm_topk and top_k > 1, scale)
+        T, E = xf.shape[0], weight.shape[0]
+        if T <= SMALL_TOKENS and T * E <= 64 * SMALL_TOKENS:
+            logits, idx, w, counts = ops.router_small_fwd(xf, weight, bias32, top_k, norm_topk and top_k > 1, scale)
+        else:
+            logits = ops.gemm_nt(xf, weight)
+            idx, w, counts = ops.router_topk_fwd(logits, bias32, top_k, norm_topk and top_k > 1, scale)
         ctx.xshape = x.shape
         ctx.save_for_backward(xf, weight, logits, idx)
         ctx.norm, ctx.scale = bool(norm_topk and top_k > 1), float(scale)
