@@ -59,6 +59,11 @@ int64_t b200moe_padded_rows_cap(int64_t M, int E);
  * returns normally.  Shows that a stalled pipeline ends in a status code, not in a hung GPU. */
 int b200moe_selftest_bounded_wait(int32_t* status, int64_t limit_cycles, b200moe_stream_t stream);
 
+/* An observer of the operations that the sequences below (b200moe_layer_*, b200moe_moe_*, b200moe_router_*,
+ * b200moe_newton_schulz) queue: called on the host with the operation's name, its number of launches and phase 0 before,
+ * 1 after they are queued.  NULL = none.  Process-wide; for measurement. */
+typedef void (*b200moe_observer_t)(const char* name, int launches, int phase);
+int b200moe_set_observer(b200moe_observer_t observer);
 /* host: keep `n` SMs free of the persistent GEMM kernels (process-wide, default 0) so that
  * communication kernels queued on another stream can run beside them.  No reference counterpart. */
 int b200moe_set_reserved_sms(int n);
@@ -311,6 +316,9 @@ int b200moe_mxfp8_expert_wgrad(const void* Atq, const void* Atsf, const void* Bt
  * w == NULL means weight 1 (the grad_hidden un-permute, kernels/sm75/moe.py:614-615). */
 int b200moe_combine(const void* rows, const float* w, const int32_t* slot_row, int64_t T, int k,
                     int64_t H, void* out, b200moe_stream_t stream);
+/* The same plus a row of its own per token: out[t] += add[t] before the one rounding (add (T,H) bf16, nullable). */
+int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k,
+                        int64_t H, void* out, b200moe_stream_t stream);
 /* Replaces _combine_bwd_kernel (kernels/sm75/moe.py:688-701): grad_eo[r] = go[tok]*w[slot],
  * grad_w[slot] = <go[tok], eo[r]> in fp32; zero rows where row_slot[r] < 0. */
 int b200moe_combine_bwd(const void* grad_out, const void* eo, const float* w,
@@ -472,6 +480,51 @@ int b200moe_axpby_bf16(const void* x, float alpha, const void* y, float beta, fl
  * 431-434); gain is the aurora gain (kernels/muon/muon_scaling.py:112), 1 for scale_mode "polar". */
 int b200moe_muon_apply(const void* xp, int E, int64_t r, int64_t c, int64_t Rp, int transposed, float gain, float decay,
                        float alpha, void* p, int p_f32, b200moe_stream_t stream);
+
+/* ---- the block as one host call each way -----------------------------------------------------
+ * The sequences of kernels/sm75/moe.py:576-618, :724-826 and router.py:221-260 out of one workspace per direction,
+ * allocated by the caller at the size the *_ws_bytes functions give (256-byte aligned).  The forward's workspace holds
+ * what the backward reads; pass it unchanged.  Nullable grad_* outputs are not computed.
+ * router: logits (T,E) bf16, picks and weights as b200moe_router_topk_fwd; counts nullable. */
+int b200moe_router_forward(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
+                           int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
+                           int32_t* status, b200moe_stream_t stream);
+size_t b200moe_router_bwd_ws_bytes(int64_t T, int64_t H, int E);
+int b200moe_router_backward(const void* x, const void* weight, const void* logits, const int64_t* idx, const float* grad_w,
+                            int64_t T, int64_t H, int E, int k, int norm_topk, float scale, void* ws, void* grad_x,
+                            void* grad_weight, int32_t* status, b200moe_stream_t stream);
+/* moe: the experts on given picks (idx (T,k), w (T,k) fp32).  E routed experts, the first n_glu with weights.
+ * row_kernels: activations as row kernels (any code, act_params, Identity / Zero experts); 0: in the GEMM epilogues
+ * (codes 0, 1, 5; act_codes NULL = SiLU).  keep = 0: no backward follows, which lets few rows per expert run over compact
+ * rows.  grad_params (E,2), row_kernels only. */
+size_t b200moe_moe_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int row_kernels);
+int b200moe_moe_forward(const void* x, const int64_t* idx, const float* w, const void* gate_up_proj, const void* down_proj,
+                        const int32_t* act_codes, const float* act_params, int64_t T, int64_t H, int64_t I, int E, int n_glu,
+                        int k, int keep, int row_kernels, void* ws, void* out, int32_t* status, b200moe_stream_t stream);
+size_t b200moe_moe_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int row_kernels);
+int b200moe_moe_backward(const void* grad_out, const float* w, const void* gate_up_proj, const void* down_proj,
+                         const int32_t* act_codes, const float* act_params, int64_t T, int64_t H, int64_t I, int E,
+                         int n_glu, int k, int row_kernels, void* fwd_ws, void* ws, void* grad_x, float* grad_w,
+                         void* grad_gate_up, void* grad_down, float* grad_params, int32_t* status, b200moe_stream_t stream);
+/* layer: router and experts (all with weights).  counts (E, nullable): rows per expert; load (E int64, nullable): the
+ * counts are added to it.  grad_x is the sum of the experts' and the router's share, rounded once. */
+size_t b200moe_layer_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k, int keep);
+int b200moe_layer_forward(const void* x, const void* gate_weight, const float* bias, const void* gate_up_proj,
+                          const void* down_proj, const int32_t* act_codes, int64_t T, int64_t H, int64_t I, int E, int k,
+                          int norm_topk, float scale, int keep, void* ws, int32_t* counts, int64_t* load, void* out,
+                          int32_t* status, b200moe_stream_t stream);
+size_t b200moe_layer_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k);
+int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate_weight, const void* gate_up_proj,
+                           const void* down_proj, const int32_t* act_codes, int64_t T, int64_t H, int64_t I, int E, int k,
+                           int norm_topk, float scale, void* fwd_ws, void* ws, void* grad_x, void* grad_gate_weight,
+                           void* grad_gate_up, void* grad_down, int32_t* status, b200moe_stream_t stream);
+/* All iterations of kernels/sm75/muon.py:83-86 on a padded stack x (E, Rp, wide): per iteration the three products of
+ * b200moe_expert_gram, _expert_linear_axpby (symmetric = 2) and _expert_linear_t.  coeffs: HOST array of (a, b, c) per
+ * iteration.  x and x_next take turns: the result is in x after an even number of iterations, else in x_next; a, a2:
+ * (E, Rp, Rp) work space. */
+int b200moe_newton_schulz(void* x, void* x_next, void* a, void* a2, const int32_t* tile_expert, const int32_t* poffs, int E,
+                          int64_t Rp, int64_t wide, const float* coeffs, int iterations, int32_t* status,
+                          b200moe_stream_t stream);
 
 #ifdef __cplusplus
 }

@@ -1,6 +1,4 @@
 """GPU: the grouped products for few rows per expert against the row-tile kernels and an fp32 reference."""
-import importlib
-
 import pytest
 import torch
 
@@ -49,8 +47,6 @@ def test_forward_without_gradient_equals_the_training_forward(pkg, T, E, k):
     with torch.no_grad():
         quiet = layer(x)
     assert torch.equal(quiet, layer(x))
-    moe_mod = importlib.import_module(pkg.__name__ + ".moe")
-    assert moe_mod.FEW_ROWS * 16 == 2560
     pkg.check_status()
 
 

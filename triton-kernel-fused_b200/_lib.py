@@ -89,6 +89,20 @@ _SIGNATURES = {
     "b200moe_ep_combine_bwd_pull": (c_int, [c_void_p] * 9 + [c_int] * 6 + [c_int64, c_int, c_int64] + [c_void_p] * 3),
     "b200moe_combine": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_void_p, c_void_p]),
     "b200moe_combine_bwd": (c_int, [c_void_p] * 5 + [c_int, c_int64, c_int64, c_void_p, c_void_p, c_void_p]),
+    "b200moe_combine_add": (c_int, [c_void_p] * 4 + [c_int64, c_int, c_int64, c_void_p, c_void_p]),
+    "b200moe_set_observer": (c_int, [c_void_p]),
+    "b200moe_router_forward": (c_int, [c_void_p] * 3 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 6),
+    "b200moe_router_bwd_ws_bytes": (c_size_t, [c_int64, c_int64, c_int]),
+    "b200moe_router_backward": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 5),
+    "b200moe_moe_fwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 5),
+    "b200moe_moe_forward": (c_int, [c_void_p] * 7 + [c_int64] * 3 + [c_int] * 5 + [c_void_p] * 4),
+    "b200moe_moe_bwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 4),
+    "b200moe_moe_backward": (c_int, [c_void_p] * 6 + [c_int64] * 3 + [c_int] * 4 + [c_void_p] * 9),
+    "b200moe_layer_fwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 3),
+    "b200moe_layer_forward": (c_int, [c_void_p] * 6 + [c_int64] * 3 + [c_int] * 3 + [c_float, c_int] + [c_void_p] * 6),
+    "b200moe_layer_bwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 2),
+    "b200moe_layer_backward": (c_int, [c_void_p] * 6 + [c_int64] * 3 + [c_int] * 3 + [c_float] + [c_void_p] * 8),
+    "b200moe_newton_schulz": (c_int, [c_void_p] * 6 + [c_int, c_int64, c_int64, c_void_p, c_int, c_void_p, c_void_p]),
     "b200moe_muon_momentum": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_float, c_int, c_void_p]),
     "b200moe_muon_row_sumsq": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
     "b200moe_muon_prescale_rows": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_float, c_float, c_void_p, c_void_p,
@@ -161,15 +175,19 @@ def ptr_table(addresses):
 
 
 def stream_of(t: torch.Tensor):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The raw handle of the current stream of t's device (torch.cuda.current_stream builds a Stream object around it,
+    which costs more than a launch)."""
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
-_status = {}
+_status = {}       # device index -> the word
 
 
 def status_word(device) -> torch.Tensor:
     """The per-device int32 word that kernels raise when a bounded wait ran out or an index was bad."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    key = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if key is None:
+        key = torch.cuda.current_device()
     t = _status.get(key)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
@@ -196,6 +214,10 @@ def raise_for_status(v: int) -> None:
 
 def padded_rows_cap(M: int, E: int) -> int:
     return int(lib().b200moe_padded_rows_cap(M, E))
+
+
+def workspace(nbytes: int, device) -> torch.Tensor:
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def require(cond: bool, msg: str) -> None:

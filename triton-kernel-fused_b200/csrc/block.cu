@@ -1,0 +1,416 @@
+// The whole block from one host call: router, permutation, expert GEMMs, activation, combine, forward and backward, as
+// one sequence of the library's own launches on the caller's stream, out of one workspace that the caller
+// allocates (the *_ws_bytes functions give its size, `carve_*` its layout).  Nothing here touches the device but the
+// launches; the forward's workspace is what a backward reads, so it must stay as the forward left it until then.
+//
+// Why: a launch from here costs the host about 2 us; through one Python call, its output allocations and argument
+// checks per kernel it cost 8 to 15 us, more than most kernels of a small batch run on the GPU.
+// Host time of a pass: one decoding token 236 -> 91 us (10 -> 6 launches), forward and backward of 512 tokens at width 256
+// 678 -> 290 us (24 -> 17), mixed activations 492 -> 254 us.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+
+namespace b200moe {
+
+typedef uint16_t bf16_t;   // storage only
+
+struct Carver {
+  char* base;
+  size_t off;
+  explicit Carver(void* p) : base(static_cast<char*>(p)), off(0) {}
+  template <class T>
+  T* take(int64_t n) {
+    off = (off + 255) & ~static_cast<size_t>(255);
+    T* p = base != nullptr ? reinterpret_cast<T*>(base + off) : nullptr;
+    off += static_cast<size_t>(n) * sizeof(T);
+    return p;
+  }
+};
+
+enum Kind { KIND_FEW = 0, KIND_TILES = 1, KIND_ROWS = 2 };
+
+struct Dims {
+  int64_t T, H, I;
+  int E, n_glu, k;        // routed experts, those with weights, picks per token
+  Kind kind;
+  int64_t M() const { return T * k; }
+  int64_t rows() const { return kind == KIND_FEW ? M() : b200moe_padded_rows_cap(M(), E); }
+};
+
+// Most rows per expert, on average, for which a forward without a backward runs over compact rows with the weights as
+// the MMA's M operand (gemm_few.cu).  Gate/up + down, us, row tiles against compact rows, at H 2048, I 1408, 64
+// experts: 4.5 rows an expert 237 / 170, 141 rows 238 / 213, 206 rows 240 / 328 (an expert then takes two tiles).
+constexpr int64_t kFewRows = 160;
+
+static Dims make_dims(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int rows_kernels) {
+  Dims d{T, H, I, E, n_glu, k, KIND_TILES};
+  if (rows_kernels) d.kind = KIND_ROWS;
+  else if (!keep && T * k <= kFewRows * E) d.kind = KIND_FEW;
+  return d;
+}
+
+static int check_dims(const char* who, const Dims& d) {
+  B200_CHECK_ARG(d.T > 0 && d.H > 0 && d.I > 0 && d.H % 8 == 0 && d.I % 8 == 0 && d.E >= 1 && d.n_glu >= 1 && d.n_glu <= d.E &&
+                     d.k >= 1 && d.T < (1LL << 31),
+                 B200MOE_E_BAD_SHAPE, "%s: T = %lld, H = %lld, I = %lld (multiples of 8), E = %d (%d with weights), k = %d", who,
+                 (long long)d.T, (long long)d.H, (long long)d.I, d.E, d.n_glu, d.k);
+  return 0;
+}
+
+struct Forward {
+  int32_t *counts, *offs, *poffs, *slot_row, *row_slot, *tile_expert, *order, *slot_pos;
+  void* scratch;
+  size_t scratch_bytes;
+  bf16_t *x_s, *gate_up, *inter, *eo;
+  bf16_t* logits;         // of the router, when it runs here
+  int64_t* idx;
+  float* w;
+};
+
+static Forward carve_forward(const Dims& d, bool router, void* ws, size_t* bytes) {
+  Carver c(ws);
+  Forward f{};
+  const int64_t M = d.M(), cap = b200moe_padded_rows_cap(M, d.E), rows = d.rows();
+  const bool few = d.kind == KIND_FEW;
+  f.counts = c.take<int32_t>(d.E);
+  f.offs = c.take<int32_t>(d.E + 1);
+  f.poffs = c.take<int32_t>(d.E + 1);
+  f.slot_row = c.take<int32_t>(M);
+  f.row_slot = c.take<int32_t>(cap);
+  f.tile_expert = c.take<int32_t>(cap / B200MOE_TILE_M);
+  if (few) {
+    f.order = c.take<int32_t>(M);
+    f.slot_pos = c.take<int32_t>(M);
+  }
+  f.scratch_bytes = b200moe_permute_ws_bytes(M, d.E);
+  f.scratch = c.take<char>(f.scratch_bytes);
+  if (router) {
+    f.logits = c.take<bf16_t>(d.T * d.E);
+    f.idx = c.take<int64_t>(M);
+    f.w = c.take<float>(M);
+  }
+  f.x_s = c.take<bf16_t>(rows * d.H);
+  if (!few) f.gate_up = c.take<bf16_t>(rows * 2 * d.I);
+  f.inter = c.take<bf16_t>(rows * d.I);
+  f.eo = c.take<bf16_t>(rows * d.H);
+  if (bytes != nullptr) *bytes = c.off;
+  return f;
+}
+
+struct Backward {
+  bf16_t *grad_eo, *grad_gu, *grad_x_s, *grad_inter;
+  float *row_da, *row_dg;
+  float* grad_w;                     // when the router's backward follows
+  bf16_t *grad_logits, *grad_x_router;
+  float* part;
+};
+
+// split-K of the router's weight gradient: about two tiles per SM
+static int64_t router_k_chunk(int64_t T, int64_t E, int64_t H) {
+  const int64_t tiles = ((E + 127) / 128) * ((H + 255) / 256);
+  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(296 / std::max<int64_t>(tiles, 1), (T + 63) / 64));
+  return ((T + slices - 1) / slices + 63) / 64 * 64;
+}
+static int64_t router_slices(int64_t T, int64_t E, int64_t H) {
+  const int64_t c = router_k_chunk(T, E, H);
+  return (T + c - 1) / c;
+}
+
+static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* bytes) {
+  Carver c(ws);
+  Backward b{};
+  const int64_t rows = d.rows();
+  b.grad_eo = c.take<bf16_t>(rows * d.H);
+  b.grad_gu = c.take<bf16_t>(rows * 2 * d.I);
+  if (d.kind == KIND_ROWS) {
+    b.grad_x_s = c.take<bf16_t>(rows * d.H);       // grad_eo is still read (Identity experts) while this is written
+    b.grad_inter = c.take<bf16_t>(rows * d.I);
+    b.row_da = c.take<float>(rows);
+    b.row_dg = c.take<float>(rows);
+  } else {
+    b.grad_x_s = b.grad_eo;                        // written after the last read of grad_eo
+  }
+  if (router) {
+    b.grad_w = c.take<float>(d.M());
+    b.grad_logits = c.take<bf16_t>(d.T * d.E);
+    b.grad_x_router = c.take<bf16_t>(d.T * d.H);
+    b.part = c.take<float>(router_slices(d.T, d.E, d.H) * d.E * d.H);
+  }
+  if (bytes != nullptr) *bytes = c.off;
+  return b;
+}
+
+#define RUN(name, launches, call)     \
+  do {                                \
+    OpScope scope__(name, launches);  \
+    const int rc__ = (call);          \
+    if (rc__) return rc__;            \
+  } while (0)
+
+static int permute(const Dims& d, const int64_t* idx, const Forward& f, int32_t* counts_out, int64_t* load, int32_t* status,
+                   b200moe_stream_t st) {
+  RUN("permute_build", d.M() > 1024 ? 2 : 1,
+      permute_build(idx, d.T, d.k, d.E, f.counts, f.offs, f.poffs, f.slot_row, f.row_slot, f.tile_expert, f.order,
+                    f.slot_pos, f.scratch, f.scratch_bytes, counts_out, load, status, st));
+  return 0;
+}
+
+static int experts_forward(const Dims& d, const void* x, const float* w, const void* gate_up_proj, const void* down_proj,
+                           const int32_t* codes, const float* params, const Forward& f, void* out, int32_t* status,
+                           b200moe_stream_t st) {
+  const int64_t rows = d.rows();
+  if (d.kind == KIND_FEW) {
+    RUN("gather_rows", 1, b200moe_gather_rows(x, f.order, f.offs + d.E, d.k, d.H, rows, f.x_s, st));
+    RUN("expert_gate_up_few", 1, b200moe_expert_gate_up_few(f.x_s, gate_up_proj, codes, f.counts, f.offs, rows, d.E, d.H, d.I,
+                                                            f.inter, status, st));
+    RUN("expert_linear_few", 1, b200moe_expert_linear_few(f.inter, down_proj, f.counts, f.offs, rows, d.E, d.H, d.I, f.eo, status, st));
+    RUN("combine", 1, b200moe_combine(f.eo, w, f.slot_pos, d.T, d.k, d.H, out, st));
+    return 0;
+  }
+  RUN("gather_rows", 1, b200moe_gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, rows, f.x_s, st));
+  if (d.kind == KIND_TILES) {
+    RUN("expert_gate_up_swiglu", 1, b200moe_expert_gate_up_act(f.x_s, gate_up_proj, codes, f.tile_expert, f.poffs, rows, 0, 0,
+                                                               d.E, d.H, d.I, f.gate_up, f.inter, status, st));
+    RUN("expert_down", 1, b200moe_expert_linear(f.inter, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, status, st));
+  } else {   // the GEMMs and the activation kernels see the rows of the experts with weights only
+    RUN("expert_linear", 1, b200moe_expert_linear(f.x_s, gate_up_proj, f.tile_expert, f.poffs, rows, d.n_glu, 2 * d.I, d.H,
+                                                  f.gate_up, status, st));
+    RUN("glu_fwd_rows", 1, b200moe_glu_fwd_rows(f.gate_up, f.tile_expert, codes, params, f.poffs + d.n_glu, rows, d.I, f.inter, st));
+    RUN("expert_linear", 1, b200moe_expert_linear(f.inter, down_proj, f.tile_expert, f.poffs, rows, d.n_glu, d.H, d.I, f.eo, status, st));
+    if (d.n_glu < d.E)
+      RUN("special_rows", 1, b200moe_special_rows(f.x_s, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, rows, f.eo, st));
+  }
+  RUN("combine", 1, b200moe_combine(f.eo, w, f.slot_row, d.T, d.k, d.H, out, st));
+  return 0;
+}
+
+// Gradients to compute (nullptr: not wanted; x != nullptr: the rows b.grad_x_s, which the caller combines per token)
+struct Grads {
+  void *x, *gate_up, *down;
+  float *w, *params;
+};
+
+static int experts_backward(const Dims& d, const void* grad_out, const float* w, const void* gate_up_proj,
+                            const void* down_proj, const int32_t* codes, const float* params, const Forward& f,
+                            const Backward& b, const Grads& g, int32_t* status, b200moe_stream_t st) {
+  const int64_t rows = d.rows();
+  const int32_t* total = f.poffs + d.E;
+  RUN("combine_bwd", 1, b200moe_combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, rows, b.grad_eo, g.w, st));
+  if (d.kind == KIND_TILES) {
+    if (g.x != nullptr || g.gate_up != nullptr) {
+      RUN("expert_down_dgrad_glu", 1,
+          b200moe_expert_down_dgrad_act(b.grad_eo, down_proj, f.gate_up, codes, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H,
+                                        d.I, b.grad_gu, status, st));
+      if (g.gate_up != nullptr)
+        RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_gu, f.x_s, f.poffs, f.counts, rows, d.E, 2 * d.I, d.H, g.gate_up, status, st));
+    }
+    if (g.down != nullptr)
+      RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_eo, f.inter, f.poffs, f.counts, rows, d.E, d.H, d.I, g.down, status, st));
+    if (g.x != nullptr)
+      RUN("expert_gate_up_dgrad", 1, b200moe_expert_linear_t(b.grad_gu, gate_up_proj, f.tile_expert, f.poffs, rows, d.E, 2 * d.I,
+                                                             d.H, b.grad_x_s, status, st));
+    return 0;
+  }
+  const int n = d.n_glu;
+  RUN("expert_linear_t", 1, b200moe_expert_linear_t(b.grad_eo, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, b.grad_inter, status, st));
+  float* da = g.params != nullptr ? b.row_da : nullptr;
+  float* dg = g.params != nullptr ? b.row_dg : nullptr;
+  RUN("glu_bwd_rows", 1, b200moe_glu_bwd_rows(b.grad_inter, f.gate_up, f.tile_expert, codes, params, f.poffs + n, rows, d.I,
+                                              b.grad_gu, da, dg, st));
+  if (g.down != nullptr)
+    RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_eo, f.inter, f.poffs, f.counts, rows, n, d.H, d.I, g.down, status, st));
+  if (g.gate_up != nullptr)
+    RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_gu, f.x_s, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, status, st));
+  if (g.x != nullptr) {
+    RUN("expert_linear_t", 1, b200moe_expert_linear_t(b.grad_gu, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, b.grad_x_s, status, st));
+    if (n < d.E)
+      RUN("special_rows", 1, b200moe_special_rows(b.grad_eo, f.tile_expert, codes, f.poffs, n, d.E, d.H, rows, b.grad_x_s, st));
+  }
+  if (g.params != nullptr) {
+    if (n < d.E)
+      B200_CUDA(cudaMemsetAsync(g.params + 2 * n, 0, sizeof(float) * 2 * (d.E - n), (cudaStream_t)st));
+    RUN("expert_row_sums", 1, b200moe_expert_row_sums(da, dg, f.poffs, n, g.params, st));
+  }
+  return 0;
+}
+
+// Up to this many tokens (four for each of 148 SMs; with more than 64 experts correspondingly fewer) logits and picks are
+// one launch of CUDA-core dot products.  GEMM + top-k against it, us, top-6 of 64 experts at H 2048: 48 tokens 15.6 / 7.5,
+// 512 tokens 16.1 / 11.7, 1024 tokens 16.1 / 20.9; 128 experts: 128 tokens 17.6 / 10.0, 256 tokens 17.6 / 16.2; 256 experts:
+// 100 tokens at H 4096 29.1 / 27.3, 256 tokens at H 1024 15.5 / 19.0.
+constexpr int64_t kSmallTokens = 592;
+
+static int router_forward(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k, int norm,
+                          float scale, void* logits, int64_t* idx, float* w, int32_t* counts, int32_t* status,
+                          b200moe_stream_t st) {
+  if (T <= kSmallTokens && T * E <= 64 * kSmallTokens) {
+    RUN("router_small_fwd", 1, b200moe_router_small_fwd(x, weight, bias, T, H, E, k, norm, scale, logits, idx, w, counts, st));
+    return 0;
+  }
+  RUN("gemm_nt", 1, b200moe_gemm_nt(x, weight, logits, T, E, H, status, st));
+  RUN("router_topk_fwd", 1, b200moe_router_topk_fwd(logits, B200MOE_LOGITS_BF16, bias, T, E, k, norm, scale, idx, w, counts, st));
+  return 0;
+}
+
+static int router_backward(const void* x, const void* weight, const void* logits, const int64_t* idx, const float* grad_w,
+                           int64_t T, int64_t H, int E, int k, int norm, float scale, void* grad_logits, float* part,
+                           void* grad_x, void* grad_weight, int32_t* status, b200moe_stream_t st) {
+  RUN("router_topk_bwd", 1, b200moe_router_topk_bwd(logits, B200MOE_LOGITS_BF16, idx, grad_w, T, E, k, norm, scale, grad_logits, st));
+  if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(grad_logits, weight, grad_x, T, H, E, status, st));
+  if (grad_weight != nullptr) {
+    OpScope scope("gemm_tn", 2);
+    int rc = b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, router_k_chunk(T, E, H), status, st);
+    if (rc) return rc;
+    rc = b200moe_splitk_reduce(part, router_slices(T, E, H), static_cast<int64_t>(E) * H, grad_weight, st);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" {
+
+// ---------------------------------------------------------------------------- router alone
+int b200moe_router_forward(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
+                           int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
+                           int32_t* status, b200moe_stream_t stream) {
+  return router_forward(x, weight, bias, T, H, E, k, norm_topk, scale, logits, idx, w, counts, status, stream);
+}
+
+size_t b200moe_router_bwd_ws_bytes(int64_t T, int64_t H, int E) {
+  if (T <= 0 || H <= 0 || E <= 0) return 0;
+  Carver c(nullptr);
+  c.take<bf16_t>(T * E);
+  c.take<float>(router_slices(T, E, H) * E * H);
+  return c.off;
+}
+
+int b200moe_router_backward(const void* x, const void* weight, const void* logits, const int64_t* idx, const float* grad_w,
+                            int64_t T, int64_t H, int E, int k, int norm_topk, float scale, void* ws, void* grad_x,
+                            void* grad_weight, int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(ws, B200MOE_E_NULL, "router_backward: null workspace");
+  Carver c(ws);
+  bf16_t* gl = c.take<bf16_t>(T * E);
+  float* part = c.take<float>(router_slices(T, E, H) * E * H);
+  return router_backward(x, weight, logits, idx, grad_w, T, H, E, k, norm_topk, scale, gl, part, grad_x, grad_weight, status, stream);
+}
+
+// ---------------------------------------------------------------------------- experts on given picks
+size_t b200moe_moe_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int row_kernels) {
+  size_t n = 0;
+  carve_forward(make_dims(T, H, I, E, n_glu, k, keep, row_kernels), false, nullptr, &n);
+  return n;
+}
+
+int b200moe_moe_forward(const void* x, const int64_t* idx, const float* w, const void* gate_up_proj, const void* down_proj,
+                        const int32_t* act_codes, const float* act_params, int64_t T, int64_t H, int64_t I, int E, int n_glu,
+                        int k, int keep, int row_kernels, void* ws, void* out, int32_t* status, b200moe_stream_t stream) {
+  const Dims d = make_dims(T, H, I, E, n_glu, k, keep, row_kernels);
+  int rc = check_dims("moe_forward", d);
+  if (rc) return rc;
+  B200_CHECK_ARG(x && idx && w && gate_up_proj && down_proj && ws && out, B200MOE_E_NULL, "moe_forward: null pointer");
+  const Forward f = carve_forward(d, false, ws, nullptr);
+  rc = permute(d, idx, f, nullptr, nullptr, status, stream);
+  if (rc) return rc;
+  return experts_forward(d, x, w, gate_up_proj, down_proj, act_codes, act_params, f, out, status, stream);
+}
+
+size_t b200moe_moe_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int row_kernels) {
+  size_t n = 0;
+  carve_backward(make_dims(T, H, I, E, n_glu, k, 1, row_kernels), false, nullptr, &n);
+  return n;
+}
+
+int b200moe_moe_backward(const void* grad_out, const float* w, const void* gate_up_proj, const void* down_proj,
+                         const int32_t* act_codes, const float* act_params, int64_t T, int64_t H, int64_t I, int E,
+                         int n_glu, int k, int row_kernels, void* fwd_ws, void* ws, void* grad_x, float* grad_w,
+                         void* grad_gate_up, void* grad_down, float* grad_params, int32_t* status, b200moe_stream_t stream) {
+  const Dims d = make_dims(T, H, I, E, n_glu, k, 1, row_kernels);
+  int rc = check_dims("moe_backward", d);
+  if (rc) return rc;
+  B200_CHECK_ARG(grad_out && w && gate_up_proj && down_proj && fwd_ws && ws && grad_w, B200MOE_E_NULL, "moe_backward: null pointer");
+  const Forward f = carve_forward(d, false, fwd_ws, nullptr);
+  const Backward b = carve_backward(d, false, ws, nullptr);
+  const Grads g{grad_x, grad_gate_up, grad_down, grad_w, grad_params};
+  rc = experts_backward(d, grad_out, w, gate_up_proj, down_proj, act_codes, act_params, f, b, g, status, stream);
+  if (rc) return rc;
+  if (grad_x != nullptr) RUN("combine", 1, b200moe_combine(b.grad_x_s, nullptr, f.slot_row, T, k, H, grad_x, stream));
+  return 0;
+}
+
+// ---------------------------------------------------------------------------- router and experts
+size_t b200moe_layer_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k, int keep) {
+  size_t n = 0;
+  carve_forward(make_dims(T, H, I, E, E, k, keep, 0), true, nullptr, &n);
+  return n;
+}
+
+int b200moe_layer_forward(const void* x, const void* gate_weight, const float* bias, const void* gate_up_proj,
+                          const void* down_proj, const int32_t* act_codes, int64_t T, int64_t H, int64_t I, int E, int k,
+                          int norm_topk, float scale, int keep, void* ws, int32_t* counts, int64_t* load, void* out,
+                          int32_t* status, b200moe_stream_t stream) {
+  const Dims d = make_dims(T, H, I, E, E, k, keep, 0);
+  int rc = check_dims("layer_forward", d);
+  if (rc) return rc;
+  B200_CHECK_ARG(x && gate_weight && gate_up_proj && down_proj && ws && out, B200MOE_E_NULL, "layer_forward: null pointer");
+  const Forward f = carve_forward(d, true, ws, nullptr);
+  rc = router_forward(x, gate_weight, bias, T, H, E, k, norm_topk, scale, f.logits, f.idx, f.w, nullptr, status, stream);
+  if (rc) return rc;
+  rc = permute(d, f.idx, f, counts, load, status, stream);
+  if (rc) return rc;
+  return experts_forward(d, x, f.w, gate_up_proj, down_proj, act_codes, nullptr, f, out, status, stream);
+}
+
+size_t b200moe_layer_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k) {
+  size_t n = 0;
+  carve_backward(make_dims(T, H, I, E, E, k, 1, 0), true, nullptr, &n);
+  return n;
+}
+
+int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate_weight, const void* gate_up_proj,
+                           const void* down_proj, const int32_t* act_codes, int64_t T, int64_t H, int64_t I, int E, int k,
+                           int norm_topk, float scale, void* fwd_ws, void* ws, void* grad_x, void* grad_gate_weight,
+                           void* grad_gate_up, void* grad_down, int32_t* status, b200moe_stream_t stream) {
+  const Dims d = make_dims(T, H, I, E, E, k, 1, 0);
+  int rc = check_dims("layer_backward", d);
+  if (rc) return rc;
+  B200_CHECK_ARG(grad_out && x && gate_weight && gate_up_proj && down_proj && fwd_ws && ws, B200MOE_E_NULL, "layer_backward: null pointer");
+  const Forward f = carve_forward(d, true, fwd_ws, nullptr);
+  const Backward b = carve_backward(d, true, ws, nullptr);
+  const Grads g{grad_x, grad_gate_up, grad_down, b.grad_w, nullptr};
+  rc = experts_backward(d, grad_out, f.w, gate_up_proj, down_proj, act_codes, nullptr, f, b, g, status, stream);
+  if (rc) return rc;
+  if (grad_x != nullptr || grad_gate_weight != nullptr) {
+    rc = router_backward(x, gate_weight, f.logits, f.idx, b.grad_w, T, H, E, k, norm_topk, scale, b.grad_logits, b.part,
+                         grad_x != nullptr ? b.grad_x_router : nullptr, grad_gate_weight, status, stream);
+    if (rc) return rc;
+  }
+  if (grad_x != nullptr)   // the experts' rows of a token and the router's share, added in fp32, one rounding
+    RUN("combine", 1, b200moe_combine_add(b.grad_x_s, nullptr, f.slot_row, b.grad_x_router, T, k, H, grad_x, stream));
+  return 0;
+}
+
+// ---------------------------------------------------------------------------- Newton-Schulz iterations
+int b200moe_newton_schulz(void* x, void* x_next, void* a, void* a2, const int32_t* tile_expert, const int32_t* poffs, int E,
+                          int64_t Rp, int64_t wide, const float* coeffs, int iterations, int32_t* status,
+                          b200moe_stream_t stream) {
+  B200_CHECK_ARG(x && x_next && a && a2 && coeffs, B200MOE_E_NULL, "newton_schulz: null pointer");
+  B200_CHECK_ARG(iterations >= 0, B200MOE_E_BAD_SHAPE, "newton_schulz: iterations = %d", iterations);
+  const int64_t rows = E * Rp;
+  for (int i = 0; i < iterations; ++i) {
+    const float ca = coeffs[3 * i], cb = coeffs[3 * i + 1], cc = coeffs[3 * i + 2];
+    RUN("expert_gram", 1, b200moe_expert_gram(x, tile_expert, poffs, rows, E, wide, 1, a, status, stream));
+    RUN("expert_linear_axpby", 1, b200moe_expert_linear_axpby(a, a, a, cc, cb, ca, 2, tile_expert, poffs, rows, E, Rp, Rp, a2, status, stream));
+    RUN("expert_linear_t", 1, b200moe_expert_linear_t(a2, x, tile_expert, poffs, rows, E, Rp, wide, x_next, status, stream));
+    std::swap(x, x_next);
+  }
+  return 0;
+}
+
+}  // extern "C"

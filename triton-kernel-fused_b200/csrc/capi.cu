@@ -51,6 +51,17 @@ __global__ void selftest_bounded_wait_kernel(int* status, long long limit_cycles
   if (threadIdx.x == 0 && !done && abort_flag != 0) atomicCAS(status, 0, abort_flag);
 }
 
+static std::atomic<b200moe_observer_t> g_observer{nullptr};
+
+OpScope::OpScope(const char* n, int l) : name(n), launches(l) {
+  b200moe_observer_t f = g_observer.load(std::memory_order_acquire);
+  if (f != nullptr) f(name, launches, 0);
+}
+OpScope::~OpScope() {
+  b200moe_observer_t f = g_observer.load(std::memory_order_acquire);
+  if (f != nullptr) f(name, launches, 1);
+}
+
 static std::atomic<int> g_reserved_sms{0};
 
 int gemm_cta_budget() {
@@ -78,6 +89,11 @@ int b200moe_selftest_bounded_wait(int32_t* status, int64_t limit_cycles, b200moe
   b200moe::selftest_bounded_wait_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status, limit_cycles);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return b200moe::cuda_fail(e, "selftest_bounded_wait launch");
+  return 0;
+}
+
+int b200moe_set_observer(b200moe_observer_t observer) {
+  b200moe::g_observer.store(observer, std::memory_order_release);
   return 0;
 }
 

@@ -15,10 +15,11 @@ __device__ __forceinline__ void fma8(float (&acc)[8], const uint4& v, float w) {
 
 constexpr int kVecBatch = 4;   // 16-byte vectors a lane keeps in flight per row it reads
 
-// out[t] = sum_j w[t,j] * rows[slot_row[t*k+j]]  (fp32 accumulate in slot order j = 0..k-1)
+// out[t] = sum_j w[t,j] * rows[slot_row[t*k+j]] (+ add[t])  (fp32 accumulate in slot order j = 0..k-1).  `add` is the
+// router's share of grad_x: adding it here saves the pass of a separate addition (headline layer: 32 us)
 __global__ void __launch_bounds__(256)
 combine_kernel(const uint4* __restrict__ rows, const float* __restrict__ w, const int* __restrict__ slot_row,
-               long long T, int k, int vec_per_row, uint4* __restrict__ out) {
+               const uint4* __restrict__ add, long long T, int k, int vec_per_row, uint4* __restrict__ out) {
   __shared__ int s_row[B200MOE_MAX_TOPK];
   __shared__ float s_w[B200MOE_MAX_TOPK];
   for (long long t = blockIdx.x; t < T; t += gridDim.x) {
@@ -35,6 +36,7 @@ combine_kernel(const uint4* __restrict__ rows, const float* __restrict__ w, cons
         const uint4 v = rows[static_cast<long long>(s_row[j]) * vec_per_row + c];
         fma8(acc, v, s_w[j]);
       }
+      if (add != nullptr) fma8(acc, add[t * vec_per_row + c], 1.0f);
       uint4 o;
       o.x = pack_bf16x2(acc[0], acc[1]);
       o.y = pack_bf16x2(acc[2], acc[3]);
@@ -107,16 +109,22 @@ extern "C" {
 
 int b200moe_combine(const void* rows, const float* w, const int32_t* slot_row, int64_t T, int k, int64_t H,
                     void* out, b200moe_stream_t stream) {
+  return b200moe_combine_add(rows, w, slot_row, nullptr, T, k, H, out, stream);
+}
+
+int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k,
+                        int64_t H, void* out, b200moe_stream_t stream) {
   B200_CHECK_ARG(rows && slot_row && out, B200MOE_E_NULL, "combine: null pointer");
   B200_CHECK_ARG(H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE, "combine: H = %lld must be a multiple of 8", (long long)H);
   B200_CHECK_ARG(k >= 1 && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "combine: k = %d", k);
-  B200_CHECK_ARG(aligned16(rows) && aligned16(out), B200MOE_E_ALIGN, "combine: pointers must be 16-byte aligned");
+  B200_CHECK_ARG(aligned16(rows) && aligned16(out) && aligned16(add), B200MOE_E_ALIGN, "combine: pointers must be 16-byte aligned");
   if (T <= 0) return 0;
   long long grid = T;
   const long long cap = static_cast<long long>(num_sms()) * 16;
   if (grid > cap) grid = cap;
   combine_kernel<<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint4*>(rows), w, slot_row, T, k, static_cast<int>(H / 8), reinterpret_cast<uint4*>(out));
+      reinterpret_cast<const uint4*>(rows), w, slot_row, reinterpret_cast<const uint4*>(add), T, k, static_cast<int>(H / 8),
+      reinterpret_cast<uint4*>(out));
   B200_CUDA(cudaGetLastError());
   return 0;
 }

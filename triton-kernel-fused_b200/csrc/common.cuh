@@ -27,6 +27,19 @@ int num_sms();
 int gemm_cta_budget();   // CTAs a persistent GEMM may occupy (num_sms() minus the reserved SMs)
 int exchange_sm_budget();   // SMs (= fat CTAs) the home-side pull kernel of the expert-parallel exchange may occupy
 
+// b200moe_permute_build; also stores the counts a second time (counts_out) and adds them to `load` (both nullable)
+int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs, int32_t* poffs,
+                  int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
+                  size_t ws_bytes, int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream);
+
+// Tells the observer set by b200moe_set_observer, if any, where an operation of a longer sequence begins and ends
+struct OpScope {
+  OpScope(const char* name, int launches);
+  ~OpScope();
+  const char* name;
+  int launches;
+};
+
 #define B200_CHECK_ARG(cond, code, ...)  \
   do {                                   \
     if (!(cond)) {                       \

@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(32 * W)
 permute_rank_kernel(const long long* __restrict__ idx, long long M, int E, const int* __restrict__ block_hist,
                     int* __restrict__ counts, int* __restrict__ offs, int* __restrict__ poffs,
                     int* __restrict__ slot_row, int* __restrict__ row_slot, int* __restrict__ tile_expert,
-                    int* __restrict__ order, int* __restrict__ slot_pos, int* __restrict__ status) {
+                    int* __restrict__ order, int* __restrict__ slot_pos, int* __restrict__ counts_out,
+                    long long* __restrict__ load, int* __restrict__ status) {
   constexpr int kPermWarps = W, kPermThreads = 32 * W;
   extern __shared__ int sh[];                          // [W][E]: ranks a warp's run starts at
   __shared__ int s_before[B200MOE_MAX_EXPERTS];        // slots of the expert in earlier CTAs
@@ -163,7 +164,10 @@ permute_rank_kernel(const long long* __restrict__ idx, long long M, int E, const
     for (int e = threadIdx.x; e <= E; e += kPermThreads) {
       offs[e] = s_off[e];
       poffs[e] = s_poff[e];
-      if (e < E) counts[e] = s_cnt[e];
+      if (e == E) continue;
+      counts[e] = s_cnt[e];
+      if (counts_out != nullptr) counts_out[e] = s_cnt[e];
+      if (load != nullptr) load[e] += s_cnt[e];
     }
   for (int e = blockIdx.x * kPermWarps + warp; e < E; e += gridDim.x * kPermWarps) {
     const int p0 = s_poff[e], p1 = s_poff[e + 1];
@@ -191,8 +195,8 @@ permute_rank_kernel(const long long* __restrict__ idx, long long M, int E, const
 
 template <int W, int PL>
 static int launch_permute(const long long* idx, long long M, int E, int* hist, int* counts, int* offs, int* poffs,
-                          int* slot_row, int* row_slot, int* tile_expert, int* order, int* slot_pos, int* status,
-                          cudaStream_t st) {
+                          int* slot_row, int* row_slot, int* tile_expert, int* order, int* slot_pos, int* counts_out,
+                          long long* load, int* status, cudaStream_t st) {
   constexpr int run = 32 * W * PL;
   const int blocks = M > run ? static_cast<int>((M + run - 1) / run) : 1;
   if (blocks > 1) {
@@ -200,7 +204,8 @@ static int launch_permute(const long long* idx, long long M, int E, int* hist, i
     B200_CUDA(cudaGetLastError());
   }
   permute_rank_kernel<W, PL><<<blocks, 32 * W, sizeof(int) * W * E, st>>>(
-      idx, M, E, hist, counts, offs, poffs, slot_row, row_slot, tile_expert, order, slot_pos, status);
+      idx, M, E, hist, counts, offs, poffs, slot_row, row_slot, tile_expert, order, slot_pos, counts_out, load,
+      status);
   B200_CUDA(cudaGetLastError());
   return 0;
 }
@@ -220,6 +225,30 @@ gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ row_slot
       for (int c = threadIdx.x; c < vec_per_row; c += blockDim.x) dst[c] = src[c];
     }
   }
+}
+
+int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs,
+                  int32_t* poffs, int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert,
+                  int32_t* order, int32_t* slot_pos, void* ws, size_t ws_bytes,
+                  int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(idx && counts && offs && poffs && slot_row && row_slot && tile_expert && ws && status,
+                 B200MOE_E_NULL, "permute_build: null pointer");
+  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
+                 "permute_build: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
+  B200_CHECK_ARG(T >= 0 && k >= 1 && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE,
+                 "permute_build: T = %lld, k = %d", (long long)T, k);
+  const int64_t M = T * k;
+  B200_CHECK_ARG(b200moe_padded_rows_cap(M, E) < (1LL << 31), B200MOE_E_BAD_SHAPE,
+                 "permute_build: %lld routed rows do not fit int32 tables", (long long)M);
+  B200_CHECK_ARG(ws_bytes >= b200moe_permute_ws_bytes(M, E), B200MOE_E_WS_TOO_SMALL,
+                 "permute_build: workspace %zu < %zu bytes", ws_bytes, b200moe_permute_ws_bytes(M, E));
+  const PermSplit split = perm_split(M);
+  auto launch = split.per_lane == 16 ? launch_permute<32, 16>
+                : split.warps == 8   ? launch_permute<8, 4>
+                : split.warps == 16  ? launch_permute<16, 4>
+                             : launch_permute<32, 4>;
+  return launch(reinterpret_cast<const long long*>(idx), M, E, reinterpret_cast<int*>(ws), counts, offs, poffs, slot_row,
+                row_slot, tile_expert, order, slot_pos, counts_out, reinterpret_cast<long long*>(load), status, (cudaStream_t)stream);
 }
 
 }  // namespace b200moe
@@ -243,24 +272,8 @@ int b200moe_permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* 
                           int32_t* poffs, int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert,
                           int32_t* order, int32_t* slot_pos, void* ws, size_t ws_bytes, int32_t* status,
                           b200moe_stream_t stream) {
-  B200_CHECK_ARG(idx && counts && offs && poffs && slot_row && row_slot && tile_expert && ws && status,
-                 B200MOE_E_NULL, "permute_build: null pointer");
-  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
-                 "permute_build: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
-  B200_CHECK_ARG(T >= 0 && k >= 1 && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE,
-                 "permute_build: T = %lld, k = %d", (long long)T, k);
-  const int64_t M = T * k;
-  B200_CHECK_ARG(b200moe_padded_rows_cap(M, E) < (1LL << 31), B200MOE_E_BAD_SHAPE,
-                 "permute_build: %lld routed rows do not fit int32 tables", (long long)M);
-  B200_CHECK_ARG(ws_bytes >= b200moe_permute_ws_bytes(M, E), B200MOE_E_WS_TOO_SMALL,
-                 "permute_build: workspace %zu < %zu bytes", ws_bytes, b200moe_permute_ws_bytes(M, E));
-  const PermSplit split = perm_split(M);
-  auto launch = split.per_lane == 16 ? launch_permute<32, 16>
-                : split.warps == 8   ? launch_permute<8, 4>
-                : split.warps == 16  ? launch_permute<16, 4>
-                                     : launch_permute<32, 4>;
-  return launch(reinterpret_cast<const long long*>(idx), M, E, reinterpret_cast<int*>(ws), counts, offs, poffs, slot_row,
-                row_slot, tile_expert, order, slot_pos, status, (cudaStream_t)stream);
+  return permute_build(idx, T, k, E, counts, offs, poffs, slot_row, row_slot, tile_expert, order, slot_pos, ws, ws_bytes,
+                       nullptr, nullptr, status, stream);
 }
 
 int b200moe_gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,

@@ -6,7 +6,8 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from .moe import moe
+from . import _lib as L
+from .moe import FUSED_CODES, _amp_cast, _code_info, _codes_on, _float32, moe
 from .mxfp8 import moe_mxfp8
 from .router import fused_mlp_router, router_bias_update
 
@@ -79,6 +80,58 @@ class LoadBalanceMixin:
                 "idle_experts": int((c == 0).sum())}
 
 
+class _Layer(torch.autograd.Function):
+    """Router and experts of a bf16 layer whose activations run in the GEMM epilogues, one native call each way
+    (csrc/block.cu): `fused_mlp_router` followed by `moe`, with the two shares of grad_x added in the last kernel.  Returns
+    (out (N,H), counts (E,) int32); `load` (E int64, or None) gets the counts added."""
+
+    @staticmethod
+    def forward(ctx, x, gate_weight, bias, gate_up_proj, down_proj, codes_dev, load, top_k, norm, scale, keep):
+        x, gate_weight, gate_up_proj, down_proj = _amp_cast(x, gate_weight, gate_up_proj, down_proj)
+        for name, t in (("x", x), ("gate_weight", gate_weight), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
+            L.require_cuda_bf16(name, t)
+        (T, H), (E, twoI, H2), dev = x.shape, gate_up_proj.shape, x.device
+        I = twoI // 2
+        L.require(H2 == H and twoI == 2 * I and tuple(down_proj.shape) == (E, H, I) and tuple(gate_weight.shape) == (E, H),
+                  f"weight shapes must be (E,H), (E,2I,H) and (E,H,I); got {tuple(gate_weight.shape)}, "
+                  f"{tuple(gate_up_proj.shape)}, {tuple(down_proj.shape)}")
+        bias32 = None if bias is None else _float32(bias.detach())
+        L.require(bias is None or (bias32.device == dev and bias32.numel() == E), "bias must have E elements on x's device")
+        L.require(gate_weight.device == gate_up_proj.device == down_proj.device == dev, "all tensors must be on one device")
+        x, gate_weight = x.contiguous(), gate_weight.contiguous()
+        gate_up_proj, down_proj = gate_up_proj.contiguous(), down_proj.contiguous()
+        lib = L.lib()
+        ws = L.workspace(lib.b200moe_layer_fwd_ws_bytes(T, H, I, E, top_k, keep), dev)
+        out = torch.empty(T, H, dtype=torch.bfloat16, device=dev)
+        counts = torch.empty(E, dtype=torch.int32, device=dev)
+        L.check(lib.b200moe_layer_forward(x.data_ptr(), gate_weight.data_ptr(), L.ptr(bias32), gate_up_proj.data_ptr(),
+                                          down_proj.data_ptr(), L.ptr(codes_dev), T, H, I, E, top_k, norm, scale, keep,
+                                          ws.data_ptr(), counts.data_ptr(), L.ptr(load), out.data_ptr(),
+                                          L.status_word(dev).data_ptr(), L.stream_of(x)))
+        if keep:
+            ctx.dims = (T, H, I, E, top_k, norm, scale)
+            ctx.save_for_backward(x, gate_weight, gate_up_proj, down_proj, codes_dev, ws)
+        ctx.mark_non_differentiable(counts)
+        return out, counts
+
+    @staticmethod
+    def backward(ctx, grad_out, grad_counts):
+        x, gate_weight, gate_up_proj, down_proj, codes_dev, ws = ctx.saved_tensors
+        T, H, I, E, k, norm, scale = ctx.dims
+        need_x, need_gate, _, need_gu, need_dn = ctx.needs_input_grad[:5]
+        dev = x.device
+        grad_out = grad_out.to(torch.bfloat16).contiguous()
+        grad = lambda need, t: torch.empty(t.shape, dtype=torch.bfloat16, device=dev) if need else None     # noqa: E731
+        gx, ggate, ggu, gdn = grad(need_x, x), grad(need_gate, gate_weight), grad(need_gu, gate_up_proj), grad(need_dn, down_proj)
+        lib = L.lib()
+        tmp = L.workspace(lib.b200moe_layer_bwd_ws_bytes(T, H, I, E, k), dev)
+        L.check(lib.b200moe_layer_backward(grad_out.data_ptr(), x.data_ptr(), gate_weight.data_ptr(), gate_up_proj.data_ptr(),
+                                           down_proj.data_ptr(), L.ptr(codes_dev), T, H, I, E, k, norm, scale, ws.data_ptr(),
+                                           tmp.data_ptr(), L.ptr(gx), L.ptr(ggate), L.ptr(ggu), L.ptr(gdn),
+                                           L.status_word(dev).data_ptr(), L.stream_of(x)))
+        return gx, ggate, None, ggu, gdn, None, None, None, None, None, None
+
+
 class MoELayer(LoadBalanceMixin, nn.Module):
     def __init__(self, H, I, E, top_k=2, norm_topk_prob=True, routed_scaling_factor=1.0, init_std=0.02,
                  precision="bf16", act_codes=None, learnable_situ=False):
@@ -117,9 +170,22 @@ class MoELayer(LoadBalanceMixin, nn.Module):
     def forward(self, x):                               # x: (B,S,H) or (N,H)
         shape = x.shape
         flat = x.reshape(-1, shape[-1])
-        idx, w, counts = fused_mlp_router(flat, self.gate.weight, self.bias, self.top_k, self.num_experts,
-                                          self.norm_topk_prob, self.routed_scaling_factor, return_counts=True)
+        # an nn.Module resolves each of its parameters and buffers by name: once each
+        weight, bias, gate_up, down, codes, params = (self.gate.weight, self.bias, self.gate_up_proj, self.down_proj,
+                                                      self.act_codes, self.act_params)
+        infos, n_glu = _code_info(codes)
+        if (self.precision == "bf16" and params is None and flat.shape[0] > 0 and n_glu == len(infos) == self.num_experts
+                and all(c in FUSED_CODES for c in infos)):
+            keep = torch.is_grad_enabled() and any(t.requires_grad for t in (flat, weight, gate_up, down))
+            load = self._load_tensor(flat.device) if self.training and flat.is_cuda else None
+            out, self.last_counts = _Layer.apply(flat, weight, bias, gate_up, down,
+                                                 _codes_on(codes, flat.device) if any(infos) else None, load, int(self.top_k),
+                                                 int(bool(self.norm_topk_prob and self.top_k > 1)),
+                                                 float(self.routed_scaling_factor), int(keep))
+            return out.reshape(shape)
+        idx, w, counts = fused_mlp_router(flat, weight, bias, self.top_k, self.num_experts, self.norm_topk_prob,
+                                          self.routed_scaling_factor, return_counts=True)
         self._record_counts(counts)
         fn = moe_mxfp8 if self.precision == "mxfp8" else moe
-        out = fn(flat, idx, w, self.gate_up_proj, self.down_proj, self.act_codes, self.act_params)
+        out = fn(flat, idx, w, gate_up, down, codes, params)
         return out.reshape(shape)

@@ -10,17 +10,10 @@ from __future__ import annotations
 import torch
 
 from . import _lib as L
-from . import ops
 
 __all__ = ["moe", "moe_grouped", "moe_per_expert", "GROUPED_MIN_TOKENS"]
 
 GROUPED_MIN_TOKENS = 4096   # kept for API compatibility (kernels/sm75/moe.py:78); one path here
-
-
-# Most rows per expert, on average, for which a forward without a backward runs over compact rows with the weights as
-# the MMA's M operand (csrc/gemm_few.cu).  Gate/up + down, us, row tiles against compact rows, at H 2048, I 1408, 64
-# experts: 4.5 rows an expert 237 / 170, 141 rows 238 / 213, 206 rows 240 / 328 (an expert then takes two tiles).
-FEW_ROWS = 160
 
 
 def _amp_cast(*ts):
@@ -31,75 +24,91 @@ def _amp_cast(*ts):
     return ts
 
 
+def _float32(t):
+    return t if t.dtype == torch.float32 and t.is_contiguous() else t.float().contiguous()
+
+
+def _codes_on(act_codes, device):
+    c = act_codes
+    if c.device != device or c.dtype != torch.int32 or not c.is_contiguous():
+        c = c.to(device=device, dtype=torch.int32).contiguous()
+    return c
+
+
+def _check_experts(hidden, idx, wt, gate_up_proj, down_proj):
+    for name, t in (("hidden", hidden), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
+        L.require_cuda_bf16(name, t)
+    L.require(hidden.dim() == 2 and gate_up_proj.dim() == 3, "hidden must be (N,H), gate_up_proj (E,2I,H)")
+    (N, H), (E, twoI, H2) = hidden.shape, gate_up_proj.shape
+    L.require(H2 == H and twoI % 2 == 0 and tuple(down_proj.shape) == (E, H, twoI // 2),
+              f"weight shapes must be (E,2I,H) and (E,H,I); got {tuple(gate_up_proj.shape)}, {tuple(down_proj.shape)}")
+    L.require(idx.is_cuda and idx.dtype == torch.int64 and idx.dim() == 2, "top_k_indices must be a CUDA int64 (N,k) tensor")
+    L.require(idx.shape == wt.shape and idx.shape[0] == N, "indices/weights must be (N,k)")
+    L.require(hidden.device == idx.device == gate_up_proj.device == down_proj.device, "all tensors must be on one device")
+
+
+def _experts_forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, codes_dev, params, E, row_kernels, keep):
+    """One native call (csrc/block.cu); a forward that is followed by a backward keeps its workspace, in which the
+    backward finds x_s, gate_up, inter, eo and the permutation tables."""
+    hidden, gate_up_proj, down_proj = hidden.contiguous(), gate_up_proj.contiguous(), down_proj.contiguous()
+    idx, w32, dev = idx.contiguous(), _float32(wt.detach()), hidden.device
+    L.require(w32.device == dev, "top_k_weights must be on hidden's device")
+    (N, H), n_glu, I, k = hidden.shape, gate_up_proj.shape[0], down_proj.shape[2], idx.shape[1]
+    lib = L.lib()
+    ws = L.workspace(lib.b200moe_moe_fwd_ws_bytes(N, H, I, E, n_glu, k, keep, row_kernels), dev)
+    out = torch.empty(N, H, dtype=torch.bfloat16, device=dev)
+    L.check(lib.b200moe_moe_forward(hidden.data_ptr(), idx.data_ptr(), w32.data_ptr(), gate_up_proj.data_ptr(),
+                                    down_proj.data_ptr(), L.ptr(codes_dev), L.ptr(params), N, H, I, E, n_glu, k, keep,
+                                    row_kernels, ws.data_ptr(), out.data_ptr(), L.status_word(dev).data_ptr(),
+                                    L.stream_of(hidden)))
+    if keep:
+        ctx.dims = (N, H, I, E, n_glu, k, row_kernels)
+        ctx.wt_dtype = wt.dtype
+        ctx.save_for_backward(ws, w32, gate_up_proj, down_proj, codes_dev, params)
+    return out
+
+
+def _experts_backward(ctx, grad_out, need, want_params):
+    """(grad_hidden, grad_wt, grad_gate_up_proj, grad_down_proj, grad_params), None where not needed."""
+    ws, w32, gate_up_proj, down_proj, codes_dev, params = ctx.saved_tensors
+    N, H, I, E, n_glu, k, row_kernels = ctx.dims
+    need_x, _, need_w, need_gu, need_dn = need
+    dev = ws.device
+    grad_out = grad_out.to(torch.bfloat16).contiguous()
+    lib, bf16 = L.lib(), dict(dtype=torch.bfloat16, device=dev)
+    grad_w = torch.empty(N, k, dtype=torch.float32, device=dev)
+    grad_x = torch.empty(N, H, **bf16) if need_x else None
+    grad_gu = torch.empty(n_glu, 2 * I, H, **bf16) if need_gu else None
+    grad_dn = torch.empty(n_glu, H, I, **bf16) if need_dn else None
+    grad_ap = torch.empty(E, 2, dtype=torch.float32, device=dev) if want_params and params is not None else None
+    tmp = L.workspace(lib.b200moe_moe_bwd_ws_bytes(N, H, I, E, n_glu, k, row_kernels), dev)
+    L.check(lib.b200moe_moe_backward(grad_out.data_ptr(), w32.data_ptr(), gate_up_proj.data_ptr(), down_proj.data_ptr(),
+                                     L.ptr(codes_dev), L.ptr(params), N, H, I, E, n_glu, k, row_kernels, ws.data_ptr(),
+                                     tmp.data_ptr(), L.ptr(grad_x), grad_w.data_ptr(), L.ptr(grad_gu), L.ptr(grad_dn),
+                                     L.ptr(grad_ap), L.status_word(dev).data_ptr(), L.stream_of(ws)))
+    return grad_x, (grad_w.to(ctx.wt_dtype) if need_w else None), grad_gu, grad_dn, grad_ap
+
+
 class _GroupedMoE(torch.autograd.Function):
-    """Forward saves x_s, gate_up, inter, eo and the permutation tables, as the reference's grouped
-    Function does (kernels/sm75/moe.py:576-599); backward follows :602-618."""
+    """Activation in the GEMM epilogues.  The forward keeps x_s, gate_up, inter, eo and the permutation tables, as the
+    reference's grouped Function does (kernels/sm75/moe.py:576-599); backward follows :602-618."""
 
     @staticmethod
     def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes, keep=True):
         """keep=False: no backward will follow (the caller knows the grad mode, which is off in here)."""
         hidden, gate_up_proj, down_proj = _amp_cast(hidden, gate_up_proj, down_proj)
-        L.require(hidden.dim() == 2, "hidden must be (N,H)")
-        for name, t in (("hidden", hidden), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
-            L.require_cuda_bf16(name, t)
-        N, H = hidden.shape
-        E, twoI, H2 = gate_up_proj.shape
-        I = twoI // 2
-        L.require(H2 == H and tuple(down_proj.shape) == (E, H, I) and twoI == 2 * I,
-                  f"weight shapes must be (E,2I,H) and (E,H,I); got {tuple(gate_up_proj.shape)}, {tuple(down_proj.shape)}")
+        _check_experts(hidden, idx, wt, gate_up_proj, down_proj)
+        E = gate_up_proj.shape[0]
         L.require(act_codes.numel() == E, "act_codes must have one code per expert")
-        L.require(tuple(idx.shape) == tuple(wt.shape) and idx.shape[0] == N, "indices/weights must be (N,k)")
-        hidden = hidden.contiguous()
-        gate_up_proj = gate_up_proj.contiguous()
-        down_proj = down_proj.contiguous()
-        w32 = wt.detach().float().contiguous()
-
         # a stack that mixes the parameter-free codes 0 / 1 / 5 keeps the fused epilogues: the code of a tile's
         # expert picks the activation there; an all-SiLU stack runs the SiLU-only instantiations
-        codes, _ = _code_info(act_codes)
-        codes_dev = None
-        if any(c != 0 for c in codes):
-            codes_dev = act_codes.to(device=hidden.device, dtype=torch.int32).contiguous()
-
-        if not keep and idx.numel() <= FEW_ROWS * E:
-            perm = ops.permute_build(idx, E, want_order=True)
-            inter = ops.expert_gate_up_few(ops.gather_compact(hidden, perm), gate_up_proj, perm, codes_dev)
-            return ops.combine_raw(ops.expert_linear_few(inter, down_proj, perm), w32, perm.slot_pos, N, perm.k)
-
-        perm = ops.permute_build(idx, E)
-        x_s = ops.gather_rows(hidden, perm)
-        gate_up, inter = ops.expert_gate_up_swiglu(x_s, gate_up_proj, perm, codes_dev)
-        eo = ops.expert_down(inter, down_proj, perm)
-        out = ops.combine(eo, w32, perm)
-
-        ctx.perm = perm
-        ctx.wt_dtype = wt.dtype
-        ctx.codes_dev = codes_dev
-        ctx.save_for_backward(x_s, gate_up, inter, eo, w32, gate_up_proj, down_proj)
-        return out
+        codes_dev = _codes_on(act_codes, hidden.device) if any(_code_info(act_codes)[0]) else None
+        return _experts_forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, codes_dev, None, E, 0, int(keep))
 
     @staticmethod
     def backward(ctx, grad_out):
-        x_s, gate_up, inter, eo, w32, gate_up_proj, down_proj = ctx.saved_tensors
-        perm = ctx.perm
-        need_x, _, need_w, need_gu, need_dn = ctx.needs_input_grad[:5]
-        grad_out = grad_out.contiguous()
-        if grad_out.dtype != torch.bfloat16:
-            grad_out = grad_out.to(torch.bfloat16)
-        grad_eo, grad_w = ops.combine_bwd(grad_out, eo, w32, perm)
-        grad_hidden = grad_gate_up_proj = grad_down_proj = None
-        if need_x or need_gu:
-            grad_gu = ops.expert_down_dgrad_glu(grad_eo, down_proj, gate_up, perm, ctx.codes_dev)
-            if need_gu:
-                grad_gate_up_proj = ops.expert_wgrad(grad_gu, x_s, perm)
-            if need_x:
-                grad_x_s = ops.expert_gate_up_dgrad(grad_gu, gate_up_proj, perm)
-                grad_hidden = ops.combine(grad_x_s, None, perm)
-        if need_dn:
-            grad_down_proj = ops.expert_wgrad(grad_eo, inter, perm)
-        grad_wt = grad_w.to(ctx.wt_dtype) if need_w else None
-        grads = (grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None, None)
-        return grads[:len(ctx.needs_input_grad)]
+        gx, gw, ggu, gdn, _ = _experts_backward(ctx, grad_out, ctx.needs_input_grad[:5], False)
+        return (gx, None, gw, ggu, gdn, None, None)[:len(ctx.needs_input_grad)]
 
 
 GLU_CODES = (0, 1, 2, 5, 6, 7)     # weight-carrying experts (kernels/sm75/moe.py:1-31)
@@ -136,67 +145,23 @@ class _PolyGLUMoE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes, act_params):
         hidden, gate_up_proj, down_proj = _amp_cast(hidden, gate_up_proj, down_proj)
-        for name, t in (("hidden", hidden), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
-            L.require_cuda_bf16(name, t)
+        _check_experts(hidden, idx, wt, gate_up_proj, down_proj)
         codes, n_glu = _code_info(act_codes)
-        E_total = len(codes)
-        N, H = hidden.shape
-        E, twoI, H2 = gate_up_proj.shape
-        I = twoI // 2
+        E_total, E = len(codes), gate_up_proj.shape[0]
         L.require(E == n_glu, f"gate_up_proj holds {E} experts but act_codes lists {n_glu} GLU experts")
-        L.require(H2 == H and tuple(down_proj.shape) == (E, H, I), "weight shapes must be (E,2I,H) and (E,H,I)")
-        L.require(tuple(idx.shape) == tuple(wt.shape) and idx.shape[0] == N, "indices/weights must be (N,k)")
-        hidden, gate_up_proj, down_proj = hidden.contiguous(), gate_up_proj.contiguous(), down_proj.contiguous()
-        w32 = wt.detach().float().contiguous()
-        codes_dev = act_codes.to(device=hidden.device, dtype=torch.int32).contiguous()
         ap32 = None
         if act_params is not None:
             L.require(tuple(act_params.shape) == (E_total, 2), "act_params must be (E,2) [alpha, gamma]")
-            ap32 = act_params.detach().float().contiguous()
-
-        import dataclasses
-        perm = ops.permute_build(idx, E_total)
-        perm_glu = dataclasses.replace(perm, E=n_glu)          # GEMMs and row kernels see the GLU rows only
-        x_s = ops.gather_rows(hidden, perm)
-        gate_up = ops.expert_linear(x_s, gate_up_proj, perm_glu)
-        inter = ops.glu_fwd_rows(gate_up, codes_dev, ap32, perm_glu)
-        eo = ops.expert_linear(inter, down_proj, perm_glu)
-        if n_glu < E_total:
-            ops.special_rows(x_s, eo, codes_dev, perm, n_glu)
-        out = ops.combine(eo, w32, perm)
-
-        ctx.perm, ctx.perm_glu, ctx.n_glu, ctx.E_total = perm, perm_glu, n_glu, E_total
-        ctx.wt_dtype = wt.dtype
-        ctx.has_params = ap32 is not None
-        ctx.save_for_backward(x_s, gate_up, inter, eo, w32, gate_up_proj, down_proj, codes_dev,
-                              ap32 if ap32 is not None else torch.empty(0, device=hidden.device))
-        return out
+            ap32 = _float32(act_params.detach())
+            L.require(ap32.device == hidden.device, "act_params must be on hidden's device")
+        return _experts_forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, _codes_on(act_codes, hidden.device), ap32,
+                                E_total, 1, 1)
 
     @staticmethod
     def backward(ctx, grad_out):
-        x_s, gate_up, inter, eo, w32, gate_up_proj, down_proj, codes_dev, ap32 = ctx.saved_tensors
-        ap32 = ap32 if ctx.has_params else None
-        perm, perm_glu, n_glu = ctx.perm, ctx.perm_glu, ctx.n_glu
-        need_x, _, need_w, need_gu, need_dn, _, need_ap = ctx.needs_input_grad
-        want_ap = bool(ctx.has_params and need_ap)
-        grad_out = grad_out.contiguous().to(torch.bfloat16)
-        grad_eo, grad_w = ops.combine_bwd(grad_out, eo, w32, perm)
-        grad_inter = ops.expert_linear_t(grad_eo, down_proj, perm_glu)
-        grad_gu, row_da, row_dg = ops.glu_bwd_rows(grad_inter, gate_up, codes_dev, ap32, perm_glu, want_ap)
-        grad_down_proj = ops.expert_wgrad(grad_eo, inter, perm_glu) if need_dn else None
-        grad_gate_up_proj = ops.expert_wgrad(grad_gu, x_s, perm_glu) if need_gu else None
-        grad_hidden = None
-        if need_x:
-            grad_x_s = ops.expert_linear_t(grad_gu, gate_up_proj, perm_glu)
-            if n_glu < ctx.E_total:
-                ops.special_rows(grad_eo, grad_x_s, codes_dev, perm, n_glu)
-            grad_hidden = ops.combine(grad_x_s, None, perm)
-        grad_ap = None
-        if want_ap:
-            grad_ap = torch.zeros(ctx.E_total, 2, dtype=torch.float32, device=x_s.device)
-            ops.expert_row_sums(row_da, row_dg, perm_glu, grad_ap)
-        grad_wt = grad_w.to(ctx.wt_dtype) if need_w else None
-        return grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None, grad_ap
+        need = ctx.needs_input_grad
+        gx, gw, ggu, gdn, gap = _experts_backward(ctx, grad_out, need[:5], need[6])
+        return gx, None, gw, ggu, gdn, None, gap
 
 
 def _empty_result(hidden, top_k_weights, *params):

@@ -15,6 +15,8 @@ dtypes, a damped aurora (beta != 0 is not reachable through the reference's cons
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib as L
@@ -141,14 +143,14 @@ def _iterate(X, E, Rp, wide, coeffs):
     A = torch.empty(rows, Rp, dtype=torch.bfloat16, device=X.device)
     A2 = torch.empty_like(A)
     Xn = torch.empty_like(X)
-    for a, b, c in coeffs:
-        # A = X X^T and B = c A A + b A + a I are symmetric: their GEMMs compute the upper tiles and store each chunk
-        # right of the diagonal tile twice, the second time transposed (A A^T = A A; axpy and identity in the epilogue)
-        ops.expert_gram(X.view(rows, wide), seg, out=A)
-        ops.expert_linear_axpby(A, A.view(E, Rp, Rp), A, c, b, a, seg, out=A2, symmetric=2)
-        ops.expert_linear_t(A2, X, seg, out=Xn.view(rows, wide))      # X = B X
-        X, Xn = Xn, X
-    return X
+    # A = X X^T and B = c A A + b A + a I are symmetric: their GEMMs compute the upper tiles and store each chunk
+    # right of the diagonal tile twice, the second time transposed (A A^T = A A; axpy and identity in the epilogue);
+    # X = B X goes to the other of two buffers.  All iterations are queued by one native call (csrc/block.cu).
+    flat = [float(v) for a, b, c in coeffs for v in (a, b, c)]
+    L.check(L.lib().b200moe_newton_schulz(X.data_ptr(), Xn.data_ptr(), A.data_ptr(), A2.data_ptr(), L.ptr(seg.tile_expert),
+                                          L.ptr(seg.poffs), E, Rp, wide, (ctypes.c_float * len(flat))(*flat), len(flat) // 3,
+                                          L.ptr(L.status_word(X.device)), L.stream_of(X)))
+    return Xn if (len(flat) // 3) % 2 else X
 
 
 def _checked_momentum(mom, E, r, c, dev):

@@ -2,6 +2,8 @@
 queue the kernels on the current CUDA stream.  No computation happens in Python."""
 from __future__ import annotations
 
+import ctypes
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -12,13 +14,32 @@ LOGITS_BF16, LOGITS_F32, SCORES_F32 = 0, 1, 2
 TILE_M = 256   # B200MOE_TILE_M: expert segments are padded to this many rows
 
 # Optional observer used by the benchmark: hook(name, kernel_launches, start_event, end_event) is
-# called for every op below with CUDA events recorded on the launching stream around it.
+# called for every op below, and for every operation inside the native sequences (block.cu), with CUDA events recorded on
+# the launching stream around it.
 _hook = None
+_native_observer = None
 
 
 def set_hook(hook):
-    global _hook
+    global _hook, _native_observer
     _hook = hook
+    if hook is None:
+        if _native_observer is not None:
+            L.lib().b200moe_set_observer(None)
+            _native_observer = None
+        return
+    open_ops = threading.local()      # a backward queues its operations from the autograd engine's thread
+
+    def observe(name, launches, phase):
+        e = torch.cuda.Event(enable_timing=True)
+        e.record()
+        if phase == 0:
+            open_ops.start = e
+        else:
+            hook(name.decode(), launches, open_ops.start, e)
+
+    _native_observer = ctypes.CFUNCTYPE(None, ctypes.c_char_p, ctypes.c_int, ctypes.c_int)(observe)
+    L.lib().b200moe_set_observer(ctypes.cast(_native_observer, ctypes.c_void_p))
 
 
 def _op(name, launches=1):
@@ -168,7 +189,7 @@ class Permutation:
         return self.poffs[self.E:]
 
 
-@_op("permute_build", 3)
+@_op("permute_build", 2)
 def permute_build(idx, E, want_order=False) -> Permutation:
     L.require(idx.is_cuda and idx.dtype == torch.int64 and idx.dim() == 2, "top_k_indices must be a CUDA int64 (N,k) tensor")
     idx = idx.contiguous()

@@ -15,13 +15,6 @@ from . import ops
 __all__ = ["fused_mlp_router", "FusedMLPRouter", "fused_router", "FusedConvRouter", "router_bias_update"]
 
 
-# Up to this many tokens (four for each of 148 SMs; with more than 64 experts correspondingly fewer) logits and picks are
-# one launch of CUDA-core dot products.  GEMM + top-k against it, us, top-6 of 64 experts at H 2048: 48 tokens 15.6 / 7.5,
-# 512 tokens 16.1 / 11.7, 1024 tokens 16.1 / 20.9; 128 experts: 128 tokens 17.6 / 10.0, 256 tokens 17.6 / 16.2; 256 experts:
-# 100 tokens at H 4096 29.1 / 27.3, 256 tokens at H 1024 15.5 / 19.0.
-SMALL_TOKENS = 592
-
-
 class FusedMLPRouter(torch.autograd.Function):
     """Returns (idx (N,k) int64, weights (N,k) fp32 final, counts (E,) int32); only `weights` is
     differentiable (kernels/sm75/router.py:229-242)."""
@@ -40,24 +33,35 @@ class FusedMLPRouter(torch.autograd.Function):
         bias32 = None
         if bias is not None:
             bias32 = bias.detach().float().contiguous()
-        T, E = xf.shape[0], weight.shape[0]
-        if T <= SMALL_TOKENS and T * E <= 64 * SMALL_TOKENS:
-            logits, idx, w, counts = ops.router_small_fwd(xf, weight, bias32, top_k, norm_topk and top_k > 1, scale)
-        else:
-            logits = ops.gemm_nt(xf, weight)
-            idx, w, counts = ops.router_topk_fwd(logits, bias32, top_k, norm_topk and top_k > 1, scale)
+        (T, H), E, dev, k = xf.shape, weight.shape[0], xf.device, int(top_k)
+        if bias32 is not None:
+            L.require(bias32.is_cuda and bias32.numel() == E, "bias must be a contiguous float32 CUDA tensor of E elements")
+        L.require(weight.device == dev, "gate_weight must be on x's device")
+        ctx.norm, ctx.scale = int(bool(norm_topk and top_k > 1)), float(scale)
+        logits = torch.empty(T, E, dtype=torch.bfloat16, device=dev)
+        idx = torch.empty(T, k, dtype=torch.int64, device=dev)
+        w = torch.empty(T, k, dtype=torch.float32, device=dev)
+        counts = torch.empty(E, dtype=torch.int32, device=dev)
+        L.check(L.lib().b200moe_router_forward(xf.data_ptr(), weight.data_ptr(), L.ptr(bias32), T, H, E, k, ctx.norm,
+                                               ctx.scale, logits.data_ptr(), idx.data_ptr(), w.data_ptr(), counts.data_ptr(),
+                                               L.status_word(dev).data_ptr(), L.stream_of(xf)))
         ctx.xshape = x.shape
         ctx.save_for_backward(xf, weight, logits, idx)
-        ctx.norm, ctx.scale = bool(norm_topk and top_k > 1), float(scale)
         ctx.mark_non_differentiable(idx, counts)
         return idx, w, counts
 
     @staticmethod
     def backward(ctx, grad_idx, grad_weights, grad_counts):
         xf, weight, logits, idx = ctx.saved_tensors
-        gl = ops.router_topk_bwd(logits, idx, grad_weights, ctx.norm, ctx.scale)
-        grad_x = ops.gemm_nn(gl, weight).view(ctx.xshape) if ctx.needs_input_grad[0] else None
-        grad_w = ops.gemm_tn(gl, xf) if ctx.needs_input_grad[1] else None
+        (T, H), E, dev = xf.shape, weight.shape[0], xf.device
+        gw = grad_weights.contiguous().float()
+        grad_x = torch.empty(ctx.xshape, dtype=torch.bfloat16, device=dev) if ctx.needs_input_grad[0] else None
+        grad_w = torch.empty(E, H, dtype=torch.bfloat16, device=dev) if ctx.needs_input_grad[1] else None
+        lib = L.lib()
+        ws = L.workspace(lib.b200moe_router_bwd_ws_bytes(T, H, E), dev)
+        L.check(lib.b200moe_router_backward(xf.data_ptr(), weight.data_ptr(), logits.data_ptr(), idx.data_ptr(), gw.data_ptr(),
+                                            T, H, E, idx.shape[1], ctx.norm, ctx.scale, ws.data_ptr(), L.ptr(grad_x),
+                                            L.ptr(grad_w), L.status_word(dev).data_ptr(), L.stream_of(xf)))
         return grad_x, grad_w, None, None, None, None, None
 
 
