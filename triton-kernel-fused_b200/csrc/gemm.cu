@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -56,6 +57,19 @@ struct Cfg {
   static constexpr int TILE_ROWS = BM * CTAS;
 };
 
+// Columns of B (and of the accumulator) a pair tile multiplies: the last tile of a ragged width is narrower, in steps that
+// keep each CTA's half of B whole in units of its shared-memory layout: 8 rows (K-major) or a 64-wide swizzle atom
+// (MN-major).  SwiGLU tiles stay whole: a narrow one gained nothing on ragged widths, and the epilogue's variable offset
+// of the up columns cost 1 % on the others.  This is what lets every width above 64 take the pair kernel: its 256-wide tiles
+// multiply no more columns than 128-wide single-CTA tiles would, at half the operand traffic per FLOP.  One layer of
+// 3001 tokens, H 1032, I 680, 32 experts, top-4: the five products that ran on 128-wide tiles 334 -> 234 us.
+template <int BN, int EPI>
+__device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
+  const int rem = p.N - n0;
+  if constexpr (EPI == EPI_SWIGLU) return BN;
+  if (p.b_mn) return rem <= BN / 2 ? BN / 2 : BN;
+  return rem >= BN ? BN : (rem + 15) / 16 * 16;
+}
 
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
@@ -155,7 +169,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
           const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
           const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
-          const int bstep = (EPI != EPI_SWIGLU && p.N - t.n0 <= BN / 2) ? BNC / 2 : BNC;
+          const int bstep = pair_cols<BN, EPI>(p, t.n0) / 2;
           // this lane's box: the coordinate that does not move with k, and the group
           int fixed, grp;
           if (isA) {
@@ -193,9 +207,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
         const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
         const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
-        // a last pair tile with at most BN/2 live columns runs as a 256 x BN/2 MMA: each CTA then
-        // supplies BN/4 columns of B, the first ones of its (still BN/2 wide) staging tile
-        const int bstep = (CTAS == 2 && EPI != EPI_SWIGLU && p.N - t.n0 <= BN / 2) ? BNC / 2 : BNC;
+        // a narrower last pair tile: each CTA supplies half of its columns of B, the first ones of its (still
+        // BN/2 wide) staging tile
+        const int bstep = (CTAS == 2) ? pair_cols<BN, EPI>(p, t.n0) / 2 : BNC;
         for (int kb = 0; kb < t.nkb; ++kb) {
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
             ok = false;
@@ -274,8 +288,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (lane == 0 && cta_rank == 0) {
-      const uint32_t idesc_full = umma_idesc_bf16(BN, p.a_mn, p.b_mn, TM);
-      const uint32_t idesc_half = umma_idesc_bf16(BN / 2, p.a_mn, p.b_mn, TM);   // narrow last pair tile
       // K-major: rows are 128 B apart, 8-row groups 1024 B apart, 16 k-elements = 32 B.
       // MN-major: 64-wide MN blocks are 64*128 B apart (LBO), 8 k-rows 1024 B apart (SBO),
       //           16 k-rows = 2048 B.
@@ -290,8 +302,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (!mbar_wait(bar_tempty + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, ST_WAIT_MMA_TMEM)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
-        const uint32_t idesc =
-            (CTAS == 2 && EPI != EPI_SWIGLU && p.N - t.n0 <= BN / 2) ? idesc_half : idesc_full;
+        const uint32_t idesc = umma_idesc_bf16(CTAS == 2 ? pair_cols<BN, EPI>(p, t.n0) : BN, p.a_mn, p.b_mn, TM);
         for (int kb = 0; kb < t.nkb; ++kb) {
           if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
             ok = false;
@@ -754,6 +765,27 @@ static int pick_bn(long long n) {
   return 128;
 }
 
+// Tile width of the grouped products: pair tiles (256 x 256 on two SMs), or single-CTA tiles 128 wide (`narrow`: the least
+// the epilogue is built for).  m_tiles = 256-row tiles, m_tiles1 = 128-row tiles over all groups.  Waves of tiles over the
+// machine decide: a wave of 128 x 128 tiles takes about 0.8 of a wave of pair tiles for half of its work per SM (0.9 with a
+// long reduction, 0.6 with a short one), so small products, whose pair tiles leave most SMs idle, run faster on it.
+// us, pair against single-CTA tiles: 8 experts x 500 rows, 264 x 136: down 9.5 / 6.6, weight gradients 14.8 / 8.5 and
+// 14.3 / 8.5; 32 experts x 375 rows, 1032 x 680: 38 / 49, 54 / 80, 36 / 55; 16 experts x 1000 rows, 1800 x 968: 72 / 107,
+// 104 / 176, 62 / 99.
+static int pick_bn_grouped(long long n, int narrow, long long m_tiles, long long m_tiles1, int cols_per_bn = 1) {
+  if (n * cols_per_bn <= 64) return narrow;
+  if (!pairs_enabled()) return std::max(pick_bn(n), narrow);
+  const long long units = gemm_cta_budget();
+  const long long pair_waves = ceil_div(m_tiles * ceil_div(n * cols_per_bn, 256), units / 2);
+  const long long cta_waves = ceil_div(m_tiles1 * ceil_div(n * cols_per_bn, 128), units);
+  return 10 * pair_waves <= 8 * cta_waves ? 256 : 128;
+}
+// the same over the padded rows of a routing decision, of which each group's last tile is taken to be half full
+static int pick_bn_rows(long long n, long long rows_cap, int E, int cols_per_bn = 1) {
+  const long long t = std::max<long long>(1, rows_cap / B200MOE_TILE_M - E / 2);
+  return pick_bn_grouped(n, 128, t, 2 * t, cols_per_bn);
+}
+
 // d1 / d2 describe the bf16 outputs as {columns, rows, groups} tensors for the TMA-store epilogue
 // (d2 = the SwiGLU `inter` output); they are ignored by the kernels that store directly.
 template <int EPI, bool POLY = false>
@@ -991,7 +1023,7 @@ int b200moe_expert_gate_up_act(const void* x_s, const void* gate_up_proj, const 
   p.sched = SCHED_GROUPED_M; p.N = (int)I; p.K = (int)H; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = gate_up; p.aux = inter; p.I = (int)I; p.status = status;
   p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
-  const int bn = (I >= 128) ? 256 : 128;   // tile covers bn/2 intermediate columns
+  const int bn = pick_bn_rows(I, rows_cap, E, 2);   // tile covers bn/2 intermediate columns
   Operand d1{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // {I, rows, 2}: group 0 = gate half, 1 = up half
   Operand d2{inter, 0, rows_cap, I, I, 1, rows_cap * I};
   if (act_codes != nullptr) {
@@ -1014,7 +1046,7 @@ int b200moe_expert_linear(const void* a, const void* w, const int32_t* tile_expe
   p.sched = SCHED_GROUPED_M; p.N = (int)N; p.K = (int)K; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
   Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
-  return dispatch_bn<EPI_STORE>(pick_bn(N) == 64 ? 128 : pick_bn(N), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
 int b200moe_expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
@@ -1073,7 +1105,7 @@ int b200moe_expert_linear_t(const void* a, const void* w, const int32_t* tile_ex
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)K; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
   Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
-  return dispatch_bn<EPI_STORE>(pick_bn(N) == 64 ? 128 : pick_bn(N), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
 int b200moe_expert_linear_push(const void* a, const void* w, int w_kn, const int32_t* tile_expert, const int32_t* poffs,
@@ -1125,7 +1157,7 @@ int b200moe_expert_down_dgrad_act(const void* grad_eo, const void* down_proj, co
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = grad_gate_up; p.aux = const_cast<void*>(gate_up);
   p.I = (int)I; p.status = status;
   p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
-  const int bn = pick_bn(I) == 64 ? 128 : pick_bn(I);
+  const int bn = pick_bn_rows(I, rows_cap, E);
   Operand d{grad_gate_up, 0, rows_cap, I, 2 * I, 2, I};   // {I, rows, 2}: grad_gate half, grad_up half
   Operand d2{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // the saved forward gate_up, same view (input)
   if (act_codes != nullptr) {
@@ -1156,7 +1188,7 @@ int b200moe_expert_wgrad(const void* A, const void* B, const int32_t* poffs, con
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)Na; p.N = (int)Nb; p.K = (int)rows_cap;
   p.num_groups = E; p.poffs = poffs; p.counts = counts; p.D = out; p.ldd = Nb; p.d_group_stride = Na * Nb;
   p.status = status;
-  const int bn = pick_bn(Nb);
+  const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
   Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
   return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn)),
                                 (cudaStream_t)stream);
