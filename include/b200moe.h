@@ -80,11 +80,12 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
                             int k, int norm_topk, float scale, int64_t* idx, float* w,
                             int32_t* counts, b200moe_stream_t stream);
 
-/* The whole router forward of a small batch in one launch: logits (T,E) bf16 = x (T,H) * weight (E,H)^T (fp32 sums),
- * then b200moe_router_topk_fwd's picks from them (kernels/sm75/router.py:221-242).  E % 8 == 0, H % 8 == 0. */
+/* The whole router forward of a small batch in one launch: logits (T,E) bf16 = x (T,H) * weight (E,H)^T, the bits that
+ * b200moe_gemm_nt gives, then b200moe_router_topk_fwd's picks from them (kernels/sm75/router.py:221-242).  E % 8 == 0,
+ * E <= 128, H % 8 == 0; counts nullable. */
 int b200moe_router_small_fwd(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
                              int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
-                             b200moe_stream_t stream);
+                             int32_t* status, b200moe_stream_t stream);
 /* Replaces _router_epilogue_bwd_kernel (kernels/sm75/router.py:86-126): grad_logits (T,E) bf16. */
 int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* idx,
                             const float* grad_w, int64_t T, int E, int k, int norm_topk, float scale,

@@ -21,8 +21,8 @@ def _composed(pkg, layer, x):
 
 
 # both sides of the small router's token limit, one pick, mixed codes, one pick without renormalisation
-@pytest.mark.parametrize("T,H,I,E,k,codes,kw", [(1, 64, 64, 8, 2, None, {}), (592, 264, 136, 16, 3, None, {}),
-                                                (593, 264, 136, 16, 1, [0, 1, 5, 0] * 4, {}),
+@pytest.mark.parametrize("T,H,I,E,k,codes,kw", [(1, 64, 64, 8, 2, None, {}), (2368, 264, 136, 16, 3, None, {}),
+                                                (2369, 264, 136, 16, 1, [0, 1, 5, 0] * 4, {}),
                                                 (2000, 512, 264, 40, 6, None, dict(norm_topk_prob=False, routed_scaling_factor=2.5))])
 def test_layer_equals_router_then_experts(pkg, T, H, I, E, k, codes, kw):
     torch.manual_seed(T)
@@ -85,7 +85,7 @@ def test_layer_on_a_side_stream(pkg):
 
 def test_observer_sees_the_operations_of_the_native_sequences(pkg):
     layer = _layer(pkg, 256, 128, 8, 2)
-    x = torch.randn(700, 256, device=DEV).to(torch.bfloat16).requires_grad_()
+    x = torch.randn(2400, 256, device=DEV).to(torch.bfloat16).requires_grad_()
     seen = []
     pkg.ops.set_hook(lambda name, launches, a, b: seen.append((name, launches, a, b)))
     try:

@@ -33,7 +33,7 @@ _SIGNATURES = {
     "b200moe_selftest_bounded_wait": (c_int, [c_void_p, c_int64, c_void_p]),
     "b200moe_router_topk_fwd": (c_int, [c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_float,
                                         c_void_p, c_void_p, c_void_p, c_void_p]),
-    "b200moe_router_small_fwd": (c_int, [c_void_p] * 3 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 5),
+    "b200moe_router_small_fwd": (c_int, [c_void_p] * 3 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 6),
     "b200moe_router_topk_bwd": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int, c_int, c_int,
                                         c_float, c_void_p, c_void_p]),
     "b200moe_router_bias_update": (c_int, [c_void_p, c_void_p, c_int, c_float, c_void_p]),

@@ -237,17 +237,15 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
   return 0;
 }
 
-// Up to this many tokens (four for each of 148 SMs; with more than 64 experts correspondingly fewer) logits and picks are
-// one launch of CUDA-core dot products.  GEMM + top-k against it, us, top-6 of 64 experts at H 2048: 48 tokens 15.6 / 7.5,
-// 512 tokens 16.1 / 11.7, 1024 tokens 16.1 / 20.9; 128 experts: 128 tokens 17.6 / 10.0, 256 tokens 17.6 / 16.2; 256 experts:
-// 100 tokens at H 4096 29.1 / 27.3, 256 tokens at H 1024 15.5 / 19.0.
-constexpr int64_t kSmallTokens = 592;
+// Up to 16 tokens for each of 148 SMs and 128 experts logits and picks are one launch (gemm_few.cu, with the times of both)
+constexpr int64_t kSmallTokens = 16 * 148;
+constexpr int kSmallExperts = 128;
 
 static int router_forward(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k, int norm,
                           float scale, void* logits, int64_t* idx, float* w, int32_t* counts, int32_t* status,
                           b200moe_stream_t st) {
-  if (T <= kSmallTokens && T * E <= 64 * kSmallTokens) {
-    RUN("router_small_fwd", 1, b200moe_router_small_fwd(x, weight, bias, T, H, E, k, norm, scale, logits, idx, w, counts, st));
+  if (T <= kSmallTokens && E <= kSmallExperts) {
+    RUN("router_small_fwd", 1, b200moe_router_small_fwd(x, weight, bias, T, H, E, k, norm, scale, logits, idx, w, counts, status, st));
     return 0;
   }
   RUN("gemm_nt", 1, b200moe_gemm_nt(x, weight, logits, T, E, H, status, st));

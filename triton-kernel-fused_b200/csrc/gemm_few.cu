@@ -15,12 +15,14 @@
 //
 // Warp roles as in gemm.cu: warp 0 TMA producer (a lane per box), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.
 #include <cuda.h>
+#include <cuda_bf16.h>
 
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
 
 #include "gemm_common.cuh"
+#include "topk.cuh"
 
 namespace b200moe {
 
@@ -283,6 +285,174 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   }
 }
 
+// ---------------------------------------------------------------------------- router of a small batch
+// Logits and top-k of 16 tokens per CTA in one launch: the gate weights are the M operand (up to 128 experts), the tokens the
+// N operand; the epilogue warps hand the bf16-rounded logits over through shared memory and each picks for two tokens.
+// Same k order, so the same logits to the bit, as the GEMM for large batches.  Bound by the chain of dependent MMAs on one
+// accumulator: about 150 cycles for each 16 of the reduction, however few rows it has (H 2048: 128 of them, 10 us).
+// us, GEMM and top-k (two launches) against this one, top-6 of 64 experts at H 2048: 1 token 15.0 / 12.5, 592 tokens 15.0 /
+// 13.9, 2368 (one wave of CTAs) 16.0 / 14.2, 4096 17.2 / 26.8; 32 experts at H 512, 2368 tokens 8.3 / 6.7.
+// (Dot products on CUDA cores, without that chain, took 5.6 us for 1 to 148 tokens, but they add in another order: about one
+// token in ten thousand then takes another expert of two that are a rounding apart.)
+struct RouterFewParams {
+  int T, H, E, k, norm;
+  float scale;
+  const float* bias;
+  __nv_bfloat16* logits;
+  long long* idx;
+  float* w;
+  int* counts;
+  int* status;
+};
+
+constexpr int kRouterTokens = 16;
+constexpr int kRouterExperts = 128;     // at most: the lanes of one accumulator
+
+struct RouterFewCfg {
+  static constexpr int W_BYTES = kRouterExperts * kFewBK * 2;
+  static constexpr int STAGE_BYTES = W_BYTES + kRouterTokens * kFewBK * 2;
+  static constexpr int NSTAGE = 11;
+  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + (2 * NSTAGE + 1) * 8 + 16 + 1024;
+};
+
+template <int VPL>
+__global__ void __launch_bounds__(kThreads, 1)
+router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const RouterFewParams p) {
+  using C = RouterFewCfg;
+  constexpr int NSTAGE = C::NSTAGE;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NSTAGE * C::STAGE_BYTES);
+  const uint32_t bar_full = smem_u32(bars);
+  const uint32_t bar_empty = smem_u32(bars + NSTAGE);
+  const uint32_t bar_done = smem_u32(bars + 2 * NSTAGE);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  __shared__ float s_logit[kRouterTokens][kRouterExperts + 1];
+  __shared__ int hist[kRouterExperts];
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * kRouterTokens;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(bar_full + 8 * s, 1);
+      mbar_init(bar_empty + 8 * s, 1);
+    }
+    mbar_init(bar_done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  for (int e = threadIdx.x; e < p.E; e += blockDim.x) hist[e] = 0;
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 32);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int nkb = (p.H + kFewBK - 1) / kFewBK;
+
+  if (warp == 0) {
+    if (lane < 2) {                        // lane 0: the weights of all experts, lane 1: the tokens
+      const bool isW = lane == 0;
+      const CUtensorMap* tm = isW ? &tmW : &tmX;
+      const uint32_t dst = isW ? 0 : C::W_BYTES;
+      const int c1 = isW ? 0 : t0;
+      const uint32_t bytes = (p.E + kRouterTokens) * kFewBK * 2;
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) break;
+        if (isW) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
+        tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, 0);
+        if (++s == NSTAGE) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16(kRouterTokens, 0, 0, 128);
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t sw = smem_u32(smem + s * C::STAGE_BYTES);
+#pragma unroll
+        for (int k = 0; k < kFewBK / 16; ++k)
+          umma_bf16(tmem_base, umma_desc_sw128(sw + 32 * k, 0, 1024), umma_desc_sw128(sw + C::W_BYTES + 32 * k, 0, 1024),
+                    idesc, (kb | k) != 0);
+        umma_commit(bar_empty + 8 * s);
+        if (++s == NSTAGE) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      if (ok) umma_commit(bar_done);
+    }
+  } else {
+    const int ew = warp - 2, q = warp & 3;     // TMEM lane quarter; the first four warps read the accumulator
+    const bool ok = mbar_wait(bar_done, 0, abort_flag, ST_WAIT_EPILOGUE);
+    __syncwarp();
+    tc_fence_after();
+    if (ok && ew < 4) {
+      uint32_t a[kRouterTokens];
+      tmem_ld16(tmem_base + (static_cast<uint32_t>(q * 32) << 16), a);
+      tmem_ld_wait();
+#pragma unroll
+      for (int t = 0; t < kRouterTokens; ++t) s_logit[t][32 * q + lane] = bf16_round(__uint_as_float(a[t]));
+    }
+    tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");    // the epilogue warps only
+    if (ok) {
+#pragma unroll 1
+      for (int tt = 2 * ew; tt < 2 * ew + 2 && t0 + tt < p.T; ++tt) {
+        const long long t = t0 + tt;
+        float sc[VPL];
+        uint32_t key[VPL];
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+          const int e = lane + 32 * i;
+          sc[i] = 0.0f;
+          key[i] = 0u;
+          if (e < p.E) {
+            const float v = s_logit[tt][e];
+            p.logits[t * p.E + e] = __float2bfloat16_rn(v);
+            sc[i] = sigmoid_f(v);
+            key[i] = select_key(sc[i] + (p.bias != nullptr ? p.bias[e] : 0.0f));
+          }
+        }
+        int my_idx;
+        float my_w;
+        topk_of_token<VPL>(sc, key, p.k, p.norm, p.scale, hist, p.counts != nullptr, my_idx, my_w);
+        if (lane < p.k) {
+          p.idx[t * p.k + lane] = my_idx;
+          p.w[t * p.k + lane] = my_w;
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (p.counts != nullptr)
+    for (int e = threadIdx.x; e < p.E; e += blockDim.x)
+      if (hist[e] != 0) atomicAdd(&p.counts[e], hist[e]);
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_flag);
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 32);
+  }
+}
+
 // ---------------------------------------------------------------------------- host side
 template <int EPI, int NT, int HALVES>
 static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows, int wgroups, const FewParams& p,
@@ -305,6 +475,25 @@ static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows,
   const long long tiles = chunks * ceil_div(p.N, TM);
   const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(gemm_cta_budget(), tiles)));
   few_rows_kernel<EPI, NT, HALVES><<<grid, kThreads, C::SMEM_BYTES, stream>>>(tmW, tmX, p);
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+template <int VPL>
+static int launch_router_few(const void* x, const void* weight, const RouterFewParams& p, cudaStream_t stream) {
+  using C = RouterFewCfg;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(router_few_kernel<VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+  });
+  if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
+  CUtensorMap tmW, tmX;   // a weight box of E rows: what the MMA reads past them ends in lanes nobody reads
+  int rc = make_map(&tmW, weight, p.H, p.E, 1, p.H, static_cast<uint64_t>(p.E) * p.H, kFewBK, p.E);
+  if (rc) return rc;
+  rc = make_map(&tmX, x, p.H, p.T, 1, p.H, static_cast<uint64_t>(p.T) * p.H, kFewBK, kRouterTokens);
+  if (rc) return rc;
+  router_few_kernel<VPL><<<(p.T + kRouterTokens - 1) / kRouterTokens, kThreads, C::SMEM_BYTES, stream>>>(tmW, tmX, p);
   B200_CUDA(cudaGetLastError());
   return 0;
 }
@@ -356,6 +545,27 @@ int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* count
   if (rows_cap <= kFewRows64 * E) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
   if (rows_cap <= kFewRows128 * E) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
   return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
+}
+
+int b200moe_router_small_fwd(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
+                             int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
+                             int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(x && weight && logits && idx && w, B200MOE_E_NULL, "router_small_fwd: null pointer");
+  B200_CHECK_ARG(E >= 1 && E <= kRouterExperts, B200MOE_E_UNSUPPORTED, "router_small_fwd: E = %d, supported 1..%d", E,
+                 kRouterExperts);
+  B200_CHECK_ARG(E % 8 == 0 && H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE,
+                 "router_small_fwd: E = %d and H = %lld must be positive multiples of 8", E, (long long)H);
+  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE,
+                 "router_small_fwd: top_k = %d must be in 1..min(E=%d, %d)", k, E, B200MOE_MAX_TOPK);
+  B200_CHECK_ARG(T >= 0 && T < (1LL << 31) && H < (1LL << 31), B200MOE_E_BAD_SHAPE, "router_small_fwd: T = %lld", (long long)T);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (counts != nullptr) B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * E, st));
+  if (T == 0) return 0;
+  RouterFewParams p{static_cast<int>(T), static_cast<int>(H), E, k, norm_topk, scale, bias, reinterpret_cast<__nv_bfloat16*>(logits),
+                    reinterpret_cast<long long*>(idx), w, counts, status};
+  if (E <= 32) return launch_router_few<1>(x, weight, p, st);
+  if (E <= 64) return launch_router_few<2>(x, weight, p, st);
+  return launch_router_few<4>(x, weight, p, st);
 }
 
 }  // extern "C"

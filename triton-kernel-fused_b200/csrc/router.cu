@@ -3,14 +3,12 @@
 // One warp owns one token; lane l holds experts l, l+32, ... (at most 8 values for E <= 256).
 #include <cuda_bf16.h>
 
-#include <type_traits>
-
 #include "common.cuh"
 #include "ptx.cuh"
+#include "topk.cuh"
 
 namespace b200moe {
 
-constexpr int kMaxVpl = B200MOE_MAX_EXPERTS / 32;  // most values a lane holds
 
 template <int KIND>
 __device__ __forceinline__ float load_in(const void* p, long long i) {
@@ -18,68 +16,12 @@ __device__ __forceinline__ float load_in(const void* p, long long i) {
   return reinterpret_cast<const float*>(p)[i];
 }
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// A selection value as an unsigned key of the same order (+0 and -0 alike; NaN above infinity).  Key 0 lies below
-// every value: experts that do not exist.  A picked expert falls to the key of -1e30, as in the reference.
-__device__ __forceinline__ uint32_t select_key(float v) {
-  const uint32_t u = __float_as_uint(v + 0.0f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-constexpr uint32_t kKnockOut = ~0xf149f2cau;   // select_key(-1e30f)
-
 // Both kernels are bound by instruction issue and by the latency of the k dependent picks, not by their few bytes per
 // token.  VPL = values per lane = ceil(E / 32) rounded up to a power of two: compiled per width, since a fixed VPL of 8
 // spends its compares on experts that do not exist (T = 16384, E = 64, k = 6: 23.9 -> 10.5 us; T = 32768, E = 128,
 // k = 8: 80 -> 26 us).  A pick is one
 // redux.max over the lanes' best keys and one redux.min over the ids that hold it (ties to the lowest expert id, as a
 // stable sort gives), instead of five shuffle rounds of (value, id) pairs.
-// The k picks of the token whose scores and selection keys a warp holds: lane j < k gets pick j and its weight.
-template <int VPL>
-__device__ __forceinline__ void topk_of_token(const float (&sc)[VPL], uint32_t (&key)[VPL], int k, int norm, float scale,
-                                              int* hist, bool count, int& my_idx, float& my_w) {
-  const int lane = threadIdx.x & 31;
-  my_idx = 0;
-  my_w = 0.0f;
-  for (int j = 0; j < k; ++j) {
-    // lane-local best: ascending i = ascending expert id, strict '>' keeps the lowest id
-    uint32_t bk = key[0];
-    int bi = lane;
-#pragma unroll
-    for (int i = 1; i < VPL; ++i) {
-      if (key[i] > bk) {
-        bk = key[i];
-        bi = lane + 32 * i;
-      }
-    }
-    const uint32_t best = __reduce_max_sync(0xffffffffu, bk);
-    bi = static_cast<int>(__reduce_min_sync(0xffffffffu, bk == best ? static_cast<unsigned>(bi) : 0xffffffffu));
-    // owner lane hands out the unbiased score and knocks the pick out
-    float wv = 0.0f;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      if (bi == lane + 32 * i) {
-        wv = sc[i];
-        key[i] = kKnockOut;
-      }
-    }
-    wv = __shfl_sync(0xffffffffu, wv, bi & 31);
-    if (lane == j) {
-      my_idx = bi;
-      my_w = wv;
-    }
-  }
-  if (count && lane < k) atomicAdd(&hist[my_idx], 1);
-  if (norm && k > 1) {
-    float tsum = 0.0f;
-    for (int j = 0; j < k; ++j) tsum += __shfl_sync(0xffffffffu, my_w, j);  // fixed order
-    tsum += 1e-20f;
-    my_w = my_w / tsum;
-  }
-  my_w = my_w * scale;
-}
-
 template <int KIND, int VPL>
 __global__ void __launch_bounds__(256)
 router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__ bias, long long T, int E,
@@ -112,104 +54,6 @@ router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__
         const float v = load_in<KIND>(input, t * E + e);
         sc[i] = (KIND == B200MOE_SCORES_F32) ? v : sigmoid_f(v);
         key[i] = select_key(sc[i] + b[i]);
-      }
-    }
-    int my_idx;
-    float my_w;
-    topk_of_token<VPL>(sc, key, k, norm, scale, hist, counts != nullptr, my_idx, my_w);
-    if (lane < k) {
-      idx_out[t * k + lane] = my_idx;
-      w_out[t * k + lane] = my_w;
-    }
-  }
-  if (counts != nullptr) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-      const int c = hist[e];
-      if (c != 0) atomicAdd(&counts[e], c);
-    }
-  }
-}
-
-// Logits and top-k of a small batch in one launch: a CTA takes TPB tokens, its warps split the experts in groups of 8
-// and, where that leaves warps over, the reduction, and a lane keeps 8 weight vectors and more in flight (each used for
-// all TPB tokens).  Bound by the latency of the weights' way from L2 (every CTA reads all E * H of them) and, with
-// more tokens, by the FMAs.  The GEMM it stands in for has one CTA per 128 tokens walk the whole reduction (32 dependent
-// k-blocks at H = 2048).  Sums are fp32 per lane, then across lanes and warps; the logits are rounded to bf16
-// before the picks, as the GEMM stores them.  48 tokens, H 2048, 64 experts, top-6: 15.6 us for GEMM and top-k, 7.5 us here.
-constexpr int kSmallWarps = 16;
-template <int VPL, int TPB>
-__global__ void __launch_bounds__(32 * kSmallWarps)
-router_small_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ weight, const float* __restrict__ bias,
-                        int T, int nvec, int E, int k, int norm, float scale, __nv_bfloat16* __restrict__ logits,
-                        long long* __restrict__ idx_out, float* __restrict__ w_out, int* __restrict__ counts) {
-  constexpr int kPart = B200MOE_MAX_EXPERTS;        // partial sums a token needs: parts * E <= 8 * 16, or E
-  __shared__ float s_part[TPB][kPart];
-  __shared__ int hist[B200MOE_MAX_EXPERTS];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int t0 = blockIdx.x * TPB;
-  const int groups = E / 8;                         // E is a multiple of 8
-  const int parts = groups < kSmallWarps ? kSmallWarps / groups : 1;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
-  for (int u = warp; u < groups * parts; u += kSmallWarps) {
-    const int g = u % groups, part = u / groups;
-    const uint4* wrow = weight + static_cast<long long>(8 * g) * nvec;
-    float acc[8][TPB];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int t = 0; t < TPB; ++t) acc[i][t] = 0.0f;
-#pragma unroll 2
-    for (int c = lane + 32 * part; c < nvec; c += 32 * parts) {
-      uint4 wv[8], xv[TPB];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) wv[i] = wrow[static_cast<long long>(i) * nvec + c];
-#pragma unroll
-      for (int t = 0; t < TPB; ++t)
-        xv[t] = t0 + t < T ? x[static_cast<long long>(t0 + t) * nvec + c] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const float2 wf = unpack_bf16x2(ww[h]);
-#pragma unroll
-          for (int t = 0; t < TPB; ++t) {
-            const float2 xf = unpack_bf16x2(h == 0 ? xv[t].x : h == 1 ? xv[t].y : h == 2 ? xv[t].z : xv[t].w);
-            acc[i][t] = fmaf(wf.x, xf.x, acc[i][t]);
-            acc[i][t] = fmaf(wf.y, xf.y, acc[i][t]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int t = 0; t < TPB; ++t) {
-        float v = acc[i][t];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) s_part[t][part * E + 8 * g + i] = v;
-      }
-  }
-  __syncthreads();
-  if (warp < TPB && t0 + warp < T) {
-    const long long t = t0 + warp;
-    float sc[VPL];
-    uint32_t key[VPL];
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int e = lane + 32 * i;
-      sc[i] = 0.0f;
-      key[i] = 0u;
-      if (e < E) {
-        float v = s_part[warp][e];
-        for (int q = 1; q < parts; ++q) v += s_part[warp][q * E + e];
-        v = bf16_round(v);
-        logits[t * E + e] = __float2bfloat16_rn(v);
-        sc[i] = sigmoid_f(v);
-        key[i] = select_key(sc[i] + (bias != nullptr ? bias[e] : 0.0f));
       }
     }
     int my_idx;
@@ -279,15 +123,6 @@ router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restr
       if (e < E) grad_logits[t * E + e] = __float2bfloat16_rn(gs[i] * (s[i] * (1.0f - s[i])));
     }
   }
-}
-
-// f(VPL) for E experts
-template <class F>
-static void by_experts(int E, F f) {
-  if (E <= 32) f(std::integral_constant<int, 1>());
-  else if (E <= 64) f(std::integral_constant<int, 2>());
-  else if (E <= 128) f(std::integral_constant<int, 4>());
-  else f(std::integral_constant<int, kMaxVpl>());
 }
 
 __global__ void router_bias_update_kernel(float* bias, const int* counts, int E, float u) {
@@ -367,37 +202,6 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
       set_error("router_topk_fwd: unknown input_kind %d", input_kind);
       return B200MOE_E_UNSUPPORTED;
   }
-  B200_CUDA(cudaGetLastError());
-  return 0;
-}
-
-int b200moe_router_small_fwd(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,
-                             int norm_topk, float scale, void* logits, int64_t* idx, float* w, int32_t* counts,
-                             b200moe_stream_t stream) {
-  B200_CHECK_ARG(x && weight && logits && idx && w, B200MOE_E_NULL, "router_small_fwd: null pointer");
-  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
-                 "router_small_fwd: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
-  B200_CHECK_ARG(E % 8 == 0 && H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE,
-                 "router_small_fwd: E = %d and H = %lld must be positive multiples of 8", E, (long long)H);
-  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE,
-                 "router_small_fwd: top_k = %d must be in 1..min(E=%d, %d)", k, E, B200MOE_MAX_TOPK);
-  B200_CHECK_ARG(T >= 0 && T < (1LL << 31) && H < (1LL << 31), B200MOE_E_BAD_SHAPE, "router_small_fwd: T = %lld", (long long)T);
-  B200_CHECK_ARG(aligned16(x) && aligned16(weight), B200MOE_E_ALIGN, "router_small_fwd: x and weight must be 16-byte aligned");
-  cudaStream_t st = (cudaStream_t)stream;
-  if (counts != nullptr) B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * E, st));
-  if (T == 0) return 0;
-  const uint4* xv = reinterpret_cast<const uint4*>(x);
-  const uint4* wv = reinterpret_cast<const uint4*>(weight);
-  __nv_bfloat16* lg = reinterpret_cast<__nv_bfloat16*>(logits);
-  long long* idx_ll = reinterpret_cast<long long*>(idx);
-  const int Ti = static_cast<int>(T), nvec = static_cast<int>(H / 8);
-  // one token a CTA while that fills no more than the SMs; four share the reads of the weights beyond
-  by_experts(E, [&](auto v) {
-    if (T <= num_sms())
-      router_small_fwd_kernel<v.value, 1><<<Ti, 32 * kSmallWarps, 0, st>>>(xv, wv, bias, Ti, nvec, E, k, norm_topk, scale, lg, idx_ll, w, counts);
-    else
-      router_small_fwd_kernel<v.value, 4><<<(Ti + 3) / 4, 32 * kSmallWarps, 0, st>>>(xv, wv, bias, Ti, nvec, E, k, norm_topk, scale, lg, idx_ll, w, counts);
-  });
   B200_CUDA(cudaGetLastError());
   return 0;
 }

@@ -103,7 +103,7 @@ def router_small_fwd(x, weight, bias, top_k, norm_topk=True, scale=1.0):
     counts = torch.empty(E, dtype=torch.int32, device=dev)
     L.check(L.lib().b200moe_router_small_fwd(L.ptr(x), L.ptr(weight), L.ptr(bias), T, H, E, int(top_k),
                                              int(bool(norm_topk)), float(scale), L.ptr(logits), L.ptr(idx), L.ptr(w),
-                                             L.ptr(counts), L.stream_of(x)))
+                                             L.ptr(counts), L.ptr(L.status_word(dev)), L.stream_of(x)))
     return logits, idx, w, counts
 
 
