@@ -780,8 +780,7 @@ def run_muon(args):
 
 def run_conv_router(args):
     """--workload conv_router: forward + backward of `fused_router` (causal K-tap conv router) on the token count and
-    width of the headline layer, once with the GEMMs that read x in place through shifted TMA boxes and once over
-    the unfolded (B*S, K*H) copy.  A line of its own for the conv-router row, not the headline metric."""
+    width of the headline layer.  A line of its own for the conv-router row, not the headline metric."""
     if int(os.environ.get("WORLD_SIZE", 1)) > 1:
         if int(os.environ.get("RANK", 0)) == 0:
             print(json.dumps({"workload": "conv_router", "unavailable": "single-GPU workload"}), flush=True)
@@ -837,12 +836,6 @@ def run_conv_router(args):
     n_warm = max(args.warmup, 3)
     steps = max(3, min(args.steps, 50))
     ms, kernels, launches, clocks = measure(steps, n_warm)
-    direct_ok = ops.conv_direct_ok
-    ops.conv_direct_ok = lambda S_, H_: False
-    try:
-        ms_u, kernels_u, _, clocks_u = measure(steps, n_warm)
-    finally:
-        ops.conv_direct_ok = direct_ok
     flops = 6.0 * B * S * K * H * E          # logits, dX and dW GEMMs
     line = {
         "metric": "conv_router_fwd_bwd_ms", "value": round(ms, 4), "unit": "ms", "n_gpus": 1, "steps": steps, "warmup": n_warm,
@@ -852,7 +845,6 @@ def run_conv_router(args):
                    "l2": "flushed between steps (256 MB write)"},
         "gemm_tflops": round(flops / (ms * 1e-3) / 1e12, 1),
         "kernels": kernels, "gpu_launches": launches, "clocks": clocks,
-        "unfolded_copy_path": {"ms_per_step": round(ms_u, 4), "kernels": kernels_u, "clocks": clocks_u},
     }
     print(json.dumps(line), flush=True)
 

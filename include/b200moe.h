@@ -133,6 +133,8 @@ int b200moe_gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, in
                            int64_t k_chunk, int32_t* status, b200moe_stream_t stream);
 int b200moe_splitk_reduce(const float* P, int64_t slices, int64_t elems, void* D,
                           b200moe_stream_t stream);
+/* The same with the result transposed: D (C,R) = bf16(sum of the slices P (slices,R,C))^T. */
+int b200moe_splitk_reduce_t(const float* P, int64_t slices, int64_t R, int64_t C, void* D, b200moe_stream_t stream);
 
 /* ---- permutation ---------------------------------------------------------------------------- */
 size_t b200moe_permute_ws_bytes(int64_t M, int E);
@@ -494,6 +496,30 @@ size_t b200moe_router_bwd_ws_bytes(int64_t T, int64_t H, int E);
 int b200moe_router_backward(const void* x, const void* weight, const void* logits, const int64_t* idx, const float* grad_w,
                             int64_t T, int64_t H, int E, int k, int norm_topk, float scale, void* ws, void* grad_x,
                             void* grad_weight, int32_t* status, b200moe_stream_t stream);
+/* conv router (FusedConvRouterCuDNN, kernels/sm75/router.py:172-218): x (B,S,H), weight (E,H,taps), logits (B*S,E).
+ * weight_rows (taps*E,H) bf16 is written by the forward and read by the backward; the forward's workspace (its size may be
+ * 0) is free afterwards.  H % 8 == 0, E % 8 == 0. */
+size_t b200moe_conv_router_fwd_ws_bytes(int64_t B, int64_t S, int64_t H, int E, int taps);
+int b200moe_conv_router_forward(const void* x, const void* weight, const float* bias, int64_t B, int64_t S, int64_t H, int E,
+                                int taps, int k, int norm_topk, float scale, void* ws, void* weight_rows, void* logits,
+                                int64_t* idx, float* w, int32_t* counts, int32_t* status, b200moe_stream_t stream);
+size_t b200moe_conv_router_bwd_ws_bytes(int64_t B, int64_t S, int64_t H, int E, int taps);
+int b200moe_conv_router_backward(const void* x, const void* weight_rows, const void* logits, const int64_t* idx,
+                                 const float* grad_w, int64_t B, int64_t S, int64_t H, int E, int taps, int k, int norm_topk,
+                                 float scale, void* ws, void* grad_x, void* grad_weight, int32_t* status,
+                                 b200moe_stream_t stream);
+/* ... and its pieces: weight_rows[j*E+e, h] = w[e,h,j] (by_expert: [e*taps+j, h]); logits[s,e] = sum_j x[s-(taps-1)+j] *
+ * weight_rows[j,e] per sequence (H % 16 == 0, any S); the gradient of the logits laid out as the operand u (B*S, taps*E) of
+ * dX = u * weight_rows and dW = u^T * x, u[s, j*E+e] = grad_logits[s+(taps-1)-j, e]; the sum of dW's split-K slices
+ * P (slices, taps*E, H) as (E,H,taps) bf16. */
+int b200moe_conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* weight_rows,
+                             b200moe_stream_t stream);
+int b200moe_conv_gemm_logits(const void* x, const void* weight_rows, void* logits, int64_t B, int64_t S, int64_t H, int64_t E,
+                             int taps, int32_t* status, b200moe_stream_t stream);
+int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* grad_w, int64_t B, int64_t S, int E, int taps,
+                          int k, int norm_topk, float scale, void* u, b200moe_stream_t stream);
+int b200moe_conv_weight_grad(const float* P, int64_t slices, int E, int64_t H, int taps, void* grad_w,
+                             b200moe_stream_t stream);
 /* moe: the experts on given picks (idx (T,k), w (T,k) fp32).  E routed experts, the first n_glu with weights.
  * row_kernels: activations as row kernels (any code, act_params, Identity / Zero experts); 0: in the GEMM epilogues
  * (codes 0, 1, 5; act_codes NULL = SiLU).  keep = 0: no backward follows, which lets few rows per expert run over compact

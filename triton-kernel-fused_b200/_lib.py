@@ -47,6 +47,7 @@ _SIGNATURES = {
     "b200moe_gemm_tn_splitk": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                        c_void_p, c_void_p]),
     "b200moe_splitk_reduce": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
+    "b200moe_splitk_reduce_t": (c_int, [c_void_p] + [c_int64] * 3 + [c_void_p, c_void_p]),
     "b200moe_permute_ws_bytes": (c_size_t, [c_int64, c_int]),
     "b200moe_permute_build": (c_int, [c_void_p, c_int64, c_int, c_int] + [c_void_p] * 8 +
                               [c_void_p, c_size_t, c_void_p, c_void_p]),
@@ -94,6 +95,14 @@ _SIGNATURES = {
     "b200moe_router_forward": (c_int, [c_void_p] * 3 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 6),
     "b200moe_router_bwd_ws_bytes": (c_size_t, [c_int64, c_int64, c_int]),
     "b200moe_router_backward": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int, c_int, c_int, c_float] + [c_void_p] * 5),
+    "b200moe_conv_router_fwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 2),
+    "b200moe_conv_router_forward": (c_int, [c_void_p] * 3 + [c_int64] * 3 + [c_int] * 4 + [c_float] + [c_void_p] * 8),
+    "b200moe_conv_router_bwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 2),
+    "b200moe_conv_router_backward": (c_int, [c_void_p] * 5 + [c_int64] * 3 + [c_int] * 4 + [c_float] + [c_void_p] * 5),
+    "b200moe_conv_weight_rows": (c_int, [c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p]),
+    "b200moe_conv_gemm_logits": (c_int, [c_void_p] * 3 + [c_int64] * 4 + [c_int, c_void_p, c_void_p]),
+    "b200moe_conv_topk_bwd": (c_int, [c_void_p] * 3 + [c_int64] * 2 + [c_int] * 4 + [c_float] + [c_void_p] * 2),
+    "b200moe_conv_weight_grad": (c_int, [c_void_p, c_int64, c_int, c_int64, c_int, c_void_p, c_void_p]),
     "b200moe_moe_fwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 5),
     "b200moe_moe_forward": (c_int, [c_void_p] * 7 + [c_int64] * 3 + [c_int] * 5 + [c_void_p] * 4),
     "b200moe_moe_bwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 4),

@@ -108,10 +108,14 @@ struct Backward {
   float* part;
 };
 
-// split-K of the router's weight gradient: about two tiles per SM
+// Split-K of the router's weight gradient dW (E, H) = gl (T, E)^T x (T, H).  Up to 128 experts the product runs as
+// dW^T = x^T gl, whose rows (H) fill the MMA's M; gl^T x would multiply E of 256 rows.  About one tile per SM; the slices
+// are summed, and transposed back, by the reduction.  T 16384, H 2048, 64 experts: product + reduction 48 -> 31 us.
+static bool router_dw_transposed(int64_t E) { return E <= 128; }
 static int64_t router_k_chunk(int64_t T, int64_t E, int64_t H) {
-  const int64_t tiles = ((E + 127) / 128) * ((H + 255) / 256);
-  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(296 / std::max<int64_t>(tiles, 1), (T + 63) / 64));
+  const int64_t tiles = router_dw_transposed(E) ? ((H + 127) / 128) * ((E + 127) / 128) : ((E + 127) / 128) * ((H + 255) / 256);
+  const int64_t per_wave = router_dw_transposed(E) ? 148 : 296;
+  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
   return ((T + slices - 1) / slices + 63) / 64 * 64;
 }
 static int64_t router_slices(int64_t T, int64_t E, int64_t H) {
@@ -260,12 +264,33 @@ static int router_backward(const void* x, const void* weight, const void* logits
   if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(grad_logits, weight, grad_x, T, H, E, status, st));
   if (grad_weight != nullptr) {
     OpScope scope("gemm_tn", 2);
-    int rc = b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, router_k_chunk(T, E, H), status, st);
+    const int64_t chunk = router_k_chunk(T, E, H), slices = router_slices(T, E, H);
+    const bool tr = router_dw_transposed(E);
+    int rc = tr ? b200moe_gemm_tn_splitk(x, grad_logits, part, H, E, T, chunk, status, st)
+                : b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, chunk, status, st);
     if (rc) return rc;
-    rc = b200moe_splitk_reduce(part, router_slices(T, E, H), static_cast<int64_t>(E) * H, grad_weight, st);
+    rc = tr ? b200moe_splitk_reduce_t(part, slices, H, E, grad_weight, st)
+            : b200moe_splitk_reduce(part, slices, static_cast<int64_t>(E) * H, grad_weight, st);
     if (rc) return rc;
   }
   return 0;
+}
+
+// ---- conv router.  logits[s] = sum_j x[s - (taps-1) + j] W_j^T with W_j (E, H): one GEMM over (tap, channel) whose
+// producer shifts its boxes of x (gemm.cu).  Backward: the top-k kernel writes u (T, taps*E), every tap's gradient beside the
+// row of x it belongs to, and dX = u [W_j], dW = u^T x are plain products that read x and write dX once, for all taps, at
+// any sequence length.  x (16, 1024, 2048), 64 experts, 4 taps: dW 69 -> 26 us against a product that shifts x tap by tap
+// (E of 256 MMA rows, x read four times).
+// (The same turn of the forward, z = x [W_j]^T and adding its rows up, reads x once as well, but adds in another order: 1 in
+// 7000 picks of close experts then differs, and a token's gradient with it.)
+static int64_t conv_k_chunk(int64_t T, int64_t rows, int64_t H) {   // one wave of pair tiles
+  const int64_t tiles = ((rows + 255) / 256) * ((H + 255) / 256);
+  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(74 / std::max<int64_t>(tiles, 1), (T + 63) / 64));
+  return ((T + slices - 1) / slices + 63) / 64 * 64;
+}
+static int64_t conv_slices(int64_t T, int64_t rows, int64_t H) {
+  const int64_t c = conv_k_chunk(T, rows, H);
+  return (T + c - 1) / c;
 }
 
 }  // namespace b200moe
@@ -297,6 +322,81 @@ int b200moe_router_backward(const void* x, const void* weight, const void* logit
   bf16_t* gl = c.take<bf16_t>(T * E);
   float* part = c.take<float>(router_slices(T, E, H) * E * H);
   return router_backward(x, weight, logits, idx, grad_w, T, H, E, k, norm_topk, scale, gl, part, grad_x, grad_weight, status, stream);
+}
+
+// ---------------------------------------------------------------------------- conv router
+// a width that is no multiple of 16 would split an MMA's 16 channels between taps: the unfolded copy keeps the sums' order
+static bool conv_in_place(int64_t H) { return H % 16 == 0; }
+
+size_t b200moe_conv_router_fwd_ws_bytes(int64_t B, int64_t S, int64_t H, int E, int taps) {
+  if (B <= 0 || S <= 0 || H <= 0 || E <= 0 || taps <= 0 || conv_in_place(H)) return 0;
+  Carver c(nullptr);
+  c.take<bf16_t>(B * S * taps * H);
+  c.take<bf16_t>(static_cast<int64_t>(E) * taps * H);
+  return c.off;
+}
+
+static int check_conv_router(const char* who, int64_t B, int64_t S, int64_t H, int E, int taps) {
+  B200_CHECK_ARG(B > 0 && S > 0 && taps >= 1 && taps <= 64 && H > 0 && H % 8 == 0 && E > 0 && E % 8 == 0 && B * S < (1LL << 31),
+                 B200MOE_E_BAD_SHAPE, "%s: B = %lld, S = %lld, H = %lld, E = %d (multiples of 8), taps = %d (1..64)", who,
+                 (long long)B, (long long)S, (long long)H, E, taps);
+  return 0;
+}
+
+int b200moe_conv_router_forward(const void* x, const void* weight, const float* bias, int64_t B, int64_t S, int64_t H, int E,
+                                int taps, int k, int norm_topk, float scale, void* ws, void* weight_rows, void* logits,
+                                int64_t* idx, float* w, int32_t* counts, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_conv_router("conv_router_forward", B, S, H, E, taps);
+  if (rc) return rc;
+  B200_CHECK_ARG(x && weight && weight_rows && logits && (ws || conv_in_place(H)), B200MOE_E_NULL, "conv_router_forward: null pointer");
+  RUN("conv_weight_rows", 1, b200moe_conv_weight_rows(weight, E, H, taps, 0, weight_rows, stream));
+  if (conv_in_place(H)) {
+    RUN("conv_gemm_fwd", 1, b200moe_conv_gemm_logits(x, weight_rows, logits, B, S, H, E, taps, status, stream));
+  } else {
+    Carver c(ws);
+    bf16_t* xu = c.take<bf16_t>(B * S * taps * H);
+    bf16_t* wf = c.take<bf16_t>(static_cast<int64_t>(E) * taps * H);
+    RUN("conv_weight_rows", 1, b200moe_conv_weight_rows(weight, E, H, taps, 1, wf, stream));
+    RUN("conv_unfold", 1, b200moe_conv_unfold(x, B, S, H, taps, xu, stream));
+    RUN("gemm_nt", 1, b200moe_gemm_nt(xu, wf, logits, B * S, E, taps * H, status, stream));
+  }
+  RUN("router_topk_fwd", 1, b200moe_router_topk_fwd(logits, B200MOE_LOGITS_BF16, bias, B * S, E, k, norm_topk, scale, idx, w, counts, stream));
+  return 0;
+}
+
+struct ConvBackward { bf16_t* u; float* part; };
+static ConvBackward carve_conv(int64_t T, int64_t H, int64_t rows, void* ws, size_t* bytes) {
+  Carver c(ws);
+  ConvBackward b;
+  b.u = c.take<bf16_t>(T * rows);
+  b.part = c.take<float>(conv_slices(T, rows, H) * rows * H);
+  if (bytes != nullptr) *bytes = c.off;
+  return b;
+}
+
+size_t b200moe_conv_router_bwd_ws_bytes(int64_t B, int64_t S, int64_t H, int E, int taps) {
+  if (B <= 0 || S <= 0 || H <= 0 || E <= 0 || taps <= 0) return 0;
+  size_t n = 0;
+  carve_conv(B * S, H, static_cast<int64_t>(E) * taps, nullptr, &n);
+  return n;
+}
+
+int b200moe_conv_router_backward(const void* x, const void* weight_rows, const void* logits, const int64_t* idx,
+                                 const float* grad_w, int64_t B, int64_t S, int64_t H, int E, int taps, int k, int norm_topk,
+                                 float scale, void* ws, void* grad_x, void* grad_weight, int32_t* status,
+                                 b200moe_stream_t stream) {
+  int rc = check_conv_router("conv_router_backward", B, S, H, E, taps);
+  if (rc) return rc;
+  B200_CHECK_ARG(x && weight_rows && ws, B200MOE_E_NULL, "conv_router_backward: null pointer");
+  const int64_t T = B * S, rows = static_cast<int64_t>(E) * taps;
+  const ConvBackward b = carve_conv(T, H, rows, ws, nullptr);
+  RUN("router_topk_bwd", 1, b200moe_conv_topk_bwd(logits, idx, grad_w, B, S, E, taps, k, norm_topk, scale, b.u, stream));
+  if (grad_x != nullptr) RUN("conv_gemm_dx", 1, b200moe_gemm_nn(b.u, weight_rows, grad_x, T, H, rows, status, stream));
+  if (grad_weight != nullptr) {
+    RUN("conv_gemm_dw", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, conv_k_chunk(T, rows, H), status, stream));
+    RUN("conv_weight_grad", 1, b200moe_conv_weight_grad(b.part, conv_slices(T, rows, H), E, H, taps, grad_weight, stream));
+  }
+  return 0;
 }
 
 // ---------------------------------------------------------------------------- experts on given picks

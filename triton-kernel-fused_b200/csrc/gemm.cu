@@ -166,7 +166,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         uint32_t ph = 0;
         bool ok = true;
         for (int tile = first_tile; tile < total && ok; tile += tile_step) {
-          const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
+          const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
           const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
           const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
           const int bstep = pair_cols<BN, EPI>(p, t.n0) / 2;
@@ -204,12 +204,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = first_tile; tile < total && ok; tile += tile_step) {
-        const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
+        const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
         const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
         const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
         // a narrower last pair tile: each CTA supplies half of its columns of B, the first ones of its (still
         // BN/2 wide) staging tile
         const int bstep = (CTAS == 2) ? pair_cols<BN, EPI>(p, t.n0) / 2 : BNC;
+        // coordinates of the A box (K-major case) and of the B boxes; a convolution operand (see GemmParams::conv_taps)
+        // replaces the flat row by (position + shift, batch).  Its divisions are done once per tile, the k-loop only counts
+        // (logits of x (16, 1024, 2048), 64 experts, 4 taps: 56 us with the divisions in the k-loop, 45 us without).
+        int a_c0 = t.k0, a_c1 = m0, a_c2 = 0, b_n0 = t.n0, b_k = t.k0, b_g = gB, b_c0 = t.k0;
+        if (CONV && p.conv_taps > 0) {
+          if (p.sched == SCHED_DENSE) {
+            a_c2 = t.g;                                            // batch
+            a_c1 = m0 - p.conv_sign * (p.conv_taps - 1);
+          } else {
+            const int tap = t.n0 / p.conv_C;
+            b_n0 = t.n0 - tap * p.conv_C;
+            b_g = t.k0 / p.conv_S;
+            b_k = t.k0 - b_g * p.conv_S + tap - (p.conv_taps - 1);
+          }
+        }
         for (int kb = 0; kb < t.nkb; ++kb) {
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
             ok = false;
@@ -218,22 +233,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
           const uint32_t sb = sa + C::A_BYTES;
           const int kk = t.k0 + kb * BK;
-          // coordinates of the B boxes (MN-major case) and of the A box (K-major case); a convolution operand
-          // (see GemmParams::conv_taps) replaces the flat row by (position + shift, batch)
-          int a_c0 = kk, a_c1 = m0, a_c2 = 0, b_n0 = t.n0, b_k = kk, b_g = gB;
-          if (CONV && p.conv_taps > 0) {
-            if (p.sched == SCHED_DENSE) {
-              const int per_tap = p.conv_C / BK, tap = kb / per_tap;
-              a_c2 = m0 / p.conv_S;
-              a_c1 = m0 - a_c2 * p.conv_S + p.conv_sign * (tap - (p.conv_taps - 1));
-              a_c0 = (kb - tap * per_tap) * BK;
-            } else {
-              const int tap = t.n0 / p.conv_C;
-              b_n0 = t.n0 - tap * p.conv_C;
-              b_g = kk / p.conv_S;
-              b_k = kk - b_g * p.conv_S + tap - (p.conv_taps - 1);
-            }
-          }
+          if (!CONV || p.conv_taps == 0) a_c0 = b_k = b_c0 = kk;
           if constexpr (CTAS == 1) {
             const uint32_t full = bar_full + 8 * s;
             mbar_arrive_expect_tx(full, C::STAGE_BYTES);
@@ -249,7 +249,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               tma_load_3d(sb, &tmB, full, kk, t.n0, 2 * gB);
               tma_load_3d(sb + (BN / 2) * BK * 2, &tmB, full, kk, t.n0, 2 * gB + 1);
             } else if (!p.b_mn) {
-              tma_load_3d(sb, &tmB, full, kk, t.n0, gB);  // box {64 k, BN rows}
+              tma_load_3d(sb, &tmB, full, b_c0, t.n0, b_g);  // box {64 k, BN rows}
             } else {
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
@@ -270,12 +270,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               // leader stages the gate rows, the peer the up rows of I-columns [n0, n0+128)
               tma_load_3d_pair(sb, &tmB, full, kk, t.n0, 2 * gB + static_cast<int>(cta_rank));
             } else if (!p.b_mn) {
-              tma_load_3d_pair(sb, &tmB, full, kk, t.n0 + bstep * static_cast<int>(cta_rank), gB);
+              tma_load_3d_pair(sb, &tmB, full, b_c0, t.n0 + bstep * static_cast<int>(cta_rank), b_g);
             } else {
 #pragma unroll
               for (int j = 0; j < BNC / 64; ++j)
                 tma_load_3d_pair(sb + j * (64 * BK * 2), &tmB, full,
                                  b_n0 + bstep * static_cast<int>(cta_rank) + 64 * j, b_k, b_g);
+            }
+          }
+          if (CONV && p.conv_taps > 0) {       // the next k-block's coordinates
+            if (p.sched == SCHED_DENSE) {
+              a_c0 += BK;
+              b_c0 += BK;
+              b_k += BK;
+              if (a_c0 >= p.conv_C) {          // next tap
+                a_c0 = 0;
+                a_c1 += p.conv_sign;
+                if (p.conv_b_taps) {
+                  b_c0 = 0;
+                  ++b_g;
+                }
+              }
+            } else {
+              b_k += BK;
+              if (kk + BK - b_g * p.conv_S >= p.conv_S) {   // next batch
+                ++b_g;
+                b_k -= p.conv_S;
+              }
             }
           }
           if (++s == NSTAGE) {
@@ -297,7 +318,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = first_tile; tile < total && ok; tile += tile_step, ++it) {
-        const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
+        const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
         const int buf = it & 1;
         if (!mbar_wait(bar_tempty + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, ST_WAIT_MMA_TMEM)) break;
         tc_fence_after();
@@ -344,7 +365,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     uint32_t epi_phase = 0;   // parity of this warp's GLU-backward load barrier
     int it = 0;
     for (int tile = first_tile; tile < total; tile += tile_step, ++it) {
-      const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base);
+      const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
       const int buf = it & 1;
       int act_code = 0;   // activation of this tile's expert (uniform over the tile)
       if constexpr (POLY && (EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD)) act_code = p.act_codes[t.g];
@@ -383,7 +404,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         // results are packed to bf16, staged per warp as 32 rows x 64 columns and written by TMA
         // stores (which clip at the tensor's bounds, so no row or column masks are needed)
         uint8_t* sbuf = bufG;   // this warp's staging box
-        const int grp = (p.sched == SCHED_GROUPED_K) ? t.g : 0;
+        const int grp = (p.sched == SCHED_GROUPED_K || (CONV && p.conv_taps > 0)) ? t.g : 0;
         if constexpr (EPI == EPI_STORE || EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {
           constexpr int W = BN / 2;
           // push mode: this lane's output row goes to a slot of another GPU's (or this GPU's) receive buffer
@@ -542,8 +563,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       } else if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32) {
-        const bool row_ok = (p.sched == SCHED_GROUPED_M) || (row < p.M);
-        const long long base = (p.sched == SCHED_GROUPED_K ? t.g * p.d_group_stride : 0) +
+        const bool conv_rows = CONV && p.conv_taps > 0 && p.sched == SCHED_DENSE;   // rows are positions of batch t.g
+        const bool row_ok = (p.sched == SCHED_GROUPED_M) || (row < (conv_rows ? p.conv_S : p.M));
+        const long long base = (p.sched == SCHED_GROUPED_K || conv_rows ? t.g * p.d_group_stride : 0) +
                                row * p.ldd + t.n0;
         constexpr int W = BN / 2;   // columns per warp
 #pragma unroll 1
@@ -898,7 +920,8 @@ int b200moe_gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, in
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
   p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
-  const int bn = pick_bn(N);
+  // up to 128 rows a pair tile would multiply nothing but padding in its second half
+  const int bn = M <= BM ? pick_bn(N) : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
   return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
                                     (cudaStream_t)stream);
 }
@@ -929,11 +952,29 @@ int b200moe_conv_gemm_fwd(const void* x, const void* wf, void* logits, int64_t B
   Operand b{wf, 0, E, K, K, 1, E * K};
   GemmParams p{};
   p.sched = SCHED_DENSE; p.M = (int)M; p.N = (int)E; p.K = (int)K; p.num_groups = 1;
-  p.D = logits; p.ldd = E; p.status = status;
+  p.D = logits; p.ldd = E; p.d_group_stride = S * E; p.status = status;
   p.conv_taps = taps; p.conv_S = (int)S; p.conv_C = (int)H; p.conv_sign = 1;
   const int bn = pick_bn(E);
-  Operand d{logits, 0, M, E, E, 1, M * E};
-  return dispatch_bn<EPI_STORE, true>(bn, a, b, &d, nullptr, p, (int)(ceil_div(M, BM) * ceil_div(E, bn)), (cudaStream_t)stream);
+  Operand d{logits, 0, S, E, E, B, S * E};
+  return dispatch_bn<EPI_STORE, true>(bn, a, b, &d, nullptr, p, (int)(B * ceil_div(S, BM) * ceil_div(E, bn)), (cudaStream_t)stream);
+}
+
+int b200moe_conv_gemm_logits(const void* x, const void* weight_rows, void* logits, int64_t B, int64_t S, int64_t H, int64_t E,
+                             int taps, int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(x && weight_rows && logits, B200MOE_E_NULL, "conv_gemm_logits: null pointer");
+  int rc = check_conv("conv_gemm_logits", B, S, H, E, taps, 1, 64);
+  if (rc) return rc;
+  B200_CHECK_ARG(H % 16 == 0, B200MOE_E_BAD_SHAPE, "conv_gemm_logits: H = %lld must be a multiple of 16", (long long)H);
+  B200_CHECK_ARG(aligned16(logits), B200MOE_E_ALIGN, "conv_gemm_logits: logits not 16-byte aligned");
+  Operand a{x, 0, S, H, H, B, S * H};                    // {H, S, B}: positions outside [0, S) read as zero
+  Operand b{weight_rows, 0, E, H, H, taps, E * H};       // {H, E, taps}
+  GemmParams p{};
+  p.sched = SCHED_DENSE; p.M = (int)(B * S); p.N = (int)E; p.K = (int)(taps * ceil_div(H, BK) * BK); p.num_groups = 1;
+  p.D = logits; p.ldd = E; p.d_group_stride = S * E; p.status = status;
+  p.conv_taps = taps; p.conv_S = (int)S; p.conv_C = (int)H; p.conv_sign = 1; p.conv_b_taps = 1;
+  const int bn = pick_bn(E);
+  Operand d{logits, 0, S, E, E, B, S * E};
+  return dispatch_bn<EPI_STORE, true>(bn, a, b, &d, nullptr, p, (int)(B * ceil_div(S, BM) * ceil_div(E, bn)), (cudaStream_t)stream);
 }
 
 int b200moe_conv_gemm_dx(const void* grad_logits, const void* wb, void* grad_x, int64_t B, int64_t S, int64_t H, int64_t E,
@@ -947,11 +988,11 @@ int b200moe_conv_gemm_dx(const void* grad_logits, const void* wb, void* grad_x, 
   Operand b{wb, 1, H, K, H, 1, H * K};            // stored (taps * E, H): MN-major
   GemmParams p{};
   p.sched = SCHED_DENSE; p.b_mn = 1; p.M = (int)M; p.N = (int)H; p.K = (int)K; p.num_groups = 1;
-  p.D = grad_x; p.ldd = H; p.status = status;
+  p.D = grad_x; p.ldd = H; p.d_group_stride = S * H; p.status = status;
   p.conv_taps = taps; p.conv_S = (int)S; p.conv_C = (int)E; p.conv_sign = -1;
   const int bn = pick_bn(H);
-  Operand d{grad_x, 0, M, H, H, 1, M * H};
-  return dispatch_bn<EPI_STORE, true>(bn, a, b, &d, nullptr, p, (int)(ceil_div(M, BM) * ceil_div(H, bn)), (cudaStream_t)stream);
+  Operand d{grad_x, 0, S, H, H, B, S * H};
+  return dispatch_bn<EPI_STORE, true>(bn, a, b, &d, nullptr, p, (int)(B * ceil_div(S, BM) * ceil_div(H, bn)), (cudaStream_t)stream);
 }
 
 int b200moe_conv_gemm_dw_splitk(const void* grad_logits, const void* x, float* P, int64_t B, int64_t S, int64_t H,

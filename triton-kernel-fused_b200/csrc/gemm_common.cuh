@@ -59,9 +59,10 @@ struct GemmParams {
   // positions, batches} and every 64-wide k-block is loaded `shift` positions away from the tile's own, positions
   // outside [0, conv_S) reading as zero (the convolution's padding), so the unfolded (rows, taps * C) copy of the
   // input is never written.  DENSE: operand A, k-block kb = (tap, channel block), shift = conv_sign * (tap -
-  // (conv_taps - 1)); row tiles must not straddle batches (conv_S % 128 == 0).  GROUPED_K by chunks (split-K
+  // (conv_taps - 1)); a row tile lies in one batch (its last one may be short).  GROUPED_K by chunks (split-K
   // weight gradient): operand B, tap = tile column / conv_C, shift = tap - (conv_taps - 1); conv_S % 64 == 0.
   int conv_taps, conv_S, conv_C, conv_sign;
+  int conv_b_taps;   // DENSE convolution: operand B is {conv_C channels, N, taps} (else {taps * conv_C, N})
 };
 
 struct Tile {
@@ -81,7 +82,8 @@ __device__ __forceinline__ int sym_tiles_per_group(const GemmParams& p, int TN, 
 __device__ __forceinline__ int total_tiles(const GemmParams& p, int TN, int TM, bool window = false) {
   const int nt = (p.N + TN - 1) / TN;
   if (p.sched == SCHED_GROUPED_M && p.sym_rows > 0) return p.num_groups * sym_tiles_per_group(p, TN, TM);
-  if (p.sched == SCHED_DENSE) return ((p.M + TM - 1) / TM) * nt;
+  if (p.sched == SCHED_DENSE)
+    return (p.conv_taps > 0 ? p.M / p.conv_S * ((p.conv_S + TM - 1) / TM) : (p.M + TM - 1) / TM) * nt;
   if (p.sched == SCHED_GROUPED_M) {
     const int rows = p.poffs[p.num_groups];
     return ((window && p.row_hi > 0 ? max(min(rows, p.row_hi) - p.row_lo, 0) : rows) / TM) * nt;
@@ -109,7 +111,7 @@ __device__ __forceinline__ const int* build_group_order(const GemmParams& p, int
 }
 
 __device__ __forceinline__ Tile get_tile(const GemmParams& p, int tile, int TN, int TM, int BK = 64,
-                                         const int* order = nullptr, int row_base = 0) {
+                                         const int* order = nullptr, int row_base = 0, bool conv = false) {
   Tile t;
   const int nt = (p.N + TN - 1) / TN;
   if (p.sched == SCHED_GROUPED_K) {
@@ -149,6 +151,11 @@ __device__ __forceinline__ Tile get_tile(const GemmParams& p, int tile, int TN, 
     t.m0 = mi * TM + row_base;   // first row of the launch's row window (0: every row)
     t.n0 = (tile - mi * nt) * TN;
     t.g = (p.sched == SCHED_GROUPED_M) ? p.tile_expert[t.m0 / B200MOE_TILE_M] : 0;
+    if (conv && p.conv_taps > 0) {   // convolution: tiles batch by batch, m0 = position, g = batch
+      const int per = (p.conv_S + TM - 1) / TM;
+      t.g = mi / per;
+      t.m0 = (mi - t.g * per) * TM;
+    }
     t.k0 = 0;
     t.nkb = (p.K + BK - 1) / BK;
   }

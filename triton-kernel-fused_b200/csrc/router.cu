@@ -3,6 +3,8 @@
 // One warp owns one token; lane l holds experts l, l+32, ... (at most 8 values for E <= 256).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "ptx.cuh"
 #include "topk.cuh"
@@ -73,16 +75,20 @@ router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__
   }
 }
 
+// taps > 1 (the conv router; rows are (batch, position), S positions): grad_logits is written as the operand of the
+// products for dX and dW, u (T, taps*E), u[s', j*E + e] = grad_logits[s' + (taps-1) - j, e], zero past the end.
 // Lane j < k reads pick j, its upstream gradient and its logit, so the dependent loads of all picks are one round trip;
 // the sums run over the picks in order.  (T = 16384, E = 64, k = 6: 14.2 -> 6.8 us.)
-template <int KIND, int VPL>
+template <int KIND, int VPL, bool PAIR>
 __global__ void __launch_bounds__(256)
 router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restrict__ idx,
-                       const float* __restrict__ grad_w, long long T, int E, int k, int norm, float scale,
+                       const float* __restrict__ grad_w, long long T, int E, int k, int norm, float scale, int S, int taps,
                        __nv_bfloat16* __restrict__ grad_logits) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
+  // expert of a lane's i-th value; PAIR (even E): neighbours two by two, so that a warp writes whole 32-bit words
+  auto expert = [lane](int i) { return PAIR ? 64 * (i >> 1) + 2 * lane + (i & 1) : lane + 32 * i; };
   for (long long t = static_cast<long long>(blockIdx.x) * wpb + warp; t < T;
        t += static_cast<long long>(gridDim.x) * wpb) {
     float s[VPL], gs[VPL];
@@ -94,7 +100,7 @@ router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restr
     }
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      const int e = lane + 32 * i;
+      const int e = expert(i);
       s[i] = (e < E) ? sigmoid_f(load_in<KIND>(logits, t * E + e)) : 0.0f;
       gs[i] = 0.0f;
     }
@@ -115,13 +121,57 @@ router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restr
       const float gj = __shfl_sync(0xffffffffu, graw, j);
 #pragma unroll
       for (int i = 0; i < VPL; ++i)
-        if (ij == lane + 32 * i) gs[i] += gj;
+        if (ij == expert(i)) gs[i] += gj;
     }
+    auto put = [&](long long row, const uint32_t (&g)[VPL]) {     // g: bf16 bits of this lane's values
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int e = lane + 32 * i;
-      if (e < E) grad_logits[t * E + e] = __float2bfloat16_rn(gs[i] * (s[i] * (1.0f - s[i])));
+      for (int i = 0; i < VPL; i += PAIR ? 2 : 1) {
+        const int e = expert(i);
+        if (e >= E) continue;
+        if constexpr (PAIR) *reinterpret_cast<uint32_t*>(grad_logits + row * E + e) = g[i] | (g[i + 1] << 16);
+        else reinterpret_cast<uint16_t*>(grad_logits)[row * E + e] = static_cast<uint16_t>(g[i]);
+      }
+    };
+    uint32_t g[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) g[i] = pack_bf16x2(gs[i] * (s[i] * (1.0f - s[i])), 0.0f);
+    if (taps == 1) {
+      put(t, g);
+      continue;
     }
+    const uint32_t zero[VPL] = {};
+    const int pos = static_cast<int>(t % S);
+    for (int j = 0; j < taps; ++j) {
+      const int back = taps - 1 - j;       // this token's gradient belongs to the row `back` positions earlier
+      if (pos >= back) put((t - back) * taps + j, g);
+      if (pos + back >= S) put(t * taps + j, zero);
+    }
+  }
+}
+
+// w (E, H, taps) -> wt (taps, E, H), wt[j, e, h] = w[e, h, j] (the operand of the conv router's products), or (E, taps, H)
+__global__ void __launch_bounds__(256)
+conv_weight_rows_kernel(const __nv_bfloat16* __restrict__ w, int E, int H, int taps, int by_expert,
+                        __nv_bfloat16* __restrict__ wt) {
+  const long long n = static_cast<long long>(E) * H;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
+    const long long e = i / H, h = i - e * H;
+    for (int j = 0; j < taps; ++j)
+      wt[(by_expert ? e * taps + j : static_cast<long long>(j) * E + e) * H + h] = w[i * taps + j];
+  }
+}
+
+// grad_w (E, H, taps) bf16 = sum over the slices of p (slices, taps*E, H) fp32
+__global__ void __launch_bounds__(256)
+conv_weight_grad_kernel(const float* __restrict__ p, long long slices, int E, int H, int taps,
+                        __nv_bfloat16* __restrict__ gw) {
+  const long long n = static_cast<long long>(E) * H, elems = n * taps;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < elems; i += gridDim.x * 256LL) {
+    const long long j = i / n, eh = i - j * n;       // consecutive threads: consecutive h of one row of p
+    float acc = 0.0f;
+#pragma unroll 8
+    for (long long q = 0; q < slices; ++q) acc += p[q * elems + i];
+    gw[eh * taps + j] = __float2bfloat16_rn(acc);
   }
 }
 
@@ -160,12 +210,44 @@ splitk_reduce_kernel(const float* __restrict__ P, long long slices, long long el
   *reinterpret_cast<uint2*>(D + i4) = o;
 }
 
+// D (C,R) = bf16( sum_s P[s] (R,C) )^T through a 32 x 32 tile in shared memory: both sides coalesced, a thread per
+// value so that all its slices are in flight at once
+__global__ void __launch_bounds__(1024)
+splitk_reduce_t_kernel(const float* __restrict__ P, long long slices, int R, int C, __nv_bfloat16* __restrict__ D) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  const long long elems = static_cast<long long>(R) * C;
+  float acc = 0.0f;
+  if (r0 + ty < R && c0 + tx < C) {
+    const float* src = P + static_cast<long long>(r0 + ty) * C + c0 + tx;
+#pragma unroll 16
+    for (long long s = 0; s < slices; ++s) acc += src[s * elems];
+  }
+  tile[ty][tx] = acc;
+  __syncthreads();
+  if (r0 + tx < R && c0 + ty < C) D[static_cast<long long>(c0 + ty) * R + r0 + tx] = __float2bfloat16_rn(tile[tx][ty]);
+}
+
 static int grid_for_tokens(long long T) {
   long long g = (T + 7) / 8;
   const long long cap = static_cast<long long>(num_sms()) * 8;
   if (g > cap) g = cap;
   if (g < 1) g = 1;
   return static_cast<int>(g);
+}
+
+template <int KIND>
+static void launch_topk_bwd(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k, int norm,
+                            float scale, int S, int taps, __nv_bfloat16* out, cudaStream_t st) {
+  const int grid = grid_for_tokens(T);
+  by_experts(E, [&](auto v) {
+    constexpr int VPL = v.value;
+    if (VPL > 1 && E % 2 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0)
+      router_topk_bwd_kernel<KIND, VPL, (VPL > 1)><<<grid, 256, 0, st>>>(logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
+    else
+      router_topk_bwd_kernel<KIND, VPL, false><<<grid, 256, 0, st>>>(logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
+  });
 }
 
 }  // namespace b200moe
@@ -214,15 +296,14 @@ int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* i
   B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "router_topk_bwd: top_k = %d", k);
   if (T <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  const int grid = grid_for_tokens(T);
   const long long* idx_ll = reinterpret_cast<const long long*>(idx);
   __nv_bfloat16* gl = reinterpret_cast<__nv_bfloat16*>(grad_logits);
   switch (input_kind) {
     case B200MOE_LOGITS_BF16:
-      by_experts(E, [&](auto v) { router_topk_bwd_kernel<B200MOE_LOGITS_BF16, v.value><<<grid, 256, 0, st>>>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, gl); });
+      launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st);
       break;
     case B200MOE_LOGITS_F32:
-      by_experts(E, [&](auto v) { router_topk_bwd_kernel<B200MOE_LOGITS_F32, v.value><<<grid, 256, 0, st>>>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, gl); });
+      launch_topk_bwd<B200MOE_LOGITS_F32>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st);
       break;
     default:
       set_error("router_topk_bwd: input_kind %d has no backward (logits are required)", input_kind);
@@ -232,11 +313,61 @@ int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* i
   return 0;
 }
 
+int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* grad_w, int64_t B, int64_t S, int E, int taps,
+                          int k, int norm_topk, float scale, void* u, b200moe_stream_t stream) {
+  B200_CHECK_ARG(logits && idx && grad_w && u, B200MOE_E_NULL, "conv_topk_bwd: null pointer");
+  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED, "conv_topk_bwd: E = %d, supported 1..%d", E,
+                 B200MOE_MAX_EXPERTS);
+  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "conv_topk_bwd: top_k = %d", k);
+  B200_CHECK_ARG(B >= 1 && S >= 1 && S < (1LL << 31) && taps >= 1 && taps <= 64, B200MOE_E_BAD_SHAPE,
+                 "conv_topk_bwd: B = %lld, S = %lld, taps = %d (1..64)", (long long)B, (long long)S, taps);
+  launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, reinterpret_cast<const long long*>(idx), grad_w, B * S, E, k, norm_topk, scale,
+                                       static_cast<int>(S), taps, reinterpret_cast<__nv_bfloat16*>(u), (cudaStream_t)stream);
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+static int weight_grid(int64_t n) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(num_sms()) * 8)));
+}
+
+int b200moe_conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, b200moe_stream_t stream) {
+  B200_CHECK_ARG(w && wt, B200MOE_E_NULL, "conv_weight_rows: null pointer");
+  B200_CHECK_ARG(E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE, "conv_weight_rows: E = %d, H = %lld, taps = %d", E,
+                 (long long)H, taps);
+  conv_weight_rows_kernel<<<weight_grid(E * H), 256, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(w), E, static_cast<int>(H), taps, by_expert, reinterpret_cast<__nv_bfloat16*>(wt));
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int b200moe_conv_weight_grad(const float* P, int64_t slices, int E, int64_t H, int taps, void* grad_w,
+                             b200moe_stream_t stream) {
+  B200_CHECK_ARG(P && grad_w, B200MOE_E_NULL, "conv_weight_grad: null pointer");
+  B200_CHECK_ARG(slices >= 1 && E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE,
+                 "conv_weight_grad: slices = %lld, E = %d, H = %lld, taps = %d", (long long)slices, E, (long long)H, taps);
+  conv_weight_grad_kernel<<<weight_grid(E * H * taps), 256, 0, (cudaStream_t)stream>>>(
+      P, slices, E, static_cast<int>(H), taps, reinterpret_cast<__nv_bfloat16*>(grad_w));
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
 int b200moe_router_bias_update(float* bias, const int32_t* counts, int E, float u, b200moe_stream_t stream) {
   B200_CHECK_ARG(bias && counts, B200MOE_E_NULL, "router_bias_update: null pointer");
   B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "router_bias_update: E = %d", E);
   if (!(u > 0.0f)) return 0;
   router_bias_update_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(bias, counts, E, u);
+  B200_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int b200moe_splitk_reduce_t(const float* P, int64_t slices, int64_t R, int64_t C, void* D, b200moe_stream_t stream) {
+  B200_CHECK_ARG(P && D, B200MOE_E_NULL, "splitk_reduce_t: null pointer");
+  B200_CHECK_ARG(slices >= 1 && R > 0 && C > 0 && R < (1LL << 31) && C <= 32 * 65535, B200MOE_E_BAD_SHAPE,
+                 "splitk_reduce_t: slices = %lld, R = %lld, C = %lld", (long long)slices, (long long)R, (long long)C);
+  const dim3 grid(static_cast<unsigned>((R + 31) / 32), static_cast<unsigned>((C + 31) / 32));
+  splitk_reduce_t_kernel<<<grid, 1024, 0, (cudaStream_t)stream>>>(P, slices, static_cast<int>(R), static_cast<int>(C),
+                                                                 reinterpret_cast<__nv_bfloat16*>(D));
   B200_CUDA(cudaGetLastError());
   return 0;
 }

@@ -92,11 +92,10 @@ def fused_mlp_router(x, gate_weight, bias, top_k, num_experts, norm_topk_prob=Tr
 
 class FusedConvRouter(torch.autograd.Function):
     """Causal-conv router (kernels/sm75/router.py:172-218, FusedConvRouterCuDNN): logits[b,s,e] =
-    sum_{j,h} x[b, s-(K-1)+j, h] * W[e,h,j], then the same sigmoid / bias / top-k epilogue.  The conv is one
-    tcgen05 GEMM whose TMA producer reads x in place, tap by tap, through a (H, S, B) tensor map (S a multiple of
-    128, H of 64; as kernels/sm120/router.py:34-85 does in one launch), or over an unfolded copy of x for other
-    shapes; backward = epilogue Jacobian, dX GEMM (the same way over grad_logits when E is a multiple of 64, else
-    plain GEMM + fold), split-K dW GEMM."""
+    sum_{j,h} x[b, s-(K-1)+j, h] * W[e,h,j], then the same sigmoid / bias / top-k epilogue.  One tcgen05 GEMM
+    whose TMA producer reads x in place, tap by tap, through an (H, S, B) tensor map (kernels/sm120/router.py:34-85 is one
+    launch too), or over an unfolded copy of x when H is no multiple of 16; the backward's top-k kernel lays the gradients
+    out tap by tap, and dX and dW are plain products with that.  One native call each way (csrc/block.cu)."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, top_k, num_experts, norm_topk=True, scale=1.0):
@@ -106,42 +105,42 @@ class FusedConvRouter(torch.autograd.Function):
         L.require_cuda_bf16("x", x)
         L.require_cuda_bf16("conv_weight", weight)
         L.require(x.dim() == 3 and weight.dim() == 3 and weight.shape[1] == x.shape[2], "need x (B,S,H) and conv_weight (E,H,K)")
-        B, S, H = x.shape
-        E, _, K = weight.shape
+        (B, S, H), (E, _, K), dev, k = x.shape, weight.shape, x.device, int(top_k)
         L.require(num_experts is None or int(num_experts) == E, "num_experts must equal conv_weight.shape[0]")
-        x = x.contiguous()
-        wf = weight.permute(0, 2, 1).reshape(E, K * H).contiguous()      # Wf[e, j*H+h] = W[e,h,j]
-        ctx.direct = ops.conv_direct_ok(S, H)
-        if ctx.direct:
-            xu = x                                                        # read in place by the GEMMs
-            logits = ops.conv_gemm_fwd(x, wf, K)
-        else:
-            xu = ops.conv_unfold(x, K)
-            logits = ops.gemm_nt(xu, wf)
+        x, weight = x.contiguous(), weight.contiguous()
         bias32 = bias.detach().float().contiguous() if bias is not None else None
-        idx, w, counts = ops.router_topk_fwd(logits, bias32, top_k, norm_topk and top_k > 1, scale)
-        ctx.shape = (B, S, H, E, K)
-        ctx.save_for_backward(xu, wf, weight, logits, idx)
-        ctx.norm, ctx.scale = bool(norm_topk and top_k > 1), float(scale)
+        if bias32 is not None:
+            L.require(bias32.is_cuda and bias32.numel() == E, "bias must be a contiguous float32 CUDA tensor of E elements")
+        L.require(weight.device == dev, "conv_weight must be on x's device")
+        ctx.norm, ctx.scale = int(bool(norm_topk and top_k > 1)), float(scale)
+        wt = torch.empty(K * E, H, dtype=torch.bfloat16, device=dev)
+        logits = torch.empty(B * S, E, dtype=torch.bfloat16, device=dev)
+        idx = torch.empty(B * S, k, dtype=torch.int64, device=dev)
+        w = torch.empty(B * S, k, dtype=torch.float32, device=dev)
+        counts = torch.empty(E, dtype=torch.int32, device=dev)
+        lib = L.lib()
+        ws = L.workspace(lib.b200moe_conv_router_fwd_ws_bytes(B, S, H, E, K), dev)
+        L.check(lib.b200moe_conv_router_forward(x.data_ptr(), weight.data_ptr(), L.ptr(bias32), B, S, H, E, K, k, ctx.norm,
+                                                ctx.scale, ws.data_ptr(), wt.data_ptr(), logits.data_ptr(), idx.data_ptr(),
+                                                w.data_ptr(), counts.data_ptr(), L.status_word(dev).data_ptr(), L.stream_of(x)))
+        ctx.shape = (B, S, H, E, K, k)
+        ctx.save_for_backward(x, wt, logits, idx)
         ctx.mark_non_differentiable(idx, counts)
         return idx, w, counts
 
     @staticmethod
     def backward(ctx, grad_idx, grad_weights, grad_counts):
-        xu, wf, weight, logits, idx = ctx.saved_tensors
-        B, S, H, E, K = ctx.shape
-        gl = ops.router_topk_bwd(logits, idx, grad_weights, ctx.norm, ctx.scale)
-        grad_x = None
-        if ctx.needs_input_grad[0]:
-            if ctx.direct and E % 64 == 0:
-                wb = weight.permute(2, 0, 1).reshape(K * E, H).contiguous()   # Wb[j*E+e, h] = W[e,h,j]
-                grad_x = ops.conv_gemm_dx(gl, wb, B, S, K)
-            else:
-                grad_x = ops.conv_fold(ops.gemm_nn(gl, wf), B, S, H, K)
-        grad_w = None
-        if ctx.needs_input_grad[1]:
-            gwf = ops.conv_gemm_dw(gl, xu, K) if ctx.direct else ops.gemm_tn(gl, xu)
-            grad_w = gwf.view(E, K, H).permute(0, 2, 1).contiguous()
+        x, wt, logits, idx = ctx.saved_tensors
+        B, S, H, E, K, k = ctx.shape
+        dev = x.device
+        gw = grad_weights.contiguous().float()
+        grad_x = torch.empty(B, S, H, dtype=torch.bfloat16, device=dev) if ctx.needs_input_grad[0] else None
+        grad_w = torch.empty(E, H, K, dtype=torch.bfloat16, device=dev) if ctx.needs_input_grad[1] else None
+        lib = L.lib()
+        ws = L.workspace(lib.b200moe_conv_router_bwd_ws_bytes(B, S, H, E, K), dev)
+        L.check(lib.b200moe_conv_router_backward(x.data_ptr(), wt.data_ptr(), logits.data_ptr(), idx.data_ptr(), gw.data_ptr(),
+                                                 B, S, H, E, K, k, ctx.norm, ctx.scale, ws.data_ptr(), L.ptr(grad_x),
+                                                 L.ptr(grad_w), L.status_word(dev).data_ptr(), L.stream_of(x)))
         return grad_x, grad_w, None, None, None, None, None
 
 
