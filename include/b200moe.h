@@ -297,7 +297,14 @@ int b200moe_mxfp8_expert_gemm(int epilogue, const void* Aq, const void* Asf, con
                               const void* Bsf, const int32_t* tile_expert, const int32_t* poffs,
                               int64_t rows_cap, int E, int64_t N, int64_t K, int64_t I, void* D, void* aux,
                               void* q_out, void* q_sf, int32_t* status, b200moe_stream_t stream);
-/* Gather fused with the row quantiser: x_s[r] = x[row_slot[r]/k] (bf16, zero pad rows) plus its codes and
+/* The forward's two products when no backward follows.  epilogue 1 (SwiGLU): only the quantised `inter` (q_out, q_sf) is
+ * written, D must be NULL; epilogue 0: D in bf16.  Rows past an expert's counts[e] live rows are not written where they
+ * fill whole blocks of 32. */
+int b200moe_mxfp8_expert_forward(int epilogue, const void* Aq, const void* Asf, const void* Bq, const void* Bsf,
+                                 const int32_t* tile_expert, const int32_t* poffs, const int32_t* counts, int64_t rows_cap,
+                                 int E, int64_t N, int64_t K, int64_t I, void* D, void* q_out, void* q_sf, int32_t* status,
+                                 b200moe_stream_t stream);
+/* Gather fused with the row quantiser: x_s (nullable)[r] = x[row_slot[r]/k] (bf16, zero pad rows) plus its codes and
  * scales (H % 32 == 0); replaces b200moe_gather_rows + b200moe_mxfp8_quant_rows. */
 int b200moe_mxfp8_gather_quant(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,
                                int64_t rows_cap, void* x_s, void* q, void* sf, b200moe_stream_t stream);

@@ -1,0 +1,26 @@
+"""GPU: the MXFP8 forward without a backward (quantising SwiGLU epilogue, no pad rows) against the training forward."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one token, experts without rows, 32-row blocks with and without live rows, more than one row tile an expert; d_model 128 takes
+# the single-CTA kernel for the down product
+@pytest.mark.parametrize("T,H,I,E,k", [(1, 128, 128, 8, 1), (33, 256, 384, 16, 2), (64, 512, 256, 8, 2), (2000, 256, 128, 8, 2)])
+def test_mxfp8_forward_without_gradient_equals_the_training_forward(pkg, T, H, I, E, k):
+    torch.manual_seed(T)
+    layer = pkg.MoELayer(H, I, E, top_k=k, precision="mxfp8").to(DEV).to(torch.bfloat16)
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    torch.empty(64 << 20, dtype=torch.uint8, device=DEV).fill_(255)      # pad rows that nobody writes hold NaN codes and scales
+    with torch.no_grad():
+        quiet = layer(x)
+    trained = layer(x)          # quantises the weights both ways after the row-wise copies were kept
+    with torch.no_grad():
+        again = layer(x)
+    pkg.check_status()
+    assert torch.isfinite(quiet).all()
+    assert torch.equal(quiet, trained.detach()) and torch.equal(again, quiet)
+    trained.float().sum().backward()
+    assert torch.isfinite(layer.gate_up_proj.grad).all()

@@ -75,6 +75,7 @@ _SIGNATURES = {
     "b200moe_mxfp8_gemm_nt": (c_int, [c_void_p] * 5 + [c_int64] * 3 + [c_void_p, c_void_p]),
     "b200moe_mxfp8_expert_gemm": (c_int, [c_int] + [c_void_p] * 6 + [c_int64, c_int, c_int64, c_int64, c_int64] +
                                   [c_void_p] * 6),
+    "b200moe_mxfp8_expert_forward": (c_int, [c_int] + [c_void_p] * 7 + [c_int64, c_int, c_int64, c_int64, c_int64] + [c_void_p] * 5),
     "b200moe_mxfp8_gather_quant_both": (c_int, [c_void_p] * 3 + [c_int, c_int64, c_int64] + [c_void_p] * 5),
     "b200moe_mxfp8_gather_quant": (c_int, [c_void_p] * 3 + [c_int, c_int64, c_int64] + [c_void_p] * 4),
     "b200moe_mxfp8_expert_wgrad": (c_int, [c_void_p] * 6 + [c_int64, c_int, c_int64, c_int64] + [c_void_p] * 3),

@@ -37,6 +37,12 @@ struct Fp8Params {
   // next GEMM's A operand): SwiGLU -> inter (I bytes per row), GLU backward -> grad_gate_up (2I per row)
   uint8_t* q_out;
   uint8_t* q_sf;
+  // optional (pair kernel, store and SwiGLU epilogues): live rows of each expert, for a forward that no backward follows.
+  // An epilogue warp whose 32 rows are all padding gives the accumulator back unread and stores nothing; with p.D ==
+  // nullptr the SwiGLU epilogue writes only the quantised `inter`, not gate_up and inter in bf16.  64 tokens of H 4096, 8
+  // experts of d_ff 14336 (16 rows an expert in tiles of 256): 175 MB of stores and a 26 us quantiser pass less, gate/up
+  // 236 -> 201 us, down 114 -> 102 us.
+  const int* live;
 };
 
 // shared-memory descriptor of a 32 x 16-byte scale atom: no swizzle, 8-row groups 128 bytes apart
@@ -244,9 +250,11 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 const float s1 = __fdividef(1.0f, 1.0f + __expf(-gf.y));
                 oh[h] = pack_bf16x2(gf.x * s0 * uf.x, gf.y * s1 * uf.y);
               }
-              *reinterpret_cast<uint4*>(gu + col) = make_uint4(og[0], og[1], og[2], og[3]);
-              *reinterpret_cast<uint4*>(gu + I + col) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
-              *reinterpret_cast<uint4*>(it_out + col) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+              if (p.D != nullptr) {
+                *reinterpret_cast<uint4*>(gu + col) = make_uint4(og[0], og[1], og[2], og[3]);
+                *reinterpret_cast<uint4*>(gu + I + col) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+                *reinterpret_cast<uint4*>(it_out + col) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+              }
 #pragma unroll
               for (int h = 0; h < 4; ++h) hq[4 * v + h] = oh[h];
             }
@@ -546,6 +554,12 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       if (!mbar_wait(bar_tfull, it & 1, abort_flag, ST_WAIT_EPILOGUE)) break;
       __syncwarp();
       tc_fence_after();
+      if (EPI != EPI_GLU_BWD && fp.live != nullptr && row0 >= p.poffs[t.g] + fp.live[t.g]) {   // nothing but pad rows
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty_leader);
+        continue;
+      }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
       const bool have_acc = t.nkb > 0;
       uint8_t* sbuf = bufG;   // this warp's staging box
@@ -606,15 +620,17 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             mx_quant_store32(oh + 16, fp.q_out + row * static_cast<long long>(I) + col0 + 32, fp.q_sf, row,
                              (col0 + 32) >> 5, I >> 7);
           }
-          staging_free(lane);
-          stage_row(sbuf, lane, acc);
-          store_box(&tmD, sbuf, lane, col0, row0, 0);    // gate half of gate_up
-          staging_free(lane);
-          stage_row(sbuf, lane, acc + 32);
-          store_box(&tmD, sbuf, lane, col0, row0, 1);    // up half
-          staging_free(lane);
-          stage_row(sbuf, lane, oh);
-          store_box(&tmD2, sbuf, lane, col0, row0, 0);   // inter
+          if (p.D != nullptr) {
+            staging_free(lane);
+            stage_row(sbuf, lane, acc);
+            store_box(&tmD, sbuf, lane, col0, row0, 0);    // gate half of gate_up
+            staging_free(lane);
+            stage_row(sbuf, lane, acc + 32);
+            store_box(&tmD, sbuf, lane, col0, row0, 1);    // up half
+            staging_free(lane);
+            stage_row(sbuf, lane, oh);
+            store_box(&tmD2, sbuf, lane, col0, row0, 0);   // inter
+          }
         }
       } else {   // EPI_GLU_BWD: accumulator = grad_inter columns [n0, n0+256), this warp 128 of them
         const int I = p.I;
@@ -784,7 +800,9 @@ static int launch_any(const void* Aq, long long a_rows, const void* Bq, long lon
     const long long groups = (g.sched == SCHED_GROUPED_K) ? g.num_groups : 1;
     rc = make_map(&tmD, g.D, g.N, rows, groups, g.ldd, g.sched == SCHED_GROUPED_K ? g.d_group_stride : rows * g.ldd, 64, 32);
   } else {
-    if (EPI == EPI_SWIGLU) {
+    if (EPI == EPI_SWIGLU && g.D == nullptr) {
+      tmD = tmA;                                                                     // quantised output only
+    } else if (EPI == EPI_SWIGLU) {
       rc = make_map(&tmD, g.D, g.I, a_rows, 2, 2LL * g.I, g.I, 64, 32);          // gate and up halves of gate_up
       if (rc == 0) rc = make_map(&tmD2, g.aux, g.I, a_rows, 1, g.I, a_rows * g.I, 64, 32);
     } else {   // GLU backward: boxes {32 columns, 32 rows}, 64-byte swizzle, for the in-place epilogue
@@ -803,6 +821,40 @@ using namespace b200moe;
 
 #define CHECK_K128(v) \
   B200_CHECK_ARG((v) > 0 && (v) % 128 == 0, B200MOE_E_BAD_SHAPE, #v " = %lld must be a positive multiple of 128", (long long)(v))
+
+static int mxfp8_grouped(int epilogue, const void* Aq, const void* Asf, const void* Bq, const void* Bsf,
+                         const int32_t* tile_expert, const int32_t* poffs, const int32_t* live, int64_t rows_cap, int E, int64_t N,
+                         int64_t K, int64_t I, void* D, void* aux, void* q_out, void* q_sf, int32_t* status,
+                         b200moe_stream_t stream) {
+  B200_CHECK_ARG(Aq && Asf && Bq && Bsf && (D || q_out) && tile_expert && poffs, B200MOE_E_NULL, "mxfp8_expert_gemm: null pointer");
+  B200_CHECK_ARG((q_out == nullptr) == (q_sf == nullptr), B200MOE_E_NULL, "mxfp8_expert_gemm: q_out and q_sf go together");
+  B200_CHECK_ARG(q_out == nullptr || (epilogue != EPI_STORE && I % 128 == 0 && aligned16(q_out)), B200MOE_E_BAD_SHAPE,
+                 "mxfp8_expert_gemm: quantised output needs the SwiGLU / GLU-backward epilogue and I %% 128 == 0");
+  CHECK_K128(K); CHECK_K128(N); CHECK_I32(rows_cap);
+  B200_CHECK_ARG(rows_cap % B200MOE_TILE_M == 0, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: rows_cap %% %d != 0", B200MOE_TILE_M);
+  B200_CHECK_ARG(E >= 1 && E * N < (1LL << 31), B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: E = %d", E);
+  Fp8Params fp{};
+  fp.g.sched = SCHED_GROUPED_M; fp.g.N = (int)N; fp.g.K = (int)K; fp.g.num_groups = E;
+  fp.g.tile_expert = tile_expert; fp.g.poffs = poffs; fp.g.D = D; fp.g.ldd = N; fp.g.aux = aux; fp.g.I = (int)I;
+  fp.g.status = status;
+  fp.sfa = (const uint8_t*)Asf; fp.sfb = (const uint8_t*)Bsf; fp.sfa_kc = fp.sfb_kc = (int)(K / 128);
+  fp.b_rows_per_group = (int)N;
+  fp.live = live;
+  fp.q_out = (uint8_t*)q_out; fp.q_sf = (uint8_t*)q_sf;
+  switch (epilogue) {
+    case EPI_STORE: return launch_any<EPI_STORE>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
+    case EPI_SWIGLU:
+      B200_CHECK_ARG(N == 2 * I && I % 64 == 0, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: SwiGLU needs N = 2I, I %% 64 == 0");
+      return launch_any<EPI_SWIGLU>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
+    case EPI_GLU_BWD:
+      B200_CHECK_ARG(aux && N == I, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: GLU backward needs N = I");
+      return launch_any<EPI_GLU_BWD>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
+    default:
+      set_error("mxfp8_expert_gemm: unknown epilogue %d", epilogue);
+      return B200MOE_E_UNSUPPORTED;
+  }
+}
+
 
 extern "C" {
 
@@ -825,32 +877,21 @@ int b200moe_mxfp8_expert_gemm(int epilogue, const void* Aq, const void* Asf, con
                               const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
                               int64_t K, int64_t I, void* D, void* aux, void* q_out, void* q_sf, int32_t* status,
                               b200moe_stream_t stream) {
-  B200_CHECK_ARG(Aq && Asf && Bq && Bsf && D && tile_expert && poffs, B200MOE_E_NULL, "mxfp8_expert_gemm: null pointer");
-  B200_CHECK_ARG((q_out == nullptr) == (q_sf == nullptr), B200MOE_E_NULL, "mxfp8_expert_gemm: q_out and q_sf go together");
-  B200_CHECK_ARG(q_out == nullptr || (epilogue != EPI_STORE && I % 128 == 0 && aligned16(q_out)), B200MOE_E_BAD_SHAPE,
-                 "mxfp8_expert_gemm: quantised output needs the SwiGLU / GLU-backward epilogue and I %% 128 == 0");
-  CHECK_K128(K); CHECK_K128(N); CHECK_I32(rows_cap);
-  B200_CHECK_ARG(rows_cap % B200MOE_TILE_M == 0, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: rows_cap %% %d != 0", B200MOE_TILE_M);
-  B200_CHECK_ARG(E >= 1 && E * N < (1LL << 31), B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: E = %d", E);
-  Fp8Params fp{};
-  fp.g.sched = SCHED_GROUPED_M; fp.g.N = (int)N; fp.g.K = (int)K; fp.g.num_groups = E;
-  fp.g.tile_expert = tile_expert; fp.g.poffs = poffs; fp.g.D = D; fp.g.ldd = N; fp.g.aux = aux; fp.g.I = (int)I;
-  fp.g.status = status;
-  fp.sfa = (const uint8_t*)Asf; fp.sfb = (const uint8_t*)Bsf; fp.sfa_kc = fp.sfb_kc = (int)(K / 128);
-  fp.b_rows_per_group = (int)N;
-  fp.q_out = (uint8_t*)q_out; fp.q_sf = (uint8_t*)q_sf;
-  switch (epilogue) {
-    case EPI_STORE: return launch_any<EPI_STORE>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
-    case EPI_SWIGLU:
-      B200_CHECK_ARG(aux && N == 2 * I && I % 64 == 0, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: SwiGLU needs N = 2I, I %% 64 == 0");
-      return launch_any<EPI_SWIGLU>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
-    case EPI_GLU_BWD:
-      B200_CHECK_ARG(aux && N == I, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: GLU backward needs N = I");
-      return launch_any<EPI_GLU_BWD>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
-    default:
-      set_error("mxfp8_expert_gemm: unknown epilogue %d", epilogue);
-      return B200MOE_E_UNSUPPORTED;
-  }
+  B200_CHECK_ARG(D, B200MOE_E_NULL, "mxfp8_expert_gemm: null pointer");
+  B200_CHECK_ARG(epilogue != EPI_SWIGLU || aux, B200MOE_E_BAD_SHAPE, "mxfp8_expert_gemm: SwiGLU needs N = 2I, I %% 64 == 0");
+  return mxfp8_grouped(epilogue, Aq, Asf, Bq, Bsf, tile_expert, poffs, nullptr, rows_cap, E, N, K, I, D, aux, q_out, q_sf,
+                       status, stream);
+}
+
+int b200moe_mxfp8_expert_forward(int epilogue, const void* Aq, const void* Asf, const void* Bq, const void* Bsf,
+                                 const int32_t* tile_expert, const int32_t* poffs, const int32_t* counts, int64_t rows_cap,
+                                 int E, int64_t N, int64_t K, int64_t I, void* D, void* q_out, void* q_sf, int32_t* status,
+                                 b200moe_stream_t stream) {
+  B200_CHECK_ARG(counts, B200MOE_E_NULL, "mxfp8_expert_forward: null pointer");
+  B200_CHECK_ARG((epilogue == EPI_STORE && D && !q_out) || (epilogue == EPI_SWIGLU && !D && q_out), B200MOE_E_UNSUPPORTED,
+                 "mxfp8_expert_forward: epilogue 0 stores D, epilogue 1 the quantised result");
+  return mxfp8_grouped(epilogue, Aq, Asf, Bq, Bsf, tile_expert, poffs, counts, rows_cap, E, N, K, I, D, nullptr, q_out, q_sf,
+                       status, stream);
 }
 
 /* grouped-K (wgrad): out[e] (Na,Nb) = At[:, rows of e] * Bt[:, rows of e]^T with At (Na, rows_cap) and

@@ -188,7 +188,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R,
   }
 }
 
-// Gather fused with the row quantiser: x_s[r] = x[row_slot[r] / k] (bf16 copy kept for the backward)
+// Gather fused with the row quantiser: x_s[r] = x[row_slot[r] / k] (bf16 copy for a caller that wants it, nullable)
 // and its e4m3 codes + scales; pad rows become zeros with scale byte 0.  One thread per 32-element block.
 __global__ void __launch_bounds__(256)
 gather_quant_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_slot,
@@ -211,9 +211,11 @@ gather_quant_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = make_uint4(0u, 0u, 0u, 0u);
     }
-    uint4* dst = reinterpret_cast<uint4*>(x_s + r * C + b * 32);
+    if (x_s != nullptr) {
+      uint4* dst = reinterpret_cast<uint4*>(x_s + r * C + b * 32);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dst[j] = v[j];
+      for (int j = 0; j < 4; ++j) dst[j] = v[j];
+    }
     mx_quant_store32(reinterpret_cast<const uint32_t*>(v), q + r * C + b * 32, sf, r, b, k_chunks);
   }
 }
@@ -252,7 +254,7 @@ int b200moe_mxfp8_quant_rows(const void* x, int64_t R, int64_t C, int64_t interl
 
 int b200moe_mxfp8_gather_quant(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,
                                int64_t rows_cap, void* x_s, void* q, void* sf, b200moe_stream_t stream) {
-  B200_CHECK_ARG(x && row_slot && total_rows && x_s && q && sf, B200MOE_E_NULL, "mxfp8_gather_quant: null pointer");
+  B200_CHECK_ARG(x && row_slot && total_rows && q && sf, B200MOE_E_NULL, "mxfp8_gather_quant: null pointer");
   B200_CHECK_ARG(H > 0 && H % 32 == 0 && k >= 1, B200MOE_E_BAD_SHAPE, "mxfp8_gather_quant: H = %lld must be a multiple of 32",
                  (long long)H);
   B200_CHECK_ARG(aligned16(x) && aligned16(x_s) && aligned16(q), B200MOE_E_ALIGN, "mxfp8_gather_quant: pointers must be aligned");

@@ -49,9 +49,21 @@ def _quantised_weights(stack, rows_fn, both_fn, both):
     return res
 
 
+def _gate_up_copies(stack, both):
+    E, twoI, H = stack.shape
+    return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * twoI, H), interleave_I=twoI // 2),
+                              lambda: ops.mxfp8_quant_both(stack, interleave_I=twoI // 2), both)
+
+
+def _down_copies(stack, both):
+    E, H, I = stack.shape
+    return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * H, I)), lambda: ops.mxfp8_quant_both(stack), both)
+
+
 class _MoEMxfp8(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes):
+    def forward(ctx, hidden, idx, wt, gate_up_proj, down_proj, act_codes, keep=True):
+        """keep=False: no backward will follow (the caller knows the grad mode, which is off in here)."""
         hidden, gate_up_proj, down_proj = _amp_cast(hidden, gate_up_proj, down_proj)
         for name, t in (("hidden", hidden), ("gate_up_proj", gate_up_proj), ("down_proj", down_proj)):
             L.require_cuda_bf16(name, t)
@@ -66,8 +78,14 @@ class _MoEMxfp8(torch.autograd.Function):
         w32 = wt.detach().float().contiguous()
         dev = hidden.device
 
-        need_x, _, _, need_gu, need_dn, _ = ctx.needs_input_grad
+        need_x, _, _, need_gu, need_dn = ctx.needs_input_grad[:5]
         perm = ops.permute_build(idx, E)
+        if not keep:   # the SwiGLU epilogue is the quantiser; no transposed activations, no gate_up, no pad rows
+            _, xq, xsf = ops.mxfp8_gather_quant(hidden, perm, keep_rows=False)
+            wq, wsf = _gate_up_copies(gate_up_proj, need_x)[:2]
+            iq, isf = ops.mxfp8_expert_forward(ops.EPI_SWIGLU, xq, xsf, wq, wsf, perm, twoI, H, I)
+            dq, dsf = _down_copies(down_proj, need_x or need_gu)[:2]
+            return ops.combine(ops.mxfp8_expert_forward(ops.EPI_STORE, iq, isf, dq, dsf, perm, H, I, I), w32, perm)
         # the gather is the quantising producer; when the gate/up weight gradient is wanted it also writes the
         # copy quantised along the token rows, and the gathered bf16 rows are never materialised
         xt = xtsf = None
@@ -78,8 +96,7 @@ class _MoEMxfp8(torch.autograd.Function):
         # tensors that the backward needs quantised along their other dimension are quantised both ways in
         # one pass over DRAM, and the transposed copy is what the backward keeps
         wgt = wgtsf = wtq = wtsf = it = itsf = None
-        res = _quantised_weights(gate_up_proj, lambda: ops.mxfp8_quant_rows(gate_up_proj.view(E * twoI, H), interleave_I=I),
-                                 lambda: ops.mxfp8_quant_both(gate_up_proj, interleave_I=I), need_x)   # + (E, H, 2I)
+        res = _gate_up_copies(gate_up_proj, need_x)   # + (E, H, 2I)
         if need_x:
             wq, wsf, wgt, wgtsf = res
         else:
@@ -95,8 +112,7 @@ class _MoEMxfp8(torch.autograd.Function):
             iq, isf, it, itsf = ops.mxfp8_quant_both(inter)                                 # + (I, rows)
         else:
             iq, isf = ops.mxfp8_quant_rows(inter)
-        res = _quantised_weights(down_proj, lambda: ops.mxfp8_quant_rows(down_proj.view(E * H, I)),
-                                 lambda: ops.mxfp8_quant_both(down_proj), need_x or need_gu)           # + (E, I, H)
+        res = _down_copies(down_proj, need_x or need_gu)   # + (E, I, H)
         if need_x or need_gu:
             dq, dsf, wtq, wtsf = res
         else:
@@ -120,7 +136,7 @@ class _MoEMxfp8(torch.autograd.Function):
         E, H, I = ctx.dims
         twoI = 2 * I
         dev = eo.device
-        need_x, _, need_w, need_gu, need_dn, _ = ctx.needs_input_grad
+        need_x, _, need_w, need_gu, need_dn = ctx.needs_input_grad[:5]
         grad_out = grad_out.contiguous().to(torch.bfloat16)
         grad_eo, grad_w = ops.combine_bwd(grad_out, eo, w32, perm)
         grad_hidden = grad_gate_up_proj = grad_down_proj = None
@@ -154,7 +170,8 @@ class _MoEMxfp8(torch.autograd.Function):
         if need_dn:
             grad_down_proj = ops.mxfp8_expert_wgrad(gt, gtsf, it, itsf, perm)
         grad_wt = grad_w.to(ctx.wt_dtype) if need_w else None
-        return grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None
+        grads = (grad_hidden, None, grad_wt, grad_gate_up_proj, grad_down_proj, None, None)
+        return grads[:len(ctx.needs_input_grad)]
 
 
 def moe_mxfp8(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, act_params=None):
@@ -164,4 +181,5 @@ def moe_mxfp8(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act
         raise ValueError("the MXFP8 path is built for pure SiLU-GLU stacks (act code 0) only")
     if hidden.shape[0] == 0:
         return _empty_result(hidden, top_k_weights, gate_up_proj, down_proj)
-    return _MoEMxfp8.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes)
+    keep = torch.is_grad_enabled() and any(t.requires_grad for t in (hidden, top_k_weights, gate_up_proj, down_proj))
+    return _MoEMxfp8.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, keep)

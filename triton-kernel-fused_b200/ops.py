@@ -437,12 +437,28 @@ def mxfp8_gather_quant_both(x, perm: Permutation):
     return q, sf, qt, sft
 
 
+@_op("mxfp8_expert_forward", 1)
+def mxfp8_expert_forward(epilogue, aq, asf, bq, bsf, perm: Permutation, N, K, I):
+    """The forward's products when no backward follows: EPI_SWIGLU -> (codes, scale atoms) of `inter`, EPI_STORE -> bf16 rows."""
+    dev = aq.device
+    d = q = qsf = None
+    if epilogue == EPI_SWIGLU:
+        q, qsf = torch.empty(perm.cap, I, dtype=torch.uint8, device=dev), _sf_empty(perm.cap, I, dev)
+    else:
+        d = torch.empty(perm.cap, N, dtype=torch.bfloat16, device=dev)
+    L.check(L.lib().b200moe_mxfp8_expert_forward(int(epilogue), L.ptr(aq), L.ptr(asf), L.ptr(bq), L.ptr(bsf),
+                                                 L.ptr(perm.tile_expert), L.ptr(perm.poffs), L.ptr(perm.counts), perm.cap,
+                                                 perm.E, N, K, I, L.ptr(d), L.ptr(q), L.ptr(qsf),
+                                                 L.ptr(L.status_word(dev)), L.stream_of(aq)))
+    return (q, qsf) if d is None else d
+
+
 @_op("mxfp8_gather_quant", 1)
-def mxfp8_gather_quant(x, perm: Permutation):
-    """Gather into the padded layout and quantise along the rows in one pass: (x_s bf16, codes, scale atoms)."""
+def mxfp8_gather_quant(x, perm: Permutation, keep_rows=True):
+    """Gather into the padded layout and quantise along the rows in one pass: (x_s bf16 or None, codes, scale atoms)."""
     L.require_cuda_bf16("hidden", x)
     H = x.shape[1]
-    x_s = torch.empty(perm.cap, H, dtype=torch.bfloat16, device=x.device)
+    x_s = torch.empty(perm.cap, H, dtype=torch.bfloat16, device=x.device) if keep_rows else None
     q = torch.empty(perm.cap, H, dtype=torch.uint8, device=x.device)
     sf = _sf_empty(perm.cap, H, x.device)
     L.check(L.lib().b200moe_mxfp8_gather_quant(L.ptr(x), L.ptr(perm.row_slot), L.ptr(perm.total_rows), perm.k, H,
