@@ -554,10 +554,10 @@ int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate
                            void* grad_gate_up, void* grad_down, int32_t* status, b200moe_stream_t stream);
 /* All iterations of kernels/sm75/muon.py:83-86 on a padded stack x (E, Rp, wide): per iteration the three products of
  * b200moe_expert_gram, _expert_linear_axpby (symmetric = 2) and _expert_linear_t.  coeffs: HOST array of (a, b, c) per
- * iteration.  x and x_next take turns: the result is in x after an even number of iterations, else in x_next; a, a2:
+ * iteration.  The first rows_live of each segment's Rp rows (less than 256 fewer) are not padding.  x and x_next take turns: the result is in x after an even number of iterations, else in x_next; a, a2:
  * (E, Rp, Rp) work space. */
 int b200moe_newton_schulz(void* x, void* x_next, void* a, void* a2, const int32_t* tile_expert, const int32_t* poffs, int E,
-                          int64_t Rp, int64_t wide, const float* coeffs, int iterations, int32_t* status,
+                          int64_t Rp, int64_t rows_live, int64_t wide, const float* coeffs, int iterations, int32_t* status,
                           b200moe_stream_t stream);
 
 #ifdef __cplusplus

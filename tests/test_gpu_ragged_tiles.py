@@ -52,3 +52,34 @@ def test_grouped_products_at_ragged_widths(pkg, N, rows):
         ref = torch.stack([sa[e == i].float().T @ sb[e == i].float() for i in range(E)])
         assert O.rel_l2(got.float(), ref) < TOL and not got[E - 1].any()
     pkg.check_status()
+
+
+# matrices whose smaller side leaves a padded remainder of 8, 56, 64, 120, 248 rows, or none; wide and tall; one iteration and several
+@pytest.mark.parametrize("E,r,c", [(3, 248, 400), (2, 264, 520), (2, 320, 264), (1, 456, 640), (4, 8, 72), (2, 512, 512)])
+def test_optimizer_iteration_over_the_live_part_equals_the_padded_products(pkg, E, r, c):
+    import ctypes
+    from importlib import import_module
+    muon, ops, lib = import_module(pkg.__name__ + ".muon"), pkg.ops, pkg.lib()
+    small, wide = min(r, c), max(r, c)
+    Rp = -(-small // 256) * 256
+    coeffs = [(3.4445, -4.7750, 2.0315), (2.0, -1.5, 0.5), (2.0, -1.5, 0.5)]
+    X = torch.zeros(E, Rp, wide, dtype=torch.bfloat16, device=DEV)
+    X[:, :small] = (torch.randn(E, small, wide, generator=torch.Generator().manual_seed(r)) / (small * wide) ** 0.5).to(torch.bfloat16)
+    seg = muon._uniform_segments(E, Rp, X.device)
+    full = lambda *s: torch.full(s, float("nan"), dtype=torch.bfloat16, device=DEV)      # noqa: E731
+    for n in (1, 3):
+        ref = X
+        for a, b, cc in coeffs[:n]:
+            A, A2, nxt = full(E * Rp, Rp), full(E * Rp, Rp), full(E * Rp, wide)
+            ops.expert_gram(ref.view(E * Rp, wide), seg, out=A)
+            ops.expert_linear_axpby(A, A.view(E, Rp, Rp), A, cc, b, a, seg, out=A2, symmetric=2)
+            ref = ops.expert_linear_t(A2, ref.view(E, Rp, wide), seg, out=nxt).view(E, Rp, wide)
+        bufs = [X.clone(), full(E, Rp, wide)]
+        A, A2 = full(E * Rp, Rp), full(E * Rp, Rp)
+        flat = [v for abc in coeffs[:n] for v in abc]
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        rc = lib.b200moe_newton_schulz(bufs[0].data_ptr(), bufs[1].data_ptr(), A.data_ptr(), A2.data_ptr(), seg.tile_expert.data_ptr(),
+                                       seg.poffs.data_ptr(), E, Rp, small, wide, (ctypes.c_float * len(flat))(*flat), n,
+                                       status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and int(status.item()) == 0
+        assert torch.equal(bufs[n % 2][:, :small], ref[:, :small])

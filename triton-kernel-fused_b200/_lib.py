@@ -112,7 +112,7 @@ _SIGNATURES = {
     "b200moe_layer_forward": (c_int, [c_void_p] * 6 + [c_int64] * 3 + [c_int] * 3 + [c_float, c_int] + [c_void_p] * 6),
     "b200moe_layer_bwd_ws_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 2),
     "b200moe_layer_backward": (c_int, [c_void_p] * 6 + [c_int64] * 3 + [c_int] * 3 + [c_float] + [c_void_p] * 8),
-    "b200moe_newton_schulz": (c_int, [c_void_p] * 6 + [c_int, c_int64, c_int64, c_void_p, c_int, c_void_p, c_void_p]),
+    "b200moe_newton_schulz": (c_int, [c_void_p] * 6 + [c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_void_p, c_void_p]),
     "b200moe_muon_momentum": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_float, c_int, c_void_p]),
     "b200moe_muon_row_sumsq": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
     "b200moe_muon_prescale_rows": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_float, c_float, c_void_p, c_void_p,

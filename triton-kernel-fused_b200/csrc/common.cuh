@@ -32,6 +32,15 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
                   size_t ws_bytes, int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream);
 
+// gemm.cu: the products of the optimizer's iteration over part of their padded extents
+int expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t K, int mirror,
+                int64_t n_live, void* out, int32_t* status, b200moe_stream_t stream);
+int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha, float beta, float diag, int symmetric,
+                        const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N, int64_t K,
+                        int64_t n_live, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream);
+int expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
+                    int64_t K, int64_t N, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream);
+
 // Tells the observer set by b200moe_set_observer, if any, where an operation of a longer sequence begins and ends
 struct OpScope {
   OpScope(const char* name, int launches);

@@ -434,7 +434,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 // 64 bytes of its row of C that lie under this sub-chunk
                 const int col0 = t.n0 + c + 32 * sub;
                 const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.aux) +
-                                                                  row * p.N + col0);
+                                                                  row * p.ldd + col0);
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                   const uint4 cv = src[v];
@@ -867,6 +867,80 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
 }
 
 
+static int check_grouped(const char* who, const void* a, const void* b, const void* c, const int32_t* tile_expert,
+                         const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I) {
+  B200_CHECK_ARG(a && b && c && poffs, B200MOE_E_NULL, "%s: null pointer", who);
+  (void)tile_expert;
+  B200_CHECK_ARG(E >= 1 && E <= 65535, B200MOE_E_BAD_SHAPE, "%s: E = %d out of range", who, E);
+  B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
+                 "%s: rows_cap = %lld must be a positive multiple of %d", who, (long long)rows_cap, B200MOE_TILE_M);
+  B200_CHECK_ARG(H > 0 && H % 8 == 0 && I > 0 && I % 8 == 0, B200MOE_E_BAD_SHAPE,
+                 "%s: H = %lld and I = %lld must be positive multiples of 8", who, (long long)H, (long long)I);
+  B200_CHECK_ARG(2 * E * I < (1LL << 31) && E * H < (1LL << 31), B200MOE_E_BAD_SHAPE, "%s: weight stack too tall", who);
+  return 0;
+}
+
+// ---- products of equal groups of padded rows (the optimizer's iteration; linear_t also the layer's).  n_live / k_live: columns
+// that are computed and the part of the reduction that is read, multiples of 64 that cover what is not padding (n_live, k_live =
+// the whole extent otherwise).  What lies past them is neither read nor, where a whole 64-column chunk is padding, written.
+int expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t K, int mirror,
+                int64_t n_live, void* out, int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(E >= 1 && rows_cap % E == 0, B200MOE_E_BAD_SHAPE, "expert_gram: %lld rows do not split into %d equal groups",
+                 (long long)rows_cap, E);
+  const int64_t R = rows_cap / E;
+  int rc = check_grouped("expert_gram", x, x, out, tile_expert, poffs, rows_cap, E, R, K);
+  if (rc) return rc;
+  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_gram: null pointer");
+  B200_CHECK_ARG(R % 256 == 0, B200MOE_E_BAD_SHAPE, "expert_gram: %lld rows per group must be a multiple of 256", (long long)R);
+  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_gram: output not aligned");
+  Operand oa{x, 0, rows_cap, K, K, 1, rows_cap * K};
+  Operand ob{x, 0, R, K, K, E, R * K};
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.N = (int)n_live; p.K = (int)K; p.num_groups = E; p.sym_rows = (int)R; p.sym_mirror = mirror ? 1 : 0;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = R; p.status = status;
+  Operand d{out, 0, rows_cap, R, R, 1, rows_cap * R};
+  return dispatch_bn<EPI_STORE_SYM>(256, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+}
+
+int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha, float beta, float diag, int symmetric,
+                        const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N, int64_t K,
+                        int64_t n_live, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_grouped("expert_linear_axpby", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
+  if (rc) return rc;
+  B200_CHECK_ARG(tile_expert && c, B200MOE_E_NULL, "expert_linear_axpby: null pointer");
+  B200_CHECK_ARG(N % 256 == 0, B200MOE_E_BAD_SHAPE, "expert_linear_axpby: N = %lld must be a multiple of 256", (long long)N);
+  B200_CHECK_ARG(aligned16(out) && aligned16(c), B200MOE_E_ALIGN, "expert_linear_axpby: pointers must be 16-byte aligned");
+  Operand oa{a, 0, rows_cap, k_live, K, 1, rows_cap * K};
+  Operand ob{w, 0, N, k_live, K, E, N * K};   // W (E, N, K): rows = output columns
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.N = (int)n_live; p.K = (int)k_live; p.num_groups = E;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
+  p.aux = const_cast<void*>(c); p.ax_alpha = alpha; p.ax_beta = beta; p.ax_diag = diag;
+  if (symmetric) {
+    B200_CHECK_ARG(rows_cap == (int64_t)E * N, B200MOE_E_BAD_SHAPE,
+                   "expert_linear_axpby: a symmetric result needs %d equal groups of N = %lld rows", E, (long long)N);
+    p.sym_rows = (int)N;
+    p.sym_mirror = symmetric > 1 ? 1 : 0;
+  }
+  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
+  return dispatch_bn<EPI_AXPBY>(256, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+}
+
+int expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
+                    int64_t K, int64_t N, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_grouped("expert_linear_t", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
+  if (rc) return rc;
+  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear_t: null pointer");
+  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_linear_t: output not aligned");
+  Operand oa{a, 0, rows_cap, k_live, K, 1, rows_cap * K};
+  Operand ob{w, 1, N, k_live, N, E, K * N};   // W[e] stored (K, N): MN-major
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)k_live; p.num_groups = E;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
+  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
+  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+}
+
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -1027,19 +1101,6 @@ static int check_row_window(const char* who, int64_t rows_cap, int64_t row_lo, i
   return 0;
 }
 
-static int check_grouped(const char* who, const void* a, const void* b, const void* c, const int32_t* tile_expert,
-                         const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I) {
-  B200_CHECK_ARG(a && b && c && poffs, B200MOE_E_NULL, "%s: null pointer", who);
-  (void)tile_expert;
-  B200_CHECK_ARG(E >= 1 && E <= 65535, B200MOE_E_BAD_SHAPE, "%s: E = %d out of range", who, E);
-  B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
-                 "%s: rows_cap = %lld must be a positive multiple of %d", who, (long long)rows_cap, B200MOE_TILE_M);
-  B200_CHECK_ARG(H > 0 && H % 8 == 0 && I > 0 && I % 8 == 0, B200MOE_E_BAD_SHAPE,
-                 "%s: H = %lld and I = %lld must be positive multiples of 8", who, (long long)H, (long long)I);
-  B200_CHECK_ARG(2 * E * I < (1LL << 31) && E * H < (1LL << 31), B200MOE_E_BAD_SHAPE, "%s: weight stack too tall", who);
-  return 0;
-}
-
 int b200moe_expert_gate_up_swiglu(const void* x_s, const void* gate_up_proj, const int32_t* tile_expert,
                                   const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
                                   void* gate_up, void* inter, int32_t* status, b200moe_stream_t stream) {
@@ -1092,61 +1153,19 @@ int b200moe_expert_linear(const void* a, const void* w, const int32_t* tile_expe
 
 int b200moe_expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
                         int64_t K, int mirror, void* out, int32_t* status, b200moe_stream_t stream) {
-  B200_CHECK_ARG(E >= 1 && rows_cap % E == 0, B200MOE_E_BAD_SHAPE, "expert_gram: %lld rows do not split into %d equal groups",
-                 (long long)rows_cap, E);
-  const int64_t R = rows_cap / E;
-  int rc = check_grouped("expert_gram", x, x, out, tile_expert, poffs, rows_cap, E, R, K);
-  if (rc) return rc;
-  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_gram: null pointer");
-  B200_CHECK_ARG(R % 256 == 0, B200MOE_E_BAD_SHAPE, "expert_gram: %lld rows per group must be a multiple of 256", (long long)R);
-  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_gram: output not aligned");
-  Operand oa{x, 0, rows_cap, K, K, 1, rows_cap * K};
-  Operand ob{x, 0, R, K, K, E, R * K};
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.N = (int)R; p.K = (int)K; p.num_groups = E; p.sym_rows = (int)R; p.sym_mirror = mirror ? 1 : 0;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = R; p.status = status;
-  Operand d{out, 0, rows_cap, R, R, 1, rows_cap * R};
-  return dispatch_bn<EPI_STORE_SYM>(256, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return expert_gram(x, tile_expert, poffs, rows_cap, E, K, mirror, E >= 1 ? rows_cap / E : 0, out, status, stream);
 }
 
 int b200moe_expert_linear_axpby(const void* a, const void* w, const void* c, float alpha, float beta, float diag,
                                 int symmetric, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
                                 int64_t N, int64_t K, void* out, int32_t* status, b200moe_stream_t stream) {
-  int rc = check_grouped("expert_linear_axpby", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
-  if (rc) return rc;
-  B200_CHECK_ARG(tile_expert && c, B200MOE_E_NULL, "expert_linear_axpby: null pointer");
-  B200_CHECK_ARG(N % 256 == 0, B200MOE_E_BAD_SHAPE, "expert_linear_axpby: N = %lld must be a multiple of 256", (long long)N);
-  B200_CHECK_ARG(aligned16(out) && aligned16(c), B200MOE_E_ALIGN, "expert_linear_axpby: pointers must be 16-byte aligned");
-  Operand oa{a, 0, rows_cap, K, K, 1, rows_cap * K};
-  Operand ob{w, 0, N, K, K, E, N * K};   // W (E, N, K): rows = output columns
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.N = (int)N; p.K = (int)K; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
-  p.aux = const_cast<void*>(c); p.ax_alpha = alpha; p.ax_beta = beta; p.ax_diag = diag;
-  if (symmetric) {
-    B200_CHECK_ARG(rows_cap == (int64_t)E * N, B200MOE_E_BAD_SHAPE,
-                   "expert_linear_axpby: a symmetric result needs %d equal groups of N = %lld rows", E, (long long)N);
-    p.sym_rows = (int)N;
-    p.sym_mirror = symmetric > 1 ? 1 : 0;
-  }
-  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
-  return dispatch_bn<EPI_AXPBY>(256, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return expert_linear_axpby(a, w, c, alpha, beta, diag, symmetric, tile_expert, poffs, rows_cap, E, N, K, N, K, out, status, stream);
 }
 
 int b200moe_expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
                             int64_t rows_cap, int E, int64_t K, int64_t N, void* out, int32_t* status,
                             b200moe_stream_t stream) {
-  int rc = check_grouped("expert_linear_t", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
-  if (rc) return rc;
-  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear_t: null pointer");
-  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_linear_t: output not aligned");
-  Operand oa{a, 0, rows_cap, K, K, 1, rows_cap * K};
-  Operand ob{w, 1, N, K, N, E, K * N};   // W[e] stored (K, N): MN-major
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)K; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
-  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
-  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return expert_linear_t(a, w, tile_expert, poffs, rows_cap, E, K, N, K, out, status, stream);
 }
 
 int b200moe_expert_linear_push(const void* a, const void* w, int w_kn, const int32_t* tile_expert, const int32_t* poffs,

@@ -132,10 +132,10 @@ def _orthogonalise_packed(u, E, r, c, coeffs, eps, rowss=None):
     if rowss is None:
         rowss = _row_sumsq(u, E * r, c)
     X = _normalise_pack(u, rowss, E, r, c, Rp, tall, eps)
-    return _iterate(X, E, Rp, wide, coeffs), Rp, tall
+    return _iterate(X, E, Rp, small, wide, coeffs), Rp, tall
 
 
-def _iterate(X, E, Rp, wide, coeffs):
+def _iterate(X, E, Rp, small, wide, coeffs):
     """X <- a X + (b A + c A A) X with A = X X^T (kernels/sm75/muon.py:83-86), evaluated as ((b A + c A A) + a I) X:
     three grouped GEMMs per iteration (two of them over the upper triangle only), X ping-pongs between two buffers."""
     seg = _uniform_segments(E, Rp, X.device)
@@ -148,7 +148,7 @@ def _iterate(X, E, Rp, wide, coeffs):
     # X = B X goes to the other of two buffers.  All iterations are queued by one native call (csrc/block.cu).
     flat = [float(v) for a, b, c in coeffs for v in (a, b, c)]
     L.check(L.lib().b200moe_newton_schulz(X.data_ptr(), Xn.data_ptr(), A.data_ptr(), A2.data_ptr(), L.ptr(seg.tile_expert),
-                                          L.ptr(seg.poffs), E, Rp, wide, (ctypes.c_float * len(flat))(*flat), len(flat) // 3,
+                                          L.ptr(seg.poffs), E, Rp, small, wide, (ctypes.c_float * len(flat))(*flat), len(flat) // 3,
                                           L.ptr(L.status_word(X.device)), L.stream_of(X)))
     return Xn if (len(flat) // 3) % 2 else X
 
