@@ -112,3 +112,35 @@ def test_small_router_against_gemm_and_top_k(pkg, T, H, E, k):
     for a, b in zip(got, (logits, *pkg.ops.router_topk_fwd(logits, bias, k, True, 1.5))):
         assert torch.equal(a, b)
     assert O.rel_l2(logits.cpu().double(), x.cpu().double() @ w.cpu().double().T) < TOL
+
+
+# row widths on both sides of every thread-group limit (32, 64, 128, 256 vectors), one vector, more than a CTA; one pick to 32
+@pytest.mark.parametrize("H,k", [(8, 1), (248, 5), (256, 8), (264, 3), (512, 2), (520, 4), (1024, 6), (1032, 32), (2048, 6), (2056, 7)])
+def test_copying_kernels_at_the_widths_of_a_row(pkg, H, k):
+    T, E = 301, 40
+    g = torch.Generator().manual_seed(H + k)
+    idx = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)])
+    x, go, add = (torch.randn(T, H, generator=g).to(torch.bfloat16) for _ in range(3))
+    w = torch.rand(T, k, generator=g)
+    ops = pkg.ops
+    perm = ops.permute_build(idx.to(DEV), E)
+    total = int(perm.poffs[-1])
+    xs = ops.gather_rows(x.to(DEV), perm)
+    rs = perm.row_slot[:total].cpu().long()
+    live = rs >= 0
+    assert torch.equal(xs[:total].cpu()[live], x[rs[live] // k]) and not xs[:total].cpu()[~live].any()
+    eo = torch.randn(perm.cap, H, generator=g).to(torch.bfloat16)
+    picked = eo[perm.slot_row.cpu().long()].double().view(T, k, H)
+    out = ops.combine(eo.to(DEV), w.to(DEV), perm)
+    assert O.rel_l2(out.cpu().double(), (picked * w.double().unsqueeze(2)).sum(1)) < TOL
+    both = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+    rows, ad = eo.to(DEV), add.to(DEV)
+    assert pkg.lib().b200moe_combine_add(rows.data_ptr(), None, perm.slot_row.data_ptr(), ad.data_ptr(), T, k, H, both.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream) == 0
+    assert O.rel_l2(both.cpu().double(), picked.sum(1) + add.double()) < TOL
+    geo, gw = ops.combine_bwd(go.to(DEV), rows, w.to(DEV), perm)
+    want = go[rs[live] // k].float() * w.flatten()[rs[live]].unsqueeze(1)
+    assert torch.equal(geo[:total].cpu()[live], want.to(torch.bfloat16)) and not geo[:total].cpu()[~live].any()
+    # H signed fp32 terms: within 1e-5 of the sum of their sizes
+    terms = go.double().unsqueeze(1) * picked
+    assert ((gw.cpu().double() - terms.sum(2)).abs() <= 1e-5 * terms.abs().sum(2)).all()

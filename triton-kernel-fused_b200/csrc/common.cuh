@@ -4,6 +4,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <type_traits>
+
 #include "../../include/b200moe.h"
 
 namespace b200moe {
@@ -62,6 +64,15 @@ struct OpScope {
     cudaError_t e__ = (call);                                             \
     if (e__ != cudaSuccess) return ::b200moe::cuda_fail(e__, #call);      \
   } while (0)
+
+// f(TPR): threads of a 256-thread CTA that share a row of nvec 16-byte vectors in the copying kernels, at least 32
+template <class F>
+inline void by_row_threads(int nvec, F f) {
+  if (nvec <= 32) f(std::integral_constant<int, 32>());
+  else if (nvec <= 64) f(std::integral_constant<int, 64>());
+  else if (nvec <= 128) f(std::integral_constant<int, 128>());
+  else f(std::integral_constant<int, 256>());
+}
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
