@@ -427,16 +427,19 @@ expert_row_sums_kernel(const float* __restrict__ row_da, const float* __restrict
 }
 
 // rows of the special experts (those after the first `first_special` experts):
-// dst[r] = src[r] for Identity (code 3), 0 otherwise (Zero, code 4)
+// dst[r] = src[r] for Identity (code 3), 0 otherwise (Zero, code 4); TPR threads share a row
+template <int TPR>
 __global__ void __launch_bounds__(256)
 special_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ tile_expert, const int* __restrict__ codes,
                     const int* __restrict__ poffs, int first_special, int num_experts, int vec_per_row,
                     uint4* __restrict__ dst) {
+  constexpr int G = 256 / TPR;
   const int r0 = poffs[first_special], r1 = poffs[num_experts];
-  for (long long r = r0 + blockIdx.x; r < r1; r += gridDim.x) {
-    const int code = codes[tile_expert[r / B200MOE_TILE_M]];
-    for (int c = threadIdx.x; c < vec_per_row; c += blockDim.x)
-      dst[r * vec_per_row + c] = (code == 3) ? src[r * vec_per_row + c] : make_uint4(0u, 0u, 0u, 0u);
+  for (long long r = r0 + static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; r < r1;
+       r += static_cast<long long>(gridDim.x) * G) {
+    const bool copy = codes[tile_expert[r / B200MOE_TILE_M]] == 3;
+    for (int c = threadIdx.x % TPR; c < vec_per_row; c += TPR)
+      dst[r * vec_per_row + c] = copy ? src[r * vec_per_row + c] : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -535,9 +538,11 @@ int b200moe_special_rows(const void* src, const int32_t* tile_expert, const int3
                  "special_rows: H = %lld, first_special = %d, num_experts = %d", (long long)H, first_special, num_experts);
   B200_CHECK_ARG(aligned16(src) && aligned16(dst), B200MOE_E_ALIGN, "special_rows: pointers must be 16-byte aligned");
   if (rows_cap <= 0 || first_special == num_experts) return 0;
-  special_rows_kernel<<<rows_grid(rows_cap), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs, first_special, num_experts,
-      static_cast<int>(H / 8), reinterpret_cast<uint4*>(dst));
+  by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
+    special_rows_kernel<tpr.value><<<rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs, first_special, num_experts,
+        static_cast<int>(H / 8), reinterpret_cast<uint4*>(dst));
+  });
   B200_CUDA(cudaGetLastError());
   return 0;
 }
