@@ -38,8 +38,9 @@ struct Fp8Params {
   uint8_t* q_out;
   uint8_t* q_sf;
   // optional (pair kernel, store and SwiGLU epilogues): live rows of each expert, for a forward that no backward follows.
-  // An epilogue warp whose 32 rows are all padding gives the accumulator back unread and stores nothing; with p.D ==
-  // nullptr the SwiGLU epilogue writes only the quantised `inter`, not gate_up and inter in bf16.  64 tokens of H 4096, 8
+  // An epilogue warp whose 32 rows are all padding gives the accumulator back unread and stores nothing, and the SwiGLU
+  // epilogue writes only the quantised `inter`, not gate_up and inter in bf16 (an instantiation of its own: tested in the
+  // training kernels both cost them 1 %).  64 tokens of H 4096, 8
   // experts of d_ff 14336 (16 rows an expert in tiles of 256): 175 MB of stores and a 26 us quantiser pass less, gate/up
   // 236 -> 201 us, down 114 -> 102 us.
   const int* live;
@@ -349,7 +350,8 @@ __device__ __forceinline__ uint32_t idesc_mxf8_pair(uint32_t sf_id) {
          (static_cast<uint32_t>(256 >> 4) << 24) | (sf_id << 29);
 }
 
-template <int EPI>
+// FWD: the instantiation for a forward that no backward follows (Fp8Params::live)
+template <int EPI, bool FWD = false>
 __global__ void __launch_bounds__(kPThreads, 1)
 gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
@@ -554,11 +556,13 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       if (!mbar_wait(bar_tfull, it & 1, abort_flag, ST_WAIT_EPILOGUE)) break;
       __syncwarp();
       tc_fence_after();
-      if (EPI != EPI_GLU_BWD && fp.live != nullptr && row0 >= p.poffs[t.g] + fp.live[t.g]) {   // nothing but pad rows
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(tempty_leader);
-        continue;
+      if constexpr (FWD) {
+        if (row0 >= p.poffs[t.g] + fp.live[t.g]) {   // nothing but pad rows
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(tempty_leader);
+          continue;
+        }
       }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
       const bool have_acc = t.nkb > 0;
@@ -620,7 +624,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             mx_quant_store32(oh + 16, fp.q_out + row * static_cast<long long>(I) + col0 + 32, fp.q_sf, row,
                              (col0 + 32) >> 5, I >> 7);
           }
-          if (p.D != nullptr) {
+          if constexpr (!FWD) {
             staging_free(lane);
             stage_row(sbuf, lane, acc);
             store_box(&tmD, sbuf, lane, col0, row0, 0);    // gate half of gate_up
@@ -713,14 +717,14 @@ static int map_sf(CUtensorMap* tm, const void* sf, long long row_blocks, long lo
   return 0;
 }
 
-template <int EPI>
+template <int EPI, bool FWD>
 static int launch_fp8_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmSFA,
                            const CUtensorMap& tmSFB, const CUtensorMap& tmD, const CUtensorMap& tmD2,
                            const Fp8Params& fp, int max_tiles, cudaStream_t stream) {
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<EPI>::kSmemBytes);
+    attr_err = cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<EPI, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<EPI>::kSmemBytes);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   int pairs = gemm_cta_budget() / 2;
@@ -738,7 +742,7 @@ static int launch_fp8_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, gemm_mxfp8_pair_kernel<EPI>, tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, gemm_mxfp8_pair_kernel<EPI, FWD>, tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp));
   return 0;
 }
 
@@ -811,8 +815,10 @@ static int launch_any(const void* Aq, long long a_rows, const void* Bq, long lon
     }
   }
   if (rc) return rc;
-  return launch_fp8_pair<EPI>(tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp, max_tiles_1cta > 0 ? (max_tiles_1cta + 3) / 4 : 0,
-                              stream);
+  const int max_pairs = max_tiles_1cta > 0 ? (max_tiles_1cta + 3) / 4 : 0;
+  if constexpr (EPI != EPI_GLU_BWD)
+    if (fp.live != nullptr) return launch_fp8_pair<EPI, true>(tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp, max_pairs, stream);
+  return launch_fp8_pair<EPI, false>(tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp, max_pairs, stream);
 }
 
 }  // namespace b200moe
