@@ -112,10 +112,13 @@ class _Layer(torch.autograd.Function):
             ctx.dims = (T, H, I, E, top_k, norm, scale)
             ctx.save_for_backward(x, gate_weight, gate_up_proj, down_proj, codes_dev, ws)
         ctx.mark_non_differentiable(counts)
+        ctx.set_materialize_grads(False)      # no zero-filled gradient for the counts: a launch and an allocation a pass
         return out, counts
 
     @staticmethod
     def backward(ctx, grad_out, grad_counts):
+        if grad_out is None:
+            return (None,) * 11
         x, gate_weight, gate_up_proj, down_proj, codes_dev, ws = ctx.saved_tensors
         T, H, I, E, k, norm, scale = ctx.dims
         need_x, need_gate, _, need_gu, need_dn = ctx.needs_input_grad[:5]

@@ -48,10 +48,13 @@ class FusedMLPRouter(torch.autograd.Function):
         ctx.xshape = x.shape
         ctx.save_for_backward(xf, weight, logits, idx)
         ctx.mark_non_differentiable(idx, counts)
+        ctx.set_materialize_grads(False)      # no zero-filled gradients for idx and counts: two launches a pass
         return idx, w, counts
 
     @staticmethod
     def backward(ctx, grad_idx, grad_weights, grad_counts):
+        if grad_weights is None:
+            return (None,) * 7
         xf, weight, logits, idx = ctx.saved_tensors
         (T, H), E, dev = xf.shape, weight.shape[0], xf.device
         gw = grad_weights.contiguous().float()
@@ -126,10 +129,13 @@ class FusedConvRouter(torch.autograd.Function):
         ctx.shape = (B, S, H, E, K, k)
         ctx.save_for_backward(x, wt, logits, idx)
         ctx.mark_non_differentiable(idx, counts)
+        ctx.set_materialize_grads(False)      # no zero-filled gradients for idx and counts: two launches a pass
         return idx, w, counts
 
     @staticmethod
     def backward(ctx, grad_idx, grad_weights, grad_counts):
+        if grad_weights is None:
+            return (None,) * 7
         x, wt, logits, idx = ctx.saved_tensors
         B, S, H, E, K, k = ctx.shape
         dev = x.device
