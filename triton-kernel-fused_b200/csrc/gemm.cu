@@ -57,18 +57,30 @@ struct Cfg {
   static constexpr int TILE_ROWS = BM * CTAS;
 };
 
-// Columns of B (and of the accumulator) a pair tile multiplies: the last tile of a ragged width is narrower, in steps that
-// keep each CTA's half of B whole in units of its shared-memory layout: 8 rows (K-major) or a 64-wide swizzle atom
-// (MN-major).  SwiGLU tiles stay whole: a narrow one gained nothing on ragged widths, and the epilogue's variable offset
-// of the up columns cost 1 % on the others.  This is what lets every width above 64 take the pair kernel: its 256-wide tiles
+// Columns of B (and of the accumulator) a pair tile multiplies: the last tile of a ragged width is narrower, in steps of 32
+// with K-major weights (the two-SM MMA with 256 rows takes an N that is a multiple of 32; a CTA's half of B then is whole
+// 8-row groups of its shared-memory layout), of 128 with MN-major ones (a 64-wide swizzle atom per CTA).  SwiGLU tiles stay
+// whole: a narrow one gained nothing on ragged widths, and the epilogue's variable offset of the up columns cost 1 % on the
+// others.  This is what lets every width above 64 take the pair kernel: its 256-wide tiles
 // multiply no more columns than 128-wide single-CTA tiles would, at half the operand traffic per FLOP.  One layer of
 // 3001 tokens, H 1032, I 680, 32 experts, top-4: the five products that ran on 128-wide tiles 334 -> 234 us.
+__host__ __device__ constexpr int pair_width(int rem, bool b_mn, int bn) {
+  return b_mn ? (rem <= bn / 2 ? bn / 2 : bn) : (rem >= bn ? bn : (rem + 31) / 32 * 32);
+}
+constexpr bool pair_widths_valid(int bn) {
+  for (int rem = 1; rem <= 2 * bn; ++rem)
+    for (int mn = 0; mn < 2; ++mn) {
+      const int w = pair_width(rem, mn != 0, bn);
+      if (w % 32 != 0 || w < 32 || w > bn || w < (rem < bn ? rem : bn)) return false;
+    }
+  return true;
+}
+static_assert(pair_widths_valid(256), "a pair tile's N must cover its columns and be a multiple of 32 up to 256");
+
 template <int BN, int EPI>
 __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
-  const int rem = p.N - n0;
   if constexpr (EPI == EPI_SWIGLU) return BN;
-  if (p.b_mn) return rem <= BN / 2 ? BN / 2 : BN;
-  return rem >= BN ? BN : (rem + 15) / 16 * 16;
+  return pair_width(p.N - n0, p.b_mn != 0, BN);
 }
 
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
