@@ -24,3 +24,22 @@ def test_mxfp8_forward_without_gradient_equals_the_training_forward(pkg, T, H, I
     assert torch.equal(quiet, trained.detach()) and torch.equal(again, quiet)
     trained.float().sum().backward()
     assert torch.isfinite(layer.gate_up_proj.grad).all()
+
+
+def test_forward_without_gradient_keeps_only_the_row_wise_copies(pkg):
+    """Trainable parameters and a trainable input under no_grad: no transposed copy is made or kept; the next training
+    forward adds them."""
+    from importlib import import_module
+    mx = import_module(pkg.__name__ + ".mxfp8")
+    layer = pkg.MoELayer(256, 128, 8, top_k=2, precision="mxfp8").to(DEV).to(torch.bfloat16)
+    x = torch.randn(40, 256, device=DEV).to(torch.bfloat16).requires_grad_()
+    kept = lambda: [len(mx._QUANTISED[id(p)][4]) for p in (layer.gate_up_proj, layer.down_proj)]     # noqa: E731
+    with torch.no_grad():
+        quiet = layer(x)
+    assert kept() == [2, 2]
+    trained = layer(x)
+    assert kept() == [4, 4] and torch.equal(quiet, trained.detach())
+    trained.float().sum().backward()
+    with torch.no_grad():
+        assert torch.equal(layer(x), quiet)
+    pkg.check_status()

@@ -33,17 +33,23 @@ WEIGHT_CACHE = os.environ.get("B200MOE_MXFP8_WEIGHT_CACHE", "1") == "1"
 _QUANTISED = {}      # id(stack) -> (weak reference, version, data pointer, has the transposed copy, tensors)
 
 
-def _quantised_weights(stack, rows_fn, both_fn, both):
+def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None):
     """(q, sf) or (q, sf, qt, sft) of an expert stack, from the cache when the stack is the same tensor, at the same
-    address, with the same autograd version as when the copies were made (every in-place update moves the version)."""
+    address, with the same autograd version as when the copies were made (every in-place update moves the version).
+    transpose_fn adds (qt, sft) to a row-wise copy that is kept already; without it both are made anew."""
     if not WEIGHT_CACHE:
         return both_fn() if both else rows_fn()
     import weakref
     key = id(stack)
     hit = _QUANTISED.get(key)
-    if hit is not None and hit[0]() is stack and hit[1] == stack._version and hit[2] == stack.data_ptr() and (hit[3] or not both):
-        return hit[4] if both or not hit[3] else hit[4][:2]
-    res = both_fn() if both else rows_fn()
+    if hit is not None and not (hit[0]() is stack and hit[1] == stack._version and hit[2] == stack.data_ptr()):
+        hit = None
+    if hit is not None and (hit[3] or not both):
+        return hit[4] if both else hit[4][:2]
+    if hit is not None and transpose_fn is not None:
+        res = hit[4] + transpose_fn()
+    else:
+        res = both_fn() if both else rows_fn()
     _QUANTISED[key] = (weakref.ref(stack, lambda _r, k=key: _QUANTISED.pop(k, None)), stack._version, stack.data_ptr(),
                        both, res)
     return res
@@ -56,8 +62,9 @@ def _gate_up_copies(stack, both):
 
 
 def _down_copies(stack, both):
-    E, H, I = stack.shape
-    return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * H, I)), lambda: ops.mxfp8_quant_both(stack), both)
+    E, H, I = stack.shape      # evaluation keeps the row-wise copy; training after it adds the other one
+    return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * H, I)), lambda: ops.mxfp8_quant_both(stack), both,
+                              lambda: ops.mxfp8_quant_transpose(stack))
 
 
 class _MoEMxfp8(torch.autograd.Function):
@@ -80,11 +87,13 @@ class _MoEMxfp8(torch.autograd.Function):
 
         need_x, _, _, need_gu, need_dn = ctx.needs_input_grad[:5]
         perm = ops.permute_build(idx, E)
-        if not keep:   # the SwiGLU epilogue is the quantiser; no transposed activations, no gate_up, no pad rows
+        # the SwiGLU epilogue is the quantiser; no transposed activations or weights (needs_input_grad tells which inputs
+        # require a gradient, also where grad mode is off and nobody will ask for one), no gate_up, no pad rows
+        if not keep:
             _, xq, xsf = ops.mxfp8_gather_quant(hidden, perm, keep_rows=False)
-            wq, wsf = _gate_up_copies(gate_up_proj, need_x)[:2]
+            wq, wsf = _gate_up_copies(gate_up_proj, False)
             iq, isf = ops.mxfp8_expert_forward(ops.EPI_SWIGLU, xq, xsf, wq, wsf, perm, twoI, H, I)
-            dq, dsf = _down_copies(down_proj, need_x or need_gu)[:2]
+            dq, dsf = _down_copies(down_proj, False)
             return ops.combine(ops.mxfp8_expert_forward(ops.EPI_STORE, iq, isf, dq, dsf, perm, H, I, I), w32, perm)
         # the gather is the quantising producer; when the gate/up weight gradient is wanted it also writes the
         # copy quantised along the token rows, and the gathered bf16 rows are never materialised
