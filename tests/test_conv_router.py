@@ -27,6 +27,18 @@ def test_conv_logits_equal_unfolded_gemm():
     assert (d[:, :10] == 0).all() and (d[:, 10:10 + K] > 0).all() and (d[:, 10 + K:] == 0).all()
 
 
+# (sequences, positions, width, experts, taps, in place?): the benchmark's shape, one sequence, a width of no whole k-block, a
+# short batch of short sequences; many short sequences, where the row tiles of the in-place product would be mostly padding
+@pytest.mark.parametrize("B,S,H,E,K,in_place", [(16, 1024, 2048, 64, 4, True), (1, 7, 256, 8, 4, True), (7, 600, 80, 16, 3, True),
+                                                (32, 8, 2048, 64, 4, True), (4096, 8, 2048, 64, 4, False), (16384, 1, 80, 16, 2, False),
+                                                (512, 16, 1040, 256, 4, False), (2, 300, 520, 64, 4, False)])
+def test_route_of_the_logits_product(pkg, B, S, H, E, K, in_place):
+    """The workspace of the forward holds the unfolded copy or nothing; the choice is made on the host."""
+    nbytes = pkg.lib().b200moe_conv_router_fwd_ws_bytes(B, S, H, E, K)
+    assert (nbytes == 0) == in_place
+    assert in_place or nbytes >= 2 * K * H * (B * S + E)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,S,H,E,K", [(2, 256, 128, 64, 4), (3, 384, 320, 128, 2), (1, 128, 64, 64, 1),
                                        (5, 128, 512, 256, 3)])

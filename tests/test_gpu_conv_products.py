@@ -60,3 +60,23 @@ def test_conv_logits_equal_the_unfolded_product(pkg, B, S, H, E, K):
     wf = w.permute(0, 2, 1).reshape(E, K * H).contiguous()
     assert torch.equal(logits, pkg.ops.gemm_nt(pkg.ops.conv_unfold(x, K), wf))
     assert int(status.item()) == 0
+
+
+# many short sequences, whose product runs over the unfolded copy, give what a few of them give, whose product runs in place
+@pytest.mark.parametrize("B,S,H,E,K,k", [(4096, 1, 64, 8, 4, 2), (2048, 5, 272, 16, 3, 4), (1500, 16, 80, 136, 2, 8)])
+def test_short_sequences_equal_a_part_of_them(pkg, B, S, H, E, K, k):
+    g = torch.Generator().manual_seed(B)
+    x = torch.randn(B, S, H, generator=g).to(torch.bfloat16).to(DEV).requires_grad_()
+    w = (torch.randn(E, H, K, generator=g) * (H * K) ** -0.5).to(torch.bfloat16).to(DEV).requires_grad_()
+    bias, G = torch.randn(E, generator=g).to(DEV) * 0.05, torch.randn(B, S, k, generator=g).to(DEV)
+    n = 40
+    ws = pkg.lib().b200moe_conv_router_fwd_ws_bytes
+    assert ws(B, S, H, E, K) > 0 and ws(n, S, H, E, K) == 0
+    idx, wt = pkg.fused_router(x, w, bias, k, E)
+    gx, gw = torch.autograd.grad(wt, (x, w), G)
+    for lo in (0, B - n):
+        part = x.detach()[lo:lo + n].requires_grad_()
+        i, p = pkg.fused_router(part, w, bias, k, E)
+        assert torch.equal(i, idx[lo:lo + n]) and torch.equal(p, wt[lo:lo + n])
+        assert torch.equal(torch.autograd.grad(p, part, G[lo:lo + n])[0], gx[lo:lo + n])
+    pkg.check_status()

@@ -325,11 +325,25 @@ int b200moe_router_backward(const void* x, const void* weight, const void* logit
 }
 
 // ---------------------------------------------------------------------------- conv router
-// a width that is no multiple of 16 would split an MMA's 16 channels between taps: the unfolded copy keeps the sums' order
-static bool conv_in_place(int64_t H) { return H % 16 == 0; }
+// In place or over an unfolded copy of x (the same k order, so the same logits to the bit).  In place the row tiles lie in one
+// sequence each and the k-blocks in one tap each, so short sequences and widths that are no multiple of 64 multiply padding;
+// the copy writes taps * H values per token and takes two more launches.  Both run waves of tiles of one accumulator chain:
+// compared are the k-blocks of their waves, 0.31 us each, with 22 of them for the launches and one per 1.9 MB of copy.  us, in
+// place / unfolded, 64 experts, 4 taps, H 2048, 16 384 tokens in sequences of 1: 4290 / 119, 16: 273 / 120, 48: 124 / 120,
+// 64: 85 / 120, 128: 47 / 120; of 4096 tokens in sequences of 16: 85 / 56, 32: 43 / 56; H 80, 16 384 tokens in sequences of 1:
+// 326 / 19, 16: 25 / 18, 32: 15 / 18.
+// A width that is no multiple of 16 would split an MMA's 16 channels between taps: always unfolded.
+static bool conv_in_place(int64_t B, int64_t S, int64_t H, int E, int taps) {
+  if (H % 16 != 0) return false;
+  auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  const int64_t cols = up(E, 128), sms = num_sms();
+  const int64_t in_place = up(B * up(S, 128) * cols, sms) * taps * up(H, 64);
+  const int64_t unfolded = up(up(B * S, 128) * cols, sms) * up(taps * H, 64);
+  return in_place - unfolded <= 22 + B * S * taps * H * 2 / 1900000;
+}
 
 size_t b200moe_conv_router_fwd_ws_bytes(int64_t B, int64_t S, int64_t H, int E, int taps) {
-  if (B <= 0 || S <= 0 || H <= 0 || E <= 0 || taps <= 0 || conv_in_place(H)) return 0;
+  if (B <= 0 || S <= 0 || H <= 0 || E <= 0 || taps <= 0 || conv_in_place(B, S, H, E, taps)) return 0;
   Carver c(nullptr);
   c.take<bf16_t>(B * S * taps * H);
   c.take<bf16_t>(static_cast<int64_t>(E) * taps * H);
@@ -348,9 +362,10 @@ int b200moe_conv_router_forward(const void* x, const void* weight, const float* 
                                 int64_t* idx, float* w, int32_t* counts, int32_t* status, b200moe_stream_t stream) {
   int rc = check_conv_router("conv_router_forward", B, S, H, E, taps);
   if (rc) return rc;
-  B200_CHECK_ARG(x && weight && weight_rows && logits && (ws || conv_in_place(H)), B200MOE_E_NULL, "conv_router_forward: null pointer");
+  const bool in_place = conv_in_place(B, S, H, E, taps);
+  B200_CHECK_ARG(x && weight && weight_rows && logits && (ws || in_place), B200MOE_E_NULL, "conv_router_forward: null pointer");
   RUN("conv_weight_rows", 1, b200moe_conv_weight_rows(weight, E, H, taps, 0, weight_rows, stream));
-  if (conv_in_place(H)) {
+  if (in_place) {
     RUN("conv_gemm_fwd", 1, b200moe_conv_gemm_logits(x, weight_rows, logits, B, S, H, E, taps, status, stream));
   } else {
     Carver c(ws);
