@@ -44,6 +44,19 @@ def test_conv_router_against_float64(pkg, B, S, H, E, K, k):
     assert O.rel_l2(wd.grad.cpu().double(), w64.grad) < 1e-2
 
 
+# weight gradient of up to 128 rows (taps * experts) on single-CTA tiles, of more on pair tiles: both sides of the line, a width
+# that is a multiple of 256 and one that is not
+@pytest.mark.parametrize("rows", [8, 128, 136])
+@pytest.mark.parametrize("H", [64, 512, 1048])
+def test_split_product_of_few_rows(pkg, rows, H):
+    g = torch.Generator().manual_seed(rows + H)
+    T = 1500
+    u, x = (torch.randn(T, n, generator=g).to(torch.bfloat16).to(DEV) for n in (rows, H))
+    got = pkg.ops.gemm_tn(u, x)
+    pkg.check_status()
+    assert O.rel_l2(got.double().cpu(), (u.double().T @ x.double()).cpu()) < 3.95e-3      # one bf16 rounding: 2^-8
+
+
 # the in-place product at ragged lengths and widths gives the logits of the unfolded product to the bit (the same k order)
 @pytest.mark.parametrize("B,S,H,E,K", [(3, 129, 80, 24, 3), (2, 300, 512, 64, 4), (4, 64, 1040, 128, 2), (2, 257, 96, 256, 4)])
 def test_conv_logits_equal_the_unfolded_product(pkg, B, S, H, E, K):

@@ -283,9 +283,10 @@ static int router_backward(const void* x, const void* weight, const void* logits
 // (E of 256 MMA rows, x read four times).
 // (The same turn of the forward, z = x [W_j]^T and adding its rows up, reads x once as well, but adds in another order: 1 in
 // 7000 picks of close experts then differs, and a token's gradient with it.)
-static int64_t conv_k_chunk(int64_t T, int64_t rows, int64_t H) {   // one wave of pair tiles
-  const int64_t tiles = ((rows + 255) / 256) * ((H + 255) / 256);
-  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(74 / std::max<int64_t>(tiles, 1), (T + 63) / 64));
+static int64_t conv_k_chunk(int64_t T, int64_t rows, int64_t H) {   // one wave of pair tiles, up to 128 rows of single-CTA tiles
+  const bool single = rows <= 128;
+  const int64_t tiles = single ? (H + 127) / 128 : ((rows + 255) / 256) * ((H + 255) / 256), per_wave = single ? 148 : 74;
+  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
   return ((T + slices - 1) / slices + 63) / 64 * 64;
 }
 static int64_t conv_slices(int64_t T, int64_t rows, int64_t H) {

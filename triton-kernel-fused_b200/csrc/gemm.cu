@@ -1006,8 +1006,11 @@ int b200moe_gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, in
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
   p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
-  // up to 128 rows a pair tile would multiply nothing but padding in its second half
-  const int bn = M <= BM ? pick_bn(N) : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
+  // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
+  // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
+  // 1024 16.1 / 6.5.
+  const int bn = M <= BM ? std::min(pick_bn(N), 128)
+                         : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
   return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
                                     (cudaStream_t)stream);
 }
