@@ -100,3 +100,29 @@ def test_observer_sees_the_operations_of_the_native_sequences(pkg):
     n = len(seen)
     layer(x)
     assert len(seen) == n
+
+
+# SMs reserved for an exchange: the split products of the routers' weight gradients take fewer slices out of the same workspace
+@pytest.mark.parametrize("reserved", [1, 40, 146])
+def test_router_gradients_with_reserved_sms(pkg, reserved):
+    g = torch.Generator().manual_seed(reserved)
+    lib = pkg.lib()
+    x = torch.randn(3000, 264, generator=g).to(torch.bfloat16).to(DEV)
+    rand = lambda *s: (torch.randn(*s, generator=g) * 0.1).to(torch.bfloat16).to(DEV).requires_grad_()     # noqa: E731
+    linear, wide, conv, wconv = rand(64, 264), rand(256, 264), rand(8, 264, 4), rand(128, 264, 3)
+    G = torch.randn(3000, 4, generator=g).to(DEV)
+
+    def grads():
+        out = [torch.autograd.grad(pkg.fused_mlp_router(x, w, None, 4, w.shape[0])[1], w, G)[0] for w in (linear, wide)]
+        return out + [torch.autograd.grad(pkg.fused_router(x.view(4, 750, 264), w, None, 4, w.shape[0])[1], w, G.view(4, 750, 4))[0]
+                      for w in (conv, wconv)]
+
+    want = grads()
+    assert lib.b200moe_set_reserved_sms(reserved) == 0
+    try:
+        got = grads()
+    finally:
+        lib.b200moe_set_reserved_sms(0)
+    pkg.check_status()
+    for a, b in zip(got, want):      # fp32 sums in another order: single bf16 results round the other way
+        assert torch.isfinite(a).all() and O.rel_l2(a.float(), b.float()) < 2e-3

@@ -201,3 +201,20 @@ def test_fixed_capacity_rows():
     for bad in (0, -1.0, float("nan")):
         with pytest.raises(ValueError):
             ep.fixed_capacity_rows(2, 8, 2, bad)
+
+
+def test_workspaces_are_sized_for_every_sm_budget():
+    """The split products take fewer slices while SMs are reserved; a workspace sized before or after holds them."""
+    lib = importlib.import_module(PKG).lib()
+    sizes = lambda: [f(*a) for f, cases in (     # noqa: E731
+        (lib.b200moe_router_bwd_ws_bytes, [(16384, 2048, 64), (100, 256, 256)]),
+        (lib.b200moe_conv_router_bwd_ws_bytes, [(16, 1024, 2048, 64, 4), (2, 100, 256, 8, 2)]),
+        (lib.b200moe_conv_router_fwd_ws_bytes, [(341, 48, 2048, 64, 4), (300, 32, 2048, 64, 4)]),
+        (lib.b200moe_layer_bwd_ws_bytes, [(16384, 2048, 1408, 64, 6)])) for a in cases]
+    full = sizes()
+    try:
+        for n in (2, 60, 146):
+            assert lib.b200moe_set_reserved_sms(n) == 0
+            assert sizes() == full
+    finally:
+        lib.b200moe_set_reserved_sms(0)

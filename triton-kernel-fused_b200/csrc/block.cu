@@ -111,16 +111,19 @@ struct Backward {
 // Split-K of the router's weight gradient dW (E, H) = gl (T, E)^T x (T, H).  Up to 128 experts the product runs as
 // dW^T = x^T gl, whose rows (H) fill the MMA's M; gl^T x would multiply E of 256 rows.  About one tile per SM; the slices
 // are summed, and transposed back, by the reduction.  T 16384, H 2048, 64 experts: product + reduction 48 -> 31 us.
-static bool router_dw_transposed(int64_t E) { return E <= 128; }
-static int64_t router_k_chunk(int64_t T, int64_t E, int64_t H) {
-  const int64_t tiles = router_dw_transposed(E) ? ((H + 127) / 128) * ((E + 127) / 128) : ((E + 127) / 128) * ((H + 255) / 256);
-  const int64_t per_wave = router_dw_transposed(E) ? 148 : 296;
-  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
-  return ((T + slices - 1) / slices + 63) / 64 * 64;
+//
+// `sms`: the SMs the GEMM may use.  A launch takes gemm_cta_budget(), which shrinks while SMs are reserved for an exchange;
+// a workspace is sized for num_sms(), which never gives fewer slices.
+struct Split { int64_t chunk, slices; };
+static Split split_k(int64_t T, int64_t tiles, int64_t per_wave) {
+  const int64_t want = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
+  const int64_t chunk = ((T + want - 1) / want + 63) / 64 * 64;
+  return {chunk, (T + chunk - 1) / chunk};
 }
-static int64_t router_slices(int64_t T, int64_t E, int64_t H) {
-  const int64_t c = router_k_chunk(T, E, H);
-  return (T + c - 1) / c;
+static bool router_dw_transposed(int64_t E) { return E <= 128; }
+static Split router_split(int64_t T, int64_t E, int64_t H, int sms) {
+  if (router_dw_transposed(E)) return split_k(T, ((H + 127) / 128) * ((E + 127) / 128), sms);
+  return split_k(T, ((E + 127) / 128) * ((H + 255) / 256), 2 * sms);
 }
 
 static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* bytes) {
@@ -141,7 +144,7 @@ static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* byt
     b.grad_w = c.take<float>(d.M());
     b.grad_logits = c.take<bf16_t>(d.T * d.E);
     b.grad_x_router = c.take<bf16_t>(d.T * d.H);
-    b.part = c.take<float>(router_slices(d.T, d.E, d.H) * d.E * d.H);
+    b.part = c.take<float>(router_split(d.T, d.E, d.H, num_sms()).slices * d.E * d.H);
   }
   if (bytes != nullptr) *bytes = c.off;
   return b;
@@ -241,14 +244,14 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
   return 0;
 }
 
-// Up to 16 tokens for each of 148 SMs and 128 experts logits and picks are one launch (gemm_few.cu, with the times of both)
-constexpr int64_t kSmallTokens = 16 * 148;
+// Up to 16 tokens per SM and 128 experts logits and picks are one launch (gemm_few.cu, with the times of both)
+constexpr int64_t kSmallTokensPerSm = 16;
 constexpr int kSmallExperts = 128;
 
 static int router_forward(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k, int norm,
                           float scale, void* logits, int64_t* idx, float* w, int32_t* counts, int32_t* status,
                           b200moe_stream_t st) {
-  if (T <= kSmallTokens && E <= kSmallExperts) {
+  if (T <= kSmallTokensPerSm * num_sms() && E <= kSmallExperts) {
     RUN("router_small_fwd", 1, b200moe_router_small_fwd(x, weight, bias, T, H, E, k, norm, scale, logits, idx, w, counts, status, st));
     return 0;
   }
@@ -264,13 +267,13 @@ static int router_backward(const void* x, const void* weight, const void* logits
   if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(grad_logits, weight, grad_x, T, H, E, status, st));
   if (grad_weight != nullptr) {
     OpScope scope("gemm_tn", 2);
-    const int64_t chunk = router_k_chunk(T, E, H), slices = router_slices(T, E, H);
+    const Split sp = router_split(T, E, H, gemm_cta_budget());
     const bool tr = router_dw_transposed(E);
-    int rc = tr ? b200moe_gemm_tn_splitk(x, grad_logits, part, H, E, T, chunk, status, st)
-                : b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, chunk, status, st);
+    int rc = tr ? b200moe_gemm_tn_splitk(x, grad_logits, part, H, E, T, sp.chunk, status, st)
+                : b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, sp.chunk, status, st);
     if (rc) return rc;
-    rc = tr ? b200moe_splitk_reduce_t(part, slices, H, E, grad_weight, st)
-            : b200moe_splitk_reduce(part, slices, static_cast<int64_t>(E) * H, grad_weight, st);
+    rc = tr ? b200moe_splitk_reduce_t(part, sp.slices, H, E, grad_weight, st)
+            : b200moe_splitk_reduce(part, sp.slices, static_cast<int64_t>(E) * H, grad_weight, st);
     if (rc) return rc;
   }
   return 0;
@@ -283,15 +286,9 @@ static int router_backward(const void* x, const void* weight, const void* logits
 // (E of 256 MMA rows, x read four times).
 // (The same turn of the forward, z = x [W_j]^T and adding its rows up, reads x once as well, but adds in another order: 1 in
 // 7000 picks of close experts then differs, and a token's gradient with it.)
-static int64_t conv_k_chunk(int64_t T, int64_t rows, int64_t H) {   // one wave of pair tiles, up to 128 rows of single-CTA tiles
-  const bool single = rows <= 128;
-  const int64_t tiles = single ? (H + 127) / 128 : ((rows + 255) / 256) * ((H + 255) / 256), per_wave = single ? 148 : 74;
-  const int64_t slices = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
-  return ((T + slices - 1) / slices + 63) / 64 * 64;
-}
-static int64_t conv_slices(int64_t T, int64_t rows, int64_t H) {
-  const int64_t c = conv_k_chunk(T, rows, H);
-  return (T + c - 1) / c;
+static Split conv_split(int64_t T, int64_t rows, int64_t H, int sms) {   // one wave of pair tiles, up to 128 rows of single-CTA tiles
+  if (rows <= 128) return split_k(T, (H + 127) / 128, sms);
+  return split_k(T, ((rows + 255) / 256) * ((H + 255) / 256), sms / 2);
 }
 
 }  // namespace b200moe
@@ -311,7 +308,7 @@ size_t b200moe_router_bwd_ws_bytes(int64_t T, int64_t H, int E) {
   if (T <= 0 || H <= 0 || E <= 0) return 0;
   Carver c(nullptr);
   c.take<bf16_t>(T * E);
-  c.take<float>(router_slices(T, E, H) * E * H);
+  c.take<float>(router_split(T, E, H, num_sms()).slices * E * H);
   return c.off;
 }
 
@@ -321,7 +318,7 @@ int b200moe_router_backward(const void* x, const void* weight, const void* logit
   B200_CHECK_ARG(ws, B200MOE_E_NULL, "router_backward: null workspace");
   Carver c(ws);
   bf16_t* gl = c.take<bf16_t>(T * E);
-  float* part = c.take<float>(router_slices(T, E, H) * E * H);
+  float* part = c.take<float>(router_split(T, E, H, num_sms()).slices * E * H);
   return router_backward(x, weight, logits, idx, grad_w, T, H, E, k, norm_topk, scale, gl, part, grad_x, grad_weight, status, stream);
 }
 
@@ -385,7 +382,7 @@ static ConvBackward carve_conv(int64_t T, int64_t H, int64_t rows, void* ws, siz
   Carver c(ws);
   ConvBackward b;
   b.u = c.take<bf16_t>(T * rows);
-  b.part = c.take<float>(conv_slices(T, rows, H) * rows * H);
+  b.part = c.take<float>(conv_split(T, rows, H, num_sms()).slices * rows * H);
   if (bytes != nullptr) *bytes = c.off;
   return b;
 }
@@ -409,8 +406,9 @@ int b200moe_conv_router_backward(const void* x, const void* weight_rows, const v
   RUN("router_topk_bwd", 1, b200moe_conv_topk_bwd(logits, idx, grad_w, B, S, E, taps, k, norm_topk, scale, b.u, stream));
   if (grad_x != nullptr) RUN("conv_gemm_dx", 1, b200moe_gemm_nn(b.u, weight_rows, grad_x, T, H, rows, status, stream));
   if (grad_weight != nullptr) {
-    RUN("conv_gemm_dw", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, conv_k_chunk(T, rows, H), status, stream));
-    RUN("conv_weight_grad", 1, b200moe_conv_weight_grad(b.part, conv_slices(T, rows, H), E, H, taps, grad_weight, stream));
+    const Split sp = conv_split(T, rows, H, gemm_cta_budget());
+    RUN("conv_gemm_dw", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, sp.chunk, status, stream));
+    RUN("conv_weight_grad", 1, b200moe_conv_weight_grad(b.part, sp.slices, E, H, taps, grad_weight, stream));
   }
   return 0;
 }
