@@ -218,3 +218,19 @@ def test_workspaces_are_sized_for_every_sm_budget():
             assert sizes() == full
     finally:
         lib.b200moe_set_reserved_sms(0)
+
+
+def test_workspace_of_nothing_is_no_bytes():
+    """Every workspace size takes an empty batch, width or stack: no bytes (the launches refuse such calls), never a signal."""
+    lib = importlib.import_module(PKG).lib()
+    full = {"moe_fwd": (4, 256, 512, 8, 8, 2, 1, 0), "moe_bwd": (4, 256, 512, 8, 8, 2, 0), "layer_fwd": (4, 256, 512, 8, 2, 1),
+            "layer_bwd": (4, 256, 512, 8, 2), "router_bwd": (4, 256, 8), "conv_router_bwd": (2, 4, 256, 8, 3),
+            "conv_router_fwd": (2, 4, 264, 8, 3)}
+    extents = {"moe_fwd": (0, 1, 2, 3, 5), "moe_bwd": (0, 1, 2, 3, 5)}
+    for name, args in full.items():
+        size = getattr(lib, f"b200moe_{name}_ws_bytes")
+        assert size(*args) > 0
+        for i in extents.get(name, range(min(5, len(args)))):
+            for v in (0, -3):
+                assert size(*args[:i], v, *args[i + 1:]) == 0, (name, i, v)
+    assert lib.b200moe_router_backward(16, 16, 16, 16, 16, 0, 256, 8, 2, 1, 1.0, 16, 16, 16, 16, None) != 0

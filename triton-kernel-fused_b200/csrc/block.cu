@@ -116,6 +116,7 @@ struct Backward {
 // a workspace is sized for num_sms(), which never gives fewer slices.
 struct Split { int64_t chunk, slices; };
 static Split split_k(int64_t T, int64_t tiles, int64_t per_wave) {
+  if (T <= 0) return {64, 0};
   const int64_t want = std::max<int64_t>(1, std::min<int64_t>(per_wave / std::max<int64_t>(tiles, 1), (T + 63) / 64));
   const int64_t chunk = ((T + want - 1) / want + 63) / 64 * 64;
   return {chunk, (T + chunk - 1) / chunk};
@@ -415,6 +416,7 @@ int b200moe_conv_router_backward(const void* x, const void* weight_rows, const v
 
 // ---------------------------------------------------------------------------- experts on given picks
 size_t b200moe_moe_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int row_kernels) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || k <= 0) return 0;
   size_t n = 0;
   carve_forward(make_dims(T, H, I, E, n_glu, k, keep, row_kernels), false, nullptr, &n);
   return n;
@@ -434,6 +436,7 @@ int b200moe_moe_forward(const void* x, const int64_t* idx, const float* w, const
 }
 
 size_t b200moe_moe_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int row_kernels) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || k <= 0) return 0;
   size_t n = 0;
   carve_backward(make_dims(T, H, I, E, n_glu, k, 1, row_kernels), false, nullptr, &n);
   return n;
@@ -458,6 +461,7 @@ int b200moe_moe_backward(const void* grad_out, const float* w, const void* gate_
 
 // ---------------------------------------------------------------------------- router and experts
 size_t b200moe_layer_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k, int keep) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || k <= 0) return 0;
   size_t n = 0;
   carve_forward(make_dims(T, H, I, E, E, k, keep, 0), true, nullptr, &n);
   return n;
@@ -480,6 +484,7 @@ int b200moe_layer_forward(const void* x, const void* gate_weight, const float* b
 }
 
 size_t b200moe_layer_bwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int k) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || k <= 0) return 0;
   size_t n = 0;
   carve_backward(make_dims(T, H, I, E, E, k, 1, 0), true, nullptr, &n);
   return n;
