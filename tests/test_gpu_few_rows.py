@@ -39,6 +39,15 @@ def test_few_rows_products(pkg, counts, H, I, codes):
     assert O.rel_l2(out[c].cpu().float(), ref) < TOL
 
 
+# wide enough that the tile follows the mean: 64, 128 and 192 rows, with experts on both sides of one and of several tiles; and one
+# wave of 64-row chunks at a mean past each of the other limits
+@pytest.mark.parametrize("counts,H,I", [([0, 63, 64, 65, 1, 0, 17, 40], 72, 1800), ([129, 100, 0, 128], 136, 2184),
+                                        ([256, 30, 0, 127, 1, 200], 264, 1224), ([193, 150, 192, 0, 385], 136, 1032),
+                                        ([576, 0, 191, 1], 1224, 136), ([193, 150, 192, 0, 385], 72, 136)])
+def test_few_rows_products_of_wide_experts(pkg, counts, H, I):
+    test_few_rows_products(pkg, counts, H, I, False)
+
+
 @pytest.mark.parametrize("T,E,k", [(1, 8, 2), (40, 16, 4), (1279, 16, 2), (1281, 16, 2)])   # both sides of the limit
 def test_forward_without_gradient_equals_the_training_forward(pkg, T, E, k):
     torch.manual_seed(T)

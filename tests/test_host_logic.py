@@ -234,3 +234,16 @@ def test_workspace_of_nothing_is_no_bytes():
             for v in (0, -3):
                 assert size(*args[:i], v, *args[i + 1:]) == 0, (name, i, v)
     assert lib.b200moe_router_backward(16, 16, 16, 16, 16, 0, 256, 8, 2, 1, 1.0, 16, 16, 16, 16, None) != 0
+
+
+def test_route_of_a_forward_without_backward():
+    """Compact rows or row tiles: the workspace of the latter is that of a forward with a backward (it holds gate_up and the
+    padded rows).  (experts, d_model, d_ff, picks, tokens, compact?): decoding; both sides of the limits on the mean rows of
+    many and of few experts; a small stack inside and past one wave of 64-row chunks; a stack of half the SMs and one of more."""
+    size = importlib.import_module(PKG).lib().b200moe_moe_fwd_ws_bytes
+    for E, H, I, k, T, compact in ((64, 2048, 1408, 6, 1, True), (64, 2048, 1408, 6, 1706, True), (64, 2048, 1408, 6, 1707, False),
+                                   (8, 4096, 14336, 2, 440, True), (8, 4096, 14336, 2, 441, False), (16, 2048, 1408, 4, 640, True),
+                                   (16, 2048, 1408, 4, 641, False), (8, 512, 256, 2, 640, True), (8, 512, 256, 2, 641, False),
+                                   (8, 1024, 1024, 2, 351, True), (8, 1024, 1024, 2, 352, False), (8, 1024, 1280, 2, 352, True)):
+        kept, quiet = (size(T, H, I, E, E, k, keep, 0) for keep in (1, 0))
+        assert (quiet < kept) == compact, (E, H, I, k, T)

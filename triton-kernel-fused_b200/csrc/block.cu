@@ -40,15 +40,10 @@ struct Dims {
   int64_t rows() const { return kind == KIND_FEW ? M() : b200moe_padded_rows_cap(M(), E); }
 };
 
-// Most rows per expert, on average, for which a forward without a backward runs over compact rows with the weights as
-// the MMA's M operand (gemm_few.cu).  Gate/up + down, us, row tiles against compact rows, at H 2048, I 1408, 64
-// experts: 4.5 rows an expert 237 / 170, 141 rows 238 / 213, 206 rows 240 / 328 (an expert then takes two tiles).
-constexpr int64_t kFewRows = 160;
-
 static Dims make_dims(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int rows_kernels) {
   Dims d{T, H, I, E, n_glu, k, KIND_TILES};
   if (rows_kernels) d.kind = KIND_ROWS;
-  else if (!keep && T * k <= kFewRows * E) d.kind = KIND_FEW;
+  else if (!keep && T > 0 && k > 0 && E > 0 && few_rows_forward(T * k, E, H, I)) d.kind = KIND_FEW;
   return d;
 }
 

@@ -34,6 +34,9 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
                   size_t ws_bytes, int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream);
 
+// gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
+bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);
+
 // gemm.cu: the products of the optimizer's iteration over part of their padded extents
 int expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t K, int mirror,
                 int64_t n_live, void* out, int32_t* status, b200moe_stream_t stream);

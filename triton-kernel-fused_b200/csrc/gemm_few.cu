@@ -498,12 +498,42 @@ static int launch_router_few(const void* x, const void* weight, const RouterFewP
   return 0;
 }
 
-// Tile by the mean rows per expert.  A larger NT keeps an expert's rows in one tile, so its weights pass through shared
-// memory once; a smaller one leaves room for more k-blocks in flight and double-buffered accumulators.  Gate/up, us, at
-// H 2048, I 1408, 64 experts: 28 rows an expert NT 64 / 128 / 192: 115 / 116 / 117; 66 rows 134 / 119 / 125; 94 rows 153 /
-// 122 / 131; 141 rows 210 / 155 / 138.  Down (one / one / two 128-row weight blocks a tile): 61 / 61 / 63, 87 / 64 / 66,
-// 107 / 70 / 69, 150 / 123 / 75.
+// Tile.  The host knows the mean rows per expert, not the counts: both rules below were timed under even routing, expert
+// frequencies ~ rank^-0.6 and rank^-1.1, and one expert in every token's picks.  us, gate/up + down with gather and combine.
+//  - Chunks of 64 rows where even the worst spread of the rows over the experts, E + M / 64 chunks, is one wave of CTAs: the
+//    smallest tile then has the shortest chain and the most SMs.  8 experts, 512 x 256, mean 140 rows, even / rank^-1.1:
+//    NT 64 25.7 / 25.6, 128 29.8 / 29.7, 192 31.7 / 34.4 (row tiles 25.4 / 25.5).
+//  - Else by the mean.  A larger NT keeps an expert's rows in one tile, so its weights pass through shared memory once; a
+//    smaller one leaves room for more k-blocks in flight and double-buffered accumulators.  64 experts, 2048 x 1408, even /
+//    rank^-1.1: mean 4 rows NT 64 184 / 154, 128 186 / 155, 192 188 / 151; 39 rows 201 / 229, 201 / 216, 204 / 205; 80 rows
+//    278 / 280, 217 / 252, 225 / 235; 140 rows 379 / 376, 304 / 297, 254 / 278.
 constexpr int64_t kFewRows64 = 40, kFewRows128 = 110;
+
+static int64_t few_blocks(int64_t N, int64_t K) { return ceil_div(std::max(N, K), 128); }   // weight blocks of an expert (either product)
+static bool few_one_wave(int64_t M, int E, int64_t N, int64_t K) { return (E + M / 64) * few_blocks(N, K) <= num_sms(); }
+
+static int few_tile(int64_t M, int E, int64_t N, int64_t K) {
+  if (M <= kFewRows64 * E || few_one_wave(M, E, N, K)) return 64;
+  return M <= kFewRows128 * E ? 128 : 192;
+}
+
+// Whether a forward without a backward runs over compact rows (this file) or row tiles (gemm.cu), same measurements, row tiles
+// against compact rows, even / rank^-1.1.  64 experts, 2048 x 1408: mean 4 rows 268 / 222 against 184 / 154, 140 rows 286 /
+// 323 against 254 / 278, 200 rows 296 / 362 against 364 / 328 (an even expert then takes two tiles): up to kFewRows.
+// Fewer than 16 experts leave few pad rows in row tiles: 8 experts, 4096 x 14336: 80 rows 577 / 579 against 521 / 517, 159
+// rows 604 / 634 against 554 / 726: up to kFewRows128.  Where one chunk per expert fills less than half of the SMs and the
+// chunks of 64 are more than one wave, the single-CTA row tiles spread the work further: 8 experts, 1024 x 1024, 140 rows
+// 35 / 37 against 39 / 39 (NT 128) and 42 / 46 (NT 192).
+// What the rules cannot see costs: 16 experts, 4096 x 1024, one pick, every token on one expert, 39 rows on average: 50
+// against 65.
+constexpr int64_t kFewRows = 160;
+
+bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I) {
+  if (M > kFewRows * E) return false;
+  if (few_one_wave(M, E, H, I)) return true;
+  if (E * few_blocks(H, I) <= num_sms() / 2) return false;
+  return E >= 16 || M <= kFewRows128 * E;
+}
 
 static int check_few(const char* who, const void* x, const void* w, const void* d, const int32_t* counts,
                      const int32_t* offs, int64_t rows_cap, int E, int64_t N, int64_t K) {
@@ -531,8 +561,9 @@ int b200moe_expert_gate_up_few(const void* x, const void* gate_up_proj, const in
   FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status};
   cudaStream_t st = (cudaStream_t)stream;
   // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
-  if (rows_cap <= kFewRows64 * E) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
-  if (rows_cap <= kFewRows128 * E) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  const int nt = few_tile(rows_cap, E, I, H);
+  if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
   return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
 }
 
@@ -542,8 +573,9 @@ int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* count
   if (rc) return rc;
   FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status};
   cudaStream_t st = (cudaStream_t)stream;
-  if (rows_cap <= kFewRows64 * E) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
-  if (rows_cap <= kFewRows128 * E) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
+  const int nt = few_tile(rows_cap, E, N, K);
+  if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
+  if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
   return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
 }
 
