@@ -93,3 +93,16 @@ def test_short_sequences_equal_a_part_of_them(pkg, B, S, H, E, K, k):
         assert torch.equal(i, idx[lo:lo + n]) and torch.equal(p, wt[lo:lo + n])
         assert torch.equal(torch.autograd.grad(p, part, G[lo:lo + n])[0], gx[lo:lo + n])
     pkg.check_status()
+
+
+def test_observer_names_the_products_that_run(pkg):
+    x = torch.randn(2, 300, 128, device=DEV).to(torch.bfloat16).requires_grad_()
+    w = torch.randn(8, 128, 4, device=DEV).to(torch.bfloat16).requires_grad_()
+    seen = []
+    pkg.ops.set_hook(lambda name, launches, a, b: seen.append(name))
+    try:
+        pkg.fused_router(x, w, None, 2, 8)[1].sum().backward()
+    finally:
+        pkg.ops.set_hook(None)
+    assert seen == ["conv_weight_rows", "conv_gemm_logits", "router_topk_fwd", "conv_topk_bwd", "gemm_nn", "gemm_tn_splitk",
+                    "conv_weight_grad"]

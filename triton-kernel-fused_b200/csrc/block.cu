@@ -360,7 +360,7 @@ int b200moe_conv_router_forward(const void* x, const void* weight, const float* 
   B200_CHECK_ARG(x && weight && weight_rows && logits && (ws || in_place), B200MOE_E_NULL, "conv_router_forward: null pointer");
   RUN("conv_weight_rows", 1, b200moe_conv_weight_rows(weight, E, H, taps, 0, weight_rows, stream));
   if (in_place) {
-    RUN("conv_gemm_fwd", 1, b200moe_conv_gemm_logits(x, weight_rows, logits, B, S, H, E, taps, status, stream));
+    RUN("conv_gemm_logits", 1, b200moe_conv_gemm_logits(x, weight_rows, logits, B, S, H, E, taps, status, stream));
   } else {
     Carver c(ws);
     bf16_t* xu = c.take<bf16_t>(B * S * taps * H);
@@ -399,11 +399,11 @@ int b200moe_conv_router_backward(const void* x, const void* weight_rows, const v
   B200_CHECK_ARG(x && weight_rows && ws, B200MOE_E_NULL, "conv_router_backward: null pointer");
   const int64_t T = B * S, rows = static_cast<int64_t>(E) * taps;
   const ConvBackward b = carve_conv(T, H, rows, ws, nullptr);
-  RUN("router_topk_bwd", 1, b200moe_conv_topk_bwd(logits, idx, grad_w, B, S, E, taps, k, norm_topk, scale, b.u, stream));
-  if (grad_x != nullptr) RUN("conv_gemm_dx", 1, b200moe_gemm_nn(b.u, weight_rows, grad_x, T, H, rows, status, stream));
+  RUN("conv_topk_bwd", 1, b200moe_conv_topk_bwd(logits, idx, grad_w, B, S, E, taps, k, norm_topk, scale, b.u, stream));
+  if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(b.u, weight_rows, grad_x, T, H, rows, status, stream));
   if (grad_weight != nullptr) {
     const Split sp = conv_split(T, rows, H, gemm_cta_budget());
-    RUN("conv_gemm_dw", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, sp.chunk, status, stream));
+    RUN("gemm_tn_splitk", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, sp.chunk, status, stream));
     RUN("conv_weight_grad", 1, b200moe_conv_weight_grad(b.part, sp.slices, E, H, taps, grad_weight, stream));
   }
   return 0;
