@@ -63,7 +63,7 @@ struct Cfg {
 // whole: a narrow one gained nothing on ragged widths, and the epilogue's variable offset of the up columns cost 1 % on the
 // others.  This is what lets every width above 64 take the pair kernel: its 256-wide tiles
 // multiply no more columns than 128-wide single-CTA tiles would, at half the operand traffic per FLOP.  One layer of
-// 3001 tokens, H 1032, I 680, 32 experts, top-4: the five products that ran on 128-wide tiles 334 -> 234 us.
+// 3001 tokens, H 1032, I 680, 32 experts, top-4: the five products that ran on 128-wide tiles 321 -> 228 us.
 __host__ __device__ constexpr int pair_width(int rem, bool b_mn, int bn) {
   return b_mn ? (rem <= bn / 2 ? bn / 2 : bn) : (rem >= bn ? bn : (rem + 31) / 32 * 32);
 }

@@ -9,8 +9,8 @@
 // (no pad rows), 16-row boxes of it are loaded up to the last live row, and the accumulator holds output columns in
 // its lanes and rows in its columns.  A box may reach past the expert's rows: they only feed accumulator columns that
 // are not stored.
-// H 2048, I 1408, 64 experts, 288 rows (4.5 an expert; 111 + 56 us at copy rate): gate/up 158 -> 111 us, down 79 -> 59 us;
-// 9000 rows (141 an expert): 159 -> 138 and 79 -> 75 us; 6 rows of one token: 21 -> 19 and 15 -> 12 us.  Loading the weights
+// H 2048, I 1408, 64 experts, 288 rows (4.5 an expert; 118 + 59 us at copy rate): gate/up 161 -> 111 us, down 80 -> 60 us;
+// 9000 rows (141 an expert): 171 -> 148 and 85 -> 78 us; 6 rows of one token: 21 -> 19 and 15 -> 12 us.  Loading the weights
 // in 16-row boxes (64 gate and 64 up rows a tile) costs 132 us in place of 111: TMA instructions bound it then.
 //
 // Warp roles as in gemm.cu: warp 0 TMA producer (a lane per box), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.

@@ -97,7 +97,7 @@ class FusedConvRouter(torch.autograd.Function):
     """Causal-conv router (kernels/sm75/router.py:172-218, FusedConvRouterCuDNN): logits[b,s,e] =
     sum_{j,h} x[b, s-(K-1)+j, h] * W[e,h,j], then the same sigmoid / bias / top-k epilogue.  One tcgen05 GEMM
     whose TMA producer reads x in place, tap by tap, through an (H, S, B) tensor map (kernels/sm120/router.py:34-85 is one
-    launch too), or over an unfolded copy of x when H is no multiple of 16; the backward's top-k kernel lays the gradients
+    launch too), or over an unfolded copy of x (H no multiple of 16, many short sequences); the backward's top-k kernel lays the gradients
     out tap by tap, and dX and dW are plain products with that.  One native call each way (csrc/block.cu)."""
 
     @staticmethod
