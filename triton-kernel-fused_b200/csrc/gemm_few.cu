@@ -512,7 +512,7 @@ constexpr int64_t kFewRows64 = 40, kFewRows128 = 110;
 static int64_t few_blocks(int64_t N, int64_t K) { return ceil_div(std::max(N, K), 128); }   // weight blocks of an expert (either product)
 static bool few_one_wave(int64_t M, int E, int64_t N, int64_t K) { return (E + M / 64) * few_blocks(N, K) <= num_sms(); }
 
-static int few_tile(int64_t M, int E, int64_t N, int64_t K) {
+static int few_nt(int64_t M, int E, int64_t N, int64_t K) {
   if (M <= kFewRows64 * E || few_one_wave(M, E, N, K)) return 64;
   return M <= kFewRows128 * E ? 128 : 192;
 }
@@ -561,7 +561,7 @@ int b200moe_expert_gate_up_few(const void* x, const void* gate_up_proj, const in
   FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status};
   cudaStream_t st = (cudaStream_t)stream;
   // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
-  const int nt = few_tile(rows_cap, E, I, H);
+  const int nt = few_nt(rows_cap, E, I, H);
   if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
   if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
   return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
@@ -573,7 +573,7 @@ int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* count
   if (rc) return rc;
   FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status};
   cudaStream_t st = (cudaStream_t)stream;
-  const int nt = few_tile(rows_cap, E, N, K);
+  const int nt = few_nt(rows_cap, E, N, K);
   if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
   if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
   return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
