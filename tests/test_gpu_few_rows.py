@@ -72,3 +72,21 @@ def test_bad_expert_index_without_gradient(pkg):
                  torch.zeros(4, dtype=torch.int32, device=DEV))
     pkg.check_status()
     assert torch.equal(out, ok)
+
+
+# serving under skewed routing: frequencies ~ rank^-1.1, and every token's first pick on one expert; compact rows with 64-, 128- and
+# 192-row tiles, and row tiles
+@pytest.mark.parametrize("T,E,k,H,I", [(60, 32, 4, 264, 136), (900, 64, 6, 136, 520), (1500, 64, 6, 264, 520), (700, 8, 2, 1032, 1032)])
+@pytest.mark.parametrize("hot", [False, True])
+def test_skewed_forward_without_gradient_equals_the_training_forward(pkg, T, E, k, H, I, hot):
+    g = torch.Generator().manual_seed(T)
+    freq = torch.arange(1, E + 1).float().pow(-1.1).expand(T, E).clone()
+    freq[:, 0] *= 1e6 if hot else 1
+    idx = torch.multinomial(freq, k, generator=g).to(DEV)
+    rand = lambda *s: (torch.randn(*s, generator=g) * 0.1).to(torch.bfloat16).to(DEV)     # noqa: E731
+    x, gu, dn, w = rand(T, H), rand(E, 2 * I, H), rand(E, H, I).requires_grad_(), torch.rand(T, k, generator=g).to(DEV)
+    codes = torch.zeros(E, dtype=torch.int32, device=DEV)
+    with torch.no_grad():
+        quiet = pkg.moe(x, idx, w, gu, dn, codes)
+    assert torch.equal(quiet, pkg.moe(x, idx, w, gu, dn, codes).detach())
+    pkg.check_status()
