@@ -27,6 +27,7 @@ template <int TPR>
 __global__ void __launch_bounds__(256)
 combine_kernel(const uint4* __restrict__ rows, const float* __restrict__ w, const int* __restrict__ slot_row,
                const uint4* __restrict__ add, long long T, int k, int vec_per_row, uint4* __restrict__ out) {
+  grid_dep_begin();
   constexpr int G = 256 / TPR;
   for (long long t = static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; t < T;
        t += static_cast<long long>(gridDim.x) * G) {
@@ -63,6 +64,7 @@ __global__ void __launch_bounds__(256)
 combine_bwd_kernel(const uint4* __restrict__ go, const uint4* __restrict__ eo, const float* __restrict__ w,
                    const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k, int vec_per_row,
                    uint4* __restrict__ grad_eo, float* __restrict__ grad_w) {
+  grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const int total = *total_rows;
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(256)
 combine_bwd_narrow_kernel(const uint4* __restrict__ go, const uint4* __restrict__ eo, const float* __restrict__ w,
                           const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k, int vec_per_row,
                           uint4* __restrict__ grad_eo, float* __restrict__ grad_w) {
+  grid_dep_begin();
   constexpr int RB = 4;
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -172,14 +175,15 @@ int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_ro
   B200_CHECK_ARG(k >= 1 && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "combine: k = %d", k);
   B200_CHECK_ARG(aligned16(rows) && aligned16(out) && aligned16(add), B200MOE_E_ALIGN, "combine: pointers must be 16-byte aligned");
   if (T <= 0) return 0;
+  cudaError_t err = cudaSuccess;
   by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
     constexpr int G = 256 / tpr.value;
     const long long grid = std::min<long long>((T + G - 1) / G, static_cast<long long>(num_sms()) * 16);
-    combine_kernel<tpr.value><<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const uint4*>(rows), w, slot_row, reinterpret_cast<const uint4*>(add), T, k, static_cast<int>(H / 8),
-        reinterpret_cast<uint4*>(out));
+    err = launch_chained(combine_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
+                         reinterpret_cast<const uint4*>(rows), w, slot_row, reinterpret_cast<const uint4*>(add), T, k,
+                         static_cast<int>(H / 8), reinterpret_cast<uint4*>(out));
   });
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(err);
   return 0;
 }
 
@@ -196,10 +200,8 @@ int b200moe_combine_bwd(const void* grad_out, const void* eo, const float* w, co
   const int nvec = static_cast<int>(H / 8), rows_per_warp = nvec <= 32 ? 4 : 1;
   const long long grid = std::min<long long>((rows_cap + 8 * rows_per_warp - 1) / (8 * rows_per_warp), static_cast<long long>(num_sms()) * 8);
   auto kernel = nvec <= 32 ? combine_bwd_narrow_kernel : combine_bwd_kernel;
-  kernel<<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint4*>(grad_out), reinterpret_cast<const uint4*>(eo), w, row_slot, total_rows, k, nvec,
-      reinterpret_cast<uint4*>(grad_eo), grad_w);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(kernel, static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const uint4*>(grad_out),
+              reinterpret_cast<const uint4*>(eo), w, row_slot, total_rows, k, nvec, reinterpret_cast<uint4*>(grad_eo), grad_w);
   return 0;
 }
 

@@ -36,6 +36,12 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);
+// its products; early: counts and weights were complete before the kernel in front of the launch began (FewParams::early)
+int expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
+                       const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, int early, void* inter,
+                       int32_t* status, b200moe_stream_t stream);
+int expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap, int E,
+                      int64_t N, int64_t K, int early, void* out, int32_t* status, b200moe_stream_t stream);
 
 // gemm.cu: the products of the optimizer's iteration over part of their padded extents
 int expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t K, int mirror,
@@ -76,6 +82,43 @@ inline void by_row_threads(int nvec, F f) {
   else if (nvec <= 128) f(std::integral_constant<int, 128>());
   else f(std::integral_constant<int, 256>());
 }
+
+// Launch whose set-up may overlap the end of the kernel before it in the stream (programmatic stream serialisation).  Every
+// kernel launched this way calls grid_dep_wait() (ptx.cuh) in all of its threads before it reads or writes anything that
+// another kernel touches, and grid_dep_launch() only after that: when a kernel's first instruction runs, the kernel two
+// before it is complete, and past its wait the one before it too.  Why: between two plain launches the SMs idle for 1.5 to 4
+// us (drain, launch, barriers, tensor memory, descriptors), as long as the small kernels of a decoding step run.  The GEMMs
+// call grid_dep_launch() when their last loads are issued: early enough to hide a launch, and at their start it made large
+// training steps 1 % slower.  us a pass, plain / chained: 48 tokens, 64 experts of 2048 x 1408 (6 launches, with the weights
+// ahead of the wait, gemm_few.cu) 205 / 192; 1500 tokens 297 / 285; forward and backward of 3001 tokens, 32 experts of 1032 x
+// 680 (18 launches) 415 / 381; mixed stack of 16 384 tokens 408 / 384.
+// With SMs reserved for an exchange (b200moe_set_reserved_sms) the launch is a plain one: CTAs that wait would sit on them.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (gemm_cta_budget() == num_sms()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#define B200_LAUNCH(kernel, grid, block, smem, stream, ...) \
+  B200_CUDA(::b200moe::launch_chained(kernel, grid, block, smem, (cudaStream_t)(stream), 1, __VA_ARGS__))
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 

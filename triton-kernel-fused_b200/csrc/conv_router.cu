@@ -14,6 +14,7 @@ namespace b200moe {
 
 __global__ void __launch_bounds__(256)
 conv_unfold_kernel(const uint4* __restrict__ x, long long B, long long S, int K, int vec_h, uint4* __restrict__ xu) {
+  grid_dep_begin();
   const long long rows = B * S;
   for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
     const long long s = r % S;
@@ -73,9 +74,8 @@ int b200moe_conv_unfold(const void* x, int64_t B, int64_t S, int64_t H, int K, v
   long long grid = B * S;
   const long long cap = static_cast<long long>(num_sms()) * 16;
   if (grid > cap) grid = cap;
-  conv_unfold_kernel<<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint4*>(x), B, S, K, static_cast<int>(H / 8), reinterpret_cast<uint4*>(xu));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(conv_unfold_kernel, static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const uint4*>(x), B, S, K,
+              static_cast<int>(H / 8), reinterpret_cast<uint4*>(xu));
   return 0;
 }
 

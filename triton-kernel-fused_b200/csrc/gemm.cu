@@ -142,6 +142,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
+  grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
   __syncthreads();
@@ -318,6 +319,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
       }
     }
+    grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (lane == 0 && cta_rank == 0) {
@@ -743,19 +745,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(units * CTAS, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = C::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (CTAS > 1) ? 1 : 0;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<BN, EPI, CTAS, POLY>, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY>, units * CTAS, kThreads, C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 

@@ -35,6 +35,9 @@ struct FewParams {
   void* D;                // (rows, N) bf16
   const int* act_codes;   // SwiGLU: activation code of each expert, nullptr = SiLU
   int* status;
+  // Counts and weights were complete before the kernel in front of this one began: the first blocks of weights are loaded
+  // before the wait for that kernel, so its end and this one's start cost no time on the memory bus.
+  int early;
 };
 
 constexpr int kFewBK = 64;      // k-block: one 128-byte swizzle row
@@ -57,9 +60,10 @@ struct FewCfg {
 
 struct FewTile { int e, m0, row0, live; };
 
-// tile -> (expert, chunk of its rows, block of output columns); pre[] = exclusive prefix of the experts' chunk counts
+// tile -> (expert, chunk of its rows, block of output columns); pre[] = exclusive prefix of the experts' chunk counts.
+// before_wait: the tables are read from L2, since an L1 line may be older than the launch
 template <int NT, int TM>
-__device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, int tile) {
+__device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, int tile, bool before_wait = false) {
   const int mt = (p.N + TM - 1) / TM;
   const int c = tile / mt;
   int lo = 0, hi = p.E;                       // the last expert with pre[e] <= c
@@ -72,8 +76,8 @@ __device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, 
   t.e = lo;
   t.m0 = (tile - c * mt) * TM;
   const int first = (c - pre[lo]) * NT;
-  t.row0 = p.offs[lo] + first;
-  t.live = min(NT, p.counts[lo] - first);
+  t.row0 = (before_wait ? __ldcg(p.offs + lo) : p.offs[lo]) + first;
+  t.live = min(NT, (before_wait ? __ldcg(p.counts + lo) : p.counts[lo]) - first);
   return t;
 }
 
@@ -117,13 +121,14 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tmem_relinquish();
   }
+  if (!p.early) grid_dep_begin();
   if (warp == 2) {                       // prefix of the chunk counts: a lane takes 8 neighbouring experts
     constexpr int V = B200MOE_MAX_EXPERTS / 32;
     int c[V], sum = 0;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int e = lane * V + i;
-      c[i] = e < p.E ? (p.counts[e] + NT - 1) / NT : 0;
+      c[i] = e < p.E ? (__ldcg(p.counts + e) + NT - 1) / NT : 0;
       sum += c[i];
     }
     int incl = sum;
@@ -152,11 +157,12 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     // ------------------------------------------------------------------ TMA producer: lanes 0.. weights, then X boxes
     const bool isW = lane < HALVES;
     const int j = isW ? lane : lane - HALVES;
-    int s = 0;
+    int s = 0, ahead = 0;                // k-blocks of the first tile whose weights are on their way
     uint32_t ph = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-      const FewTile t = few_tile<NT, TM>(p, pre, tile);
+      const bool first = p.early && tile == static_cast<int>(blockIdx.x);
+      const FewTile t = few_tile<NT, TM>(p, pre, tile, first);
       const int nb = (t.live + kFewBox - 1) / kFewBox;
       const bool active = isW || j < nb;
       int c1, c2 = 0;
@@ -169,22 +175,35 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       const CUtensorMap* tm = isW ? &tmW : &tmX;
       const uint32_t dst = isW ? j * (128 * kFewBK * 2) : C::W_BYTES + j * (kFewBox * kFewBK * 2);
       const uint32_t bytes = C::W_BYTES + nb * (kFewBox * kFewBK * 2);
+      if (first) {
+        ahead = min(NSTAGE, nkb);        // every stage is empty
+        for (int kb = 0; kb < ahead; ++kb) {
+          if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * kb, bytes);
+          if (isW) tma_load_3d(smem_u32(smem + kb * C::STAGE_BYTES) + dst, tm, bar_full + 8 * kb, kb * kFewBK, c1, c2);
+        }
+        __syncwarp();
+        grid_dep_begin();                // what X holds comes from the kernel before
+      }
       for (int kb = 0; kb < nkb; ++kb) {
         if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
           ok = false;
           break;
         }
-        if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
-        if (active) tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, c2);
+        const bool have = kb < ahead;    // of the first tile only: `ahead` is 0 after it
+        if (lane == 0 && !have) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
+        if (active && !(have && isW))
+          tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, c2);
         if (++s == NSTAGE) {
           s = 0;
           ph ^= 1;
         }
       }
+      ahead = 0;
       ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
+    if (p.early) grid_dep_begin();
     if (lane == 0) {
       int s = 0, it = 0;
       uint32_t ph = 0;
@@ -226,6 +245,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     // ------------------------------------------------------------------ epilogue: lane = output column, register = row
     const int q = warp & 3;              // TMEM lane quarter this warp may read
     const int half = (warp - 2) >> 2;    // even or odd 16-row groups
+    if (p.early) grid_dep_begin();
     int it = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
       const FewTile t = few_tile<NT, TM>(p, pre, tile);
@@ -342,12 +362,15 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     mbar_init(bar_done, 1);
     *abort_flag = 0;
     fence_mbar_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
   }
   for (int e = threadIdx.x; e < p.E; e += blockDim.x) hist[e] = 0;
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), 32);
     tmem_relinquish();
   }
+  grid_dep_begin();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -474,8 +497,7 @@ static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows,
   const long long chunks = std::min<long long>(rows_cap, p.E + rows_cap / NT);   // at most
   const long long tiles = chunks * ceil_div(p.N, TM);
   const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(gemm_cta_budget(), tiles)));
-  few_rows_kernel<EPI, NT, HALVES><<<grid, kThreads, C::SMEM_BYTES, stream>>>(tmW, tmX, p);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH((few_rows_kernel<EPI, NT, HALVES>), grid, kThreads, C::SMEM_BYTES, stream, tmW, tmX, p);
   return 0;
 }
 
@@ -493,8 +515,7 @@ static int launch_router_few(const void* x, const void* weight, const RouterFewP
   if (rc) return rc;
   rc = make_map(&tmX, x, p.H, p.T, 1, p.H, static_cast<uint64_t>(p.T) * p.H, kFewBK, kRouterTokens);
   if (rc) return rc;
-  router_few_kernel<VPL><<<(p.T + kRouterTokens - 1) / kRouterTokens, kThreads, C::SMEM_BYTES, stream>>>(tmW, tmX, p);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(router_few_kernel<VPL>, (p.T + kRouterTokens - 1) / kRouterTokens, kThreads, C::SMEM_BYTES, stream, tmW, tmX, p);
   return 0;
 }
 
@@ -547,6 +568,32 @@ static int check_few(const char* who, const void* x, const void* w, const void* 
   return 0;
 }
 
+int expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
+                       const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, int early, void* inter,
+                       int32_t* status, b200moe_stream_t stream) {
+  int rc = check_few("expert_gate_up_few", x, gate_up_proj, inter, counts, offs, rows_cap, E, I, H);
+  if (rc) return rc;
+  FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status, early};
+  cudaStream_t st = (cudaStream_t)stream;
+  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
+  const int nt = few_nt(rows_cap, E, I, H);
+  if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+}
+
+int expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap, int E,
+                      int64_t N, int64_t K, int early, void* out, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_few("expert_linear_few", x, w, out, counts, offs, rows_cap, E, N, K);
+  if (rc) return rc;
+  FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status, early};
+  cudaStream_t st = (cudaStream_t)stream;
+  const int nt = few_nt(rows_cap, E, N, K);
+  if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
+  if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
+  return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
+}
+
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -556,27 +603,12 @@ extern "C" {
 int b200moe_expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
                                const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, void* inter,
                                int32_t* status, b200moe_stream_t stream) {
-  int rc = check_few("expert_gate_up_few", x, gate_up_proj, inter, counts, offs, rows_cap, E, I, H);
-  if (rc) return rc;
-  FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status};
-  cudaStream_t st = (cudaStream_t)stream;
-  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
-  const int nt = few_nt(rows_cap, E, I, H);
-  if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
-  if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
-  return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  return expert_gate_up_few(x, gate_up_proj, act_codes, counts, offs, rows_cap, E, H, I, 0, inter, status, stream);
 }
 
 int b200moe_expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap,
                               int E, int64_t N, int64_t K, void* out, int32_t* status, b200moe_stream_t stream) {
-  int rc = check_few("expert_linear_few", x, w, out, counts, offs, rows_cap, E, N, K);
-  if (rc) return rc;
-  FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status};
-  cudaStream_t st = (cudaStream_t)stream;
-  const int nt = few_nt(rows_cap, E, N, K);
-  if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
-  if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
-  return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
+  return expert_linear_few(x, w, counts, offs, rows_cap, E, N, K, 0, out, status, stream);
 }
 
 int b200moe_router_small_fwd(const void* x, const void* weight, const float* bias, int64_t T, int64_t H, int E, int k,

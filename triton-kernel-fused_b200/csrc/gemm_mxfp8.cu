@@ -112,6 +112,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tmem_relinquish();
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
+  grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
   __syncthreads();
@@ -150,6 +151,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
       }
     }
+    grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
     if (lane == 0) {   // ---------------------------------------------------------- MMA issuer
       int s = 0, it = 0;
@@ -401,6 +403,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     tmem_relinquish_pair();
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
+  grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
   __syncthreads();
@@ -448,6 +451,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
       }
     }
+    grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
     if (lane == 0 && cta_rank == 0) {   // --------------------------------------------- MMA issuer (leader)
       int s = 0, it = 0;
@@ -730,19 +734,8 @@ static int launch_fp8_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const
   int pairs = gemm_cta_budget() / 2;
   if (max_tiles > 0 && max_tiles < pairs) pairs = max_tiles;
   if (pairs < 1) pairs = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pairs * 2, 1, 1);
-  cfg.blockDim = dim3(kPThreads, 1, 1);
-  cfg.dynamicSmemBytes = PairCfg<EPI>::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, gemm_mxfp8_pair_kernel<EPI, FWD>, tmA, tmB, tmSFA, tmSFB, tmD, tmD2, fp));
+  B200_CUDA(launch_chained(gemm_mxfp8_pair_kernel<EPI, FWD>, pairs * 2, kPThreads, PairCfg<EPI>::kSmemBytes, stream, 2, tmA, tmB, tmSFA,
+                           tmSFB, tmD, tmD2, fp));
   return 0;
 }
 
@@ -769,8 +762,7 @@ static int launch_fp8(const CUtensorMap& tmA, const CUtensorMap& tmB, const Fp8P
   int grid = gemm_cta_budget();
   if (max_tiles > 0 && max_tiles < grid) grid = max_tiles;
   if (grid < 1) grid = 1;
-  gemm_mxfp8_kernel<EPI><<<grid, kThreads, kFSmemBytes, stream>>>(tmA, tmB, fp);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(gemm_mxfp8_kernel<EPI>, grid, kThreads, kFSmemBytes, stream, tmA, tmB, fp);
   return 0;
 }
 

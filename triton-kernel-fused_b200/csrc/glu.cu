@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(kRowThreads)
 glu_fwd_vec_kernel(const uint4* __restrict__ gate_up, const int* __restrict__ tile_expert, const int* __restrict__ codes,
                    const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
                    uint4* __restrict__ inter) {
+  grid_dep_begin();
   constexpr int RPB = kRowThreads / TPR;   // rows a CTA works on at a time; divides the 256-row tile
   __shared__ float red[kRowThreads / 32];
   const int total = *total_rows;
@@ -239,6 +240,7 @@ glu_bwd_vec_kernel(const uint4* __restrict__ grad_inter, const uint4* __restrict
                    const int* __restrict__ tile_expert, const int* __restrict__ codes,
                    const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
                    uint4* __restrict__ grad_gate_up, float* __restrict__ row_da, float* __restrict__ row_dg) {
+  grid_dep_begin();
   constexpr int RPB = kRowThreads / TPR;
   __shared__ float red[kRowThreads / 32];
   const int total = *total_rows;
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(256)
 glu_fwd_rows_kernel(const __nv_bfloat16* __restrict__ gate_up, const int* __restrict__ tile_expert,
                     const int* __restrict__ codes, const float* __restrict__ params, const int* __restrict__ total_rows,
                     int I, __nv_bfloat16* __restrict__ inter) {
+  grid_dep_begin();
   __shared__ float red[8];
   const int total = *total_rows;
   for (long long r = blockIdx.x; r < total; r += gridDim.x) {
@@ -321,6 +324,7 @@ glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ grad_inter, const __nv_bfl
                     const int* __restrict__ tile_expert, const int* __restrict__ codes,
                     const float* __restrict__ params, const int* __restrict__ total_rows, int I,
                     __nv_bfloat16* __restrict__ grad_gate_up, float* __restrict__ row_da, float* __restrict__ row_dg) {
+  grid_dep_begin();
   __shared__ float red[8];
   const int total = *total_rows;
   for (long long r = blockIdx.x; r < total; r += gridDim.x) {
@@ -411,6 +415,7 @@ constexpr int kSumThreads = 1024;
 __global__ void __launch_bounds__(kSumThreads)
 expert_row_sums_kernel(const float* __restrict__ row_da, const float* __restrict__ row_dg, const int* __restrict__ poffs,
                        float* __restrict__ out) {
+  grid_dep_begin();
   __shared__ float red[kSumThreads / 32];
   const int e = blockIdx.x;
   float a = 0.0f, b = 0.0f;
@@ -433,6 +438,7 @@ __global__ void __launch_bounds__(256)
 special_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ tile_expert, const int* __restrict__ codes,
                     const int* __restrict__ poffs, int first_special, int num_experts, int vec_per_row,
                     uint4* __restrict__ dst) {
+  grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int r0 = poffs[first_special], r1 = poffs[num_experts];
   for (long long r = r0 + static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; r < r1;
@@ -481,18 +487,17 @@ int b200moe_glu_fwd_rows(const void* gate_up, const int32_t* tile_expert, const 
   if (rows_cap <= 0) return 0;
   if (rows_in_registers(I, gate_up, inter, inter)) {
     const int nvec = static_cast<int>(I / 8);
+    cudaError_t err = cudaSuccess;
     by_row_width(nvec, [&](auto tpr, auto vpt) {
-      glu_fwd_vec_kernel<tpr.value, vpt.value><<<rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)), kRowThreads, 0, (cudaStream_t)stream>>>(
-          reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes, act_params, total_rows, nvec,
-          reinterpret_cast<uint4*>(inter));
+      err = launch_chained(glu_fwd_vec_kernel<tpr.value, vpt.value>, rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)),
+                           kRowThreads, 0, (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes,
+                           act_params, total_rows, nvec, reinterpret_cast<uint4*>(inter));
     });
-    B200_CUDA(cudaGetLastError());
+    B200_CUDA(err);
     return 0;
   }
-  glu_fwd_rows_kernel<<<rows_grid(rows_cap), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert, act_codes, act_params, total_rows, static_cast<int>(I),
-      reinterpret_cast<__nv_bfloat16*>(inter));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(glu_fwd_rows_kernel, rows_grid(rows_cap), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert,
+              act_codes, act_params, total_rows, static_cast<int>(I), reinterpret_cast<__nv_bfloat16*>(inter));
   return 0;
 }
 
@@ -506,18 +511,19 @@ int b200moe_glu_bwd_rows(const void* grad_inter, const void* gate_up, const int3
   if (rows_cap <= 0) return 0;
   if (rows_in_registers(I, grad_inter, gate_up, grad_gate_up)) {
     const int nvec = static_cast<int>(I / 8);
+    cudaError_t err = cudaSuccess;
     by_row_width(nvec, [&](auto tpr, auto vpt) {
-      glu_bwd_vec_kernel<tpr.value, vpt.value><<<rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)), kRowThreads, 0, (cudaStream_t)stream>>>(
-          reinterpret_cast<const uint4*>(grad_inter), reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes,
-          act_params, total_rows, nvec, reinterpret_cast<uint4*>(grad_gate_up), row_da, row_dg);
+      err = launch_chained(glu_bwd_vec_kernel<tpr.value, vpt.value>, rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)),
+                           kRowThreads, 0, (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(grad_inter),
+                           reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes, act_params, total_rows, nvec,
+                           reinterpret_cast<uint4*>(grad_gate_up), row_da, row_dg);
     });
-    B200_CUDA(cudaGetLastError());
+    B200_CUDA(err);
     return 0;
   }
-  glu_bwd_rows_kernel<<<rows_grid(rows_cap), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(grad_inter), reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert,
-      act_codes, act_params, total_rows, static_cast<int>(I), reinterpret_cast<__nv_bfloat16*>(grad_gate_up), row_da, row_dg);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(glu_bwd_rows_kernel, rows_grid(rows_cap), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(grad_inter),
+              reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert, act_codes, act_params, total_rows, static_cast<int>(I),
+              reinterpret_cast<__nv_bfloat16*>(grad_gate_up), row_da, row_dg);
   return 0;
 }
 
@@ -525,8 +531,7 @@ int b200moe_expert_row_sums(const float* row_da, const float* row_dg, const int3
                             b200moe_stream_t stream) {
   B200_CHECK_ARG(row_da && row_dg && poffs && out, B200MOE_E_NULL, "expert_row_sums: null pointer");
   B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_row_sums: E = %d", E);
-  expert_row_sums_kernel<<<E, kSumThreads, 0, (cudaStream_t)stream>>>(row_da, row_dg, poffs, out);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(expert_row_sums_kernel, E, kSumThreads, 0, stream, row_da, row_dg, poffs, out);
   return 0;
 }
 
@@ -538,12 +543,13 @@ int b200moe_special_rows(const void* src, const int32_t* tile_expert, const int3
                  "special_rows: H = %lld, first_special = %d, num_experts = %d", (long long)H, first_special, num_experts);
   B200_CHECK_ARG(aligned16(src) && aligned16(dst), B200MOE_E_ALIGN, "special_rows: pointers must be 16-byte aligned");
   if (rows_cap <= 0 || first_special == num_experts) return 0;
+  cudaError_t err = cudaSuccess;
   by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
-    special_rows_kernel<tpr.value><<<rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs, first_special, num_experts,
-        static_cast<int>(H / 8), reinterpret_cast<uint4*>(dst));
+    err = launch_chained(special_rows_kernel<tpr.value>, rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0,
+                         (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs,
+                         first_special, num_experts, static_cast<int>(H / 8), reinterpret_cast<uint4*>(dst));
   });
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(err);
   return 0;
 }
 

@@ -36,6 +36,7 @@ static PermSplit perm_split(long long M) {
 template <int W, int PL>
 __global__ void __launch_bounds__(32 * W)
 permute_hist_kernel(const long long* __restrict__ idx, long long M, int E, int* __restrict__ block_hist) {
+  grid_dep_begin();
   constexpr int kPermThreads = 32 * W;
   __shared__ int h[B200MOE_MAX_EXPERTS];
   for (int e = threadIdx.x; e < E; e += kPermThreads) h[e] = 0;
@@ -58,6 +59,7 @@ permute_rank_kernel(const long long* __restrict__ idx, long long M, int E, const
                     int* __restrict__ slot_row, int* __restrict__ row_slot, int* __restrict__ tile_expert,
                     int* __restrict__ order, int* __restrict__ slot_pos, int* __restrict__ counts_out,
                     long long* __restrict__ load, int* __restrict__ status) {
+  grid_dep_begin();
   constexpr int kPermWarps = W, kPermThreads = 32 * W;
   extern __shared__ int sh[];                          // [W][E]: ranks a warp's run starts at
   __shared__ int s_before[B200MOE_MAX_EXPERTS];        // slots of the expert in earlier CTAs
@@ -202,13 +204,10 @@ static int launch_permute(const long long* idx, long long M, int E, int* hist, i
   constexpr int run = 32 * W * PL;
   const int blocks = M > run ? static_cast<int>((M + run - 1) / run) : 1;
   if (blocks > 1) {
-    permute_hist_kernel<W, PL><<<blocks, 32 * W, 0, st>>>(idx, M, E, hist);
-    B200_CUDA(cudaGetLastError());
+    B200_LAUNCH((permute_hist_kernel<W, PL>), blocks, 32 * W, 0, st, idx, M, E, hist);
   }
-  permute_rank_kernel<W, PL><<<blocks, 32 * W, sizeof(int) * W * E, st>>>(
-      idx, M, E, hist, counts, offs, poffs, slot_row, row_slot, tile_expert, order, slot_pos, counts_out, load,
-      status);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH((permute_rank_kernel<W, PL>), blocks, 32 * W, sizeof(int) * W * E, st, idx, M, E, hist, counts, offs, poffs,
+              slot_row, row_slot, tile_expert, order, slot_pos, counts_out, load, status);
   return 0;
 }
 
@@ -219,6 +218,7 @@ template <int TPR>
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ row_slot,
                    const int* __restrict__ total_rows, int k, int vec_per_row, uint4* __restrict__ x_s) {
+  grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int total = *total_rows;
   for (long long r = static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; r < total;
@@ -286,13 +286,15 @@ int b200moe_gather_rows(const void* x, const int32_t* row_slot, const int32_t* t
   B200_CHECK_ARG(k >= 1, B200MOE_E_BAD_SHAPE, "gather_rows: k = %d", k);
   B200_CHECK_ARG(aligned16(x) && aligned16(x_s), B200MOE_E_ALIGN, "gather_rows: pointers must be 16-byte aligned");
   if (rows_cap <= 0) return 0;
+  cudaError_t err = cudaSuccess;
   by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
     constexpr int G = 256 / tpr.value;
     const long long grid = std::min<long long>((rows_cap + G - 1) / G, static_cast<long long>(num_sms()) * 16);
-    gather_rows_kernel<tpr.value><<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const uint4*>(x), row_slot, total_rows, k, static_cast<int>(H / 8), reinterpret_cast<uint4*>(x_s));
+    err = launch_chained(gather_rows_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
+                         reinterpret_cast<const uint4*>(x), row_slot, total_rows, k, static_cast<int>(H / 8),
+                         reinterpret_cast<uint4*>(x_s));
   });
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(err);
   return 0;
 }
 

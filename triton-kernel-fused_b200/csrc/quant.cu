@@ -33,6 +33,7 @@ __device__ __forceinline__ long long interleaved_row(long long r, long long I) {
 __global__ void __launch_bounds__(256)
 quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, long long C, long long interleave_I,
                   uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+  grid_dep_begin();
   const long long blocks_per_row = C >> 5;
   const long long k_chunks = (C + 127) >> 7;
   const long long total = R * blocks_per_row;
@@ -62,8 +63,8 @@ template <bool ROWS, bool GATHER = false>
 __global__ void __launch_bounds__(256, 4)
 quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R, long long C, long long interleave_I,
                   uint8_t* __restrict__ q_t, uint8_t* __restrict__ sf_t, uint8_t* __restrict__ q_r,
-                  uint8_t* __restrict__ sf_r, const int* __restrict__ row_slot = nullptr,
-                  const int* __restrict__ total_rows = nullptr, int k = 1) {
+                  uint8_t* __restrict__ sf_r, const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k) {
+  grid_dep_begin();
   // source row of matrix row r (nullptr = zero row)
   auto src_row = [&](long long g, long long r) -> const __nv_bfloat16* {
     if constexpr (GATHER) {
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(256)
 gather_quant_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_slot,
                     const int* __restrict__ total_rows, int k, long long C, __nv_bfloat16* __restrict__ x_s,
                     uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+  grid_dep_begin();
   const long long blocks_per_row = C >> 5;
   const long long k_chunks = (C + 127) >> 7;
   const long long total = static_cast<long long>(*total_rows) * blocks_per_row;
@@ -245,10 +247,8 @@ int b200moe_mxfp8_quant_rows(const void* x, int64_t R, int64_t C, int64_t interl
   long long grid = (total + 255) / 256;
   const long long cap = static_cast<long long>(num_sms()) * 32;
   if (grid > cap) grid = cap;
-  quant_rows_kernel<<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), R, C, interleave_I, reinterpret_cast<uint8_t*>(q),
-      reinterpret_cast<uint8_t*>(sf));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(quant_rows_kernel, static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), R, C,
+              interleave_I, reinterpret_cast<uint8_t*>(q), reinterpret_cast<uint8_t*>(sf));
   return 0;
 }
 
@@ -263,10 +263,8 @@ int b200moe_mxfp8_gather_quant(const void* x, const int32_t* row_slot, const int
   long long grid = (total + 255) / 256;
   const long long cap = static_cast<long long>(num_sms()) * 32;
   if (grid > cap) grid = cap;
-  gather_quant_kernel<<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), row_slot, total_rows, k, H, reinterpret_cast<__nv_bfloat16*>(x_s),
-      reinterpret_cast<uint8_t*>(q), reinterpret_cast<uint8_t*>(sf));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(gather_quant_kernel, static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), row_slot,
+              total_rows, k, H, reinterpret_cast<__nv_bfloat16*>(x_s), reinterpret_cast<uint8_t*>(q), reinterpret_cast<uint8_t*>(sf));
   return 0;
 }
 
@@ -276,15 +274,9 @@ static int launch_quant_tile(const void* x, long long G, long long R, long long 
   long long grid = tiles;
   const long long cap = static_cast<long long>(num_sms()) * 8;
   if (grid > cap) grid = cap;
-  if (q_r != nullptr)
-    quant_tile_kernel<true><<<static_cast<int>(grid), 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), G, R, C, interleave_I, reinterpret_cast<uint8_t*>(q_t),
-        reinterpret_cast<uint8_t*>(sf_t), reinterpret_cast<uint8_t*>(q_r), reinterpret_cast<uint8_t*>(sf_r));
-  else
-    quant_tile_kernel<false><<<static_cast<int>(grid), 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), G, R, C, 0, reinterpret_cast<uint8_t*>(q_t),
-        reinterpret_cast<uint8_t*>(sf_t), nullptr, nullptr);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(q_r != nullptr ? quant_tile_kernel<true> : quant_tile_kernel<false>, static_cast<int>(grid), 256, 0, stream,
+              reinterpret_cast<const __nv_bfloat16*>(x), G, R, C, q_r != nullptr ? interleave_I : 0, reinterpret_cast<uint8_t*>(q_t),
+              reinterpret_cast<uint8_t*>(sf_t), reinterpret_cast<uint8_t*>(q_r), reinterpret_cast<uint8_t*>(sf_r), nullptr, nullptr, 1);
   return 0;
 }
 
@@ -303,11 +295,9 @@ int b200moe_mxfp8_gather_quant_both(const void* x, const int32_t* row_slot, cons
   long long grid = tiles;
   const long long cap = static_cast<long long>(num_sms()) * 8;
   if (grid > cap) grid = cap;
-  quant_tile_kernel<true, true><<<static_cast<int>(grid), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), 1, rows_cap, H, 0, reinterpret_cast<uint8_t*>(q_t),
-      reinterpret_cast<uint8_t*>(sf_t), reinterpret_cast<uint8_t*>(q_rows), reinterpret_cast<uint8_t*>(sf_rows), row_slot,
-      total_rows, k);
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH((quant_tile_kernel<true, true>), static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), 1,
+              rows_cap, H, 0, reinterpret_cast<uint8_t*>(q_t), reinterpret_cast<uint8_t*>(sf_t), reinterpret_cast<uint8_t*>(q_rows),
+              reinterpret_cast<uint8_t*>(sf_rows), row_slot, total_rows, k);
   return 0;
 }
 

@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256)
 router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__ bias, long long T, int E,
                        int k, int norm, float scale, long long* __restrict__ idx_out,
                        float* __restrict__ w_out, int* __restrict__ counts) {
+  grid_dep_begin();
   __shared__ int hist[B200MOE_MAX_EXPERTS];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(256)
 router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restrict__ idx,
                        const float* __restrict__ grad_w, long long T, int E, int k, int norm, float scale, int S, int taps,
                        __nv_bfloat16* __restrict__ grad_logits) {
+  grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
@@ -153,6 +155,7 @@ router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restr
 __global__ void __launch_bounds__(256)
 conv_weight_rows_kernel(const __nv_bfloat16* __restrict__ w, int E, int H, int taps, int by_expert,
                         __nv_bfloat16* __restrict__ wt) {
+  grid_dep_begin();
   const long long n = static_cast<long long>(E) * H;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
     const long long e = i / H, h = i - e * H;
@@ -165,6 +168,7 @@ conv_weight_rows_kernel(const __nv_bfloat16* __restrict__ w, int E, int H, int t
 __global__ void __launch_bounds__(256)
 conv_weight_grad_kernel(const float* __restrict__ p, long long slices, int E, int H, int taps,
                         __nv_bfloat16* __restrict__ gw) {
+  grid_dep_begin();
   const long long n = static_cast<long long>(E) * H, elems = n * taps;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < elems; i += gridDim.x * 256LL) {
     const long long j = i / n, eh = i - j * n;       // consecutive threads: consecutive h of one row of p
@@ -197,6 +201,7 @@ __global__ void router_bias_update_kernel(float* bias, const int* counts, int E,
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ P, long long slices, long long elems,
                      __nv_bfloat16* __restrict__ D) {
+  grid_dep_begin();
   const long long i4 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i4 >= elems) return;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -214,6 +219,7 @@ splitk_reduce_kernel(const float* __restrict__ P, long long slices, long long el
 // value so that all its slices are in flight at once
 __global__ void __launch_bounds__(1024)
 splitk_reduce_t_kernel(const float* __restrict__ P, long long slices, int R, int C, __nv_bfloat16* __restrict__ D) {
+  grid_dep_begin();
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -238,16 +244,17 @@ static int grid_for_tokens(long long T) {
 }
 
 template <int KIND>
-static void launch_topk_bwd(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k, int norm,
+static cudaError_t launch_topk_bwd(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k, int norm,
                             float scale, int S, int taps, __nv_bfloat16* out, cudaStream_t st) {
   const int grid = grid_for_tokens(T);
+  cudaError_t err = cudaSuccess;
   by_experts(E, [&](auto v) {
     constexpr int VPL = v.value;
-    if (VPL > 1 && E % 2 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0)
-      router_topk_bwd_kernel<KIND, VPL, (VPL > 1)><<<grid, 256, 0, st>>>(logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
-    else
-      router_topk_bwd_kernel<KIND, VPL, false><<<grid, 256, 0, st>>>(logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
+    const bool pair = VPL > 1 && E % 2 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0;
+    err = launch_chained(pair ? router_topk_bwd_kernel<KIND, VPL, (VPL > 1)> : router_topk_bwd_kernel<KIND, VPL, false>, grid, 256, 0,
+                         st, 1, logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
   });
+  return err;
 }
 
 }  // namespace b200moe
@@ -270,21 +277,22 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
   if (T == 0) return 0;
   const int grid = grid_for_tokens(T);
   long long* idx_ll = reinterpret_cast<long long*>(idx);
+  cudaError_t err = cudaSuccess;
   switch (input_kind) {
     case B200MOE_LOGITS_BF16:
-      by_experts(E, [&](auto v) { router_topk_fwd_kernel<B200MOE_LOGITS_BF16, v.value><<<grid, 256, 0, st>>>(input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
+      by_experts(E, [&](auto v) { err = launch_chained(router_topk_fwd_kernel<B200MOE_LOGITS_BF16, v.value>, grid, 256, 0, st, 1, input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
       break;
     case B200MOE_LOGITS_F32:
-      by_experts(E, [&](auto v) { router_topk_fwd_kernel<B200MOE_LOGITS_F32, v.value><<<grid, 256, 0, st>>>(input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
+      by_experts(E, [&](auto v) { err = launch_chained(router_topk_fwd_kernel<B200MOE_LOGITS_F32, v.value>, grid, 256, 0, st, 1, input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
       break;
     case B200MOE_SCORES_F32:
-      by_experts(E, [&](auto v) { router_topk_fwd_kernel<B200MOE_SCORES_F32, v.value><<<grid, 256, 0, st>>>(input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
+      by_experts(E, [&](auto v) { err = launch_chained(router_topk_fwd_kernel<B200MOE_SCORES_F32, v.value>, grid, 256, 0, st, 1, input, bias, T, E, k, norm_topk, scale, idx_ll, w, counts); });
       break;
     default:
       set_error("router_topk_fwd: unknown input_kind %d", input_kind);
       return B200MOE_E_UNSUPPORTED;
   }
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(err);
   return 0;
 }
 
@@ -300,16 +308,15 @@ int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* i
   __nv_bfloat16* gl = reinterpret_cast<__nv_bfloat16*>(grad_logits);
   switch (input_kind) {
     case B200MOE_LOGITS_BF16:
-      launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st);
+      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st));
       break;
     case B200MOE_LOGITS_F32:
-      launch_topk_bwd<B200MOE_LOGITS_F32>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st);
+      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_F32>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st));
       break;
     default:
       set_error("router_topk_bwd: input_kind %d has no backward (logits are required)", input_kind);
       return B200MOE_E_UNSUPPORTED;
   }
-  B200_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -321,9 +328,9 @@ int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* g
   B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "conv_topk_bwd: top_k = %d", k);
   B200_CHECK_ARG(B >= 1 && S >= 1 && S < (1LL << 31) && taps >= 1 && taps <= 64, B200MOE_E_BAD_SHAPE,
                  "conv_topk_bwd: B = %lld, S = %lld, taps = %d (1..64)", (long long)B, (long long)S, taps);
-  launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, reinterpret_cast<const long long*>(idx), grad_w, B * S, E, k, norm_topk, scale,
-                                       static_cast<int>(S), taps, reinterpret_cast<__nv_bfloat16*>(u), (cudaStream_t)stream);
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, reinterpret_cast<const long long*>(idx), grad_w, B * S, E, k, norm_topk,
+                                                 scale, static_cast<int>(S), taps, reinterpret_cast<__nv_bfloat16*>(u),
+                                                 (cudaStream_t)stream));
   return 0;
 }
 
@@ -335,9 +342,8 @@ int b200moe_conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_e
   B200_CHECK_ARG(w && wt, B200MOE_E_NULL, "conv_weight_rows: null pointer");
   B200_CHECK_ARG(E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE, "conv_weight_rows: E = %d, H = %lld, taps = %d", E,
                  (long long)H, taps);
-  conv_weight_rows_kernel<<<weight_grid(E * H), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(w), E, static_cast<int>(H), taps, by_expert, reinterpret_cast<__nv_bfloat16*>(wt));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(conv_weight_rows_kernel, weight_grid(E * H), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(w), E,
+              static_cast<int>(H), taps, by_expert, reinterpret_cast<__nv_bfloat16*>(wt));
   return 0;
 }
 
@@ -346,9 +352,8 @@ int b200moe_conv_weight_grad(const float* P, int64_t slices, int E, int64_t H, i
   B200_CHECK_ARG(P && grad_w, B200MOE_E_NULL, "conv_weight_grad: null pointer");
   B200_CHECK_ARG(slices >= 1 && E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE,
                  "conv_weight_grad: slices = %lld, E = %d, H = %lld, taps = %d", (long long)slices, E, (long long)H, taps);
-  conv_weight_grad_kernel<<<weight_grid(E * H * taps), 256, 0, (cudaStream_t)stream>>>(
-      P, slices, E, static_cast<int>(H), taps, reinterpret_cast<__nv_bfloat16*>(grad_w));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(conv_weight_grad_kernel, weight_grid(E * H * taps), 256, 0, stream, P, slices, E, static_cast<int>(H), taps,
+              reinterpret_cast<__nv_bfloat16*>(grad_w));
   return 0;
 }
 
@@ -366,9 +371,8 @@ int b200moe_splitk_reduce_t(const float* P, int64_t slices, int64_t R, int64_t C
   B200_CHECK_ARG(slices >= 1 && R > 0 && C > 0 && R < (1LL << 31) && C <= 32 * 65535, B200MOE_E_BAD_SHAPE,
                  "splitk_reduce_t: slices = %lld, R = %lld, C = %lld", (long long)slices, (long long)R, (long long)C);
   const dim3 grid(static_cast<unsigned>((R + 31) / 32), static_cast<unsigned>((C + 31) / 32));
-  splitk_reduce_t_kernel<<<grid, 1024, 0, (cudaStream_t)stream>>>(P, slices, static_cast<int>(R), static_cast<int>(C),
-                                                                 reinterpret_cast<__nv_bfloat16*>(D));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(splitk_reduce_t_kernel, grid, 1024, 0, stream, P, slices, static_cast<int>(R), static_cast<int>(C),
+              reinterpret_cast<__nv_bfloat16*>(D));
   return 0;
 }
 
@@ -379,8 +383,7 @@ int b200moe_splitk_reduce(const float* P, int64_t slices, int64_t elems, void* D
                  (long long)elems);
   const long long threads = elems / 4;
   const int grid = static_cast<int>((threads + 255) / 256);
-  splitk_reduce_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(P, slices, elems, reinterpret_cast<__nv_bfloat16*>(D));
-  B200_CUDA(cudaGetLastError());
+  B200_LAUNCH(splitk_reduce_kernel, grid, 256, 0, stream, P, slices, elems, reinterpret_cast<__nv_bfloat16*>(D));
   return 0;
 }
 
