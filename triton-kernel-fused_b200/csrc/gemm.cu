@@ -159,60 +159,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (each CTA)
-    if constexpr (CTAS == 2 && !CONV) {
-      // Pair tiles: the up to four boxes of a stage (one or two of A, one or two of B) are issued by four lanes in
-      // ONE instruction, each lane with its own tensor map, destination and coordinates, instead of by one lane
-      // in up to four instructions.  The producer's time between "stage free" and "loads issued" is what an empty
-      // ring waits for: with both operands MN-major (the weight-gradient GEMMs, four boxes per stage) the
-      // one-lane producer could not keep up with the MMAs, and this form made those launches 12-13 % faster.
-      if (lane < 4) {
-        const bool isA = lane < 2;
-        const int j = lane & 1;
-        const bool mn = isA ? (p.a_mn != 0) : (EPI != EPI_SWIGLU && p.b_mn != 0);
-        const int nbox = !mn ? 1 : (isA ? BM / 64 : BNC / 64);
-        const bool active = j < nbox;
-        const CUtensorMap* tm = isA ? &tmA : &tmB;
-        const uint32_t dst_off = (isA ? 0u : static_cast<uint32_t>(C::A_BYTES)) + static_cast<uint32_t>(j) * (64 * BK * 2);
-        const uint32_t full0 = mapa_shared(bar_full, 0);
-        const bool expects = (lane == 0 && cta_rank == 0);
-        int s = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int tile = first_tile; tile < total && ok; tile += tile_step) {
-          const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
-          const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
-          const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
-          const int bstep = pair_cols<BN, EPI>(p, t.n0) / 2;
-          // this lane's box: the coordinate that does not move with k, and the group
-          int fixed, grp;
-          if (isA) {
-            fixed = m0 + (mn ? 64 * j : 0);
-            grp = 0;
-          } else if constexpr (EPI == EPI_SWIGLU) {
-            fixed = t.n0;
-            grp = 2 * gB + static_cast<int>(cta_rank);
-          } else {
-            fixed = t.n0 + bstep * static_cast<int>(cta_rank) + (mn ? 64 * j : 0);
-            grp = gB;
-          }
-          int kk = t.k0;
-          for (int kb = 0; kb < t.nkb; ++kb, kk += BK) {
-            if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
-              ok = false;
-              break;
-            }
-            if (expects) mbar_arrive_expect_tx(bar_full + 8 * s, 2 * C::STAGE_BYTES);
-            if (active)
-              tma_load_3d_pair(smem_u32(smem + s * C::STAGE_BYTES) + dst_off, tm, full0 + 8 * s, mn ? fixed : kk,
-                               mn ? kk : fixed, grp);
-            if (++s == NSTAGE) {
-              s = 0;
-              ph ^= 1;
-            }
-          }
-        }
-      }
-    } else if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -322,7 +269,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       // K-major: rows are 128 B apart, 8-row groups 1024 B apart, 16 k-elements = 32 B.
       // MN-major: 64-wide MN blocks are 64*128 B apart (LBO), 8 k-rows 1024 B apart (SBO),
       //           16 k-rows = 2048 B.

@@ -121,7 +121,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int total = total_tiles(p, TN, BM);
 
   if (warp == 0) {
-    if (lane == 0) {   // ---------------------------------------------------------- producer
+    if (elect_one()) {   // ------------------------------------------------------- producer
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -153,7 +153,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
-    if (lane == 0) {   // ---------------------------------------------------------- MMA issuer
+    if (elect_one()) {   // ------------------------------------------------------- MMA issuer
       int s = 0, it = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -415,14 +415,8 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------ producer (each CTA)
-    // The four boxes of a stage (A, B, the A scale atom, the two B scale atoms) are issued by four lanes in ONE
-    // instruction, each lane with its own tensor map, destination and coordinates: four instructions from one lane
-    // took longer than the MMAs of a stage, and the ring ran dry.
-    if (lane < 4) {
-      const CUtensorMap* tm = lane == 0 ? &tmA : lane == 1 ? &tmB : lane == 2 ? &tmSFA : &tmSFB;
-      const uint32_t dst_off = lane == 0 ? 0u : lane == 1 ? kATile : lane == 2 ? kATile + kBTile : kATile + kBTile + kSfAtom;
+    if (elect_one()) {
       const uint32_t full0 = mapa_shared(bar_full, 0);              // the leader's barrier counts both CTAs
-      const bool expects = (lane == 0 && cta_rank == 0);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -430,20 +424,21 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         const Tile t = get_tile(p, tile, TN, TM, FBK, order);
         const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
         const int m0 = t.m0 + BM * cta_rank;
-        const int rb_a = m0 >> 7;
         const int rb_b = static_cast<int>((static_cast<long long>(gB) * fp.b_rows_per_group + t.n0) >> 7);
-        // data boxes: (k, row, group); scale atoms: (0, k chunk of 128, 128-row block)
-        const int c1_fixed = lane == 0 ? m0 : t.n0 + 128 * cta_rank;
-        const int c2 = lane == 0 ? 0 : lane == 1 ? gB : lane == 2 ? rb_a : rb_b;
         for (int kb = 0; kb < t.nkb; ++kb) {
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
             ok = false;
             break;
           }
-          if (expects) mbar_arrive_expect_tx(bar_full + 8 * s, 2 * (kATile + kBTile + 3 * kSfAtom));
+          const uint32_t full = full0 + 8 * s;
+          if (cta_rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2 * (kATile + kBTile + 3 * kSfAtom));
+          const uint32_t sa = smem_u32(smem + s * kPStage);
           const int kk = t.k0 + kb * FBK;
-          tma_load_3d_pair(smem_u32(smem + s * kPStage) + dst_off, tm, full0 + 8 * s, lane < 2 ? kk : 0,
-                           lane < 2 ? c1_fixed : (kk >> 7), c2);
+          // data boxes: (k, row, group); scale atoms: (0, k chunk of 128, 128-row block)
+          tma_load_3d_pair(sa, &tmA, full, kk, m0, 0);
+          tma_load_3d_pair(sa + kATile, &tmB, full, kk, t.n0 + 128 * cta_rank, gB);
+          tma_load_3d_pair(sa + kATile + kBTile, &tmSFA, full, 0, kk >> 7, m0 >> 7);
+          tma_load_3d_pair(sa + kATile + kBTile + kSfAtom, &tmSFB, full, 0, kk >> 7, rb_b);
           if (++s == kPStages) {
             s = 0;
             ph ^= 1;
@@ -453,7 +448,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     }
     grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
-    if (lane == 0 && cta_rank == 0) {   // --------------------------------------------- MMA issuer (leader)
+    if (cta_rank == 0 && elect_one()) {   // ------------------------------------------- MMA issuer (leader)
       int s = 0, it = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -500,7 +495,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // own, stages ahead of the MMAs, instead of in the MMA thread's instruction stream directly before the
     // MMAs that read them.  A stage's scale columns are free again once the stage itself was refilled: the
     // producer waited for the commit that followed the MMAs reading them.
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
