@@ -90,3 +90,47 @@ def test_skewed_forward_without_gradient_equals_the_training_forward(pkg, T, E, 
         quiet = pkg.moe(x, idx, w, gu, dn, codes)
     assert torch.equal(quiet, pkg.moe(x, idx, w, gu, dn, codes).detach())
     pkg.check_status()
+
+
+def test_few_rows_products_into_unaligned_memory(pkg):
+    """Results that are not 16-byte aligned are written value by value, and nothing beside them."""
+    L, ops = pkg.lib(), pkg.ops
+    for counts, H, I in (([5, 0, 40], 72, 136), ([180, 150, 170, 192] * 8, 136, 1032)):     # 64- and 192-row tiles
+        E, M = len(counts), sum(counts)
+        g = torch.Generator().manual_seed(M)
+        idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(M, generator=g)].view(M, 1).to(DEV)
+        x = torch.randn(M, H, generator=g).to(torch.bfloat16).to(DEV)
+        gu = (torch.randn(E, 2 * I, H, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+        dn = (torch.randn(E, H, I, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+        perm = ops.permute_build(idx, E, want_order=True)
+        xs = ops.gather_compact(x, perm)
+        inter = ops.expert_gate_up_few(xs, gu, perm, None)
+        out = ops.expert_linear_few(inter, dn, perm)
+        st, stream = torch.zeros(1, dtype=torch.int32, device=DEV), torch.cuda.current_stream().cuda_stream
+        for shift in (1, 4):
+            a, b = (torch.full((M * w + 16,), 7.0, dtype=torch.bfloat16, device=DEV) for w in (I, H))
+            assert L.b200moe_expert_gate_up_few(xs.data_ptr(), gu.data_ptr(), None, perm.counts.data_ptr(), perm.offs.data_ptr(), M, E,
+                                                H, I, a.data_ptr() + 2 * shift, st.data_ptr(), stream) == 0
+            assert L.b200moe_expert_linear_few(inter.data_ptr(), dn.data_ptr(), perm.counts.data_ptr(), perm.offs.data_ptr(), M, E, H,
+                                               I, b.data_ptr() + 2 * shift, st.data_ptr(), stream) == 0
+            for got, want in ((a, inter), (b, out)):
+                n = want.numel()
+                assert torch.equal(got[shift:shift + n], want.flatten())
+                assert (got[:shift] == 7).all() and (got[shift + n:] == 7).all()
+        assert int(st) == 0
+
+
+# k-blocks of 64 channels in pairs: one, an odd number, a remainder of 8; experts up to one and several per lane
+@pytest.mark.parametrize("H,E,k", [(8, 8, 1), (64, 32, 4), (72, 40, 8), (192, 64, 6), (200, 128, 8), (1032, 128, 2)])
+def test_small_router_equals_the_large_batch(pkg, H, E, k):
+    g = torch.Generator().manual_seed(H)
+    T = 16 * torch.cuda.get_device_properties(0).multi_processor_count      # the most tokens of one launch
+    x = torch.randn(T + 1, H, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E, H, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    bias = (torch.randn(E, generator=g) * 0.1).to(DEV)
+    big = pkg.fused_mlp_router(x, w, bias, k, E, return_counts=True)
+    for n in (1, 17, T):
+        idx, wt, counts = pkg.fused_mlp_router(x[:n], w, bias, k, E, return_counts=True)
+        assert torch.equal(idx, big[0][:n]) and torch.equal(wt, big[1][:n])
+        assert torch.equal(counts.cpu(), torch.bincount(idx.flatten().cpu(), minlength=E).int())
+    pkg.check_status()

@@ -360,6 +360,24 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t 
 }
 
 
+// A gate|up stack (E, 2I, K) as {K, 8, 2, I/8, E}: a box of {64, 8, 2, 8, 1} holds eight groups of 8 gate rows and the 8 up rows of
+// the same columns, so that a 16-lane block of an accumulator has gate and up of 8 columns in the same threads
+static inline int make_map_gate_up(CUtensorMap* tm, const void* base, uint64_t K, uint64_t I, uint64_t E, uint32_t groups) {
+  EncodeTiledFn fn = get_encode_fn();
+  B200_CHECK_ARG(fn != nullptr, B200MOE_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  B200_CHECK_ARG(aligned16(base), B200MOE_E_ALIGN, "tensor base %p is not 16-byte aligned", base);
+  cuuint64_t dims[5] = {K, 8, 2, I / 8, E};
+  cuuint64_t strides[4] = {K * 2, I * K * 2, 16 * K, 4 * I * K};
+  cuuint32_t box[5] = {64, 8, 2, groups, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  B200_CHECK_ARG(r == CUDA_SUCCESS, B200MOE_E_CUDA, "cuTensorMapEncodeTiled failed (%d): gate|up stack of %llu x %llu x %llu", (int)r,
+                 (unsigned long long)E, (unsigned long long)(2 * I), (unsigned long long)K);
+  return 0;
+}
+
 static inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
 }  // namespace b200moe

@@ -9,11 +9,14 @@
 // (no pad rows), 16-row boxes of it are loaded up to the last live row, and the accumulator holds output columns in
 // its lanes and rows in its columns.  A box may reach past the expert's rows: they only feed accumulator columns that
 // are not stored.
-// H 2048, I 1408, 64 experts, 288 rows (4.5 an expert; 118 + 59 us at copy rate): gate/up 161 -> 111 us, down 80 -> 60 us;
-// 9000 rows (141 an expert): 171 -> 148 and 85 -> 78 us; 6 rows of one token: 21 -> 19 and 15 -> 12 us.  Loading the weights
-// in 16-row boxes (64 gate and 64 up rows a tile) costs 132 us in place of 111: TMA instructions bound it then.
+// H 2048, I 1408, 64 experts, us as row tiles / here: 288 rows (4.5 an expert; 118 + 59 us at copy rate): gate/up 161 / 108, down 80 /
+// 60; 9000 rows (141 an expert): 171 / 151 and 85 / 75; 6 rows of one token: 21 / 12.3 and 15 / 9.2.
+// A large tile is bound by the bytes that leave L2 (weights in and out, X once per 128 columns) and wants them in flight: with a
+// stage less the 9000 rows take 157 us.  A small one is bound by latencies and by what a stage costs the two threads that
+// issue it: one lane for all boxes, elected (ptx.cuh), 128-row weight boxes that hold gate and up (make_map_gate_up), and tiles of 64
+// columns where even they are one wave; with a lane per box and tiles of 128 one token took 18.3 and 11.1 us.
 //
-// Warp roles as in gemm.cu: warp 0 TMA producer (a lane per box), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.
+// Warp roles as in gemm.cu: warp 0 TMA producer (one lane), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -35,25 +38,30 @@ struct FewParams {
   void* D;                // (rows, N) bf16
   const int* act_codes;   // SwiGLU: activation code of each expert, nullptr = SiLU
   int* status;
+  int aligned;            // D is 16-byte aligned
   // Counts and weights were complete before the kernel in front of this one began: the first blocks of weights are loaded
   // before the wait for that kernel, so its end and this one's start cost no time on the memory bus.
   int early;
 };
 
 constexpr int kFewBK = 64;      // k-block: one 128-byte swizzle row
-constexpr int kFewBox = 16;     // rows of X per TMA box = granularity of the MMA's N
+constexpr int kFewBox = 16;     // rows of X of the small TMA box = granularity of the MMA's N
+constexpr int kFewBig = 64;     // rows of the large one: a box costs the producer 45 cycles, whatever its size
 
-// NT: most rows of one tile.  HALVES: 128-row weight blocks per stage, each with an accumulator of its own (SwiGLU:
-// gate and up).  A CTA streams HALVES * 16 KB of weights for every live * 128 bytes of X a k-block.
-template <int NT, int HALVES>
+// NT: most rows of one tile.  HALVES: 128-row weight blocks per stage, each with an accumulator of its own.  A SwiGLU block is 64
+// gate rows and the 64 up rows of the same columns, eight and eight (make_map_gate_up).
+// A CTA streams HALVES * 16 KB of weights for every live * 128 bytes of X a k-block.
+template <int EPI, int NT, int HALVES>
 struct FewCfg {
+  static constexpr int BLOCK_COLS = EPI == EPI_SWIGLU ? 64 : 128;   // output columns of a weight block
+  static constexpr int TM = BLOCK_COLS * HALVES;
   static constexpr int W_BYTES = HALVES * 128 * kFewBK * 2;
   static constexpr int X_BYTES = NT * kFewBK * 2;
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
-  static constexpr int kFit = (232448 - 1024 - 2048) / STAGE_BYTES;
-  static constexpr int NSTAGE = kFit > 8 ? 8 : kFit;
-  static constexpr int ACC_COLS = HALVES * NT;                  // one tile's accumulators
+  static constexpr int ACC_COLS = HALVES * NT;                      // one tile's accumulators
   static constexpr int NBUF = 2 * ACC_COLS <= 512 ? 2 : 1;
+  static constexpr int kFit = (232448 - 3072) / STAGE_BYTES;
+  static constexpr int NSTAGE = kFit > 8 ? 8 : kFit;
   static constexpr int TMEM_COLS = NBUF * ACC_COLS > 256 ? 512 : NBUF * ACC_COLS > 128 ? 256 : 128;
   static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + (2 * NSTAGE + 2 * NBUF) * 8 + 16 + 1024;
 };
@@ -83,12 +91,11 @@ __device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, 
 
 template <int EPI, int NT, int HALVES>
 __global__ void __launch_bounds__(kThreads, 1)
-few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const FewParams p) {
-  using C = FewCfg<NT, HALVES>;
+few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                const __grid_constant__ CUtensorMap tmXbig, const FewParams p) {
+  using C = FewCfg<EPI, NT, HALVES>;
   constexpr int NSTAGE = C::NSTAGE, NBUF = C::NBUF;
-  constexpr int TM = (EPI == EPI_SWIGLU) ? 128 : 128 * HALVES;   // output columns of a tile
-  static_assert(EPI != EPI_SWIGLU || HALVES == 2, "SwiGLU needs the gate and the up accumulator");
-  static_assert(HALVES + NT / kFewBox <= 32, "a lane per box");
+  constexpr int TM = C::TM;                               // output columns of a tile
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -116,6 +123,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     fence_mbar_init();
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
+    if (NT > kFewBig) tma_prefetch_desc(&tmXbig);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -154,57 +162,59 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const int nkb = (p.K + kFewBK - 1) / kFewBK;
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer: lanes 0.. weights, then X boxes
-    const bool isW = lane < HALVES;
-    const int j = isW ? lane : lane - HALVES;
-    int s = 0, ahead = 0;                // k-blocks of the first tile whose weights are on their way
-    uint32_t ph = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-      const bool first = p.early && tile == static_cast<int>(blockIdx.x);
-      const FewTile t = few_tile<NT, TM>(p, pre, tile, first);
-      const int nb = (t.live + kFewBox - 1) / kFewBox;
-      const bool active = isW || j < nb;
-      int c1, c2 = 0;
-      if (isW) {
-        c1 = (EPI == EPI_SWIGLU) ? t.m0 : t.m0 + 128 * j;
-        c2 = (EPI == EPI_SWIGLU) ? 2 * t.e + j : t.e;
-      } else {
-        c1 = t.row0 + kFewBox * j;
-      }
-      const CUtensorMap* tm = isW ? &tmW : &tmX;
-      const uint32_t dst = isW ? j * (128 * kFewBK * 2) : C::W_BYTES + j * (kFewBox * kFewBK * 2);
-      const uint32_t bytes = C::W_BYTES + nb * (kFewBox * kFewBK * 2);
-      if (first) {
-        ahead = min(NSTAGE, nkb);        // every stage is empty
-        for (int kb = 0; kb < ahead; ++kb) {
-          if (lane == 0) mbar_arrive_expect_tx(bar_full + 8 * kb, bytes);
-          if (isW) tma_load_3d(smem_u32(smem + kb * C::STAGE_BYTES) + dst, tm, bar_full + 8 * kb, kb * kFewBK, c1, c2);
+    // ------------------------------------------------------------------ TMA producer
+    // One lane issues all boxes of a stage: about 210 cycles a k-block for its waits and 45 a box (measured before it was elected).
+    // With a lane per box of 16 rows, the whole warp waiting, it was 510 + 54 a box: at 144 rows twice what the MMAs take.
+    if (elect_one()) {
+      int s = 0, ahead = 0;              // k-blocks of the first tile whose weights are on their way
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+        const bool first = p.early && tile == static_cast<int>(blockIdx.x);
+        const FewTile t = few_tile<NT, TM>(p, pre, tile, first);
+        const int nbig = NT > kFewBig ? (t.live + kFewBox - 1) / kFewBig : 0;
+        const int nsmall = max(0, (t.live - nbig * kFewBig + kFewBox - 1) / kFewBox);
+        const uint32_t bytes = C::W_BYTES + nbig * (kFewBig * kFewBK * 2) + nsmall * (kFewBox * kFewBK * 2);
+        auto load_w = [&](int kb, int st) {
+          const uint32_t dst = smem_u32(smem + st * C::STAGE_BYTES);
+          mbar_arrive_expect_tx(bar_full + 8 * st, bytes);
+#pragma unroll
+          for (int h = 0; h < HALVES; ++h) {
+            if constexpr (EPI == EPI_SWIGLU)
+              tma_load_5d(dst + h * (128 * kFewBK * 2), &tmW, bar_full + 8 * st, kb * kFewBK, 0, 0, t.m0 / 8 + 8 * h, t.e);
+            else
+              tma_load_3d(dst + h * (128 * kFewBK * 2), &tmW, bar_full + 8 * st, kb * kFewBK, t.m0 + 128 * h, t.e);
+          }
+        };
+        if (first) {
+          ahead = min(NSTAGE, nkb);      // every stage is empty
+          for (int kb = 0; kb < ahead; ++kb) load_w(kb, kb);
+          grid_dep_begin();              // what X holds comes from the kernel before
         }
-        __syncwarp();
-        grid_dep_begin();                // what X holds comes from the kernel before
-      }
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
-          ok = false;
-          break;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
+            ok = false;
+            break;
+          }
+          if (kb >= ahead) load_w(kb, s);          // `ahead` is 0 after the first tile
+          const uint32_t dst = smem_u32(smem + s * C::STAGE_BYTES) + C::W_BYTES;
+          for (int j = 0; j < nbig; ++j)
+            tma_load_3d(dst + j * (kFewBig * kFewBK * 2), &tmXbig, bar_full + 8 * s, kb * kFewBK, t.row0 + kFewBig * j, 0);
+          for (int j = 0; j < nsmall; ++j)
+            tma_load_3d(dst + nbig * (kFewBig * kFewBK * 2) + j * (kFewBox * kFewBK * 2), &tmX, bar_full + 8 * s, kb * kFewBK,
+                        t.row0 + kFewBig * nbig + kFewBox * j, 0);
+          if (++s == NSTAGE) {
+            s = 0;
+            ph ^= 1;
+          }
         }
-        const bool have = kb < ahead;    // of the first tile only: `ahead` is 0 after it
-        if (lane == 0 && !have) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
-        if (active && !(have && isW))
-          tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, c2);
-        if (++s == NSTAGE) {
-          s = 0;
-          ph ^= 1;
-        }
+        ahead = 0;
       }
-      ahead = 0;
-      ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (p.early) grid_dep_begin();
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0, it = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -242,9 +252,12 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue: lane = output column, register = row
+    // ------------------------------------------------------------------ epilogue: TMEM lane = weight row, column = row of X
+    // A warp turns 16 rows of its share of a block's columns at a time, in registers, and writes 16 bytes a lane.
     const int q = warp & 3;              // TMEM lane quarter this warp may read
     const int half = (warp - 2) >> 2;    // even or odd 16-row groups
+    constexpr int G = (NT + 31) / 32;    // groups of a warp, at most
+    constexpr int WC = C::BLOCK_COLS / 4;                    // columns of a block in this quarter: 32, or 16 with gate and up
     if (p.early) grid_dep_begin();
     int it = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
@@ -256,41 +269,90 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       __syncwarp();
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::ACC_COLS;
-      for (int c = 16 * half; c < t.live; c += 32) {
-        uint32_t a[HALVES][16];
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h) tmem_ld16(taddr + h * NT + c, a[h]);
+      // bf16 values of one group, rounded before the activation as where gate and up are stored: v[h][4b + j] = rows (tokens) 8b + 2
+      // (lane % 4) and the next one of column block h, j: gate and up, or the two column blocks of a 16-lane load
+      auto fetch = [&](int hb, int c, uint32_t (&v)[2][4]) {
+        uint32_t r[2][8];
+        tmem_ld_blocks16(taddr + hb * NT + c, r[0]);
+        tmem_ld_blocks16(taddr + (16u << 16) + hb * NT + c, r[1]);
         tmem_ld_wait();
-        const int nr = min(16, t.live - c);                  // live rows of this group
-        __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(t.row0 + c) * p.N;
-        if constexpr (EPI == EPI_SWIGLU) {
-          const int col = t.m0 + 32 * q + lane;
-          auto rows = [&](auto tag) {
-            constexpr int CODE = decltype(tag)::value;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              // gate and up are rounded to bf16 before the activation, as where they are stored
-              const float g = bf16_round(__uint_as_float(a[0][i])), u = bf16_round(__uint_as_float(a[HALVES - 1][i]));
-              if (i < nr && col < p.N) d[static_cast<long long>(i) * p.N + col] = __float2bfloat16_rn(glu_fwd_val<CODE>(g, u));
-            }
-          };
-          if (code == 1) rows(std::integral_constant<int, 1>());
-          else if (code == 5) rows(std::integral_constant<int, 5>());
-          else rows(std::integral_constant<int, 0>());
-        } else {
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h) {
-            const int col = t.m0 + 128 * h + 32 * q + lane;
+          for (int i = 0; i < 4; ++i) v[h][i] = pack_bf16x2(__uint_as_float(r[h][2 * i]), __uint_as_float(r[h][2 * i + 1]));
+      };
+      auto put = [&](auto tag, int hb, int c, const uint32_t (&v)[2][4]) {
+        constexpr int CODE = decltype(tag)::value;
+        // 16-byte pieces: 8 output columns (piece) of a row of X
+        auto write = [&](int row, int piece, uint32_t (&w)[4]) {
+          const int col = t.m0 + C::BLOCK_COLS * hb + WC * q + 8 * piece;
+          if (row >= t.live || col >= p.N) return;
+          __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(t.row0 + row) * p.N + col;
+          if (p.aligned) {
+            *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (i < nr && col < p.N)
-                d[static_cast<long long>(i) * p.N + col] = __float2bfloat16_rn(__uint_as_float(a[h][i]));
+            for (int i = 0; i < 8; ++i) reinterpret_cast<uint16_t*>(d)[i] = static_cast<uint16_t>(w[i >> 1] >> (16 * (i & 1)));
+          }
+        };
+        const int j = lane & 3;
+        if constexpr (EPI == EPI_SWIGLU) {      // two pieces, two blocks of 8 rows
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int h = i & 1, b = i >> 1;
+            const float2 g = unpack_bf16x2(v[h][2 * b]), u = unpack_bf16x2(v[h][2 * b + 1]);
+            w[i] = movmatrix_trans(pack_bf16x2(glu_fwd_val<CODE>(g.x, u.x), glu_fwd_val<CODE>(g.y, u.y)));
+          }
+          quad_transpose(w, lane);
+          write(c + 8 * (j >> 1) + (lane >> 2), j & 1, w);
+        } else {                                // four pieces a block of 8 rows
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            uint32_t w[4] = {movmatrix_trans(v[0][2 * b]), movmatrix_trans(v[0][2 * b + 1]), movmatrix_trans(v[1][2 * b]),
+                             movmatrix_trans(v[1][2 * b + 1])};
+            quad_transpose(w, lane);
+            write(c + 8 * b + (lane >> 2), j, w);
           }
         }
+      };
+      auto by_code = [&](auto f) {       // uniform over the tile
+        if (EPI == EPI_SWIGLU && code == 1) f(std::integral_constant<int, 1>());
+        else if (EPI == EPI_SWIGLU && code == 5) f(std::integral_constant<int, 5>());
+        else f(std::integral_constant<int, 0>());
+      };
+      if constexpr (NBUF == 1) {         // the only accumulators: drained before anything else, so that the MMAs go on
+        uint32_t v[G][HALVES][2][4];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          if (16 * half + 32 * g < t.live)
+#pragma unroll
+            for (int hb = 0; hb < HALVES; ++hb) fetch(hb, 16 * half + 32 * g, v[g][hb]);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+        by_code([&](auto tag) {
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+            if (16 * half + 32 * g < t.live)
+#pragma unroll
+              for (int hb = 0; hb < HALVES; ++hb) put(tag, hb, 16 * half + 32 * g, v[g][hb]);
+        });
+      } else {
+        by_code([&](auto tag) {
+#pragma unroll 1
+          for (int c = 16 * half; c < t.live; c += 32)
+#pragma unroll
+            for (int hb = 0; hb < HALVES; ++hb) {
+              uint32_t v[2][4];
+              fetch(hb, c, v);
+              put(tag, hb, c, v);
+            }
+        });
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
     }
   }
 
@@ -308,12 +370,14 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 // ---------------------------------------------------------------------------- router of a small batch
 // Logits and top-k of 16 tokens per CTA in one launch: the gate weights are the M operand (up to 128 experts), the tokens the
 // N operand; the epilogue warps hand the bf16-rounded logits over through shared memory and each picks for two tokens.
-// Same k order, so the same logits to the bit, as the GEMM for large batches.  Bound by the chain of dependent MMAs on one
-// accumulator: about 150 cycles for each 16 of the reduction, however few rows it has (H 2048: 128 of them, 10 us).
-// us, GEMM and top-k (two launches) against this one, top-6 of 64 experts at H 2048: 1 token 15.0 / 12.5, 592 tokens 15.0 /
-// 13.9, 2368 (one wave of CTAs) 16.0 / 14.2, 4096 17.2 / 26.8; 32 experts at H 512, 2368 tokens 8.3 / 6.7.
-// (Dot products on CUDA cores, without that chain, took 5.6 us for 1 to 148 tokens, but they add in another order: about one
-// token in ten thousand then takes another expert of two that are a rounding apart.)
+// Same k order, so the same logits to the bit, as the GEMM for large batches.  Bound by the issue of its loads and MMAs (H 2048: 128
+// MMAs of 28 cycles or more, one CTA per 16 tokens) and by launch, top-k and tear-down around them: two k-blocks a stage, one elected
+// thread each for loads and MMAs, a warp per token for the picks.
+// us, top-6 of 64 experts at H 2048: 1 token 8.1, 48 tokens 8.4, 1500 tokens 8.9 (one k-block a stage, two lanes loading, two tokens a
+// warp: 12.9, 14.4, 14.8; GEMM and top-k as two launches 15.0 ... 16.0); 64 tokens, 8 experts at H 4096 22.9 -> 12.6.  Past one wave of
+// CTAs, 2368 tokens, the two launches are the faster ones (4096 tokens 17.2).
+// (Dot products on CUDA cores took 5.6 us for 1 to 148 tokens, but they add in another order: about one token in ten
+// thousand then takes another expert of two that are a rounding apart.)
 struct RouterFewParams {
   int T, H, E, k, norm;
   float scale;
@@ -327,16 +391,19 @@ struct RouterFewParams {
 
 constexpr int kRouterTokens = 16;
 constexpr int kRouterExperts = 128;     // at most: the lanes of one accumulator
+constexpr int kRouterThreads = 64 + 32 * kRouterTokens;   // a warp per token picks
 
 struct RouterFewCfg {
+  static constexpr int KB = 2;          // k-blocks a stage
   static constexpr int W_BYTES = kRouterExperts * kFewBK * 2;
-  static constexpr int STAGE_BYTES = W_BYTES + kRouterTokens * kFewBK * 2;
-  static constexpr int NSTAGE = 11;
+  static constexpr int KB_BYTES = W_BYTES + kRouterTokens * kFewBK * 2;
+  static constexpr int STAGE_BYTES = KB * KB_BYTES;
+  static constexpr int NSTAGE = 5;
   static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + (2 * NSTAGE + 1) * 8 + 16 + 1024;
 };
 
 template <int VPL>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kRouterThreads, 1)
 router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const RouterFewParams p) {
   using C = RouterFewCfg;
   constexpr int NSTAGE = C::NSTAGE;
@@ -378,18 +445,18 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int nkb = (p.H + kFewBK - 1) / kFewBK;
 
   if (warp == 0) {
-    if (lane < 2) {                        // lane 0: the weights of all experts, lane 1: the tokens
-      const bool isW = lane == 0;
-      const CUtensorMap* tm = isW ? &tmW : &tmX;
-      const uint32_t dst = isW ? 0 : C::W_BYTES;
-      const int c1 = isW ? 0 : t0;
-      const uint32_t bytes = (p.E + kRouterTokens) * kFewBK * 2;
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
-      for (int kb = 0; kb < nkb; ++kb) {
+      for (int kb = 0; kb < nkb; kb += C::KB) {
+        const int n = min(C::KB, nkb - kb);
         if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) break;
-        if (isW) mbar_arrive_expect_tx(bar_full + 8 * s, bytes);
-        tma_load_3d(smem_u32(smem + s * C::STAGE_BYTES) + dst, tm, bar_full + 8 * s, kb * kFewBK, c1, 0);
+        mbar_arrive_expect_tx(bar_full + 8 * s, n * (p.E + kRouterTokens) * kFewBK * 2);
+        for (int i = 0; i < n; ++i) {
+          const uint32_t dst = smem_u32(smem + s * C::STAGE_BYTES + i * C::KB_BYTES);
+          tma_load_3d(dst, &tmW, bar_full + 8 * s, (kb + i) * kFewBK, 0, 0);
+          tma_load_3d(dst + C::W_BYTES, &tmX, bar_full + 8 * s, (kb + i) * kFewBK, t0, 0);
+        }
         if (++s == NSTAGE) {
           s = 0;
           ph ^= 1;
@@ -397,22 +464,25 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(kRouterTokens, 0, 0, 128);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb) {
+      for (int kb = 0; kb < nkb; kb += C::KB) {
+        const int n = min(C::KB, nkb - kb);
         if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t sw = smem_u32(smem + s * C::STAGE_BYTES);
+        for (int i = 0; i < n; ++i) {
+          const uint32_t sw = smem_u32(smem + s * C::STAGE_BYTES + i * C::KB_BYTES);
 #pragma unroll
-        for (int k = 0; k < kFewBK / 16; ++k)
-          umma_bf16(tmem_base, umma_desc_sw128(sw + 32 * k, 0, 1024), umma_desc_sw128(sw + C::W_BYTES + 32 * k, 0, 1024),
-                    idesc, (kb | k) != 0);
+          for (int k = 0; k < kFewBK / 16; ++k)
+            umma_bf16(tmem_base, umma_desc_sw128(sw + 32 * k, 0, 1024), umma_desc_sw128(sw + C::W_BYTES + 32 * k, 0, 1024),
+                      idesc, (kb | i | k) != 0);
+        }
         umma_commit(bar_empty + 8 * s);
         if (++s == NSTAGE) {
           s = 0;
@@ -423,6 +493,9 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     }
   } else {
     const int ew = warp - 2, q = warp & 3;     // TMEM lane quarter; the first four warps read the accumulator
+    float b[VPL];                              // on its way while the products run
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) b[i] = (p.bias != nullptr && lane + 32 * i < p.E) ? p.bias[lane + 32 * i] : 0.0f;
     const bool ok = mbar_wait(bar_done, 0, abort_flag, ST_WAIT_EPILOGUE);
     __syncwarp();
     tc_fence_after();
@@ -434,32 +507,29 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       for (int t = 0; t < kRouterTokens; ++t) s_logit[t][32 * q + lane] = bf16_round(__uint_as_float(a[t]));
     }
     tc_fence_before();
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");    // the epilogue warps only
-    if (ok) {
-#pragma unroll 1
-      for (int tt = 2 * ew; tt < 2 * ew + 2 && t0 + tt < p.T; ++tt) {
-        const long long t = t0 + tt;
-        float sc[VPL];
-        uint32_t key[VPL];
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kRouterTokens) : "memory");    // the epilogue warps only
+    const long long t = t0 + ew;
+    if (ok && t < p.T) {
+      float sc[VPL];
+      uint32_t key[VPL];
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-          const int e = lane + 32 * i;
-          sc[i] = 0.0f;
-          key[i] = 0u;
-          if (e < p.E) {
-            const float v = s_logit[tt][e];
-            p.logits[t * p.E + e] = __float2bfloat16_rn(v);
-            sc[i] = sigmoid_f(v);
-            key[i] = select_key(sc[i] + (p.bias != nullptr ? p.bias[e] : 0.0f));
-          }
+      for (int i = 0; i < VPL; ++i) {
+        const int e = lane + 32 * i;
+        sc[i] = 0.0f;
+        key[i] = 0u;
+        if (e < p.E) {
+          const float v = s_logit[ew][e];
+          p.logits[t * p.E + e] = __float2bfloat16_rn(v);
+          sc[i] = sigmoid_f(v);
+          key[i] = select_key(sc[i] + b[i]);
         }
-        int my_idx;
-        float my_w;
-        topk_of_token<VPL>(sc, key, p.k, p.norm, p.scale, hist, p.counts != nullptr, my_idx, my_w);
-        if (lane < p.k) {
-          p.idx[t * p.k + lane] = my_idx;
-          p.w[t * p.k + lane] = my_w;
-        }
+      }
+      int my_idx;
+      float my_w;
+      topk_of_token<VPL>(sc, key, p.k, p.norm, p.scale, hist, p.counts != nullptr, my_idx, my_w);
+      if (lane < p.k) {
+        p.idx[t * p.k + lane] = my_idx;
+        p.w[t * p.k + lane] = my_w;
       }
     }
   }
@@ -478,9 +548,8 @@ router_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
 // ---------------------------------------------------------------------------- host side
 template <int EPI, int NT, int HALVES>
-static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows, int wgroups, const FewParams& p,
-                      cudaStream_t stream) {
-  using C = FewCfg<NT, HALVES>;
+static int launch_few(const void* x, const void* w, int64_t rows_cap, const FewParams& p, cudaStream_t stream) {
+  using C = FewCfg<EPI, NT, HALVES>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -488,16 +557,19 @@ static int launch_few(const void* x, const void* w, int64_t rows_cap, int wrows,
                                     C::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
-  CUtensorMap tmW, tmX;
-  int rc = make_map(&tmW, w, p.K, wrows, wgroups, p.K, static_cast<uint64_t>(wrows) * p.K, kFewBK, 128);
+  CUtensorMap tmW, tmX, tmXbig;
+  int rc = EPI == EPI_SWIGLU ? make_map_gate_up(&tmW, w, p.K, p.N, p.E, 8)
+                             : make_map(&tmW, w, p.K, p.N, p.E, p.K, static_cast<uint64_t>(p.N) * p.K, kFewBK, 128);
   if (rc) return rc;
   rc = make_map(&tmX, x, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, kFewBK, kFewBox);
   if (rc) return rc;
-  constexpr int TM = (EPI == EPI_SWIGLU) ? 128 : 128 * HALVES;
+  tmXbig = tmX;
+  if (NT > kFewBig) rc = make_map(&tmXbig, x, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, kFewBK, kFewBig);
+  if (rc) return rc;
   const long long chunks = std::min<long long>(rows_cap, p.E + rows_cap / NT);   // at most
-  const long long tiles = chunks * ceil_div(p.N, TM);
+  const long long tiles = chunks * ceil_div(p.N, C::TM);
   const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(gemm_cta_budget(), tiles)));
-  B200_LAUNCH((few_rows_kernel<EPI, NT, HALVES>), grid, kThreads, C::SMEM_BYTES, stream, tmW, tmX, p);
+  B200_LAUNCH((few_rows_kernel<EPI, NT, HALVES>), grid, kThreads, C::SMEM_BYTES, stream, tmW, tmX, tmXbig, p);
   return 0;
 }
 
@@ -515,7 +587,7 @@ static int launch_router_few(const void* x, const void* weight, const RouterFewP
   if (rc) return rc;
   rc = make_map(&tmX, x, p.H, p.T, 1, p.H, static_cast<uint64_t>(p.T) * p.H, kFewBK, kRouterTokens);
   if (rc) return rc;
-  B200_LAUNCH(router_few_kernel<VPL>, (p.T + kRouterTokens - 1) / kRouterTokens, kThreads, C::SMEM_BYTES, stream, tmW, tmX, p);
+  B200_LAUNCH(router_few_kernel<VPL>, (p.T + kRouterTokens - 1) / kRouterTokens, kRouterThreads, C::SMEM_BYTES, stream, tmW, tmX, p);
   return 0;
 }
 
@@ -536,6 +608,11 @@ static bool few_one_wave(int64_t M, int E, int64_t N, int64_t K) { return (E + M
 static int few_nt(int64_t M, int E, int64_t N, int64_t K) {
   if (M <= kFewRows64 * E || few_one_wave(M, E, N, K)) return 64;
   return M <= kFewRows128 * E ? 128 : 192;
+}
+
+// Gate/up blocks of 64 columns instead of 128, where even they are one wave: half the chain of a tile, twice the SMs that stream.
+static bool few_narrow(int64_t M, int E, int64_t I) {
+  return (std::min<int64_t>(E, M) + M / 64) * ceil_div(I, 64) <= num_sms();
 }
 
 // Whether a forward without a backward runs over compact rows (this file) or row tiles (gemm.cu), same measurements, row tiles
@@ -573,25 +650,25 @@ int expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* a
                        int32_t* status, b200moe_stream_t stream) {
   int rc = check_few("expert_gate_up_few", x, gate_up_proj, inter, counts, offs, rows_cap, E, I, H);
   if (rc) return rc;
-  FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status, early};
+  FewParams p{E, static_cast<int>(I), static_cast<int>(H), counts, offs, inter, act_codes, status, aligned16(inter), early};
   cudaStream_t st = (cudaStream_t)stream;
-  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
   const int nt = few_nt(rows_cap, E, I, H);
-  if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
-  if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
-  return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p.N, 2 * E, p, st);
+  if (nt == 64 && few_narrow(rows_cap, E, I)) return launch_few<EPI_SWIGLU, 64, 1>(x, gate_up_proj, rows_cap, p, st);
+  if (nt == 64) return launch_few<EPI_SWIGLU, 64, 2>(x, gate_up_proj, rows_cap, p, st);
+  if (nt == 128) return launch_few<EPI_SWIGLU, 128, 2>(x, gate_up_proj, rows_cap, p, st);
+  return launch_few<EPI_SWIGLU, 192, 2>(x, gate_up_proj, rows_cap, p, st);
 }
 
 int expert_linear_few(const void* x, const void* w, const int32_t* counts, const int32_t* offs, int64_t rows_cap, int E,
                       int64_t N, int64_t K, int early, void* out, int32_t* status, b200moe_stream_t stream) {
   int rc = check_few("expert_linear_few", x, w, out, counts, offs, rows_cap, E, N, K);
   if (rc) return rc;
-  FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status, early};
+  FewParams p{E, static_cast<int>(N), static_cast<int>(K), counts, offs, out, nullptr, status, aligned16(out), early};
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = few_nt(rows_cap, E, N, K);
-  if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p.N, E, p, st);
-  if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p.N, E, p, st);
-  return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p.N, E, p, st);
+  if (nt == 64) return launch_few<EPI_STORE, 64, 1>(x, w, rows_cap, p, st);
+  if (nt == 128) return launch_few<EPI_STORE, 128, 1>(x, w, rows_cap, p, st);
+  return launch_few<EPI_STORE, 192, 2>(x, w, rows_cap, p, st);
 }
 
 }  // namespace b200moe

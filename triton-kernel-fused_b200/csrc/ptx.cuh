@@ -110,6 +110,15 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm,
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1, int c2, int c3,
+                                            int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+      : "memory");
+}
+
 // 3-D tiled store, this CTA's shared memory -> global, tracked by the thread's bulk async-group.
 // Elements outside the tensor's bounds are not written.  c0 * element size must be a multiple of 16.
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* tm, uint32_t src, int c0, int c1, int c2) {
@@ -271,6 +280,37 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+// 16 lanes x 16 consecutive fp32 columns as 8 x 8 blocks: thread t holds of column block b (columns 8b ...) r[4b], r[4b+1] = lane
+// t / 4, columns 2 (t % 4) and the next one, and r[4b+2], r[4b+3] = lane t / 4 + 8, the same columns.  The lane field of taddr
+// is the quarter's first lane or that plus 16.  Packed to bf16 two by two these are the fragments movmatrix turns.
+__device__ __forceinline__ void tmem_ld_blocks16(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+// an 8 x 8 block of 16-bit values, transposed among the threads of a warp
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t m) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(m));
+  return d;
+}
+// 4 x 4 words among each four neighbouring threads: word i of thread j becomes what word j of thread i was
+__device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int lane) {
+  const bool odd = (lane & 1) != 0, high = (lane & 2) != 0;
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? w[i] : w[i + 1], 1);
+    if (odd) w[i] = r;
+    else w[i + 1] = r;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, high ? w[i] : w[i + 2], 2);
+    if (high) w[i] = r;
+    else w[i + 2] = r;
+  }
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
