@@ -201,6 +201,25 @@ def test_quantised_weights_are_reused_until_the_stack_changes(pkg):
     pkg.check_status()
 
 
+# rows an expert gets: none, one, both sides of a 16-row step and of 64- and 128-row chunks, several chunks; one k-block, an odd number
+# and an even number of them; enough rows for the row tiles
+@pytest.mark.parametrize("counts,H,I", [([1], 128, 128), ([0, 1, 15, 16, 17, 0, 63, 64], 256, 384), ([65, 0, 47, 50] + [1] * 28, 640, 256), ([0, 180] + [0] * 6, 384, 256),
+                                        ([65, 128, 129, 0], 384, 128), ([200, 0, 30, 127, 260], 640, 256),
+                                        ([700, 0, 0, 0, 0, 0, 0, 0], 256, 640), ([300, 520], 128, 256)])
+def test_mxfp8_forward_without_gradient_equals_the_training_forward(pkg, counts, H, I):
+    E, M = len(counts), sum(counts)
+    g = torch.Generator().manual_seed(M + H)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(M, generator=g)].view(M, 1).to(DEV)
+    x = (torch.randn(M, H, generator=g) * torch.logspace(-3, 3, M)[:, None]).to(torch.bfloat16).to(DEV)
+    gu = (torch.randn(E, 2 * I, H, generator=g) * 0.1).to(torch.bfloat16).to(DEV).requires_grad_()
+    dn = (torch.randn(E, H, I, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    w, codes = torch.rand(M, 1, generator=g).to(DEV) + 0.5, torch.zeros(E, dtype=torch.int32, device=DEV)
+    with torch.no_grad():
+        quiet = pkg.moe_mxfp8(x, idx, w, gu, dn, codes)
+    assert torch.equal(quiet, pkg.moe_mxfp8(x, idx, w, gu, dn, codes).detach())
+    pkg.check_status()
+
+
 def test_mxfp8_rejects_unaligned_width(pkg):
     x = torch.zeros(8, 192, dtype=torch.bfloat16, device=DEV)
     idx = torch.zeros(8, 1, dtype=torch.int64, device=DEV)

@@ -24,6 +24,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "few_tiles.cuh"
 #include "gemm_common.cuh"
 #include "topk.cuh"
 
@@ -66,29 +67,6 @@ struct FewCfg {
   static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + (2 * NSTAGE + 2 * NBUF) * 8 + 16 + 1024;
 };
 
-struct FewTile { int e, m0, row0, live; };
-
-// tile -> (expert, chunk of its rows, block of output columns); pre[] = exclusive prefix of the experts' chunk counts.
-// before_wait: the tables are read from L2, since an L1 line may be older than the launch
-template <int NT, int TM>
-__device__ __forceinline__ FewTile few_tile(const FewParams& p, const int* pre, int tile, bool before_wait = false) {
-  const int mt = (p.N + TM - 1) / TM;
-  const int c = tile / mt;
-  int lo = 0, hi = p.E;                       // the last expert with pre[e] <= c
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (pre[mid] <= c) lo = mid;
-    else hi = mid;
-  }
-  FewTile t;
-  t.e = lo;
-  t.m0 = (tile - c * mt) * TM;
-  const int first = (c - pre[lo]) * NT;
-  t.row0 = (before_wait ? __ldcg(p.offs + lo) : p.offs[lo]) + first;
-  t.live = min(NT, (before_wait ? __ldcg(p.counts + lo) : p.counts[lo]) - first);
-  return t;
-}
-
 template <int EPI, int NT, int HALVES>
 __global__ void __launch_bounds__(kThreads, 1)
 few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -130,29 +108,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     tmem_relinquish();
   }
   if (!p.early) grid_dep_begin();
-  if (warp == 2) {                       // prefix of the chunk counts: a lane takes 8 neighbouring experts
-    constexpr int V = B200MOE_MAX_EXPERTS / 32;
-    int c[V], sum = 0;
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int e = lane * V + i;
-      c[i] = e < p.E ? (__ldcg(p.counts + e) + NT - 1) / NT : 0;
-      sum += c[i];
-    }
-    int incl = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    int run = incl - sum;
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      pre[lane * V + i] = run;
-      run += c[i];
-    }
-    if (lane == 31) pre[B200MOE_MAX_EXPERTS] = run;
-  }
+  if (warp == 2) few_prefix<NT>(p.counts, p.E, lane, pre);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -171,7 +127,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       bool ok = true;
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
         const bool first = p.early && tile == static_cast<int>(blockIdx.x);
-        const FewTile t = few_tile<NT, TM>(p, pre, tile, first);
+        const FewTile t = few_tile<NT, TM>(p.counts, p.offs, p.E, p.N, pre, tile, first);
         const int nbig = NT > kFewBig ? (t.live + kFewBox - 1) / kFewBig : 0;
         const int nsmall = max(0, (t.live - nbig * kFewBig + kFewBox - 1) / kFewBox);
         const uint32_t bytes = C::W_BYTES + nbig * (kFewBig * kFewBK * 2) + nsmall * (kFewBox * kFewBK * 2);
@@ -219,7 +175,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++it) {
-        const FewTile t = few_tile<NT, TM>(p, pre, tile);
+        const FewTile t = few_tile<NT, TM>(p.counts, p.offs, p.E, p.N, pre, tile);
         const uint32_t idesc = umma_idesc_bf16((t.live + kFewBox - 1) / kFewBox * kFewBox, 0, 0, 128);
         const int buf = it % NBUF;
         if (!mbar_wait(bar_tempty + 8 * buf, ((it / NBUF) & 1) ^ 1, abort_flag, ST_WAIT_MMA_TMEM)) break;
@@ -261,7 +217,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     if (p.early) grid_dep_begin();
     int it = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
-      const FewTile t = few_tile<NT, TM>(p, pre, tile);
+      const FewTile t = few_tile<NT, TM>(p.counts, p.offs, p.E, p.N, pre, tile);
       const int buf = it % NBUF;
       int code = 0;
       if (EPI == EPI_SWIGLU && p.act_codes != nullptr) code = p.act_codes[t.e];
@@ -269,20 +225,10 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       __syncwarp();
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::ACC_COLS;
-      // bf16 values of one group, rounded before the activation as where gate and up are stored: v[h][4b + j] = rows (tokens) 8b + 2
-      // (lane % 4) and the next one of column block h, j: gate and up, or the two column blocks of a 16-lane load
-      auto fetch = [&](int hb, int c, uint32_t (&v)[2][4]) {
-        uint32_t r[2][8];
-        tmem_ld_blocks16(taddr + hb * NT + c, r[0]);
-        tmem_ld_blocks16(taddr + (16u << 16) + hb * NT + c, r[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) v[h][i] = pack_bf16x2(__uint_as_float(r[h][2 * i]), __uint_as_float(r[h][2 * i + 1]));
-      };
+      // bf16 values of one group, rounded before the activation as where gate and up are stored; a 16-lane block of a SwiGLU
+      // tile is 8 columns of gate (v[h][2b]) and the same of up (v[h][2b + 1])
+      auto fetch = [&](int hb, int c, uint32_t (&v)[2][4]) { few_fetch(taddr + hb * NT + c, v); };
       auto put = [&](auto tag, int hb, int c, const uint32_t (&v)[2][4]) {
-        constexpr int CODE = decltype(tag)::value;
         // 16-byte pieces: 8 output columns (piece) of a row of X
         auto write = [&](int row, int piece, uint32_t (&w)[4]) {
           const int col = t.m0 + C::BLOCK_COLS * hb + WC * q + 8 * piece;
@@ -302,6 +248,7 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           for (int i = 0; i < 4; ++i) {
             const int h = i & 1, b = i >> 1;
             const float2 g = unpack_bf16x2(v[h][2 * b]), u = unpack_bf16x2(v[h][2 * b + 1]);
+            constexpr int CODE = decltype(tag)::value;
             w[i] = movmatrix_trans(pack_bf16x2(glu_fwd_val<CODE>(g.x, u.x), glu_fwd_val<CODE>(g.y, u.y)));
           }
           quad_transpose(w, lane);
@@ -309,9 +256,8 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         } else {                                // four pieces a block of 8 rows
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            uint32_t w[4] = {movmatrix_trans(v[0][2 * b]), movmatrix_trans(v[0][2 * b + 1]), movmatrix_trans(v[1][2 * b]),
-                             movmatrix_trans(v[1][2 * b + 1])};
-            quad_transpose(w, lane);
+            uint32_t w[4];
+            few_turn(v, b, lane, w);
             write(c + 8 * b + (lane >> 2), j, w);
           }
         }

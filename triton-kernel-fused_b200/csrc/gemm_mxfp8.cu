@@ -11,6 +11,7 @@
 // SwiGLU over 64-interleaved gate|up weight rows, GLU backward).
 #include <stdlib.h>
 
+#include "few_tiles.cuh"
 #include "gemm_common.cuh"
 #include "mxfp8_quant.cuh"
 
@@ -700,6 +701,239 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Few rows per expert (decoding), forward only: the weights are the M operand, 128 rows of them a tile, and the expert's rows
+// the N operand in steps of 16, as in gemm_few.cu.  The row-tile kernel above gives every expert with a row 256 rows of MMAs, operand
+// loads and scale copies.
+// Bound: HBM, by the one read of the weights.  A stage is two k-blocks (256 elements: 32 KB of weights), so that a block's boxes,
+// scale atoms (neighbouring k-chunks are contiguous) and barriers are paid for once per 32 KB.
+// SwiGLU: a weight block is 64 gate and the 64 up rows of the same columns (lanes 0-63 and 64-127), so gate and up meet through
+// shared memory, where a thread then quantises 32 columns of a row as the row quantiser does.
+// 64 tokens of H 4096, 8 experts of d_ff 14336, top-2 (146 + 73 us at copy rate): gate/up 193 -> 146, down 101 -> 76 us.
+struct FewFp8Params {
+  int E, N, K, I;
+  const int* counts;        // rows of each expert
+  const int* poffs;         // its first row, a multiple of 256
+  const uint8_t* sfw;       // scale atoms of the weights and of X
+  const uint8_t* sfx;
+  __nv_bfloat16* D;         // store: (rows, N)
+  uint8_t* q_out;           // SwiGLU: (rows, I) codes and their scale atoms
+  uint8_t* q_sf;
+  int* status;
+};
+
+template <int EPI, int NT>
+struct FewFp8Cfg {
+  static constexpr int KB = 2;                                     // k-blocks a stage
+  static constexpr int X_BYTES = NT * FBK;
+  static constexpr int STAGE_BYTES = KB * (kATile + X_BYTES + 2 * kSfAtom);
+  static constexpr int ROW_BYTES = 256 + 16;                       // staged rows of 128 bf16 values, 16 bytes apart in the banks
+  static constexpr int EPI_ROWS = 64;
+  static constexpr int EPI_BYTES = EPI == EPI_SWIGLU ? EPI_ROWS * ROW_BYTES : 0;
+  static constexpr int NSTAGE = (232448 - 4096 - EPI_BYTES) / STAGE_BYTES;
+  static constexpr int SF_COLS = 8 * KB;                           // tensor-memory columns a stage's scales take
+  static constexpr int SF_BASE = 2 * NT;                           // behind two accumulators
+  static constexpr int TMEM_COLS = SF_BASE + SF_COLS * NSTAGE <= 256 ? 256 : 512;
+  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + EPI_BYTES + (2 * NSTAGE + 4) * 8 + 16 + 1024;
+};
+
+template <int EPI, int NT>
+__global__ void __launch_bounds__(kThreads, 1)
+few_mxfp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                 const __grid_constant__ CUtensorMap tmXbig, const FewFp8Params p) {
+  using C = FewFp8Cfg<EPI, NT>;
+  constexpr int NSTAGE = C::NSTAGE, TM = 128, kBox = 16, kBig = 64;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* rows = smem + NSTAGE * C::STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(rows + C::EPI_BYTES);
+  const uint32_t bar_full = smem_u32(bars);
+  const uint32_t bar_empty = smem_u32(bars + NSTAGE);
+  const uint32_t bar_tfull = smem_u32(bars + 2 * NSTAGE);
+  const uint32_t bar_tempty = smem_u32(bars + 2 * NSTAGE + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTAGE + 4);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  __shared__ int pre[B200MOE_MAX_EXPERTS + 1];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(bar_full + 8 * s, 1);
+      mbar_init(bar_empty + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_tfull + 8 * b, 1);
+      mbar_init(bar_tempty + 8 * b, kEpiWarps);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmXbig);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  grid_dep_wait();
+  if (warp == 2) few_prefix<NT>(p.counts, p.E, lane, pre);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int total = pre[p.E] * (p.N / TM);       // N is a multiple of 128
+  const int nkb = p.K / FBK;
+  // a stage: per k-block the weights and X, then the scale atoms of the weights' k-blocks and of X's
+  constexpr int kSfOff = C::KB * (kATile + C::X_BYTES);
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+        const FewTile t = few_tile<NT, TM>(p.counts, p.poffs, p.E, p.N, pre, tile);
+        const int nbig = (t.live + kBox - 1) / kBig;
+        const int nsmall = max(0, (t.live - nbig * kBig + kBox - 1) / kBox);
+        const uint8_t* sfw = p.sfw + ((static_cast<long long>(t.e) * p.N + t.m0) >> 7) * nkb * kSfAtom;
+        const uint8_t* sfx = p.sfx + static_cast<long long>(t.row0 >> 7) * nkb * kSfAtom;
+        for (int kb = 0; kb < nkb; kb += C::KB) {
+          const int n = min(C::KB, nkb - kb);
+          if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
+            ok = false;
+            break;
+          }
+          const uint32_t full = bar_full + 8 * s, st = smem_u32(smem + s * C::STAGE_BYTES);
+          mbar_arrive_expect_tx(full, n * (kATile + (nbig * kBig + nsmall * kBox) * FBK + 2 * kSfAtom));
+          for (int i = 0; i < n; ++i) tma_load_3d(st + i * kATile, &tmW, full, (kb + i) * FBK, t.m0, t.e);
+          bulk_load_1d(st + kSfOff, sfw + kb * kSfAtom, n * kSfAtom, full);
+          bulk_load_1d(st + kSfOff + C::KB * kSfAtom, sfx + kb * kSfAtom, n * kSfAtom, full);
+          for (int i = 0; i < n; ++i) {
+            const uint32_t dst = st + C::KB * kATile + i * C::X_BYTES;
+            for (int j = 0; j < nbig; ++j) tma_load_3d(dst + j * kBig * FBK, &tmXbig, full, (kb + i) * FBK, t.row0 + kBig * j, 0);
+            for (int j = 0; j < nsmall; ++j)
+              tma_load_3d(dst + (nbig * kBig + j * kBox) * FBK, &tmX, full, (kb + i) * FBK, t.row0 + kBig * nbig + kBox * j, 0);
+          }
+          if (++s == NSTAGE) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+    }
+    grid_dep_launch();   // the last loads are on their way
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      int s = 0, it = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++it) {
+        const FewTile t = few_tile<NT, TM>(p.counts, p.poffs, p.E, p.N, pre, tile);
+        const int n16 = (t.live + kBox - 1) / kBox * kBox, buf = it & 1;
+        const uint32_t sfx_col = (t.row0 & 127) >> 5;      // the chunk's rows inside their 128-row atom: 32 a column
+        if (!mbar_wait(bar_tempty + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, ST_WAIT_MMA_TMEM)) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * NT;
+        for (int kb = 0; kb < nkb; kb += C::KB) {
+          const int n = min(C::KB, nkb - kb);
+          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t st = smem_u32(smem + s * C::STAGE_BYTES);
+          const uint32_t sf = tmem_base + C::SF_BASE + s * C::SF_COLS;
+          for (int i = 0; i < n; ++i) {
+            tmem_cp_sf(sf + 8 * i, sf_desc(st + kSfOff + i * kSfAtom));
+            tmem_cp_sf(sf + 8 * i + 4, sf_desc(st + kSfOff + (C::KB + i) * kSfAtom));
+          }
+          for (int i = 0; i < n; ++i) {
+            const uint32_t sw = st + i * kATile, sx = st + C::KB * kATile + i * C::X_BYTES;
+#pragma unroll
+            for (int k = 0; k < FBK / 32; ++k)
+              umma_mxf8(d_tmem, umma_desc_sw128(sw + k * 32, 0, 1024), umma_desc_sw128(sx + k * 32, 0, 1024), idesc_mxf8(n16, k),
+                        sf + 8 * i, sf + 8 * i + 4 + sfx_col, (kb | i | k) != 0);
+          }
+          umma_commit(bar_empty + 8 * s);
+          if (++s == NSTAGE) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (!ok) break;
+        umma_commit(bar_tfull + 8 * buf);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue: TMEM lane = weight row, column = row of X
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    int it = 0;
+    bool ok = true;      // a warp that gave up goes on to the barriers of the others
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
+      const FewTile t = few_tile<NT, TM>(p.counts, p.poffs, p.E, p.N, pre, tile);
+      const int buf = it & 1;
+      ok = ok && mbar_wait(bar_tfull + 8 * buf, (it >> 1) & 1, abort_flag, ST_WAIT_EPILOGUE);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * NT;
+      for (int c0 = 0; c0 < t.live; c0 += C::EPI_ROWS) {
+        const int c1 = min(t.live, c0 + C::EPI_ROWS);
+        if (ok)
+#pragma unroll 1
+          for (int c = c0 + 16 * half; c < c1; c += 32) {
+            uint32_t v[2][4];
+            few_fetch(taddr + c, v);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              uint32_t w[4];
+              few_turn(v, b, lane, w);
+              const int row = c + 8 * b + (lane >> 2), col = 32 * q + 8 * (lane & 3);
+              const uint4 o = make_uint4(w[0], w[1], w[2], w[3]);
+              if constexpr (EPI == EPI_SWIGLU) *reinterpret_cast<uint4*>(rows + (row - c0) * C::ROW_BYTES + 2 * col) = o;
+              else if (row < t.live) *reinterpret_cast<uint4*>(p.D + static_cast<long long>(t.row0 + row) * p.N + t.m0 + col) = o;
+            }
+          }
+        if constexpr (EPI == EPI_SWIGLU) {
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+          const int task = threadIdx.x - 64, r = task >> 1, blk = task & 1;     // a row of 64, 32 of its columns
+          if (ok && r < C::EPI_ROWS && c0 + r < t.live) {
+            const uint4* g4 = reinterpret_cast<const uint4*>(rows + r * C::ROW_BYTES + 64 * blk);
+            const uint4* u4 = g4 + 8;                                            // 64 columns on
+            uint32_t oh[16];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint4 g = g4[i], u = u4[i];
+              const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                const float2 gf = unpack_bf16x2(gw[h]), uf = unpack_bf16x2(uw[h]);
+                oh[4 * i + h] = pack_bf16x2(glu_fwd_val<0>(gf.x, uf.x), glu_fwd_val<0>(gf.y, uf.y));
+              }
+            }
+            const long long row = t.row0 + c0 + r;
+            const int col = t.m0 / 2 + 32 * blk;
+            mx_quant_store32(oh, p.q_out + row * p.I + col, p.q_sf, row, col >> 5, p.I >> 7);
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");      // the staged rows have been read
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_flag);
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
 // scale atoms seen as a {128 x u32, k-chunks, row-blocks} tensor, no swizzle; box = `atoms` row-blocks
 static int map_sf(CUtensorMap* tm, const void* sf, long long row_blocks, long long k_chunks, int atoms) {
   EncodeTiledFn fn = get_encode_fn();
@@ -766,6 +1000,28 @@ static int map_fp8(CUtensorMap* tm, const void* q, long long rows, long long K, 
   return make_map(tm, q, K, rows, groups, K, rows * K, FBK, 128, 1);
 }
 
+template <int EPI, int NT>
+static int launch_few_fp8(const void* Xq, const void* Wq, int64_t rows_cap, const FewFp8Params& p, cudaStream_t stream) {
+  using C = FewFp8Cfg<EPI, NT>;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(few_mxfp8_kernel<EPI, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+  });
+  if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
+  CUtensorMap tmW, tmX, tmXbig;
+  int rc = map_fp8(&tmW, Wq, p.N, p.K, p.E);
+  if (rc) return rc;
+  rc = make_map(&tmX, Xq, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, FBK, 16, 1);
+  if (rc) return rc;
+  rc = make_map(&tmXbig, Xq, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, FBK, 64, 1);
+  if (rc) return rc;
+  const long long chunks = p.E + rows_cap / NT;   // at most
+  const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(gemm_cta_budget(), chunks * (p.N / 128))));
+  B200_LAUNCH((few_mxfp8_kernel<EPI, NT>), grid, kThreads, C::SMEM_BYTES, stream, tmW, tmX, tmXbig, p);
+  return 0;
+}
+
 // Launch with pair tiles when the output is at least one 256-wide tile (and pairs are enabled).
 template <int EPI>
 static int launch_any(const void* Aq, long long a_rows, const void* Bq, long long b_rows, long long b_groups,
@@ -812,6 +1068,13 @@ static int launch_any(const void* Aq, long long a_rows, const void* Bq, long lon
 
 using namespace b200moe;
 
+// Mean rows per expert up to which a forward runs on few_mxfp8_kernel, and up to which in chunks of 64 rows instead of 128, as the host
+// knows the mean: by the most rows that the padded ones can hold.  us of a whole block, row tiles / here, even and rank^-1.1 routing.
+// 8 experts, 4096 x 14336: mean 16 rows 307, 308 / 234, 234; 48 rows 315, 314 / 239, 285 (chunks of 64); 100 rows 325, 346 / 260, 314 (of
+// 128; of 64 362, 364); 128 rows 331, 347 / 323, 322; 160 rows 335, 358 / 410, 396.  64 experts, 2048 x 1408: 16 rows 164, 165 / 127, 130;
+// 128 rows 180, 200 / 163, 180; 200 rows 188, 229 / 202, 214.  16 experts, 1024 x 1024: 16 rows 32, 32 / 23, 23; 160 rows 39, 44 / 39, 37.
+constexpr int64_t kFewFp8Rows = 128, kFewFp8Small = 32;
+
 #define CHECK_K128(v) \
   B200_CHECK_ARG((v) > 0 && (v) % 128 == 0, B200MOE_E_BAD_SHAPE, #v " = %lld must be a positive multiple of 128", (long long)(v))
 
@@ -834,6 +1097,17 @@ static int mxfp8_grouped(int epilogue, const void* Aq, const void* Asf, const vo
   fp.b_rows_per_group = (int)N;
   fp.live = live;
   fp.q_out = (uint8_t*)q_out; fp.q_sf = (uint8_t*)q_sf;
+  // M <= most, the rows that fill the padded ones at best: the host does not know the counts
+  const int64_t most = rows_cap - static_cast<int64_t>(E) * B200MOE_TILE_M;
+  if (live != nullptr && most <= kFewFp8Rows * E && E <= B200MOE_MAX_EXPERTS && (epilogue == EPI_STORE || N == 2 * I)) {
+    B200_CHECK_ARG(epilogue != EPI_STORE || aligned16(D), B200MOE_E_ALIGN, "mxfp8_expert_forward: output not 16-byte aligned");
+    FewFp8Params f{E, (int)N, (int)K, (int)I, live, poffs, fp.sfb, fp.sfa, reinterpret_cast<__nv_bfloat16*>(D), fp.q_out, fp.q_sf, status};
+    const bool small = most <= kFewFp8Small * E;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (epilogue == EPI_STORE)
+      return small ? launch_few_fp8<EPI_STORE, 64>(Aq, Bq, rows_cap, f, st) : launch_few_fp8<EPI_STORE, 128>(Aq, Bq, rows_cap, f, st);
+    return small ? launch_few_fp8<EPI_SWIGLU, 64>(Aq, Bq, rows_cap, f, st) : launch_few_fp8<EPI_SWIGLU, 128>(Aq, Bq, rows_cap, f, st);
+  }
   switch (epilogue) {
     case EPI_STORE: return launch_any<EPI_STORE>(Aq, rows_cap, Bq, N, E, K, fp, 0, (cudaStream_t)stream);
     case EPI_SWIGLU:
