@@ -6,8 +6,10 @@ fallback: if the library is missing or a call fails, a Python exception is raise
 from __future__ import annotations
 
 import ctypes
+import importlib
 import os
 import subprocess
+import sys
 import threading
 
 import torch
@@ -15,6 +17,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(_HERE, "libb200moe.so")
+FAST_PATH = os.path.join(_HERE, "_fast.so")
 
 _lock = threading.Lock()
 _lib = None
@@ -136,14 +139,15 @@ _ERRORS = {-1: ValueError, -2: ValueError, -3: ValueError, -4: ValueError, -5: R
 
 
 def build(verbose: bool = False) -> str:
-    """Compile libb200moe.so for sm_100a with nvcc (works without a GPU) and return its path."""
-    cmd = ["make", "-C", _CSRC, "-j", str(min(8, os.cpu_count() or 1))]
+    """Compile libb200moe.so for sm_100a with nvcc and _fast.so with the host compiler (works without a GPU); returns the
+    library's path."""
+    cmd = ["make", "-C", _CSRC, "-j", str(min(8, os.cpu_count() or 1)), f"PYTHON={sys.executable}"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         print(res.stdout[-4000:])
         print(res.stderr[-4000:])
-    if res.returncode != 0 or not os.path.exists(LIB_PATH):
-        raise RuntimeError("building libb200moe.so failed (see output above)")
+    if res.returncode != 0 or not os.path.exists(LIB_PATH) or not os.path.exists(FAST_PATH):
+        raise RuntimeError("building libb200moe.so and _fast.so failed (see output above)")
     return LIB_PATH
 
 
@@ -165,6 +169,22 @@ def lib():
                 fn.argtypes = args
             _lib = handle
     return _lib
+
+
+_fast = None
+
+
+def fast():
+    """The compiled autograd functions (csrc/fast.cpp), or None while a compiler or tracer has to see the Python ones."""
+    global _fast
+    if torch.compiler.is_compiling() or torch.jit.is_tracing():
+        return None
+    if _fast is None:
+        lib()
+        if not os.path.exists(FAST_PATH):
+            raise RuntimeError(f"{FAST_PATH} is missing: build it with `make -C {_CSRC}` (or __graft_entry__.build())")
+        _fast = importlib.import_module("._fast", __package__)
+    return _fast
 
 
 def check(rc: int) -> None:

@@ -82,7 +82,8 @@ class LoadBalanceMixin:
 
 class _Layer(torch.autograd.Function):
     """Router and experts of a bf16 layer whose activations run in the GEMM epilogues, one native call each way
-    (csrc/block.cu): `fused_mlp_router` followed by `moe`, with the two shares of grad_x added in the last kernel.  Returns
+    (csrc/block.cu): `fused_mlp_router` followed by `moe`, with the two shares of grad_x added in the last kernel.  Plain calls take
+    its compiled form (csrc/fast.cpp).  Returns
     (out (N,H), counts (E,) int32); `load` (E int64, or None) gets the counts added."""
 
     @staticmethod
@@ -172,20 +173,26 @@ class MoELayer(LoadBalanceMixin, nn.Module):
 
     def forward(self, x):                               # x: (B,S,H) or (N,H)
         shape = x.shape
-        flat = x.reshape(-1, shape[-1])
+        flat = x if x.dim() == 2 else x.reshape(-1, shape[-1])
         # an nn.Module resolves each of its parameters and buffers by name: once each
         weight, bias, gate_up, down, codes, params = (self.gate.weight, self.bias, self.gate_up_proj, self.down_proj,
                                                       self.act_codes, self.act_params)
         infos, n_glu = _code_info(codes)
         if (self.precision == "bf16" and params is None and flat.shape[0] > 0 and n_glu == len(infos) == self.num_experts
                 and all(c in FUSED_CODES for c in infos)):
-            keep = torch.is_grad_enabled() and any(t.requires_grad for t in (flat, weight, gate_up, down))
             load = self._load_tensor(flat.device) if self.training and flat.is_cuda else None
-            out, self.last_counts = _Layer.apply(flat, weight, bias, gate_up, down,
-                                                 _codes_on(codes, flat.device) if any(infos) else None, load, int(self.top_k),
-                                                 int(bool(self.norm_topk_prob and self.top_k > 1)),
-                                                 float(self.routed_scaling_factor), int(keep))
-            return out.reshape(shape)
+            codes_dev = _codes_on(codes, flat.device) if any(infos) else None
+            k, scale = int(self.top_k), float(self.routed_scaling_factor)
+            norm = int(bool(self.norm_topk_prob and k > 1))
+            fast = L.fast() if flat.is_cuda else None
+            res = None
+            if fast is not None:
+                res = fast.layer(flat, weight, bias, gate_up, down, codes_dev, load, L.status_word(flat.device), k, norm, scale)
+            if res is None:
+                keep = torch.is_grad_enabled() and any(t.requires_grad for t in (flat, weight, gate_up, down))
+                res = _Layer.apply(flat, weight, bias, gate_up, down, codes_dev, load, k, norm, scale, int(keep))
+            out, self.__dict__["last_counts"] = res       # a plain attribute: nn.Module.__setattr__ would look for parameters first
+            return out if out.dim() == len(shape) else out.reshape(shape)
         idx, w, counts = fused_mlp_router(flat, weight, bias, self.top_k, self.num_experts, self.norm_topk_prob,
                                           self.routed_scaling_factor, return_counts=True)
         self._record_counts(counts)

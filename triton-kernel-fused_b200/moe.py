@@ -213,7 +213,15 @@ def moe(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes
         out = moe(hidden.to(bf), top_k_indices, top_k_weights, _bf16_copy(gate_up_proj), _bf16_copy(down_proj),
                   act_codes, act_params)
         return out.to(hidden.dtype)
-    if act_params is None and n_glu == len(codes) and all(c in FUSED_CODES for c in codes):
+    fused = act_params is None and n_glu == len(codes) and all(c in FUSED_CODES for c in codes)
+    fast = L.fast() if hidden.is_cuda else None
+    if fast is not None:
+        codes_dev = None if fused and not any(codes) else _codes_on(act_codes, hidden.device)
+        out = fast.experts(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, codes_dev, act_params,
+                           L.status_word(hidden.device), len(codes), n_glu, int(not fused))
+        if out is not None:
+            return out
+    if fused:
         keep = torch.is_grad_enabled() and any(t.requires_grad for t in (hidden, top_k_weights, gate_up_proj, down_proj))
         return _GroupedMoE.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, keep)
     return _PolyGLUMoE.apply(hidden, top_k_indices, top_k_weights, gate_up_proj, down_proj, act_codes, act_params)

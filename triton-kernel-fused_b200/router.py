@@ -98,7 +98,8 @@ class FusedConvRouter(torch.autograd.Function):
     sum_{j,h} x[b, s-(K-1)+j, h] * W[e,h,j], then the same sigmoid / bias / top-k epilogue.  One tcgen05 GEMM
     whose TMA producer reads x in place, tap by tap, through an (H, S, B) tensor map (kernels/sm120/router.py:34-85 is one
     launch too), or over an unfolded copy of x (H no multiple of 16, many short sequences); the backward's top-k kernel lays the gradients
-    out tap by tap, and dX and dW are plain products with that.  One native call each way (csrc/block.cu)."""
+    out tap by tap, and dX and dW are plain products with that.  One native call each way (csrc/block.cu); plain calls
+    take the compiled form of this Function (csrc/fast.cpp)."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, top_k, num_experts, norm_topk=True, scale=1.0):
@@ -158,6 +159,14 @@ def fused_router(x, conv_weight, bias, top_k, num_experts, norm_topk_prob=True, 
     if x.numel() == 0:
         idx, w, counts = _empty_routing(x, conv_weight, top_k)
     else:
+        fast = L.fast() if x.is_cuda else None
+        res = None
+        if fast is not None:
+            res = fast.conv_router(x, conv_weight, bias, L.status_word(x.device), int(top_k),
+                                   conv_weight.shape[0] if num_experts is None else int(num_experts),
+                                   int(bool(norm_topk_prob and top_k > 1)), float(routed_scaling_factor))
+        if res is not None:
+            return res if return_counts else res[:2]
         idx, w, counts = FusedConvRouter.apply(x, conv_weight, bias, top_k, num_experts, norm_topk_prob,
                                                routed_scaling_factor)
     idx = idx.view(B, S, top_k)
