@@ -355,6 +355,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (glu_col0 < p.I) glu_load(0);
         if (glu_col0 + 32 < p.I) glu_load(1);
       }
+      // single-CTA GLU backward: gate and up of a step (16 rows x CW columns) as they lie in memory, the first one's on their way
+      // while the MMAs run, the next one's while one is computed
+      constexpr int CW = (EPI == EPI_SWIGLU ? BN / 4 : BN / 2) >= 64 ? 64 : 32;      // columns at a time (epilogues without TMA)
+      constexpr int NP = CW / 32;
+      constexpr bool kGluRegs = !TMA_EPI && EPI == EPI_GLU_BWD;
+      [[maybe_unused]] uint4 gv[2][NP], uv[2][NP];
+      auto glu_fetch = [&](int step) {
+        if constexpr (kGluRegs) {
+          const int col0 = t.n0 + half * (BN / 2) + (step >> 1) * CW;
+          const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.aux) +
+                                     static_cast<long long>(row0 + 16 * (step & 1)) * (2LL * p.I) + col0;
+#pragma unroll
+          for (int s2 = 0; s2 < 2; ++s2) {
+            epi_pieces<NP>(src + 16LL * s2 * p.I, 2LL * p.I, p.I - col0, lane, gv[s2]);
+            epi_pieces<NP>(src + 16LL * s2 * p.I + p.I, 2LL * p.I, p.I - col0, lane, uv[s2]);
+          }
+        }
+      };
+      glu_fetch(0);
       if (!mbar_wait(bar_tfull + 8 * buf, (it >> 1) & 1, abort_flag, ST_WAIT_EPILOGUE)) break;
       __syncwarp();
       tc_fence_after();
@@ -523,128 +542,97 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
           }
         }
-      } else if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32) {
-        const bool conv_rows = CONV && p.conv_taps > 0 && p.sched == SCHED_DENSE;   // rows are positions of batch t.g
-        const bool row_ok = (p.sched == SCHED_GROUPED_M) || (row < (conv_rows ? p.conv_S : p.M));
-        const long long base = (p.sched == SCHED_GROUPED_K || conv_rows ? t.g * p.d_group_stride : 0) +
-                               row * p.ldd + t.n0;
-        constexpr int W = BN / 2;   // columns per warp
+      } else {
+        // Single-CTA tiles up to 128 wide, and fp32 partial sums: from tensor memory through registers.  16 rows x 64 (or 32) columns at a
+        // time are read as 8 x 8 blocks; among the four threads that hold a row's blocks a 4 x 4 exchange of packed words gives each one
+        // block's 16 bytes, and a second one between neighbouring rows lets a warp read or write 128 contiguous bytes of 4 rows per
+        // instruction.  (Each lane writing 16-byte pieces of its own row: 512 tokens of H 256, I 512, 8 experts: gate/up 7.4 us against
+        // 6.3, GLU backward 12.1 against 8.6, the five other products 32.6 against 31.)
+        const uint32_t lower = taddr + (16u << 16);      // rows 16 ... of the warp
+        if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32) {
+          constexpr int W = BN / 2;                     // columns per warp
+          const bool conv_rows = CONV && p.conv_taps > 0 && p.sched == SCHED_DENSE;   // rows are positions of batch t.g
+          const int rows_end = (p.sched == SCHED_GROUPED_M) ? 0x7fffffff : (conv_rows ? p.conv_S : p.M);
+          const long long base = ((p.sched == SCHED_GROUPED_K || conv_rows) ? t.g * p.d_group_stride : 0) +
+                                 static_cast<long long>(row0) * p.ldd + t.n0 + half * W;
+          const int live = min(W, p.N - t.n0 - half * W);                             // columns of this warp
 #pragma unroll 1
-        for (int c0 = half * W; c0 < (half + 1) * W; c0 += 32) {
-          if (t.n0 + c0 >= p.N) break;
-          uint32_t r[32];
-          if (have_acc) {
-            tmem_ld32(taddr + c0, r);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = 0u;
-          }
-          if (row_ok) {
-            if constexpr (EPI == EPI_STORE) {
-              __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + base + c0;
-#pragma unroll
-              for (int v = 0; v < 4; ++v)
-                if (t.n0 + c0 + v * 8 < p.N) *reinterpret_cast<uint4*>(d + v * 8) = pack8(r + v * 8);
-            } else {
-              float* d = reinterpret_cast<float*>(p.D) + base + c0;
-#pragma unroll
-              for (int v = 0; v < 8; ++v)
-                if (t.n0 + c0 + v * 4 < p.N)
-                  *reinterpret_cast<uint4*>(d + v * 4) = make_uint4(r[v * 4 + 0], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_SWIGLU) {
-        // accumulator columns [0,BN/2) = gate, [BN/2,BN) = up for I-columns [n0, n0+BN/2)
-        const int I = p.I;
-        __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(p.D) + row * (2LL * I);
-        __nv_bfloat16* it_out = reinterpret_cast<__nv_bfloat16*>(p.aux) + row * static_cast<long long>(I);
-        constexpr int W = BN / 4;   // I-columns per warp
-#pragma unroll 1
-        for (int c0 = half * W; c0 < (half + 1) * W; c0 += 32) {
-          if (t.n0 + c0 >= I) break;
-          uint32_t g[32], u[32];
-          tmem_ld32(taddr + c0, g);
-          tmem_ld32(taddr + BN / 2 + c0, u);
-          tmem_ld_wait();
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int col = t.n0 + c0 + v * 8;
-            if (col < I) {
-              uint32_t og[4], ou[4], oh[4];
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                og[h] = pack_bf16x2(__uint_as_float(g[v * 8 + 2 * h]), __uint_as_float(g[v * 8 + 2 * h + 1]));
-                ou[h] = pack_bf16x2(__uint_as_float(u[v * 8 + 2 * h]), __uint_as_float(u[v * 8 + 2 * h + 1]));
-              }
-              glu_fwd_pairs_by_code<POLY>(act_code, og, ou, oh, 4);
-              *reinterpret_cast<uint4*>(gu + col) = make_uint4(og[0], og[1], og[2], og[3]);
-              *reinterpret_cast<uint4*>(gu + I + col) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
-              *reinterpret_cast<uint4*>(it_out + col) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
-            }
-          }
-        }
-      } else {  // EPI_GLU_BWD: accumulator = grad_inter columns [n0, n0+BN)
-        const int I = p.I;
-        const __nv_bfloat16* gu = reinterpret_cast<const __nv_bfloat16*>(p.aux) + row * (2LL * I);
-        __nv_bfloat16* ggu = reinterpret_cast<__nv_bfloat16*>(p.D) + row * (2LL * I);
-        constexpr int W = BN / 2;
-        constexpr int NCH = W / 32;
-        // the saved gate/up values of chunk c+1 are fetched while chunk c is computed
-        uint4 gv[2][4], uv[2][4];
-        auto fetch = [&](int c, int slot) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int col = t.n0 + half * W + c * 32 + v * 8;
-            if (col < I) {
-              gv[slot][v] = __ldg(reinterpret_cast<const uint4*>(gu + col));
-              uv[slot][v] = __ldg(reinterpret_cast<const uint4*>(gu + I + col));
-            } else {
-              gv[slot][v] = make_uint4(0u, 0u, 0u, 0u);
-              uv[slot][v] = make_uint4(0u, 0u, 0u, 0u);
-            }
-          }
-        };
-        fetch(0, 0);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          const int c0 = half * W + c * 32;
-          if (t.n0 + c0 < I) {          // warp-uniform
-            uint32_t r[32];
-            tmem_ld32(taddr + c0, r);
-            if (c + 1 < NCH) fetch(c + 1, (c + 1) & 1);
+          for (int c = 0; c < live; c += CW) {
+            uint32_t r[2][NP][16];
+            epi_load<NP>(taddr + half * W + c, have_acc, r[0]);
+            epi_load<NP>(lower + half * W + c, have_acc, r[1]);
             tmem_ld_wait();
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c0 + v * 8;
-              if (col < I) {
-                const uint4 g4 = gv[c & 1][v], u4 = uv[c & 1][v];
-                const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
-                const uint32_t uw[4] = {u4.x, u4.y, u4.z, u4.w};
-                uint32_t og[4], ou[4];
-                auto bwd8 = [&](auto code_tag) {
-                  constexpr int CODE = decltype(code_tag)::value;
+            for (int i = 0; i < 4; ++i) {
+              const int rows = rows_end - row0 - 8 * i;
+              if constexpr (EPI == EPI_STORE_F32) {
+                float* d = reinterpret_cast<float*>(p.D) + base + static_cast<long long>(8 * i + (lane >> 2)) * p.ldd + c + 2 * (lane & 3);
 #pragma unroll
-                  for (int h = 0; h < 4; ++h) {
-                    const float2 gf = unpack_bf16x2(gw[h]);
-                    const float2 uf = unpack_bf16x2(uw[h]);
-                    // grad_inter is rounded to bf16 first: the reference materialises it in bf16
-                    const float go0 = bf16_round(__uint_as_float(r[v * 8 + 2 * h]));
-                    const float go1 = bf16_round(__uint_as_float(r[v * 8 + 2 * h + 1]));
-                    float gg0, gu0, gg1, gu1;
-                    glu_bwd_val<CODE>(gf.x, uf.x, go0, gg0, gu0);
-                    glu_bwd_val<CODE>(gf.y, uf.y, go1, gg1, gu1);
-                    og[h] = pack_bf16x2(gg0, gg1);
-                    ou[h] = pack_bf16x2(gu0, gu1);
-                  }
-                };
-                if (POLY && act_code == 1) bwd8(std::integral_constant<int, 1>{});
-                else if (POLY && act_code == 5) bwd8(std::integral_constant<int, 5>{});
-                else bwd8(std::integral_constant<int, 0>{});
-                *reinterpret_cast<uint4*>(ggu + col) = make_uint4(og[0], og[1], og[2], og[3]);
-                *reinterpret_cast<uint4*>(ggu + I + col) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+                for (int b = 0; b < 4 * NP; ++b)
+                  if ((lane >> 2) < rows && c + 8 * b < live)
+                    *reinterpret_cast<uint2*>(d + 8 * b) = make_uint2(r[i >> 1][b / 4][4 * (b % 4) + 2 * (i & 1)], r[i >> 1][b / 4][4 * (b % 4) + 2 * (i & 1) + 1]);
+              } else {
+                uint32_t w[NP][4];
+#pragma unroll
+                for (int j = 0; j < NP; ++j) epi_pack(r[i >> 1][j], i & 1, w[j]);
+                epi_put<NP>(reinterpret_cast<__nv_bfloat16*>(p.D) + base + static_cast<long long>(8 * i) * p.ldd + c, p.ldd, rows, live - c, lane, w);
               }
+            }
+          }
+        } else if constexpr (EPI == EPI_SWIGLU) {
+          // accumulator columns [0,BN/2) = gate, [BN/2,BN) = up for I-columns [n0, n0+BN/2)
+          const int I = p.I, c = half * (BN / 4), col0 = t.n0 + c;
+          if (col0 < I) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              uint32_t g[NP][16], u[NP][16];
+              epi_load<NP>((h ? lower : taddr) + c, true, g);
+              epi_load<NP>((h ? lower : taddr) + BN / 2 + c, true, u);
+              tmem_ld_wait();
+#pragma unroll
+              for (int s2 = 0; s2 < 2; ++s2) {
+                const long long r8 = row0 + 16 * h + 8 * s2;
+                uint32_t gw[NP][4], uw[NP][4], hw[NP][4];
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                  epi_pack(g[i], s2, gw[i]);
+                  epi_pack(u[i], s2, uw[i]);
+                  glu_fwd_pairs_by_code<POLY>(act_code, gw[i], uw[i], hw[i], 4);
+                }
+                __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(p.D) + r8 * (2LL * I) + col0;
+                epi_put<NP>(gu, 2LL * I, 8, I - col0, lane, gw);
+                epi_put<NP>(gu + I, 2LL * I, 8, I - col0, lane, uw);
+                epi_put<NP>(reinterpret_cast<__nv_bfloat16*>(p.aux) + r8 * I + col0, I, 8, I - col0, lane, hw);
+              }
+            }
+          }
+        } else {  // EPI_GLU_BWD: accumulator = grad_inter columns [n0, n0+BN)
+          constexpr int W = BN / 2;
+          const int I = p.I;
+#pragma unroll 1
+          for (int step = 0; step < W / CW * 2; ++step) {
+            const int c = half * W + (step >> 1) * CW, col0 = t.n0 + c;
+            if (col0 >= I) break;
+            uint32_t gw[2][NP][4], uw[2][NP][4], r[NP][16];
+#pragma unroll
+            for (int s2 = 0; s2 < 2; ++s2) {
+              epi_words<NP>(gv[s2], lane, gw[s2]);
+              epi_words<NP>(uv[s2], lane, uw[s2]);
+            }
+            if (step + 1 < W / CW * 2) glu_fetch(step + 1);
+            epi_load<NP>(((step & 1) ? lower : taddr) + c, true, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int s2 = 0; s2 < 2; ++s2) {
+#pragma unroll
+              for (int i = 0; i < NP; ++i) {
+                uint32_t iw[4];
+                epi_pack(r[i], s2, iw);                         // rounded to bf16: the reference materialises grad_inter in bf16
+                glu_bwd_pairs<POLY>(act_code, iw, gw[s2][i], uw[s2][i]);      // now grad_gate, grad_up
+              }
+              __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row0 + 16 * (step & 1) + 8 * s2) * (2LL * I) + col0;
+              epi_put<NP>(d, 2LL * I, 8, I - col0, lane, gw[s2]);
+              epi_put<NP>(d + I, 2LL * I, 8, I - col0, lane, uw[s2]);
             }
           }
         }

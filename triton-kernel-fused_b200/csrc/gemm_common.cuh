@@ -266,6 +266,28 @@ __device__ __forceinline__ void glu_bwd32(const uint32_t (&r)[32], const uint4 (
   glu_bwd32_code<0>(r, g, u, og, ou);
 }
 
+// four packed pairs in place: gi = grad_inter, already rounded; g, u = gate, up -> grad_gate, grad_up
+template <int CODE>
+__device__ __forceinline__ void glu_bwd_pairs_code(const uint32_t (&gi)[4], uint32_t (&g)[4], uint32_t (&u)[4]) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const float2 gf = unpack_bf16x2(g[b]), uf = unpack_bf16x2(u[b]), go = unpack_bf16x2(gi[b]);
+    float gg0, gu0, gg1, gu1;
+    glu_bwd_val<CODE>(gf.x, uf.x, go.x, gg0, gu0);
+    glu_bwd_val<CODE>(gf.y, uf.y, go.y, gg1, gu1);
+    g[b] = pack_bf16x2(gg0, gg1);
+    u[b] = pack_bf16x2(gu0, gu1);
+  }
+}
+template <bool POLY>
+__device__ __forceinline__ void glu_bwd_pairs(int code, const uint32_t (&gi)[4], uint32_t (&g)[4], uint32_t (&u)[4]) {
+  if constexpr (POLY) {
+    if (code == 1) return glu_bwd_pairs_code<1>(gi, g, u);
+    if (code == 5) return glu_bwd_pairs_code<5>(gi, g, u);
+  }
+  glu_bwd_pairs_code<0>(gi, g, u);
+}
+
 // the same with grad_inter already rounded and packed: gi[i] = columns (2i, 2i+1)
 __device__ __forceinline__ void glu_bwd32_packed(const uint32_t* gi, const uint4 (&g)[4], const uint4 (&u)[4],
                                                  uint32_t* og, uint32_t* ou) {
@@ -286,6 +308,65 @@ __device__ __forceinline__ void glu_bwd32_packed(const uint32_t* gi, const uint4
       ou[4 * v + h] = pack_bf16x2(go.x * (gf.x * s0), go.y * (gf.y * s1));
     }
   }
+}
+
+// ---- between tensor memory and global memory through registers, 8 rows x 32 NP columns at a time (NP: 1 or 2)
+// Accumulator columns from taddr on, of 16 rows: tmem_ld_wait before they are used
+template <int NP>
+__device__ __forceinline__ void epi_load(uint32_t taddr, bool have_acc, uint32_t (&r)[NP][16]) {
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    if (have_acc) {
+      tmem_ld_blocks32(taddr + 32 * i, r[i]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[i][j] = 0u;
+    }
+  }
+}
+// word b: columns 8b + 2 (lane % 4) and the next one of row 8 s2 + lane / 4, as bf16
+__device__ __forceinline__ void epi_pack(const uint32_t (&r)[16], int s2, uint32_t (&w)[4]) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) w[b] = pack_bf16x2(__uint_as_float(r[4 * b + 2 * s2]), __uint_as_float(r[4 * b + 2 * s2 + 1]));
+}
+// row and column of a lane's i-th 16-byte piece: whole 128 bytes of a row per eight lanes, or 64 per four
+template <int NP>
+__device__ __forceinline__ int epi_row(int lane, int i) { return NP == 2 ? ((lane >> 2) & ~1) + i : lane >> 2; }
+template <int NP>
+__device__ __forceinline__ int epi_col(int lane) { return NP == 2 ? line_col(lane) : 8 * (lane & 3); }
+// words of row lane / 4 -> memory; `at`: first row and column; rows, cols: how many exist from there on
+template <int NP>
+__device__ __forceinline__ void epi_put(__nv_bfloat16* at, long long ld, int rows, int cols, int lane, uint32_t (&w)[NP][4]) {
+#pragma unroll
+  for (int i = 0; i < NP; ++i) quad_transpose(w[i], lane);
+  if constexpr (NP == 2) line_exchange(w[0], w[1], lane);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int r = epi_row<NP>(lane, i), c = epi_col<NP>(lane);
+    if (r < rows && c < cols) *reinterpret_cast<uint4*>(at + r * ld + c) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+  }
+}
+// the way back in two halves, so that loads can be on their way: pieces as they lie in memory, then words of row lane / 4
+template <int NP>
+__device__ __forceinline__ void epi_pieces(const __nv_bfloat16* at, long long ld, int cols, int lane, uint4 (&v)[NP]) {
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int r = epi_row<NP>(lane, i), c = epi_col<NP>(lane);
+    v[i] = c < cols ? __ldg(reinterpret_cast<const uint4*>(at + r * ld + c)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+template <int NP>
+__device__ __forceinline__ void epi_words(const uint4 (&v)[NP], int lane, uint32_t (&w)[NP][4]) {
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    w[i][0] = v[i].x;
+    w[i][1] = v[i].y;
+    w[i][2] = v[i].z;
+    w[i][3] = v[i].w;
+  }
+  if constexpr (NP == 2) line_exchange(w[0], w[1], lane);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) quad_transpose(w[i], lane);
 }
 
 // One lane = one row of a 32-row staging box: 64 bf16 (32 packed registers) go to the 128-byte

@@ -290,6 +290,15 @@ __device__ __forceinline__ void tmem_ld_blocks16(uint32_t taddr, uint32_t (&r)[8
                : "r"(taddr)
                : "memory");
 }
+// the same over 32 columns: four column blocks
+__device__ __forceinline__ void tmem_ld_blocks32(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 // an 8 x 8 block of 16-bit values, transposed among the threads of a warp
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t m) {
   uint32_t d;
@@ -312,6 +321,19 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int lane) {
     else w[i + 2] = r;
   }
 }
+// Pieces of 16 bytes, a from the first and b from the second 64 bytes of a row's 128, rows t / 4 of a warp's threads: afterwards a belongs
+// to the even and b to the odd row of two neighbouring ones, and the threads of both rows hold one row's 128 bytes between
+// them (columns: line_col).  Its own inverse.
+__device__ __forceinline__ void line_exchange(uint32_t (&a)[4], uint32_t (&b)[4], int lane) {
+  const bool odd = (lane & 4) != 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? a[i] : b[i], 4);
+    if (odd) a[i] = r;
+    else b[i] = r;
+  }
+}
+__device__ __forceinline__ int line_col(int lane) { return ((lane & 4) << 3) + 8 * (lane & 3); }   // of 64 columns
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
