@@ -52,6 +52,20 @@ def test_argument_errors_are_python_exceptions():
     assert lib.b200moe_combine(None, None, None, 4, 2, 64, None, None) == -6
 
 
+@pytest.mark.parametrize("cap,N,K", [(8 * 256 + 512, 256, 512), (8 * 256 + 256 * 1024, 256, 512), (8 * 256 + 512, 128, 256)])
+def test_unaligned_mxfp8_scales_are_refused(cap, N, K):
+    """Scale buffers are sources of bulk copies: off a 16-byte boundary every product refuses them before it launches anything
+    (few rows per expert, row tiles, single-CTA tiles).  The addresses are never read."""
+    lib = load_pkg().lib()
+    ok, off = 1 << 20, (1 << 20) + 4
+    for a, b in ((off, ok), (ok, off)):
+        assert lib.b200moe_mxfp8_expert_forward(0, ok, a, ok, b, ok, ok, ok, cap, 8, N, K, K, ok, None, None, None, None) == -2
+        assert lib.b200moe_mxfp8_expert_forward(1, ok, a, ok, b, ok, ok, ok, cap, 8, 2 * N, K, N, None, ok, ok, None, None) == -2
+        assert lib.b200moe_mxfp8_expert_gemm(0, ok, a, ok, b, ok, ok, cap, 8, N, K, K, ok, None, None, None, None, None) == -2
+        assert lib.b200moe_mxfp8_expert_wgrad(ok, a, ok, b, ok, ok, cap, 8, N, K, ok, None, None) == -2
+        assert lib.b200moe_mxfp8_gemm_nt(ok, a, ok, b, ok, 512, N, K, None, None) == -2
+
+
 def test_missing_library_fails_loudly(tmp_path, monkeypatch):
     pkg = load_pkg()
     from importlib import import_module

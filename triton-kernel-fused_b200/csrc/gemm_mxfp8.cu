@@ -934,11 +934,16 @@ few_mxfp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   }
 }
 
+// Every kernel here loads scale atoms with bulk or tensor copies, whose source has to be 16-byte aligned
+static int check_scales(const void* sfa, const void* sfb) {
+  B200_CHECK_ARG(aligned16(sfa) && aligned16(sfb), B200MOE_E_ALIGN, "scale buffers %p, %p must be 16-byte aligned", sfa, sfb);
+  return 0;
+}
+
 // scale atoms seen as a {128 x u32, k-chunks, row-blocks} tensor, no swizzle; box = `atoms` row-blocks
 static int map_sf(CUtensorMap* tm, const void* sf, long long row_blocks, long long k_chunks, int atoms) {
   EncodeTiledFn fn = get_encode_fn();
   B200_CHECK_ARG(fn != nullptr, B200MOE_E_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  B200_CHECK_ARG(aligned16(sf), B200MOE_E_ALIGN, "scale buffer is not 16-byte aligned");
   cuuint64_t dims[3] = {128, (cuuint64_t)k_chunks, (cuuint64_t)row_blocks};
   cuuint64_t strides[2] = {512, (cuuint64_t)k_chunks * 512};
   cuuint32_t box[3] = {128, 1, (cuuint32_t)atoms};
@@ -1003,6 +1008,8 @@ static int map_fp8(CUtensorMap* tm, const void* q, long long rows, long long K, 
 template <int EPI, int NT>
 static int launch_few_fp8(const void* Xq, const void* Wq, int64_t rows_cap, const FewFp8Params& p, cudaStream_t stream) {
   using C = FewFp8Cfg<EPI, NT>;
+  int rc = check_scales(p.sfx, p.sfw);
+  if (rc) return rc;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -1010,7 +1017,7 @@ static int launch_few_fp8(const void* Xq, const void* Wq, int64_t rows_cap, cons
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   CUtensorMap tmW, tmX, tmXbig;
-  int rc = map_fp8(&tmW, Wq, p.N, p.K, p.E);
+  rc = map_fp8(&tmW, Wq, p.N, p.K, p.E);
   if (rc) return rc;
   rc = make_map(&tmX, Xq, p.K, rows_cap, 1, p.K, static_cast<uint64_t>(rows_cap) * p.K, FBK, 16, 1);
   if (rc) return rc;
@@ -1026,8 +1033,10 @@ static int launch_few_fp8(const void* Xq, const void* Wq, int64_t rows_cap, cons
 template <int EPI>
 static int launch_any(const void* Aq, long long a_rows, const void* Bq, long long b_rows, long long b_groups,
                       long long K, const Fp8Params& fp, int max_tiles_1cta, cudaStream_t stream) {
+  int rc = check_scales(fp.sfa, fp.sfb);
+  if (rc) return rc;
   CUtensorMap tmA, tmB;
-  int rc = map_fp8(&tmA, Aq, a_rows, K, 1);
+  rc = map_fp8(&tmA, Aq, a_rows, K, 1);
   if (rc) return rc;
   rc = map_fp8(&tmB, Bq, b_rows, K, b_groups);
   if (rc) return rc;
