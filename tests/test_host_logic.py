@@ -1,5 +1,7 @@
 """CPU: host-side logic of the package that needs no kernel launch."""
 import importlib
+import os
+import re
 
 import torch
 
@@ -247,3 +249,23 @@ def test_route_of_a_forward_without_backward():
                                    (8, 1024, 1024, 2, 351, True), (8, 1024, 1024, 2, 352, False), (8, 1024, 1280, 2, 352, True)):
         kept, quiet = (size(T, H, I, E, E, k, keep, 0) for keep in (1, 0))
         assert (quiet < kept) == compact, (E, H, I, k, T)
+
+
+def test_chained_kernels_promise_no_constant_data():
+    """A chained kernel (one with a grid_dep_wait) starts while the kernel before it still writes what it reads: none of its
+    pointers may be __restrict__, nothing in its file read through the non-coherent path, and it waits."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), PKG, "csrc")
+    seen = 0
+    sources = {f: re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read()) for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))}
+    for name, text in sources.items():
+        for kernel in re.split(r"(?=\b__global__\b)", text)[1:]:
+            head, body = kernel.split("{", 1)
+            if not re.search(r"\bgrid_dep_(wait|begin|launch)\(", body):
+                continue
+            seen += 1
+            assert "__restrict__" not in head, (name, head)
+            assert re.search(r"\bgrid_dep_(wait|begin)\(", body), (name, head)
+            assert not re.search(r"__ldg\(|ld\.global\.nc", text), name
+    assert seen >= 25
+    for shared in ("common.cuh", "ptx.cuh", "gemm_common.cuh", "few_tiles.cuh", "topk.cuh", "mxfp8_quant.cuh"):
+        assert not re.search(r"__ldg\(|ld\.global\.nc", sources[shared]), shared

@@ -25,8 +25,8 @@ constexpr int kVecBatch = 4;   // 16-byte vectors a lane keeps in flight per row
 // H 2048, top-8 223 -> 214 us.
 template <int TPR>
 __global__ void __launch_bounds__(256)
-combine_kernel(const uint4* __restrict__ rows, const float* __restrict__ w, const int* __restrict__ slot_row,
-               const uint4* __restrict__ add, long long T, int k, int vec_per_row, uint4* __restrict__ out) {
+combine_kernel(const uint4* rows, const float* w, const int* slot_row, const uint4* add, long long T, int k,
+               int vec_per_row, uint4* out) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   for (long long t = static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; t < T;
@@ -61,9 +61,8 @@ combine_kernel(const uint4* __restrict__ rows, const float* __restrict__ w, cons
 // One warp per routed row, 2 * kVecBatch independent 16-byte loads in flight per lane; the dot product is
 // reduced by shuffles in a fixed order.
 __global__ void __launch_bounds__(256)
-combine_bwd_kernel(const uint4* __restrict__ go, const uint4* __restrict__ eo, const float* __restrict__ w,
-                   const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k, int vec_per_row,
-                   uint4* __restrict__ grad_eo, float* __restrict__ grad_w) {
+combine_bwd_kernel(const uint4* go, const uint4* eo, const float* w, const int* row_slot, const int* total_rows, int k,
+                   int vec_per_row, uint4* grad_eo, float* grad_w) {
   grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -116,9 +115,8 @@ combine_bwd_kernel(const uint4* __restrict__ go, const uint4* __restrict__ eo, c
 // in flight here too (the kernel above keeps two: 20 000 tokens of H 256, top-8: 82 -> 70 us; for wider rows it is the
 // faster one: 64 vectors 18 against 24 us, 256 vectors 200 against 248 us).
 __global__ void __launch_bounds__(256)
-combine_bwd_narrow_kernel(const uint4* __restrict__ go, const uint4* __restrict__ eo, const float* __restrict__ w,
-                          const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k, int vec_per_row,
-                          uint4* __restrict__ grad_eo, float* __restrict__ grad_w) {
+combine_bwd_narrow_kernel(const uint4* go, const uint4* eo, const float* w, const int* row_slot, const int* total_rows,
+                          int k, int vec_per_row, uint4* grad_eo, float* grad_w) {
   grid_dep_begin();
   constexpr int RB = 4;
   const int lane = threadIdx.x & 31;

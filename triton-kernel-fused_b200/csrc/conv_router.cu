@@ -13,7 +13,7 @@
 namespace b200moe {
 
 __global__ void __launch_bounds__(256)
-conv_unfold_kernel(const uint4* __restrict__ x, long long B, long long S, int K, int vec_h, uint4* __restrict__ xu) {
+conv_unfold_kernel(const uint4* x, long long B, long long S, int K, int vec_h, uint4* xu) {
   grid_dep_begin();
   const long long rows = B * S;
   for (long long r = blockIdx.x; r < rows; r += gridDim.x) {

@@ -352,7 +352,7 @@ __device__ __forceinline__ void epi_pieces(const __nv_bfloat16* at, long long ld
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     const int r = epi_row<NP>(lane, i), c = epi_col<NP>(lane);
-    v[i] = c < cols ? __ldg(reinterpret_cast<const uint4*>(at + r * ld + c)) : make_uint4(0u, 0u, 0u, 0u);
+    v[i] = c < cols ? *reinterpret_cast<const uint4*>(at + r * ld + c) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 template <int NP>

@@ -277,8 +277,8 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int col = t.n0 + c0 + v * 8;
-            g4[v] = col < I ? __ldg(reinterpret_cast<const uint4*>(gu + col)) : make_uint4(0u, 0u, 0u, 0u);
-            u4[v] = col < I ? __ldg(reinterpret_cast<const uint4*>(gu + I + col)) : make_uint4(0u, 0u, 0u, 0u);
+            g4[v] = col < I ? *reinterpret_cast<const uint4*>(gu + col) : make_uint4(0u, 0u, 0u, 0u);
+            u4[v] = col < I ? *reinterpret_cast<const uint4*>(gu + I + col) : make_uint4(0u, 0u, 0u, 0u);
           }
           uint32_t r[32], og[16], ou[16];
           tmem_ld32(taddr + c0, r);

@@ -147,9 +147,8 @@ __device__ __forceinline__ void glu_fwd_row(const uint4 (&g)[VPT], const uint4 (
 
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(kRowThreads)
-glu_fwd_vec_kernel(const uint4* __restrict__ gate_up, const int* __restrict__ tile_expert, const int* __restrict__ codes,
-                   const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
-                   uint4* __restrict__ inter) {
+glu_fwd_vec_kernel(const uint4* gate_up, const int* tile_expert, const int* codes, const float* params,
+                   const int* total_rows, int nvec, uint4* inter) {
   grid_dep_begin();
   constexpr int RPB = kRowThreads / TPR;   // rows a CTA works on at a time; divides the 256-row tile
   __shared__ float red[kRowThreads / 32];
@@ -236,10 +235,9 @@ __device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (
 
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(kRowThreads)
-glu_bwd_vec_kernel(const uint4* __restrict__ grad_inter, const uint4* __restrict__ gate_up,
-                   const int* __restrict__ tile_expert, const int* __restrict__ codes,
-                   const float* __restrict__ params, const int* __restrict__ total_rows, int nvec,
-                   uint4* __restrict__ grad_gate_up, float* __restrict__ row_da, float* __restrict__ row_dg) {
+glu_bwd_vec_kernel(const uint4* grad_inter, const uint4* gate_up, const int* tile_expert, const int* codes,
+                   const float* params, const int* total_rows, int nvec, uint4* grad_gate_up, float* row_da,
+                   float* row_dg) {
   grid_dep_begin();
   constexpr int RPB = kRowThreads / TPR;
   __shared__ float red[kRowThreads / 32];
@@ -287,9 +285,8 @@ glu_bwd_vec_kernel(const uint4* __restrict__ grad_inter, const uint4* __restrict
 
 // ---------------------------------------------------------------------------- one value per thread
 __global__ void __launch_bounds__(256)
-glu_fwd_rows_kernel(const __nv_bfloat16* __restrict__ gate_up, const int* __restrict__ tile_expert,
-                    const int* __restrict__ codes, const float* __restrict__ params, const int* __restrict__ total_rows,
-                    int I, __nv_bfloat16* __restrict__ inter) {
+glu_fwd_rows_kernel(const __nv_bfloat16* gate_up, const int* tile_expert, const int* codes, const float* params,
+                    const int* total_rows, int I, __nv_bfloat16* inter) {
   grid_dep_begin();
   __shared__ float red[8];
   const int total = *total_rows;
@@ -320,10 +317,9 @@ glu_fwd_rows_kernel(const __nv_bfloat16* __restrict__ gate_up, const int* __rest
 
 // grad_gate_up = [grad_gate | grad_up]; optional per-row d(alpha), d(gamma) for learnable SiTU.
 __global__ void __launch_bounds__(256)
-glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ grad_inter, const __nv_bfloat16* __restrict__ gate_up,
-                    const int* __restrict__ tile_expert, const int* __restrict__ codes,
-                    const float* __restrict__ params, const int* __restrict__ total_rows, int I,
-                    __nv_bfloat16* __restrict__ grad_gate_up, float* __restrict__ row_da, float* __restrict__ row_dg) {
+glu_bwd_rows_kernel(const __nv_bfloat16* grad_inter, const __nv_bfloat16* gate_up, const int* tile_expert,
+                    const int* codes, const float* params, const int* total_rows, int I, __nv_bfloat16* grad_gate_up,
+                    float* row_da, float* row_dg) {
   grid_dep_begin();
   __shared__ float red[8];
   const int total = *total_rows;
@@ -413,8 +409,7 @@ glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ grad_inter, const __nv_bfl
 // of its loads: 1024 threads keep a segment's rows in flight in a few rounds (3000 rows an expert: 8.7 -> 4.1 us with 256 -> 1024).
 constexpr int kSumThreads = 1024;
 __global__ void __launch_bounds__(kSumThreads)
-expert_row_sums_kernel(const float* __restrict__ row_da, const float* __restrict__ row_dg, const int* __restrict__ poffs,
-                       float* __restrict__ out) {
+expert_row_sums_kernel(const float* row_da, const float* row_dg, const int* poffs, float* out) {
   grid_dep_begin();
   __shared__ float red[kSumThreads / 32];
   const int e = blockIdx.x;
@@ -435,9 +430,8 @@ expert_row_sums_kernel(const float* __restrict__ row_da, const float* __restrict
 // dst[r] = src[r] for Identity (code 3), 0 otherwise (Zero, code 4); TPR threads share a row
 template <int TPR>
 __global__ void __launch_bounds__(256)
-special_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ tile_expert, const int* __restrict__ codes,
-                    const int* __restrict__ poffs, int first_special, int num_experts, int vec_per_row,
-                    uint4* __restrict__ dst) {
+special_rows_kernel(const uint4* src, const int* tile_expert, const int* codes, const int* poffs, int first_special,
+                    int num_experts, int vec_per_row, uint4* dst) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int r0 = poffs[first_special], r1 = poffs[num_experts];

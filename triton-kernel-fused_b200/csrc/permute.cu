@@ -35,7 +35,7 @@ static PermSplit perm_split(long long M) {
 
 template <int W, int PL>
 __global__ void __launch_bounds__(32 * W)
-permute_hist_kernel(const long long* __restrict__ idx, long long M, int E, int* __restrict__ block_hist) {
+permute_hist_kernel(const long long* idx, long long M, int E, int* block_hist) {
   grid_dep_begin();
   constexpr int kPermThreads = 32 * W;
   __shared__ int h[B200MOE_MAX_EXPERTS];
@@ -54,11 +54,9 @@ permute_hist_kernel(const long long* __restrict__ idx, long long M, int E, int* 
 
 template <int W, int PL>
 __global__ void __launch_bounds__(32 * W)
-permute_rank_kernel(const long long* __restrict__ idx, long long M, int E, const int* __restrict__ block_hist,
-                    int* __restrict__ counts, int* __restrict__ offs, int* __restrict__ poffs,
-                    int* __restrict__ slot_row, int* __restrict__ row_slot, int* __restrict__ tile_expert,
-                    int* __restrict__ order, int* __restrict__ slot_pos, int* __restrict__ counts_out,
-                    long long* __restrict__ load, int* __restrict__ status) {
+permute_rank_kernel(const long long* idx, long long M, int E, const int* block_hist, int* counts, int* offs, int* poffs,
+                    int* slot_row, int* row_slot, int* tile_expert, int* order, int* slot_pos, int* counts_out,
+                    long long* load, int* status) {
   grid_dep_begin();
   constexpr int kPermWarps = W, kPermThreads = 32 * W;
   extern __shared__ int sh[];                          // [W][E]: ranks a warp's run starts at
@@ -216,8 +214,7 @@ static int launch_permute(const long long* idx, long long M, int E, int* hist, i
 // whole CTA a row 20 000 tokens of H 256, top-8 take 84 us (36 here), 16 384 of H 512, top-2 21 us (11 here).
 template <int TPR>
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ row_slot,
-                   const int* __restrict__ total_rows, int k, int vec_per_row, uint4* __restrict__ x_s) {
+gather_rows_kernel(const uint4* x, const int* row_slot, const int* total_rows, int k, int vec_per_row, uint4* x_s) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int total = *total_rows;

@@ -145,7 +145,8 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
 }
 
 // ---------------------------------------------------------------- chained launches (launch_chained, common.cuh)
-// the kernel before this one in the stream is complete and its writes are visible
+// the kernel before this one in the stream is complete and its writes are visible; the clobber keeps every load and store of what
+// another kernel touches behind it
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the next kernel's CTAs may be placed once every CTA has got here (call it after grid_dep_wait only)
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -31,8 +31,7 @@ __device__ __forceinline__ long long interleaved_row(long long r, long long I) {
 // re-ordered per 64 so that each group of 128 output rows holds gate rows j..j+63 then up rows
 // j..j+63 (the SwiGLU GEMM then sees gate and up of the same columns in one 128-wide tile).
 __global__ void __launch_bounds__(256)
-quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, long long C, long long interleave_I,
-                  uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+quant_rows_kernel(const __nv_bfloat16* x, long long R, long long C, long long interleave_I, uint8_t* q, uint8_t* sf) {
   grid_dep_begin();
   const long long blocks_per_row = C >> 5;
   const long long k_chunks = (C + 127) >> 7;
@@ -44,7 +43,7 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, long long C,
     const uint4* src = reinterpret_cast<const uint4*>(x + r * C + b * 32);
     uint4 v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __ldg(src + j);
+    for (int j = 0; j < 4; ++j) v[j] = src[j];
     const long long dr = interleave_I > 0 ? interleaved_row(r, interleave_I) : r;
     mx_quant_store32(reinterpret_cast<const uint32_t*>(v), q + dr * C + b * 32, sf, dr, b, k_chunks);
   }
@@ -61,9 +60,8 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long R, long long C,
 // row_slot[r] >= 0, and a zero row otherwise: the gathered matrix itself is never written.
 template <bool ROWS, bool GATHER = false>
 __global__ void __launch_bounds__(256, 4)
-quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R, long long C, long long interleave_I,
-                  uint8_t* __restrict__ q_t, uint8_t* __restrict__ sf_t, uint8_t* __restrict__ q_r,
-                  uint8_t* __restrict__ sf_r, const int* __restrict__ row_slot, const int* __restrict__ total_rows, int k) {
+quant_tile_kernel(const __nv_bfloat16* x, long long G, long long R, long long C, long long interleave_I, uint8_t* q_t,
+                  uint8_t* sf_t, uint8_t* q_r, uint8_t* sf_r, const int* row_slot, const int* total_rows, int k) {
   grid_dep_begin();
   // source row of matrix row r (nullptr = zero row)
   auto src_row = [&](long long g, long long r) -> const __nv_bfloat16* {
@@ -101,7 +99,7 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R,
           uint4 v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            v[j] = srow != nullptr ? __ldg(reinterpret_cast<const uint4*>(srow + cb) + j) : make_uint4(0u, 0u, 0u, 0u);
+            v[j] = srow != nullptr ? reinterpret_cast<const uint4*>(srow + cb)[j] : make_uint4(0u, 0u, 0u, 0u);
           const long long dr = interleave_I > 0 ? interleaved_row(gr, interleave_I) : gr;
           mx_quant_store32(reinterpret_cast<const uint32_t*>(v), q_r + dr * C + cb, sf_r, dr, cb >> 5, kc_r);
         }
@@ -127,14 +125,14 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R,
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int t = __shfl_sync(0xffffffffu, my_tok, i);
-          v[i] = (in && t >= 0) ? __ldg(reinterpret_cast<const uint32_t*>(x + static_cast<long long>(t) * C + c)) : 0u;
+          v[i] = (in && t >= 0) ? *reinterpret_cast<const uint32_t*>(x + static_cast<long long>(t) * C + c) : 0u;
         }
       }
       if (r0 < R && c < C) {
         if constexpr (!GATHER) {
           const __nv_bfloat16* src = x + (g * R + r0) * C + c;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(src + i * C));
+          for (int i = 0; i < 32; ++i) v[i] = *reinterpret_cast<const uint32_t*>(src + i * C);
         }
         uint32_t m = 0u;
 #pragma unroll
@@ -192,9 +190,8 @@ quant_tile_kernel(const __nv_bfloat16* __restrict__ x, long long G, long long R,
 // Gather fused with the row quantiser: x_s[r] = x[row_slot[r] / k] (bf16 copy for a caller that wants it, nullable)
 // and its e4m3 codes + scales; pad rows become zeros with scale byte 0.  One thread per 32-element block.
 __global__ void __launch_bounds__(256)
-gather_quant_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ row_slot,
-                    const int* __restrict__ total_rows, int k, long long C, __nv_bfloat16* __restrict__ x_s,
-                    uint8_t* __restrict__ q, uint8_t* __restrict__ sf) {
+gather_quant_kernel(const __nv_bfloat16* x, const int* row_slot, const int* total_rows, int k, long long C,
+                    __nv_bfloat16* x_s, uint8_t* q, uint8_t* sf) {
   grid_dep_begin();
   const long long blocks_per_row = C >> 5;
   const long long k_chunks = (C + 127) >> 7;
@@ -208,7 +205,7 @@ gather_quant_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__
     if (slot >= 0) {
       const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<long long>(slot / k) * C + b * 32);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = __ldg(src + j);
+      for (int j = 0; j < 4; ++j) v[j] = src[j];
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = make_uint4(0u, 0u, 0u, 0u);

@@ -26,9 +26,8 @@ __device__ __forceinline__ float load_in(const void* p, long long i) {
 // stable sort gives), instead of five shuffle rounds of (value, id) pairs.
 template <int KIND, int VPL>
 __global__ void __launch_bounds__(256)
-router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__ bias, long long T, int E,
-                       int k, int norm, float scale, long long* __restrict__ idx_out,
-                       float* __restrict__ w_out, int* __restrict__ counts) {
+router_topk_fwd_kernel(const void* input, const float* bias, long long T, int E, int k, int norm, float scale,
+                       long long* idx_out, float* w_out, int* counts) {
   grid_dep_begin();
   __shared__ int hist[B200MOE_MAX_EXPERTS];
   const int lane = threadIdx.x & 31;
@@ -82,9 +81,8 @@ router_topk_fwd_kernel(const void* __restrict__ input, const float* __restrict__
 // the sums run over the picks in order.  (T = 16384, E = 64, k = 6: 14.2 -> 6.8 us.)
 template <int KIND, int VPL, bool PAIR>
 __global__ void __launch_bounds__(256)
-router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restrict__ idx,
-                       const float* __restrict__ grad_w, long long T, int E, int k, int norm, float scale, int S, int taps,
-                       __nv_bfloat16* __restrict__ grad_logits) {
+router_topk_bwd_kernel(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k,
+                       int norm, float scale, int S, int taps, __nv_bfloat16* grad_logits) {
   grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -153,8 +151,7 @@ router_topk_bwd_kernel(const void* __restrict__ logits, const long long* __restr
 
 // w (E, H, taps) -> wt (taps, E, H), wt[j, e, h] = w[e, h, j] (the operand of the conv router's products), or (E, taps, H)
 __global__ void __launch_bounds__(256)
-conv_weight_rows_kernel(const __nv_bfloat16* __restrict__ w, int E, int H, int taps, int by_expert,
-                        __nv_bfloat16* __restrict__ wt) {
+conv_weight_rows_kernel(const __nv_bfloat16* w, int E, int H, int taps, int by_expert, __nv_bfloat16* wt) {
   grid_dep_begin();
   const long long n = static_cast<long long>(E) * H;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
@@ -166,8 +163,7 @@ conv_weight_rows_kernel(const __nv_bfloat16* __restrict__ w, int E, int H, int t
 
 // grad_w (E, H, taps) bf16 = sum over the slices of p (slices, taps*E, H) fp32
 __global__ void __launch_bounds__(256)
-conv_weight_grad_kernel(const float* __restrict__ p, long long slices, int E, int H, int taps,
-                        __nv_bfloat16* __restrict__ gw) {
+conv_weight_grad_kernel(const float* p, long long slices, int E, int H, int taps, __nv_bfloat16* gw) {
   grid_dep_begin();
   const long long n = static_cast<long long>(E) * H, elems = n * taps;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < elems; i += gridDim.x * 256LL) {
@@ -199,8 +195,7 @@ __global__ void router_bias_update_kernel(float* bias, const int* counts, int E,
 
 // D[i] = bf16( sum_s P[s][i] ), 4 elements per thread
 __global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ P, long long slices, long long elems,
-                     __nv_bfloat16* __restrict__ D) {
+splitk_reduce_kernel(const float* P, long long slices, long long elems, __nv_bfloat16* D) {
   grid_dep_begin();
   const long long i4 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i4 >= elems) return;
@@ -218,7 +213,7 @@ splitk_reduce_kernel(const float* __restrict__ P, long long slices, long long el
 // D (C,R) = bf16( sum_s P[s] (R,C) )^T through a 32 x 32 tile in shared memory: both sides coalesced, a thread per
 // value so that all its slices are in flight at once
 __global__ void __launch_bounds__(1024)
-splitk_reduce_t_kernel(const float* __restrict__ P, long long slices, int R, int C, __nv_bfloat16* __restrict__ D) {
+splitk_reduce_t_kernel(const float* P, long long slices, int R, int C, __nv_bfloat16* D) {
   grid_dep_begin();
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
