@@ -12,7 +12,7 @@
 // H 2048, I 1408, 64 experts, us as row tiles / here: 288 rows (4.5 an expert; 118 + 59 us at copy rate): gate/up 161 / 108, down 80 /
 // 60; 9000 rows (141 an expert): 171 / 151 and 85 / 75; 6 rows of one token: 21 / 12.3 and 15 / 9.2.
 // A large tile is bound by the bytes that leave L2 (weights in and out, X once per 128 columns) and wants them in flight: with a
-// stage less the 9000 rows take 157 us.  A small one is bound by latencies and by what a stage costs the two threads that
+// stage less gate/up of 9000 rows takes 157 us (beside 151 then).  A small one is bound by latencies and by what a stage costs the two threads that
 // issue it: one lane for all boxes, elected (ptx.cuh), 128-row weight boxes that hold gate and up (make_map_gate_up), and tiles of 64
 // columns where even they are one wave; with a lane per box and tiles of 128 one token took 18.3 and 11.1 us.
 //
@@ -267,7 +267,10 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         else if (EPI == EPI_SWIGLU && code == 5) f(std::integral_constant<int, 5>());
         else f(std::integral_constant<int, 0>());
       };
-      if constexpr (NBUF == 1) {         // the only accumulators: drained before anything else, so that the MMAs go on
+      // The only accumulators of a plain product are drained before anything else, so that the MMAs go on (9000 rows, us: 90 / 88).
+      // Gate and up are not: their 96 words a thread beside the activations do not fit its registers (gate/up of 9000 rows 164 us,
+      // spilled; 146 as here, and drained one block at a time 147).
+      if constexpr (NBUF == 1 && EPI == EPI_STORE) {
         uint32_t v[G][HALVES][2][4];
 #pragma unroll
         for (int g = 0; g < G; ++g)
@@ -277,13 +280,11 @@ few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
-        by_code([&](auto tag) {
 #pragma unroll
-          for (int g = 0; g < G; ++g)
-            if (16 * half + 32 * g < t.live)
+        for (int g = 0; g < G; ++g)
+          if (16 * half + 32 * g < t.live)
 #pragma unroll
-              for (int hb = 0; hb < HALVES; ++hb) put(tag, hb, 16 * half + 32 * g, v[g][hb]);
-        });
+            for (int hb = 0; hb < HALVES; ++hb) put(std::integral_constant<int, 0>(), hb, 16 * half + 32 * g, v[g][hb]);
       } else {
         by_code([&](auto tag) {
 #pragma unroll 1
