@@ -43,3 +43,31 @@ def test_forward_without_gradient_keeps_only_the_row_wise_copies(pkg):
     with torch.no_grad():
         assert torch.equal(layer(x), quiet)
     pkg.check_status()
+
+
+def test_kept_copies_are_complete_on_another_stream(pkg):
+    """Copies that a busy stream has only queued, read at once by a call on another stream; then freed while that call runs."""
+    g = torch.Generator().manual_seed(8)
+    idx = torch.stack([torch.randperm(8, generator=g)[:2] for _ in range(64)]).to(DEV)
+    x = torch.randn(64, 256, generator=g).to(torch.bfloat16).to(DEV)
+    w, codes = torch.rand(64, 2, generator=g).to(DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    dn = (torch.randn(8, 256, 512, generator=g) * 0.1).to(torch.bfloat16).to(DEV)
+    side = torch.cuda.Stream()
+    for fn, dtype in ((pkg.moe_mxfp8, torch.bfloat16), (pkg.moe, torch.float32)):
+        gu = (torch.randn(8, 1024, 256, generator=g) * 0.1).to(dtype).to(DEV)
+        args = lambda: (x.to(dtype), idx, w, gu, dn.to(dtype), codes)     # noqa: E731
+        with torch.no_grad():
+            want = fn(*args())
+            for _ in range(3):
+                a = args()
+                torch.cuda.synchronize()
+                gu.mul_(1.0)                       # another version: new copies, of the same values
+                torch.cuda._sleep(20_000_000)      # the main stream is busy for about 10 ms
+                fn(*a)
+                with torch.cuda.stream(side):
+                    got = fn(*a)
+                gu.mul_(1.0)
+                fn(*a)                             # the old copies go; their memory is written on the main stream
+                torch.cuda.synchronize()
+                assert torch.equal(got, want)
+    pkg.check_status()

@@ -269,3 +269,67 @@ def test_chained_kernels_promise_no_constant_data():
     assert seen >= 25
     for shared in ("common.cuh", "ptx.cuh", "gemm_common.cuh", "few_tiles.cuh", "topk.cuh", "mxfp8_quant.cuh"):
         assert not re.search(r"__ldg\(|ld\.global\.nc", sources[shared]), shared
+
+
+def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
+    """Quantised and bf16 copies that one stream made: a call on another stream waits for it before it reads them, until they are
+    known to be complete, and records itself as a user of their memory; the stream that made them does neither."""
+    moe_mod, mx, L = (importlib.import_module(PKG + n) for n in (".moe", ".mxfp8", "._lib"))
+    log = []
+
+    class Event:
+        done = False
+
+        def query(self):
+            return self.done
+
+    class Stream:
+        def __init__(self, name):
+            self.name, self.cuda_stream = name, hash(name)
+
+        def record_event(self):
+            log.append(("record", self.name))
+            return Event()
+
+        def wait_event(self, e):
+            log.append(("wait", self.name))
+
+    class Copy:
+        is_cuda, device = True, torch.device("cuda", 0)
+
+        def record_stream(self, s):
+            log.append(("used by", s.name))
+
+        def to(self, _):
+            return self
+
+        detach = lambda self: self     # noqa: E731
+
+    now = [Stream("a")]
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: now[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(L, "stream_of", lambda t: now[0].cuda_stream)
+
+    class Master(Copy):
+        requires_grad, _version = False, 0
+
+    stack, master = torch.zeros(2), Master()
+    q = (Copy(), Copy())
+    for get in (lambda: mx._quantised_weights(stack, lambda: q, None, False), lambda: moe_mod._bf16_copy(master)):
+        now[0] = Stream("a")
+        n = len(log)
+        res = get()
+        copies = res if isinstance(res, tuple) else (res,)
+        assert log[n:] == [("record", "a")]
+        get()
+        assert log[n + 1:] == []
+        now[0], n = Stream("b"), len(log)
+        assert get() is res or get() == res
+        assert ("wait", "b") in log[n:] and log[n:].count(("used by", "b")) % len(copies) == 0 and ("used by", "b") in log[n:]
+        assert log[n:].index(("wait", "b")) < log[n:].index(("used by", "b"))
+        Event.done, n = True, len(log)
+        get()
+        assert ("wait", "b") not in log[n:] and ("used by", "b") in log[n:]
+        Event.done = False
+    del mx._QUANTISED[id(stack)]
+    del moe_mod._BF16_COPIES[id(master)]

@@ -175,7 +175,34 @@ def _empty_result(hidden, top_k_weights, *params):
     return out
 
 
-_BF16_COPIES = {}     # id(parameter) -> (weak reference, version, bf16 copy)
+class StackCopies:
+    """Copies of a weight stack that outlive the call that made them.  The stream that wrote them need not be the one that reads
+    them next: until they are known to be complete a reader on another stream waits for the writer's event, and their memory is
+    not handed out again before that stream is done with it.  (While a graph is being captured neither is possible, nor needed:
+    torch.cuda.graph waits for the device before it begins.)"""
+
+    def __init__(self, tensors):
+        self.tensors = tensors
+        self.stream = self.event = None
+        if tensors[0].is_cuda and not torch.cuda.is_current_stream_capturing():
+            self.stream = L.stream_of(tensors[0])
+            self.event = torch.cuda.current_stream(tensors[0].device).record_event()
+
+    def here(self):
+        """The tensors, for the current stream."""
+        if (self.stream is not None and L.stream_of(self.tensors[0]) != self.stream
+                and not torch.cuda.is_current_stream_capturing()):
+            now = torch.cuda.current_stream(self.tensors[0].device)
+            if self.event is not None and self.event.query():
+                self.event = None
+            if self.event is not None:
+                now.wait_event(self.event)
+            for t in self.tensors:
+                t.record_stream(now)
+        return self.tensors
+
+
+_BF16_COPIES = {}     # id(parameter) -> (weak reference, version, StackCopies of the bf16 copy)
 
 
 def _bf16_copy(t):
@@ -189,9 +216,9 @@ def _bf16_copy(t):
     key = id(t)
     hit = _BF16_COPIES.get(key)
     if hit is not None and hit[0]() is t and hit[1] == t._version:
-        return hit[2]
+        return hit[2].here()[0]
     c = t.detach().to(torch.bfloat16)
-    _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, c)
+    _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, StackCopies((c,)))
     return c
 
 

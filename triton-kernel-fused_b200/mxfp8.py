@@ -17,7 +17,7 @@ import torch
 
 from . import _lib as L
 from . import ops
-from .moe import _amp_cast, _code_info, _empty_result
+from .moe import StackCopies, _amp_cast, _code_info, _empty_result
 
 __all__ = ["moe_mxfp8", "FUSE_QUANT_EPILOGUE"]
 
@@ -30,7 +30,7 @@ FUSE_QUANT_EPILOGUE = os.environ.get("B200MOE_MXFP8_FUSE_QUANT", "0") == "1"
 # Quantised copies of the expert stacks are reused while the stacks are unchanged (B200MOE_MXFP8_WEIGHT_CACHE=0: off).
 # They cost one byte per weight and direction: 2 x the bf16 stack's bytes when both directions are kept.
 WEIGHT_CACHE = os.environ.get("B200MOE_MXFP8_WEIGHT_CACHE", "1") == "1"
-_QUANTISED = {}      # id(stack) -> (weak reference, version, data pointer, has the transposed copy, tensors)
+_QUANTISED = {}      # id(stack) -> (weak reference, version, data pointer, has the transposed copy, tensors, StackCopies)
 
 
 def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None):
@@ -45,13 +45,13 @@ def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None):
     if hit is not None and not (hit[0]() is stack and hit[1] == stack._version and hit[2] == stack.data_ptr()):
         hit = None
     if hit is not None and (hit[3] or not both):
-        return hit[4] if both else hit[4][:2]
+        return hit[5].here() if both else hit[5].here()[:2]
     if hit is not None and transpose_fn is not None:
-        res = hit[4] + transpose_fn()
+        res = hit[5].here() + transpose_fn()
     else:
         res = both_fn() if both else rows_fn()
     _QUANTISED[key] = (weakref.ref(stack, lambda _r, k=key: _QUANTISED.pop(k, None)), stack._version, stack.data_ptr(),
-                       both, res)
+                       both, res, StackCopies(res))
     return res
 
 
