@@ -71,3 +71,46 @@ def test_kept_copies_are_complete_on_another_stream(pkg):
                 torch.cuda.synchronize()
                 assert torch.equal(got, want)
     pkg.check_status()
+
+
+def test_captured_passes_use_the_weights_of_the_replay(pkg):
+    """Training passes captured after eager ones (whose copies are kept): replays after an update of the weights give what an eager
+    pass on the new weights gives.  A forward captured on new weights leaves eager calls before its first replay right."""
+    torch.manual_seed(4)
+    layer = pkg.MoELayer(256, 128, 8, top_k=2, precision="mxfp8").to(DEV).to(torch.bfloat16)
+    x = torch.randn(96, 256, device=DEV).to(torch.bfloat16).requires_grad_()
+    params = [x, *layer.parameters()]
+
+    def step():
+        for p in params:
+            p.grad = None
+        out = layer(x)
+        out.backward(out.detach())
+        return [out.detach()] + [p.grad for p in params]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        res = step()
+    for scale in (-1.5, 0.5):
+        with torch.no_grad():
+            for p in layer.parameters():
+                p.mul_(scale)
+        graph.replay()
+        got = [t.clone() for t in res]
+        assert all(torch.equal(a, b) for a, b in zip(got, step()))
+    with torch.no_grad():
+        layer.gate_up_proj.mul_(2.0)
+        layer.down_proj.mul_(0.25)
+        forward = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(forward):
+            out = layer(x)
+        eager = layer(x).clone()
+        forward.replay()
+        assert torch.equal(out, eager) and eager.abs().max() > 0
+    pkg.check_status()

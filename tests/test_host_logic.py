@@ -307,7 +307,7 @@ def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
 
     now = [Stream("a")]
     monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: now[0])
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(L, "capturing", lambda: False)
     monkeypatch.setattr(L, "stream_of", lambda t: now[0].cuda_stream)
 
     class Master(Copy):
@@ -333,3 +333,31 @@ def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
         Event.done = False
     del mx._QUANTISED[id(stack)]
     del moe_mod._BF16_COPIES[id(master)]
+
+
+def test_copies_made_under_capture_are_not_kept(monkeypatch):
+    """A copy queued into a graph is filled by replays only and lies in the graph's memory: no later call may get it.  A captured
+    forward reads kept copies; a captured pass with a backward makes its own, because its weights change between replays."""
+    moe_mod, mx, L = (importlib.import_module(PKG + n) for n in (".moe", ".mxfp8", "._lib"))
+    capturing = [True]
+    monkeypatch.setattr(L, "capturing", lambda: capturing[0])
+    stack, made = torch.zeros(2, 4, 8), []
+    get = lambda **kw: mx._quantised_weights(stack, lambda: made.append(0) or (torch.zeros(1), torch.zeros(1)), None, False, **kw)     # noqa: E731
+    get()
+    assert id(stack) not in mx._QUANTISED
+    capturing[0] = False
+    kept = get()
+    assert len(made) == 2 and get()[0] is kept[0]
+    capturing[0] = True
+    assert get()[0] is kept[0] and get(keep=True)[0] is not kept[0] and len(made) == 3
+    capturing[0] = False
+    assert get(keep=True)[0] is kept[0]
+    w = torch.randn(2, 8, 4)
+    capturing[0] = True
+    a = moe_mod._bf16_copy(w)
+    assert id(w) not in moe_mod._BF16_COPIES
+    capturing[0] = False
+    b = moe_mod._bf16_copy(w)
+    assert b is not a
+    capturing[0] = True
+    assert moe_mod._bf16_copy(w) is b

@@ -210,6 +210,11 @@ def stream_of(t: torch.Tensor):
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
+def capturing() -> bool:
+    """Whether the current stream is being captured into a graph (False where there is no GPU)."""
+    return torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()
+
+
 _status = {}       # device index -> the word
 
 

@@ -184,14 +184,13 @@ class StackCopies:
     def __init__(self, tensors):
         self.tensors = tensors
         self.stream = self.event = None
-        if tensors[0].is_cuda and not torch.cuda.is_current_stream_capturing():
+        if tensors[0].is_cuda:
             self.stream = L.stream_of(tensors[0])
             self.event = torch.cuda.current_stream(tensors[0].device).record_event()
 
     def here(self):
         """The tensors, for the current stream."""
-        if (self.stream is not None and L.stream_of(self.tensors[0]) != self.stream
-                and not torch.cuda.is_current_stream_capturing()):
+        if self.stream is not None and L.stream_of(self.tensors[0]) != self.stream and not L.capturing():
             now = torch.cuda.current_stream(self.tensors[0].device)
             if self.event is not None and self.event.query():
                 self.event = None
@@ -218,6 +217,8 @@ def _bf16_copy(t):
     if hit is not None and hit[0]() is t and hit[1] == t._version:
         return hit[2].here()[0]
     c = t.detach().to(torch.bfloat16)
+    if L.capturing():      # the graph's memory, which only a replay fills
+        return c
     _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, StackCopies((c,)))
     return c
 

@@ -4,8 +4,8 @@ run on tcgen05 block-scaled MMAs over e4m3 operands with E8M0 block-32 scales.
 The reference has no MXFP8 path; the signature mirrors `moe` (kernels/sm75/moe.py:838) and the
 numerics follow the OCP MX convention (see include/b200moe.h).  Master weights stay bf16; their quantised
 copies are kept until the weights change (autograd version counter: an optimizer step invalidates them, the
-micro-batches of a gradient-accumulation step and inference calls reuse them; `WEIGHT_CACHE = False` turns it
-off); each GEMM quantises its operands along its own reduction dimension
+micro-batches of a gradient-accumulation step and inference calls reuse them, a captured training pass makes its
+own; `WEIGHT_CACHE = False` turns it off); each GEMM quantises its operands along its own reduction dimension
 (row-wise for forward/dgrad activations, transposed copies for weights in dgrad and for both
 operands of the wgrads).  Needs d_model % 128 == 0 and d_ff % 128 == 0.
 """
@@ -33,11 +33,15 @@ WEIGHT_CACHE = os.environ.get("B200MOE_MXFP8_WEIGHT_CACHE", "1") == "1"
 _QUANTISED = {}      # id(stack) -> (weak reference, version, data pointer, has the transposed copy, tensors, StackCopies)
 
 
-def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None):
+def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None, keep=False):
     """(q, sf) or (q, sf, qt, sft) of an expert stack, from the cache when the stack is the same tensor, at the same
     address, with the same autograd version as when the copies were made (every in-place update moves the version).
-    transpose_fn adds (qt, sft) to a row-wise copy that is kept already; without it both are made anew."""
-    if not WEIGHT_CACHE:
+    transpose_fn adds (qt, sft) to a row-wise copy that is kept already; without it both are made anew.
+    Under graph capture no copy is kept: its memory is the graph's, and only a replay fills it.  keep (a backward follows): a
+    captured pass makes its own copies, since its weights change between replays; a captured forward alone reads those
+    there are, so it has to be captured again when the weights change."""
+    capturing = L.capturing()
+    if not WEIGHT_CACHE or (capturing and keep):
         return both_fn() if both else rows_fn()
     import weakref
     key = id(stack)
@@ -50,21 +54,23 @@ def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None):
         res = hit[5].here() + transpose_fn()
     else:
         res = both_fn() if both else rows_fn()
+    if capturing:
+        return res
     _QUANTISED[key] = (weakref.ref(stack, lambda _r, k=key: _QUANTISED.pop(k, None)), stack._version, stack.data_ptr(),
                        both, res, StackCopies(res))
     return res
 
 
-def _gate_up_copies(stack, both):
+def _gate_up_copies(stack, both, keep):
     E, twoI, H = stack.shape
     return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * twoI, H), interleave_I=twoI // 2),
-                              lambda: ops.mxfp8_quant_both(stack, interleave_I=twoI // 2), both)
+                              lambda: ops.mxfp8_quant_both(stack, interleave_I=twoI // 2), both, keep=keep)
 
 
-def _down_copies(stack, both):
+def _down_copies(stack, both, keep):
     E, H, I = stack.shape      # evaluation keeps the row-wise copy; training after it adds the other one
     return _quantised_weights(stack, lambda: ops.mxfp8_quant_rows(stack.view(E * H, I)), lambda: ops.mxfp8_quant_both(stack), both,
-                              lambda: ops.mxfp8_quant_transpose(stack))
+                              lambda: ops.mxfp8_quant_transpose(stack), keep)
 
 
 class _MoEMxfp8(torch.autograd.Function):
@@ -91,9 +97,9 @@ class _MoEMxfp8(torch.autograd.Function):
         # require a gradient, also where grad mode is off and nobody will ask for one), no gate_up, no pad rows
         if not keep:
             _, xq, xsf = ops.mxfp8_gather_quant(hidden, perm, keep_rows=False)
-            wq, wsf = _gate_up_copies(gate_up_proj, False)
+            wq, wsf = _gate_up_copies(gate_up_proj, False, keep)
             iq, isf = ops.mxfp8_expert_forward(ops.EPI_SWIGLU, xq, xsf, wq, wsf, perm, twoI, H, I)
-            dq, dsf = _down_copies(down_proj, False)
+            dq, dsf = _down_copies(down_proj, False, keep)
             return ops.combine(ops.mxfp8_expert_forward(ops.EPI_STORE, iq, isf, dq, dsf, perm, H, I, I), w32, perm)
         # the gather is the quantising producer; when the gate/up weight gradient is wanted it also writes the
         # copy quantised along the token rows, and the gathered bf16 rows are never materialised
@@ -105,7 +111,7 @@ class _MoEMxfp8(torch.autograd.Function):
         # tensors that the backward needs quantised along their other dimension are quantised both ways in
         # one pass over DRAM, and the transposed copy is what the backward keeps
         wgt = wgtsf = wtq = wtsf = it = itsf = None
-        res = _gate_up_copies(gate_up_proj, need_x)   # + (E, H, 2I)
+        res = _gate_up_copies(gate_up_proj, need_x, keep)   # + (E, H, 2I)
         if need_x:
             wq, wsf, wgt, wgtsf = res
         else:
@@ -121,7 +127,7 @@ class _MoEMxfp8(torch.autograd.Function):
             iq, isf, it, itsf = ops.mxfp8_quant_both(inter)                                 # + (I, rows)
         else:
             iq, isf = ops.mxfp8_quant_rows(inter)
-        res = _down_copies(down_proj, need_x or need_gu)   # + (E, I, H)
+        res = _down_copies(down_proj, need_x or need_gu, keep)   # + (E, I, H)
         if need_x or need_gu:
             dq, dsf, wtq, wtsf = res
         else:
