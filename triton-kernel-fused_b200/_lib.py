@@ -11,6 +11,7 @@ import os
 import subprocess
 import sys
 import threading
+import warnings
 
 import torch
 
@@ -171,20 +172,30 @@ def lib():
     return _lib
 
 
-_fast = None
+_fast = None       # the module; False: there is none that fits
 
 
 def fast():
-    """The compiled autograd functions (csrc/fast.cpp), or None while a compiler or tracer has to see the Python ones."""
+    """The compiled autograd functions (csrc/fast.cpp), or None: while a compiler or tracer has to see the Python ones, and where the
+    module was not built or was built for another torch (a warning, once).  The Python Functions do the same work, at more host time."""
     global _fast
     if torch.compiler.is_compiling() or torch.jit.is_tracing():
         return None
     if _fast is None:
         lib()
-        if not os.path.exists(FAST_PATH):
-            raise RuntimeError(f"{FAST_PATH} is missing: build it with `make -C {_CSRC}` (or __graft_entry__.build())")
-        _fast = importlib.import_module("._fast", __package__)
-    return _fast
+        why = "is missing"
+        if os.path.exists(FAST_PATH):
+            try:
+                _fast = importlib.import_module("._fast", __package__)
+                if _fast.torch_version == torch.__version__.split("+")[0]:
+                    return _fast
+                why = f"was built for torch {_fast.torch_version}, this is {torch.__version__}"
+            except ImportError as e:
+                why = f"cannot be loaded ({e})"
+        _fast = False
+        warnings.warn(f"{FAST_PATH} {why}: the Python autograd Functions run instead, with the same results and more host time a "
+                      f"call; build it with `make -C {_CSRC}` (or __graft_entry__.build())", RuntimeWarning, stacklevel=2)
+    return _fast or None
 
 
 def check(rc: int) -> None:

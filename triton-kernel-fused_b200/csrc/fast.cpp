@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
+#include <torch/version.h>
 
 #include "../../include/b200moe.h"
 
@@ -276,6 +277,7 @@ optional<std::tuple<Tensor, Tensor, Tensor>> conv_router(const Tensor& x, const 
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.attr("torch_version") = TORCH_VERSION;
   m.def("layer", torch::wrap_pybind_function_no_gil(layer));
   m.def("experts", torch::wrap_pybind_function_no_gil(experts));
   m.def("conv_router", torch::wrap_pybind_function_no_gil(conv_router));
