@@ -16,7 +16,7 @@ from .conftest import PKG_NAME, ROOT, load_pkg
 @pytest.mark.skipif(shutil.which("nvcc") is None, reason="no nvcc")
 def test_few_rows_kernels_do_not_spill(tmp_path):
     """Their epilogues hold whole accumulators in registers: an instantiation that spills them is slower than one that reads
-    tensor memory twice (gate/up of 9000 rows 164 against 146 us)."""
+    and writes a group at a time (gate/up of 9000 rows 164 against 146 us)."""
     src = os.path.join(ROOT, PKG_NAME, "csrc", "gemm_few.cu")
     res = subprocess.run(["nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
                           "-c", src, "-o", str(tmp_path / "few.o")], capture_output=True, text=True)

@@ -4,19 +4,38 @@ import importlib
 
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+class Spy:
+    """The module, noting of each call whether it took it (True) or left it to the Python Function (False)."""
+
+    def __init__(self, module):
+        self.taken = []
+        for name in ("layer", "experts", "conv_router"):
+            setattr(self, name, self._noting(getattr(module, name)))
+
+    def _noting(self, fn):
+        def call(*a):
+            self.taken.append(True)       # so is one that raises: a native error, a checkpoint's end of its second forward
+            res = fn(*a)
+            self.taken[-1] = res is not None
+            return res
+        return call
+
+
 @pytest.fixture()
-def python_only(pkg, monkeypatch):
+def spy(pkg, monkeypatch):
+    """The compiled functions under a Spy; `spy.off` takes them away."""
     L = importlib.import_module(pkg.__name__ + "._lib")
     real = L.fast
-
-    def switch(on):
-        monkeypatch.setattr(L, "fast", (lambda: None) if on else real)
-    return switch
+    s = Spy(real())
+    s.off = False
+    monkeypatch.setattr(L, "fast", lambda: None if s.off or real() is None else s)
+    return s
 
 
 def _rand(*s, seed=0):
@@ -49,10 +68,9 @@ def _call(pkg, kind, x_grad=True):
 
 @pytest.mark.parametrize("kind", ["layer", "codes", "moe", "poly", "conv"])
 @pytest.mark.parametrize("x_grad", [True, False])
-def test_compiled_equals_python(pkg, python_only, kind, x_grad):
+def test_compiled_equals_python(pkg, spy, kind, x_grad):
     res = []
-    for on in (True, False):
-        python_only(on)
+    for spy.off in (True, False):
         outs, leaves = _call(pkg, kind, x_grad)
         outs[0].backward(torch.ones_like(outs[0]) * 0.25)
         with torch.no_grad():
@@ -61,13 +79,14 @@ def test_compiled_equals_python(pkg, python_only, kind, x_grad):
         one = torch.autograd.grad(some[0].sum(), leaves2[1])[0]
         assert not quiet[0].requires_grad and outs[0].requires_grad
         res.append([t for t in (*outs, *[p.grad for p in leaves], quiet[0], one)])
+        assert spy.taken == ([] if spy.off else [True] * 3)
     pkg.check_status()
     for a, b in zip(*res):
         assert (a is None and b is None) or (a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b))
 
 
 @pytest.mark.parametrize("kind", ["layer", "poly", "conv"])
-def test_saved_tensors_pass_through_hooks(pkg, kind):
+def test_saved_tensors_pass_through_hooks(pkg, spy, kind):
     outs, leaves = _call(pkg, kind)
     outs[0].sum().backward()
     want = [p.grad.clone() for p in leaves]
@@ -75,24 +94,42 @@ def test_saved_tensors_pass_through_hooks(pkg, kind):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(), lambda t: t.to(DEV)):
         outs, leaves = _call(pkg, kind)
     outs[0].sum().backward()
+    assert spy.taken == [True, True]
     assert len(packed) >= 4 and all(torch.equal(a, p.grad) for a, p in zip(want, leaves))
     pkg.check_status()
 
 
-def test_calls_that_are_not_plain_take_the_python_function(pkg, python_only):
+class Passing(TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+def test_calls_that_are_not_plain_take_the_python_function(pkg, spy):
+    def declined(f):
+        """f's result; every compiled function that it called left the call to Python."""
+        n = len(spy.taken)
+        try:
+            return f()
+        finally:
+            assert spy.taken[n:] and not any(spy.taken[n:])
+
     layer = pkg.MoELayer(64, 72, 8, top_k=2).to(DEV).to(torch.bfloat16)
     wide = _rand(40, 128)
     x = wide[:, :64]                                   # rows 128 apart: made contiguous by the Python Function
     with torch.no_grad():
-        assert torch.equal(layer(x), layer(x.contiguous()))
+        want = layer(x.contiguous())
+        assert spy.taken == [True]
+        assert torch.equal(declined(lambda: layer(x)), want)
+        with Passing():                                # a mode that has to see the allocations
+            assert torch.equal(declined(lambda: layer(x.contiguous())), want)
         f32 = layer.float()                            # cast under autocast
         with torch.autocast("cuda", dtype=torch.bfloat16):
-            cast = f32(x.float())
+            cast = declined(lambda: f32(x.float()))
         assert torch.equal(cast, layer.to(torch.bfloat16)(x.contiguous()))
     with pytest.raises(ValueError):
-        layer(x.float())                               # no autocast: refused
+        declined(lambda: layer(x.float()))             # no autocast: refused
     with pytest.raises(ValueError):
-        layer(torch.zeros(4, 56, dtype=torch.bfloat16, device=DEV))
+        declined(lambda: layer(torch.zeros(4, 56, dtype=torch.bfloat16, device=DEV)))
     with pytest.raises(ValueError):                    # native errors keep their Python types
         pkg.fused_router(_rand(1, 8, 64), _rand(16, 64, 4), None, 17, 16)
     xs = x.contiguous()
@@ -100,13 +137,13 @@ def test_calls_that_are_not_plain_take_the_python_function(pkg, python_only):
                       lambda: torch.func.grad(lambda a: layer(a).float().sum())(xs),
                       lambda: torch.func.jvp(lambda a: layer(a), (xs,), (xs,))):
         errors = []
-        for on in (True, False):
-            python_only(on)
+        for spy.off in (True, False):
             with pytest.raises(Exception) as e:
-                transform()
+                transform() if spy.off else declined(transform)
             errors.append(type(e.value))
         assert errors[0] is errors[1]
-    python_only(False)
+    n = len(spy.taken)
     y = torch.utils.checkpoint.checkpoint(layer, xs.clone().requires_grad_(), use_reentrant=False)
     y.sum().backward()
+    assert spy.taken[n:] == [True, True]
     pkg.check_status()
