@@ -167,7 +167,7 @@ static int experts_forward(const Dims& d, const void* x, const float* w, const v
   const int64_t rows = d.rows();
   if (d.kind == KIND_FEW) {
     RUN("gather_rows", 1, b200moe_gather_rows(x, f.order, f.offs + d.E, d.k, d.H, rows, f.x_s, st));
-    // early: the gather began after the permutation's end, and that after whatever wrote the weights
+    // early: past its wait the gather has the permutation behind it, and the permutation whatever wrote the weights
     RUN("expert_gate_up_few", 1, expert_gate_up_few(f.x_s, gate_up_proj, codes, f.counts, f.offs, rows, d.E, d.H, d.I, 1, f.inter,
                                                     status, st));
     RUN("expert_linear_few", 1, expert_linear_few(f.inter, down_proj, f.counts, f.offs, rows, d.E, d.H, d.I, 1, f.eo, status, st));

@@ -36,7 +36,7 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);
-// its products; early: counts and weights were complete before the kernel in front of the launch began (FewParams::early)
+// its products; early: counts and weights were complete when the kernel in front had passed its wait (FewParams::early)
 int expert_gate_up_few(const void* x, const void* gate_up_proj, const int32_t* act_codes, const int32_t* counts,
                        const int32_t* offs, int64_t rows_cap, int E, int64_t H, int64_t I, int early, void* inter,
                        int32_t* status, b200moe_stream_t stream);

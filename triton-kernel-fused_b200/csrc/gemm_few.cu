@@ -10,10 +10,10 @@
 // its lanes and rows in its columns.  A box may reach past the expert's rows: they only feed accumulator columns that
 // are not stored.
 // H 2048, I 1408, 64 experts, us as row tiles / here: 288 rows (4.5 an expert; 118 + 59 us at copy rate): gate/up 161 / 108, down 80 /
-// 60; 9000 rows (141 an expert): 171 / 151 and 85 / 75; 6 rows of one token: 21 / 12.3 and 15 / 9.2.
+// 60; 9000 rows (141 an expert): 171 / 136 and 85 / 75; 6 rows of one token: 21 / 12.3 and 15 / 9.2.
 // A large tile is bound by the bytes that leave L2 (weights in and out, X once per 128 columns) and wants them in flight: with a
-// stage less gate/up of 9000 rows takes 157 us (beside 151 then).  A small one is bound by latencies and by what a stage costs the two threads that
-// issue it: one lane for all boxes, elected (ptx.cuh), 128-row weight boxes that hold gate and up (make_map_gate_up), and tiles of 64
+// stage less gate/up of 9000 rows took 157 us in place of 151.  A small one is bound by latencies and by what a stage costs the
+// two threads that issue it: one lane for all boxes, elected (ptx.cuh), 128-row weight boxes that hold gate and up (make_map_gate_up), and tiles of 64
 // columns where even they are one wave; with a lane per box and tiles of 128 one token took 18.3 and 11.1 us.
 //
 // Warp roles as in gemm.cu: warp 0 TMA producer (one lane), warp 1 TMEM owner + MMA issuer, warps 2-9 epilogue.
@@ -40,8 +40,9 @@ struct FewParams {
   const int* act_codes;   // SwiGLU: activation code of each expert, nullptr = SiLU
   int* status;
   int aligned;            // D is 16-byte aligned
-  // Counts and weights were complete before the kernel in front of this one began: the first blocks of weights are loaded
-  // before the wait for that kernel, so its end and this one's start cost no time on the memory bus.
+  // Counts and weights were complete when the kernel in front had passed its own wait, so before this one began (its CTAs are
+  // placed after that): the first blocks of weights are loaded before the wait for that kernel, so its end and this one's start
+  // cost no time on the memory bus.
   int early;
 };
 
@@ -539,14 +540,17 @@ static int launch_router_few(const void* x, const void* weight, const RouterFewP
 }
 
 // Tile.  The host knows the mean rows per expert, not the counts: both rules below were timed under even routing, expert
-// frequencies ~ rank^-0.6 and rank^-1.1, and one expert in every token's picks.  us, gate/up + down with gather and combine.
+// frequencies ~ rank^-0.6 and rank^-1.1, and one expert in every token's picks.  us of gate/up + down with permutation, gather
+// and combine, L2 flushed before each.
 //  - Chunks of 64 rows where even the worst spread of the rows over the experts, E + M / 64 chunks, is one wave of CTAs: the
 //    smallest tile then has the shortest chain and the most SMs.  8 experts, 512 x 256, mean 140 rows, even / rank^-1.1:
-//    NT 64 25.7 / 25.6, 128 29.8 / 29.7, 192 31.7 / 34.4 (row tiles 25.4 / 25.5).
+//    NT 64 30 / 30, 128 34 / 34, 192 38 / 40 (row tiles 34 / 34).
 //  - Else by the mean.  A larger NT keeps an expert's rows in one tile, so its weights pass through shared memory once; a
 //    smaller one leaves room for more k-blocks in flight and double-buffered accumulators.  64 experts, 2048 x 1408, even /
-//    rank^-1.1: mean 4 rows NT 64 184 / 154, 128 186 / 155, 192 188 / 151; 39 rows 201 / 229, 201 / 216, 204 / 205; 80 rows
-//    278 / 280, 217 / 252, 225 / 235; 140 rows 379 / 376, 304 / 297, 254 / 278.
+//    rank^-1.1: mean 4 rows NT 64 197 / 164, 128 200 / 166, 192 201 / 164; 39 rows 211 / 217, 211 / 217, 211 / 211; 80 rows
+//    252 / 246, 221 / 232, 221 / 227; 110 rows 266 / 291, 229 / 257, 231 / 246; 140 rows 345 / 340, 285 / 274, 245 / 268.
+//    kFewRows128 stands where an NT 192 that spilled put it: between 40 and 110 rows the two are now within 2 % under even
+//    routing and NT 192 leads under a skewed one, most with few experts (8 of 4096 x 14336, 80 rows 594 against 520).
 constexpr int64_t kFewRows64 = 40, kFewRows128 = 110;
 
 static int64_t few_blocks(int64_t N, int64_t K) { return ceil_div(std::max(N, K), 128); }   // weight blocks of an expert (either product)
@@ -563,14 +567,14 @@ static bool few_narrow(int64_t M, int E, int64_t I) {
 }
 
 // Whether a forward without a backward runs over compact rows (this file) or row tiles (gemm.cu), same measurements, row tiles
-// against compact rows, even / rank^-1.1.  64 experts, 2048 x 1408: mean 4 rows 268 / 222 against 184 / 154, 140 rows 286 /
-// 323 against 254 / 278, 200 rows 296 / 362 against 364 / 328 (an even expert then takes two tiles): up to kFewRows.
-// Fewer than 16 experts leave few pad rows in row tiles: 8 experts, 4096 x 14336: 80 rows 577 / 579 against 521 / 517, 159
-// rows 604 / 634 against 554 / 726: up to kFewRows128.  Where one chunk per expert fills less than half of the SMs and the
-// chunks of 64 are more than one wave, the single-CTA row tiles spread the work further: 8 experts, 1024 x 1024, 140 rows
-// 35 / 37 against 39 / 39 (NT 128) and 42 / 46 (NT 192).
-// What the rules cannot see costs: 16 experts, 4096 x 1024, one pick, every token on one expert, 39 rows on average: 50
-// against 65.
+// against compact rows, even / rank^-1.1.  64 experts, 2048 x 1408: mean 4 rows 274 / 225 against 197 / 164, 140 rows 289 /
+// 330 against 245 / 268, 200 rows 304 / 386 against 342 / 325 (an even expert then takes two tiles): up to kFewRows.
+// Fewer than 16 experts leave few pad rows in row tiles: 8 experts, 4096 x 14336: 80 rows 586 / 608 against 492 / 596, 110 rows
+// 610 / 746 against 520 / 709: up to kFewRows128.  Both limits on few experts were drawn with a slower NT 192 and now give some
+// away: 159 rows there 618 / 841 against 534 / 726, and where one chunk per expert fills less than half of the SMs and the
+// chunks of 64 are more than one wave, 8 experts of 1024 x 1024, 140 rows 56 / 49 against 46 / 41 (NT 128).
+// Every token's one pick on one expert, the spread the host cannot see: 16 experts, 4096 x 1024, 39 rows on average 76 against
+// 72, 60 rows 61 against 59, 159 rows 102 against 90.
 constexpr int64_t kFewRows = 160;
 
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I) {

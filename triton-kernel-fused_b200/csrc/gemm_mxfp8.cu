@@ -1082,6 +1082,11 @@ using namespace b200moe;
 // 8 experts, 4096 x 14336: mean 16 rows 307, 308 / 234, 234; 48 rows 315, 314 / 239, 285 (chunks of 64); 100 rows 325, 346 / 260, 314 (of
 // 128; of 64 362, 364); 128 rows 331, 347 / 323, 322; 160 rows 335, 358 / 410, 396.  64 experts, 2048 x 1408: 16 rows 164, 165 / 127, 130;
 // 128 rows 180, 200 / 163, 180; 200 rows 188, 229 / 202, 214.  16 experts, 1024 x 1024: 16 rows 32, 32 / 23, 23; 160 rows 39, 44 / 39, 37.
+// The two products alone, L2 flushed before each, one expert in every token's two picks: 8 experts of 4096 x 14336, 32 rows 341 / 286,
+// 64 rows 376 / 320, 128 rows 488 / 370; 64 of 2048 x 1408, 128 rows 185 / 161.  Experts that do not fill the SMs need no term of their
+// own: 8 of 256 x 256, 128 rows 24 / 17 even, 22 / 17 skewed; 16 of 1024 x 1024 38 / 30, 42 / 34.  What it costs: every row on one
+// expert (one pick each), whose weights then pass through shared memory once a chunk: 8 of 4096 x 14336, 32 rows 101 / 109, 96 rows
+// 163 / 206, 128 rows 210 / 251; 64 of 2048 x 1408, 128 rows 81 / 91; 256 of 512 x 512, 128 rows 56 / 73.
 constexpr int64_t kFewFp8Rows = 128, kFewFp8Small = 32;
 
 #define CHECK_K128(v) \
