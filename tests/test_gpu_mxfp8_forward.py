@@ -58,16 +58,18 @@ def test_kept_copies_are_complete_on_another_stream(pkg):
         args = lambda: (x.to(dtype), idx, w, gu, dn.to(dtype), codes)     # noqa: E731
         with torch.no_grad():
             want = fn(*args())
-            for _ in range(3):
+            for maker in (torch.cuda.current_stream(), torch.cuda.Stream()) * 2:
                 a = args()
                 torch.cuda.synchronize()
-                gu.mul_(1.0)                       # another version: new copies, of the same values
-                torch.cuda._sleep(20_000_000)      # the main stream is busy for about 10 ms
-                fn(*a)
+                with torch.cuda.stream(maker):
+                    gu.mul_(1.0)                       # another version: new copies, of the same values
+                    torch.cuda._sleep(20_000_000)      # the stream is busy for about 10 ms
+                    fn(*a)
                 with torch.cuda.stream(side):
                     got = fn(*a)
-                gu.mul_(1.0)
-                fn(*a)                             # the old copies go; their memory is written on the main stream
+                with torch.cuda.stream(maker):
+                    gu.mul_(1.0)
+                    fn(*a)                             # the old copies go; new ones are written on the same stream
                 torch.cuda.synchronize()
                 assert torch.equal(got, want)
     pkg.check_status()

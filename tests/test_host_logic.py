@@ -273,7 +273,7 @@ def test_chained_kernels_promise_no_constant_data():
 
 def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
     """Quantised and bf16 copies that one stream made: a call on another stream waits for it before it reads them, until they are
-    known to be complete, and records itself as a user of their memory; the stream that made them does neither."""
+    known to be complete, and records itself as a user of their memory; the stream that made them does neither (the default stream records its event when one is asked for)."""
     moe_mod, mx, L = (importlib.import_module(PKG + n) for n in (".moe", ".mxfp8", "._lib"))
     log = []
 
@@ -285,7 +285,7 @@ def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
 
     class Stream:
         def __init__(self, name):
-            self.name, self.cuda_stream = name, hash(name)
+            self.name, self.cuda_stream = name, 0 if name == "default" else hash(name)
 
         def record_event(self):
             log.append(("record", self.name))
@@ -307,32 +307,32 @@ def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
 
     now = [Stream("a")]
     monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: now[0])
-    monkeypatch.setattr(L, "capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "default_stream", lambda d=None: Stream("default"))
+    monkeypatch.setattr(L, "capturing", lambda t: False)
     monkeypatch.setattr(L, "stream_of", lambda t: now[0].cuda_stream)
 
     class Master(Copy):
         requires_grad, _version = False, 0
 
-    stack, master = torch.zeros(2), Master()
-    q = (Copy(), Copy())
-    for get in (lambda: mx._quantised_weights(stack, lambda: q, None, False), lambda: moe_mod._bf16_copy(master)):
-        now[0] = Stream("a")
-        n = len(log)
-        res = get()
-        copies = res if isinstance(res, tuple) else (res,)
-        assert log[n:] == [("record", "a")]
-        get()
-        assert log[n + 1:] == []
-        now[0], n = Stream("b"), len(log)
-        assert get() is res or get() == res
-        assert ("wait", "b") in log[n:] and log[n:].count(("used by", "b")) % len(copies) == 0 and ("used by", "b") in log[n:]
-        assert log[n:].index(("wait", "b")) < log[n:].index(("used by", "b"))
-        Event.done, n = True, len(log)
-        get()
-        assert ("wait", "b") not in log[n:] and ("used by", "b") in log[n:]
-        Event.done = False
-    del mx._QUANTISED[id(stack)]
-    del moe_mod._BF16_COPIES[id(master)]
+    for maker in ("a", "default"):
+        stack, master, q = torch.zeros(2), Master(), (Copy(), Copy())
+        for get in (lambda: mx._quantised_weights(stack, lambda: q, None, False), lambda: moe_mod._bf16_copy(master)):
+            now[0], Event.done = Stream(maker), False
+            log.clear()
+            res = get()
+            users = [("used by", "b")] * (len(res) if isinstance(res, tuple) else 1)
+            get()
+            made = [] if maker == "default" else [("record", "a")]
+            assert log == made
+            now[0] = Stream("b")
+            assert get() == res
+            assert log == [("record", maker), ("wait", "b")] + users
+            Event.done = True
+            log.clear()
+            get()
+            get()
+            assert log == 2 * users
+        del mx._QUANTISED[id(stack)], moe_mod._BF16_COPIES[id(master)]
 
 
 def test_copies_made_under_capture_are_not_kept(monkeypatch):
@@ -340,7 +340,7 @@ def test_copies_made_under_capture_are_not_kept(monkeypatch):
     forward reads kept copies; a captured pass with a backward makes its own, because its weights change between replays."""
     moe_mod, mx, L = (importlib.import_module(PKG + n) for n in (".moe", ".mxfp8", "._lib"))
     capturing = [True]
-    monkeypatch.setattr(L, "capturing", lambda: capturing[0])
+    monkeypatch.setattr(L, "capturing", lambda t: capturing[0])
     stack, made = torch.zeros(2, 4, 8), []
     get = lambda **kw: mx._quantised_weights(stack, lambda: made.append(0) or (torch.zeros(1), torch.zeros(1)), None, False, **kw)     # noqa: E731
     get()

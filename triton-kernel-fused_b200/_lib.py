@@ -221,9 +221,9 @@ def stream_of(t: torch.Tensor):
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
-def capturing() -> bool:
-    """Whether the current stream is being captured into a graph (False where there is no GPU)."""
-    return torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()
+def capturing(t: torch.Tensor) -> bool:
+    """Whether the current stream of t's device is being captured into a graph."""
+    return t.is_cuda and torch._C._cuda_isCurrentStreamCapturing()
 
 
 _status = {}       # device index -> the word

@@ -180,25 +180,34 @@ class StackCopies:
     them next: until they are known to be complete a reader on another stream waits for the writer's event, and their memory is
     not handed out again before that stream is done with it.  (While a graph is being captured neither is possible, nor needed:
     torch.cuda.graph waits for the device before it begins.)"""
+    __slots__ = ("tensors", "stream", "event")
 
     def __init__(self, tensors):
         self.tensors = tensors
         self.stream = self.event = None
         if tensors[0].is_cuda:
             self.stream = L.stream_of(tensors[0])
-            self.event = torch.cuda.current_stream(tensors[0].device).record_event()
+            # on the default stream, which is there for good, only when one is asked for: an event of a stack's first pass costs it 15 us
+            self.event = True if self.stream == 0 else torch.cuda.current_stream(tensors[0].device).record_event()
 
     def here(self):
         """The tensors, for the current stream."""
-        if self.stream is not None and L.stream_of(self.tensors[0]) != self.stream and not L.capturing():
-            now = torch.cuda.current_stream(self.tensors[0].device)
-            if self.event is not None and self.event.query():
-                self.event = None
-            if self.event is not None:
-                now.wait_event(self.event)
-            for t in self.tensors:
-                t.record_stream(now)
+        if self.stream is not None and L.stream_of(self.tensors[0]) != self.stream:
+            self._elsewhere(self.tensors[0])
         return self.tensors
+
+    def _elsewhere(self, t):
+        if L.capturing(t):
+            return
+        now = torch.cuda.current_stream(t.device)
+        if self.event is True:
+            self.event = torch.cuda.default_stream(t.device).record_event()
+        if self.event is not None and self.event.query():
+            self.event = None
+        if self.event is not None:
+            now.wait_event(self.event)
+        for t in self.tensors:
+            t.record_stream(now)
 
 
 _BF16_COPIES = {}     # id(parameter) -> (weak reference, version, StackCopies of the bf16 copy)
@@ -217,7 +226,7 @@ def _bf16_copy(t):
     if hit is not None and hit[0]() is t and hit[1] == t._version:
         return hit[2].here()[0]
     c = t.detach().to(torch.bfloat16)
-    if L.capturing():      # the graph's memory, which only a replay fills
+    if L.capturing(c):     # the graph's memory, which only a replay fills
         return c
     _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, StackCopies((c,)))
     return c

@@ -40,22 +40,21 @@ def _quantised_weights(stack, rows_fn, both_fn, both, transpose_fn=None, keep=Fa
     Under graph capture no copy is kept: its memory is the graph's, and only a replay fills it.  keep (a backward follows): a
     captured pass makes its own copies, since its weights change between replays; a captured forward alone reads those
     there are, so it has to be captured again when the weights change."""
-    capturing = L.capturing()
-    if not WEIGHT_CACHE or (capturing and keep):
+    if not WEIGHT_CACHE:
         return both_fn() if both else rows_fn()
     import weakref
     key = id(stack)
     hit = _QUANTISED.get(key)
     if hit is not None and not (hit[0]() is stack and hit[1] == stack._version and hit[2] == stack.data_ptr()):
         hit = None
+    if (hit is None or keep) and L.capturing(stack):
+        return both_fn() if both else rows_fn()
     if hit is not None and (hit[3] or not both):
         return hit[5].here() if both else hit[5].here()[:2]
     if hit is not None and transpose_fn is not None:
         res = hit[5].here() + transpose_fn()
     else:
         res = both_fn() if both else rows_fn()
-    if capturing:
-        return res
     _QUANTISED[key] = (weakref.ref(stack, lambda _r, k=key: _QUANTISED.pop(k, None)), stack._version, stack.data_ptr(),
                        both, res, StackCopies(res))
     return res
