@@ -304,6 +304,7 @@ def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
             return self
 
         detach = lambda self: self     # noqa: E731
+        data_ptr = lambda self: 16     # noqa: E731
 
     now = [Stream("a")]
     monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: now[0])
@@ -361,3 +362,13 @@ def test_copies_made_under_capture_are_not_kept(monkeypatch):
     assert b is not a
     capturing[0] = True
     assert moe_mod._bf16_copy(w) is b
+
+
+def test_bf16_copies_follow_assigned_data():
+    """Assigning `.data` (what module.to() and weight swaps do) moves no version counter: the copy is made anew all the same."""
+    moe_mod = importlib.import_module(PKG + ".moe")
+    w = torch.randn(2, 8, 4)
+    a = moe_mod._bf16_copy(w)
+    w.data = torch.randn(2, 8, 4)
+    b = moe_mod._bf16_copy(w)
+    assert b is not a and torch.equal(b, w.to(torch.bfloat16)) and moe_mod._bf16_copy(w) is b

@@ -210,12 +210,12 @@ class StackCopies:
             t.record_stream(now)
 
 
-_BF16_COPIES = {}     # id(parameter) -> (weak reference, version, StackCopies of the bf16 copy)
+_BF16_COPIES = {}     # id(parameter) -> (weak reference, version, data pointer, StackCopies of the bf16 copy)
 
 
 def _bf16_copy(t):
     """bf16 copy of an fp16 / fp32 expert stack, kept until the tensor changes (its autograd version counter moves
-    on every in-place update, e.g. an optimizer step) or is freed.  Callers with fp32 master weights would otherwise
+    on every in-place update, e.g. an optimizer step; its address when `.data` is assigned) or is freed.  Callers with fp32 master weights would otherwise
     pay a full copy of both stacks on every call.  Tensors that need a gradient are cast afresh, so that autograd
     carries the gradient back through the cast."""
     if t.requires_grad and torch.is_grad_enabled():
@@ -223,12 +223,12 @@ def _bf16_copy(t):
     import weakref
     key = id(t)
     hit = _BF16_COPIES.get(key)
-    if hit is not None and hit[0]() is t and hit[1] == t._version:
-        return hit[2].here()[0]
+    if hit is not None and hit[0]() is t and hit[1] == t._version and hit[2] == t.data_ptr():
+        return hit[3].here()[0]
     c = t.detach().to(torch.bfloat16)
     if L.capturing(c):     # the graph's memory, which only a replay fills
         return c
-    _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, StackCopies((c,)))
+    _BF16_COPIES[key] = (weakref.ref(t, lambda _r, k=key: _BF16_COPIES.pop(k, None)), t._version, t.data_ptr(), StackCopies((c,)))
     return c
 
 
