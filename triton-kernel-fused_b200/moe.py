@@ -215,9 +215,9 @@ _BF16_COPIES = {}     # id(parameter) -> (weak reference, version, data pointer,
 
 def _bf16_copy(t):
     """bf16 copy of an fp16 / fp32 expert stack, kept until the tensor changes (its autograd version counter moves
-    on every in-place update, e.g. an optimizer step; its address when `.data` is assigned) or is freed.  Callers with fp32 master weights would otherwise
-    pay a full copy of both stacks on every call.  Tensors that need a gradient are cast afresh, so that autograd
-    carries the gradient back through the cast."""
+    on every in-place update, e.g. an optimizer step; its address when `.data` is assigned) or is freed.  Callers with
+    fp32 master weights would otherwise pay a full copy of both stacks on every call.  Tensors that need a gradient are
+    cast afresh, so that autograd carries the gradient back through the cast.  Under graph capture nothing is kept."""
     if t.requires_grad and torch.is_grad_enabled():
         return t.to(torch.bfloat16)
     import weakref
