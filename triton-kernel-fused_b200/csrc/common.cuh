@@ -88,8 +88,8 @@ inline void by_row_threads(int nvec, F f) {
 // another kernel touches, and grid_dep_launch() only after that: when a kernel's first instruction runs, the kernel two
 // before it is complete, and past its wait the one before it too.  Its pointers are neither __restrict__ nor read by __ldg: both
 // promise the compiler data that stays as it is for the kernel's whole life, which begins before the wait, so it could load ahead
-// of the wait or past the coherent cache.  (Taking the promises out cost nothing: combine of 98 304 rows of 2048 96.4 / 96.3 us,
-// both quantisers of them 186 / 184, GLU backward of 1408 columns 457 / 457.)  Why: between two plain launches the SMs idle for 1.5 to 4
+// of the wait or past the coherent cache.  (Taking the promises out cost next to nothing: combine of 98 304 rows of 2048 96.4 /
+// 96.3 us, both quantisers of them 186 / 184, GLU backward of 1408 columns 457 / 457, the conv router's pass 115.0 / 115.3.)  Why: between two plain launches the SMs idle for 1.5 to 4
 // us (drain, launch, barriers, tensor memory, descriptors), as long as the small kernels of a decoding step run.  The GEMMs
 // call grid_dep_launch() when their last loads are issued: early enough to hide a launch, and at their start it made large
 // training steps 1 % slower.  us a pass, plain / chained: 48 tokens, 64 experts of 2048 x 1408 (6 launches, with the weights
