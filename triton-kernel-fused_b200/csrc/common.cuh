@@ -29,10 +29,27 @@ int num_sms();
 int gemm_cta_budget();   // CTAs a persistent GEMM may occupy (num_sms() minus the reserved SMs)
 int exchange_sm_budget();   // SMs (= fat CTAs) the home-side pull kernel of the expert-parallel exchange may occupy
 
+// Routing weight of each padded row (pads: 0).  row_w == nullptr: not wanted
+struct RowWeights {
+  float* row_w;
+  const float* slot_w;   // (T, k)
+};
 // b200moe_permute_build; also stores the counts a second time (counts_out) and adds them to `load` (both nullable)
 int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs, int32_t* poffs,
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
-                  size_t ws_bytes, int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream);
+                  size_t ws_bytes, int32_t* counts_out, int64_t* load, const RowWeights& rows, int32_t* status, b200moe_stream_t stream);
+
+// combine.cu: grad_w[slot] = sum over `parts` of dots[part][row], dots (parts, ld)
+int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, const int32_t* total_rows, float* grad_w, b200moe_stream_t stream);
+
+// gemm.cu: whether a block's rows are weighted by the epilogues of its GLU products, and those products
+bool weighted_rows(int64_t M, int E, int64_t H, int64_t I);
+int expert_gate_up_weighted(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+                            const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I, void* gate_up, void* inter, int32_t* status,
+                            b200moe_stream_t stream);
+int expert_down_dgrad_weighted(const void* go_s, const void* down_proj, const void* gate_up, const int32_t* act_codes, const float* row_w,
+                               const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
+                               void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream);
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);

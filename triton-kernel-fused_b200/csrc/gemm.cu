@@ -86,7 +86,8 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
-template <int BN, int EPI, int CTAS, bool POLY = false>
+// WEIGHTED: the GLU epilogues of a block whose rows are weighted where their activations are made (expert_gate_up_weighted).
+template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
@@ -332,6 +333,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       if constexpr (POLY && (EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD)) act_code = p.act_codes[t.g];
       const int row0 = t.m0 + BM * static_cast<int>(cta_rank) + q * 32;   // first row of this warp
       const long long row = static_cast<long long>(row0) + lane;
+      const float row_w = WEIGHTED ? p.row_w[row] : 1.0f;
       // GLU backward works on four 32-column sub-chunks per warp with two sets of (gate, up) boxes of
       // 32 rows x 32 columns (2 KB, 64-byte swizzle): a set is loaded by TMA, overwritten in place with
       // grad_gate / grad_up and stored by TMA while the other set is loading or being computed on.  The saved
@@ -486,7 +488,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 og[16 * sub + i] = pack_bf16x2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
                 ou[16 * sub + i] = pack_bf16x2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
               }
-              glu_fwd_pairs_by_code<POLY>(act_code, og + 16 * sub, ou + 16 * sub, oh + 16 * sub, 16);
+              glu_fwd_pairs_by_code<POLY>(act_code, og + 16 * sub, ou + 16 * sub, oh + 16 * sub, 16, row_w);
             }
             staging_free(lane);
             stage_row(sbuf, lane, og);
@@ -500,6 +502,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         } else {  // EPI_GLU_BWD: accumulator = grad_inter columns [n0, n0+BN); this warp: 128 of them
           constexpr int W = BN / 2;
+          float dot = 0.0f;
 #pragma unroll 1
           for (int sub = 0; sub < W / 32; ++sub) {
             const int col = glu_col0 + 32 * sub;
@@ -520,7 +523,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
             tmem_ld_wait();
             uint32_t og[16], ou[16];
-            glu_bwd32<POLY>(r, g4, u4, og, ou, act_code);
+            glu_bwd32<POLY>(r, g4, u4, og, ou, act_code, row_w, WEIGHTED ? &dot : nullptr);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {              // results replace the inputs in place
               const int off = lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4);
@@ -541,6 +544,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               glu_load(sub + 2);
             }
           }
+          if constexpr (WEIGHTED)
+            if (glu_col0 < p.I) p.dots[(glu_col0 / W) * p.dots_ld + row] = dot;
         }
       } else {
         // Single-CTA tiles up to 128 wide, and fp32 partial sums: from tensor memory through registers.  16 rows x 64 (or 32) columns at a
@@ -667,21 +672,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------------------- host side
-template <int BN, int EPI, int CTAS, bool POLY = false>
+template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD, const CUtensorMap& tmD2,
                   const GemmParams& p, int max_tiles, cudaStream_t stream) {
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY>, units * CTAS, kThreads, C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, units * CTAS, kThreads, C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 
@@ -748,7 +753,7 @@ static int pick_bn_rows(long long n, long long rows_cap, int E, int cols_per_bn 
 
 // d1 / d2 describe the bf16 outputs as {columns, rows, groups} tensors for the TMA-store epilogue
 // (d2 = the SwiGLU `inter` output); they are ignored by the kernels that store directly.
-template <int EPI, bool POLY = false>
+template <int EPI, bool POLY = false, bool WEIGHTED = false>
 static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand* d1, const Operand* d2,
                        GemmParams& p, int max_tiles, cudaStream_t stream) {
   const bool pair = (bn == 256) && (p.sched != SCHED_DENSE) && pairs_enabled();
@@ -787,8 +792,11 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
       }
     }
   }
-  if (pair) return launch<256, EPI, 2, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
-  if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
+  if (pair) return launch<256, EPI, 2, POLY, WEIGHTED>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
+  if constexpr (WEIGHTED) {
+    set_error("internal: weighted epilogues are built for pair tiles");
+    return B200MOE_E_UNSUPPORTED;
+  } else if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
     if (bn == 256) return launch<256, EPI, 1>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     set_error("tile width %d not built for this epilogue", bn);
     return B200MOE_E_UNSUPPORTED;
@@ -877,6 +885,101 @@ int expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, co
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
   Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
   return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+}
+
+// row window of a grouped-M launch: (0, 0) = every row, else tile-aligned 0 <= row_lo < row_hi <= rows_cap
+static int check_row_window(const char* who, int64_t rows_cap, int64_t row_lo, int64_t row_hi) {
+  if (row_lo == 0 && row_hi == 0) return 0;
+  B200_CHECK_ARG(row_lo >= 0 && row_lo < row_hi && row_hi <= rows_cap && row_lo % B200MOE_TILE_M == 0 &&
+                     row_hi % B200MOE_TILE_M == 0,
+                 B200MOE_E_BAD_SHAPE, "%s: row window [%lld, %lld) must be tile-aligned and inside %lld rows", who,
+                 (long long)row_lo, (long long)row_hi, (long long)rows_cap);
+  return 0;
+}
+
+static int gate_up(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+                   const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
+                   int32_t* status, b200moe_stream_t stream) {
+  int rc = check_grouped("expert_gate_up_swiglu", x_s, gate_up_proj, gate_up, tile_expert, poffs, rows_cap, E, H, I);
+  if (rc) return rc;
+  rc = check_row_window("expert_gate_up_swiglu", rows_cap, row_lo, row_hi);
+  if (rc) return rc;
+  B200_CHECK_ARG(inter && tile_expert, B200MOE_E_NULL, "expert_gate_up_swiglu: null pointer");
+  B200_CHECK_ARG(aligned16(gate_up) && aligned16(inter), B200MOE_E_ALIGN, "expert_gate_up_swiglu: outputs not aligned");
+  Operand a{x_s, 0, rows_cap, H, H, 1, rows_cap * H};
+  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
+  Operand b{gate_up_proj, 0, I, H, H, 2LL * E, I * H};
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.N = (int)I; p.K = (int)H; p.num_groups = E;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = gate_up; p.aux = inter; p.I = (int)I; p.status = status;
+  p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
+  const int bn = pick_bn_rows(I, rows_cap, E, 2);   // tile covers bn/2 intermediate columns
+  Operand d1{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // {I, rows, 2}: group 0 = gate half, 1 = up half
+  Operand d2{inter, 0, rows_cap, I, I, 1, rows_cap * I};
+  p.act_codes = act_codes;
+  if (row_w != nullptr) {
+    p.row_w = row_w;
+    return act_codes != nullptr ? dispatch_bn<EPI_SWIGLU, true, true>(256, a, b, &d1, &d2, p, 0, (cudaStream_t)stream)
+                                : dispatch_bn<EPI_SWIGLU, false, true>(256, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
+  }
+  if (act_codes != nullptr) return dispatch_bn<EPI_SWIGLU, true>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
+  return dispatch_bn<EPI_SWIGLU>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
+}
+
+static int down_dgrad(const void* grad_eo, const void* down_proj, const void* gate_up, const int32_t* act_codes, const float* row_w,
+                      const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I,
+                      void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_grouped("expert_down_dgrad_glu", grad_eo, down_proj, grad_gate_up, tile_expert, poffs, rows_cap, E, H, I);
+  if (rc) return rc;
+  rc = check_row_window("expert_down_dgrad_glu", rows_cap, row_lo, row_hi);
+  if (rc) return rc;
+  B200_CHECK_ARG(gate_up && tile_expert, B200MOE_E_NULL, "expert_down_dgrad_glu: null pointer");
+  B200_CHECK_ARG(aligned16(grad_gate_up) && aligned16(gate_up), B200MOE_E_ALIGN, "expert_down_dgrad_glu: not aligned");
+  Operand a{grad_eo, 0, rows_cap, H, H, 1, rows_cap * H};
+  Operand b{down_proj, 1, I, H, I, E, H * I};   // W_d[e] stored (K=H, N=I): MN-major
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)I; p.K = (int)H; p.num_groups = E;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = grad_gate_up; p.aux = const_cast<void*>(gate_up);
+  p.I = (int)I; p.status = status;
+  p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
+  const int bn = pick_bn_rows(I, rows_cap, E);
+  Operand d{grad_gate_up, 0, rows_cap, I, 2 * I, 2, I};   // {I, rows, 2}: grad_gate half, grad_up half
+  Operand d2{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // the saved forward gate_up, same view (input)
+  p.act_codes = act_codes;
+  if (row_w != nullptr) {
+    p.row_w = row_w; p.dots = dots; p.dots_ld = rows_cap;
+    return act_codes != nullptr ? dispatch_bn<EPI_GLU_BWD, true, true>(256, a, b, &d, &d2, p, 0, (cudaStream_t)stream)
+                                : dispatch_bn<EPI_GLU_BWD, false, true>(256, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
+  }
+  if (act_codes != nullptr) return dispatch_bn<EPI_GLU_BWD, true>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
+  return dispatch_bn<EPI_GLU_BWD>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
+}
+
+// ---- a routed row weighted where its activations are made, not where it is added up: inter = w act(gate) up, so the down product's rows
+// need no weight any more, the weight gradients no weighted copy of the upstream gradient, and grad_inter = w (go W_down) and the
+// weight's own gradient (go W_down) . (act(gate) up) both come out of one accumulator: the experts' results are not read a second time,
+// and go is rounded once less.  Pays where those results have left L2 by then (from about half of its 126 MB on).  us, go into expert order with its
+// weights and dots / without: 98 304 rows of H 2048 234 / 135 (a pass 4907 / 4772), 262 144 rows 655 / 410 (8422 / 8235), 32 768 rows of H 2056
+// 88 / 49 (2305 / 2281), of H 1024 36 / 21 (529 / 520), 16 384 rows of H 1024 16 / 11 but 307 / 306 a pass.
+bool weighted_rows(int64_t M, int E, int64_t H, int64_t I) {
+  // (Where a forward without a backward takes the few-rows kernels, which leave the weights to the combine, it would round elsewhere.)
+  if (M * H * 2 < (64LL << 20) || !pairs_enabled() || I <= 64 || few_rows_forward(M, E, H, I)) return false;
+  const int64_t tiles = std::max<int64_t>(1, ceil_div(M, B200MOE_TILE_M) + E / 2), pairs = num_sms() / 2;   // as pick_bn_rows
+  // both products on pair tiles by the rule of pick_bn_grouped
+  auto on_pairs = [&](int64_t n) { return 10 * ceil_div(tiles * ceil_div(n, 256), pairs) <= 8 * ceil_div(2 * tiles * ceil_div(n, 128), 2 * pairs); };
+  return on_pairs(2 * I) && on_pairs(I);
+}
+
+int expert_gate_up_weighted(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+                            const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I, void* gate_up_out, void* inter, int32_t* status,
+                            b200moe_stream_t stream) {
+  return gate_up(x_s, gate_up_proj, act_codes, row_w, tile_expert, poffs, rows_cap, 0, 0, E, H, I, gate_up_out, inter, status, stream);
+}
+
+int expert_down_dgrad_weighted(const void* go_s, const void* down_proj, const void* gate_up_saved, const int32_t* act_codes, const float* row_w,
+                               const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
+                               void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
+  return down_dgrad(go_s, down_proj, gate_up_saved, act_codes, row_w, tile_expert, poffs, rows_cap, 0, 0, E, H, I, grad_gate_up, dots, status, stream);
 }
 
 }  // namespace b200moe
@@ -1032,16 +1135,6 @@ int b200moe_conv_gemm_dw_splitk(const void* grad_logits, const void* x, float* P
                                     (cudaStream_t)stream);
 }
 
-// row window of a grouped-M launch: (0, 0) = every row, else tile-aligned 0 <= row_lo < row_hi <= rows_cap
-static int check_row_window(const char* who, int64_t rows_cap, int64_t row_lo, int64_t row_hi) {
-  if (row_lo == 0 && row_hi == 0) return 0;
-  B200_CHECK_ARG(row_lo >= 0 && row_lo < row_hi && row_hi <= rows_cap && row_lo % B200MOE_TILE_M == 0 &&
-                     row_hi % B200MOE_TILE_M == 0,
-                 B200MOE_E_BAD_SHAPE, "%s: row window [%lld, %lld) must be tile-aligned and inside %lld rows", who,
-                 (long long)row_lo, (long long)row_hi, (long long)rows_cap);
-  return 0;
-}
-
 int b200moe_expert_gate_up_swiglu(const void* x_s, const void* gate_up_proj, const int32_t* tile_expert,
                                   const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
                                   void* gate_up, void* inter, int32_t* status, b200moe_stream_t stream) {
@@ -1053,27 +1146,7 @@ int b200moe_expert_gate_up_act(const void* x_s, const void* gate_up_proj, const 
                                const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo,
                                int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
                                int32_t* status, b200moe_stream_t stream) {
-  int rc = check_grouped("expert_gate_up_swiglu", x_s, gate_up_proj, gate_up, tile_expert, poffs, rows_cap, E, H, I);
-  if (rc) return rc;
-  rc = check_row_window("expert_gate_up_swiglu", rows_cap, row_lo, row_hi);
-  if (rc) return rc;
-  B200_CHECK_ARG(inter && tile_expert, B200MOE_E_NULL, "expert_gate_up_swiglu: null pointer");
-  B200_CHECK_ARG(aligned16(gate_up) && aligned16(inter), B200MOE_E_ALIGN, "expert_gate_up_swiglu: outputs not aligned");
-  Operand a{x_s, 0, rows_cap, H, H, 1, rows_cap * H};
-  // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
-  Operand b{gate_up_proj, 0, I, H, H, 2LL * E, I * H};
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.N = (int)I; p.K = (int)H; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = gate_up; p.aux = inter; p.I = (int)I; p.status = status;
-  p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
-  const int bn = pick_bn_rows(I, rows_cap, E, 2);   // tile covers bn/2 intermediate columns
-  Operand d1{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // {I, rows, 2}: group 0 = gate half, 1 = up half
-  Operand d2{inter, 0, rows_cap, I, I, 1, rows_cap * I};
-  if (act_codes != nullptr) {
-    p.act_codes = act_codes;
-    return dispatch_bn<EPI_SWIGLU, true>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
-  }
-  return dispatch_bn<EPI_SWIGLU>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
+  return ::b200moe::gate_up(x_s, gate_up_proj, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, gate_up, inter, status, stream);
 }
 
 int b200moe_expert_linear(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
@@ -1145,27 +1218,8 @@ int b200moe_expert_down_dgrad_act(const void* grad_eo, const void* down_proj, co
                                   const int32_t* act_codes, const int32_t* tile_expert, const int32_t* poffs,
                                   int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I,
                                   void* grad_gate_up, int32_t* status, b200moe_stream_t stream) {
-  int rc = check_grouped("expert_down_dgrad_glu", grad_eo, down_proj, grad_gate_up, tile_expert, poffs, rows_cap, E, H, I);
-  if (rc) return rc;
-  rc = check_row_window("expert_down_dgrad_glu", rows_cap, row_lo, row_hi);
-  if (rc) return rc;
-  B200_CHECK_ARG(gate_up && tile_expert, B200MOE_E_NULL, "expert_down_dgrad_glu: null pointer");
-  B200_CHECK_ARG(aligned16(grad_gate_up) && aligned16(gate_up), B200MOE_E_ALIGN, "expert_down_dgrad_glu: not aligned");
-  Operand a{grad_eo, 0, rows_cap, H, H, 1, rows_cap * H};
-  Operand b{down_proj, 1, I, H, I, E, H * I};   // W_d[e] stored (K=H, N=I): MN-major
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)I; p.K = (int)H; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = grad_gate_up; p.aux = const_cast<void*>(gate_up);
-  p.I = (int)I; p.status = status;
-  p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
-  const int bn = pick_bn_rows(I, rows_cap, E);
-  Operand d{grad_gate_up, 0, rows_cap, I, 2 * I, 2, I};   // {I, rows, 2}: grad_gate half, grad_up half
-  Operand d2{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // the saved forward gate_up, same view (input)
-  if (act_codes != nullptr) {
-    p.act_codes = act_codes;
-    return dispatch_bn<EPI_GLU_BWD, true>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
-  }
-  return dispatch_bn<EPI_GLU_BWD>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
+  return ::b200moe::down_dgrad(grad_eo, down_proj, gate_up, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, grad_gate_up,
+                               nullptr, status, stream);
 }
 
 int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_proj, const int32_t* tile_expert,
