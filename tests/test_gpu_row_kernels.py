@@ -60,6 +60,38 @@ def test_glu_rows_against_float64(pkg, I):
             assert not da[sl].any() and not dg[sl].any()
 
 
+# both sides of the limits between two and three vectors a thread
+@pytest.mark.parametrize("I", [768, 776, 1536, 1544, 3072, 3080, 6144, 6152])
+def test_glu_rows_of_three_vectors_a_thread(pkg, I):
+    test_glu_rows_against_float64(pkg, I)
+
+
+def test_glu_rows_of_special_values(pkg):
+    """Infinite, NaN and huge gates give what the formulas give in fp32, and nothing beside them."""
+    codes = [0, 1, 5]                                         # (a Norm code spreads such a gate over its row)
+    vals = torch.tensor([0.0, 1e-30, 30.0, 87.0, 88.5, 104.0, 1e4, 1e30, float("inf"), float("nan")]).to(torch.bfloat16)
+    vals = torch.cat([vals, -vals])
+    rows = 256 * len(codes)
+    gate_up = torch.ones(rows, 16, dtype=torch.bfloat16)
+    gate_up[:, 3] = vals[torch.arange(rows) % len(vals)]
+    perm = types.SimpleNamespace(cap=rows, E=3, tile_expert=torch.arange(3, dtype=torch.int32, device=DEV),
+                                 poffs=torch.arange(4, dtype=torch.int32, device=DEV) * 256,
+                                 total_rows=torch.tensor([rows], dtype=torch.int32, device=DEV))
+    cd, pd = torch.tensor(codes, dtype=torch.int32, device=DEV), torch.ones(3, 2, device=DEV)
+    inter = pkg.ops.glu_fwd_rows(gate_up.to(DEV), cd, pd, perm).cpu().float()
+    ggu, _, _ = pkg.ops.glu_bwd_rows(torch.ones(rows, 8, dtype=torch.bfloat16, device=DEV), gate_up.to(DEV), cd, pd, perm, True)
+    for e, code in enumerate(codes):
+        sl = slice(256 * e, 256 * (e + 1))
+        g = gate_up[sl, 3].float()
+        s = 1 / (1 + torch.exp(-g))
+        want = {0: g * s, 1: torch.fmax(g, torch.zeros(())).square(), 5: (2 / (1 + torch.exp(-2 * g)) - 1) * s}[code]
+        for got in (inter[sl, 3], ggu.cpu().float()[sl, 8 + 3]):      # grad_up is the activation too
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.to(torch.bfloat16).isinf())
+            ok = want.to(torch.bfloat16).isfinite()
+            assert ((got - want)[ok].abs() <= 2 ** -8 * want[ok].abs() + 1e-35).all()      # one rounding; results of 2^-126 and less may be 0
+    assert torch.isfinite(inter[:, torch.arange(8) != 3]).all()
+
+
 @pytest.mark.parametrize("E,k", [(1, 1), (31, 8), (32, 32), (33, 5), (64, 8), (65, 8), (128, 8), (129, 32), (256, 32)])
 def test_router_kernels_at_the_widths_of_a_lane(pkg, E, k):
     N = 1000

@@ -6,14 +6,15 @@
 // Semantics follow kernels/sm75/moe.py:163-232 (_glu_fwd_row_kernel, _glu_bwd_row_kernel) and
 // :859-881 (_act_eager) of the reference; math in fp32, bf16 in and out.
 //
-// Bound: HBM (forward 3 I, backward 5 I bf16 values a row) and, close behind it, the exponentials.  The kernels that
+// Bound: HBM (forward 3 I, backward 5 I bf16 values a row) and, close behind it, the instructions of the activations.  The kernels that
 // carry the path (`glu_*_vec_kernel`) hold a row in registers: TPR threads share a row, each with VPT 16-byte vectors of
 // every operand, all loaded before the first use, so a row is read once however many reductions its activation needs.
 // Rows of one CTA lie inside one 256-row tile and share its expert, so the activation code is uniform over the CTA and
 // the element loops are compiled per code.  The one-value-per-thread kernels below them read each value with a
 // 2-byte access, once per reduction; they remain for d_ff that is no multiple of 8 or above 8192 and for unaligned
-// buffers.  32 768 rows, d_ff 768, codes 0 1 2 5 6 7 in turn: forward 86 -> 40 us,
-// backward 194 -> 78 us (56 us of it at copy rate for both).
+// buffers.  32 768 rows, codes 0 1 2 5 6 7 in turn, L2 flushed before, us (at copy rate): d_ff 768 forward 37 (25), backward 57 (41);
+// d_ff 1032 55 (33), 94 (55); 8192 rows of d_ff 4096 51 (31), 78 (52).  With divisions, rows of 64 x 2 and 128 x 2 vectors, and the
+// Norm codes' activations kept across the second reduction they took 53 / 98, 84 / 164 and 63 / 111.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -73,6 +74,20 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
   return v;
 }
 
+// Reciprocal of 1 or more by the special-function unit, within one unit in the last place.  The correctly rounded division took more
+// instructions than the exponential beside it (forward 53 -> 44 us, backward 98 -> 80 of the rows above).
+__device__ __forceinline__ float rcp_above_1(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// tanh(x) from e = exp(-2x): of the rounding errors only that of e is absolute (2 / (1 + e) - 1 has that of the quotient as well, next to
+// which a small tanh is lost).  An infinite e is -1, a NaN stays one.
+__device__ __forceinline__ float tanh_of_exp(float e) {
+  asm("min.NaN.f32 %0, %0, 0f7149F2CA;" : "+f"(e));     // 1e30
+  return (1.0f - e) * rcp_above_1(1.0f + e);
+}
+
 // activation value and its derivative with respect to gn (gn = gate, or gate / rms for the Norm codes).  Code 5:
 // dal = d(act)/d(alpha), t5s = act / gamma
 template <int CODE>
@@ -82,15 +97,15 @@ __device__ __forceinline__ void act_eval(float gn, float alpha, float gamma, flo
     act = r * r;
     d = 2.0f * r;
   } else {
-    const float sig = sigmoidf_(gn);
+    const float e = expf(-gn), sig = rcp_above_1(1.0f + e);
     if constexpr (CODE == 5) {
-      const float t5 = tanh_via_sigmoid(alpha * gn);
+      const float t5 = tanh_of_exp(expf(-2.0f * (alpha * gn)));
       t5s = t5 * sig;
       act = gamma * t5s;
       d = gamma * (alpha * (1.0f - t5 * t5) * sig + t5s * (1.0f - sig));
       dal = gamma * gn * (1.0f - t5 * t5) * sig;
     } else if constexpr (CODE == 7) {
-      const float tg = tanh_via_sigmoid(gn);
+      const float tg = tanh_of_exp(e * e);
       act = tg * sig;
       d = (1.0f - tg * tg) * sig + tg * sig * (1.0f - sig);
     } else {
@@ -187,49 +202,50 @@ __device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (
                                             uint4* gg, uint4* gu, int t, int nvec, float alpha, float gamma, float* red,
                                             float& da, float& dg) {
   constexpr bool NORM = CODE == 2 || CODE == 6 || CODE == 7;
-  float inv_r = 1.0f, S = 0.0f;
-  float act[NORM ? 8 * VPT : 8], d[NORM ? 8 * VPT : 8];
-  float dal = 0.0f, t5s = 0.0f;
-  if constexpr (NORM) {   // RMS coupling term: mean of go * up * f'(gn) * gn
-    inv_r = row_rms_inv<TPR, VPT>(g, nvec * 8, red);
-    float part = 0.0f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      float gf[8], uf[8], of[8];
-      unpack8(g[i], gf);
-      unpack8(u[i], uf);
-      unpack8(go[i], of);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float gn = gf[j] * inv_r;
-        act_eval<CODE>(gn, alpha, gamma, act[8 * i + j], d[8 * i + j], dal, t5s);
-        part += of[j] * uf[j] * d[8 * i + j] * gn;
-      }
-    }
-    S = row_sum<TPR>(part, red) / static_cast<float>(nvec * 8);
-  }
+  float inv_r = 1.0f, part = 0.0f;
+  float wd[NORM ? VPT : 1][8];            // Norm codes: go * up * f'(gn), kept until the row's coupling term is known
+  if constexpr (NORM) inv_r = row_rms_inv<TPR, VPT>(g, nvec * 8, red);
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = t + TPR * i;
-    if (c >= nvec) continue;
     float gf[8], uf[8], of[8];
     unpack8(g[i], gf);
     unpack8(u[i], uf);
     unpack8(go[i], of);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int q = NORM ? 8 * i + j : j;
-      if constexpr (!NORM) act_eval<CODE>(gf[j], alpha, gamma, act[q], d[q], dal, t5s);
-      const float gi = of[j], w = gi * uf[j];
+      const float gn = NORM ? gf[j] * inv_r : gf[j];
+      float act, d, dal = 0.0f, t5s = 0.0f;
+      act_eval<CODE>(gn, alpha, gamma, act, d, dal, t5s);
+      const float w = of[j] * uf[j];
       if constexpr (CODE == 5) {
         da += w * dal;
         dg += w * t5s;
       }
-      gf[j] = NORM ? (w * d[q] - S * (gf[j] * inv_r)) * inv_r : w * d[q];
-      uf[j] = gi * act[q];
+      uf[j] = of[j] * act;
+      if constexpr (NORM) {
+        wd[i][j] = w * d;
+        part += wd[i][j] * gn;
+      } else {
+        gf[j] = w * d;
+      }
     }
-    gg[c] = pack8(gf);
-    gu[c] = pack8(uf);
+    if (c < nvec) {
+      gu[c] = pack8(uf);
+      if constexpr (!NORM) gg[c] = pack8(gf);
+    }
+  }
+  if constexpr (NORM) {   // RMS coupling term: mean of go * up * f'(gn) * gn
+    const float S = row_sum<TPR>(part, red) / static_cast<float>(nvec * 8);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c = t + TPR * i;
+      float gf[8];
+      unpack8(g[i], gf);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) gf[j] = (wd[i][j] - S * (gf[j] * inv_r)) * inv_r;
+      if (c < nvec) gg[c] = pack8(gf);
+    }
   }
 }
 
@@ -456,14 +472,18 @@ constexpr int64_t kMaxVecWidth = 8192;
 static bool rows_in_registers(int64_t I, const void* a, const void* b, const void* c) {
   return I % 8 == 0 && I <= kMaxVecWidth && aligned16(a) && aligned16(b) && aligned16(c);
 }
-// f(TPR, VPT): the narrowest row group that holds nvec vectors; two vectors of each operand a thread keep the backward
-// near 100 registers, so a wider row takes more threads first
+// f(TPR, VPT): the narrowest row group that holds nvec vectors, of two or three vectors of each operand a thread, so that at most a
+// third of its lanes is idle (d_ff 768: 32 x 3, 1032: 64 x 3); beside more registers, fewer warps a row need fewer barriers
 template <class F>
 static void by_row_width(int nvec, F f) {
-  if (nvec <= 64) f(std::integral_constant<int, 32>(), std::integral_constant<int, 2>());
-  else if (nvec <= 128) f(std::integral_constant<int, 64>(), std::integral_constant<int, 2>());
-  else if (nvec <= 256) f(std::integral_constant<int, 128>(), std::integral_constant<int, 2>());
-  else if (nvec <= 512) f(std::integral_constant<int, 256>(), std::integral_constant<int, 2>());
+  auto width = [&](auto tpr) {
+    if (nvec <= 2 * tpr.value) f(tpr, std::integral_constant<int, 2>());
+    else f(tpr, std::integral_constant<int, 3>());
+  };
+  if (nvec <= 96) width(std::integral_constant<int, 32>());
+  else if (nvec <= 192) width(std::integral_constant<int, 64>());
+  else if (nvec <= 384) width(std::integral_constant<int, 128>());
+  else if (nvec <= 768) width(std::integral_constant<int, 256>());
   else f(std::integral_constant<int, 256>(), std::integral_constant<int, 4>());
 }
 
