@@ -39,6 +39,10 @@ struct Dims {
   Kind kind;
   int64_t M() const { return T * k; }
   int64_t rows() const { return kind == KIND_FEW ? M() : b200moe_padded_rows_cap(M(), E); }
+  // elements between rows of the workspace's buffers (row_pitch; the few-rows kernels take dense ones)
+  int64_t ldh() const { return kind == KIND_FEW ? H : row_pitch(H); }
+  int64_t ldi() const { return kind == KIND_FEW ? I : row_pitch(I); }
+  int64_t ld2() const { return row_pitch(2 * I); }
 };
 
 static Dims make_dims(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int rows_kernels) {
@@ -91,10 +95,10 @@ static Forward carve_forward(const Dims& d, bool router, void* ws, size_t* bytes
     f.idx = c.take<int64_t>(M);
     f.w = c.take<float>(M);
   }
-  f.x_s = c.take<bf16_t>(rows * d.H);
-  if (!few) f.gate_up = c.take<bf16_t>(rows * 2 * d.I);
-  f.inter = c.take<bf16_t>(rows * d.I);
-  f.eo = c.take<bf16_t>(rows * d.H);
+  f.x_s = c.take<bf16_t>(rows * d.ldh());
+  if (!few) f.gate_up = c.take<bf16_t>(rows * d.ld2());
+  f.inter = c.take<bf16_t>(rows * d.ldi());
+  f.eo = c.take<bf16_t>(rows * d.ldh());
   if (bytes != nullptr) *bytes = c.off;
   return f;
 }
@@ -131,11 +135,11 @@ static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* byt
   Carver c(ws);
   Backward b{};
   const int64_t rows = d.rows();
-  b.grad_eo = c.take<bf16_t>(rows * d.H);
-  b.grad_gu = c.take<bf16_t>(rows * 2 * d.I);
+  b.grad_eo = c.take<bf16_t>(rows * d.ldh());
+  b.grad_gu = c.take<bf16_t>(rows * d.ld2());
   if (d.kind == KIND_ROWS) {
-    b.grad_x_s = c.take<bf16_t>(rows * d.H);       // grad_eo is still read (Identity experts) while this is written
-    b.grad_inter = c.take<bf16_t>(rows * d.I);
+    b.grad_x_s = c.take<bf16_t>(rows * d.ldh());       // grad_eo is still read (Identity experts) while this is written
+    b.grad_inter = c.take<bf16_t>(rows * d.ldi());
     b.row_da = c.take<float>(rows);
     b.row_dg = c.take<float>(rows);
   } else {
@@ -180,27 +184,20 @@ static int experts_forward(const Dims& d, const void* x, const float* w, const v
     RUN("combine", 1, b200moe_combine(f.eo, w, f.slot_pos, d.T, d.k, d.H, out, st));
     return 0;
   }
-  RUN("gather_rows", 1, b200moe_gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, rows, f.x_s, st));
-  if (d.kind == KIND_WEIGHTED) {
-    RUN("expert_gate_up_swiglu", 1, expert_gate_up_weighted(f.x_s, gate_up_proj, codes, f.row_w, f.tile_expert, f.poffs, rows, d.E, d.H, d.I,
-                                                            f.gate_up, f.inter, status, st));
-    RUN("expert_down", 1, b200moe_expert_linear(f.inter, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, status, st));
-    RUN("combine", 1, b200moe_combine(f.eo, nullptr, f.slot_row, d.T, d.k, d.H, out, st));   // the rows carry their weights
-    return 0;
-  }
-  if (d.kind == KIND_TILES) {
-    RUN("expert_gate_up_swiglu", 1, b200moe_expert_gate_up_act(f.x_s, gate_up_proj, codes, f.tile_expert, f.poffs, rows, 0, 0,
-                                                               d.E, d.H, d.I, f.gate_up, f.inter, status, st));
-    RUN("expert_down", 1, b200moe_expert_linear(f.inter, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, status, st));
+  const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
+  RUN("gather_rows", 1, gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, ldh, rows, f.x_s, st));
+  if (d.kind != KIND_ROWS) {   // weighted rows carry their weights from the activations on
+    RUN("expert_gate_up_swiglu", 1, expert_gate_up(f.x_s, ldh, gate_up_proj, codes, f.row_w, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H, d.I,
+                                                   f.gate_up, ld2, f.inter, ldi, status, st));
+    RUN("expert_down", 1, expert_linear(f.inter, ldi, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, ldh, status, st));
   } else {   // the GEMMs and the activation kernels see the rows of the experts with weights only
-    RUN("expert_linear", 1, b200moe_expert_linear(f.x_s, gate_up_proj, f.tile_expert, f.poffs, rows, d.n_glu, 2 * d.I, d.H,
-                                                  f.gate_up, status, st));
-    RUN("glu_fwd_rows", 1, b200moe_glu_fwd_rows(f.gate_up, f.tile_expert, codes, params, f.poffs + d.n_glu, rows, d.I, f.inter, st));
-    RUN("expert_linear", 1, b200moe_expert_linear(f.inter, down_proj, f.tile_expert, f.poffs, rows, d.n_glu, d.H, d.I, f.eo, status, st));
+    RUN("expert_linear", 1, expert_linear(f.x_s, ldh, gate_up_proj, f.tile_expert, f.poffs, rows, d.n_glu, 2 * d.I, d.H, f.gate_up, ld2, status, st));
+    RUN("glu_fwd_rows", 1, glu_fwd_rows(f.gate_up, ld2, f.tile_expert, codes, params, f.poffs + d.n_glu, rows, d.I, f.inter, ldi, st));
+    RUN("expert_linear", 1, expert_linear(f.inter, ldi, down_proj, f.tile_expert, f.poffs, rows, d.n_glu, d.H, d.I, f.eo, ldh, status, st));
     if (d.n_glu < d.E)
-      RUN("special_rows", 1, b200moe_special_rows(f.x_s, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, rows, f.eo, st));
+      RUN("special_rows", 1, special_rows(f.x_s, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, ldh, rows, f.eo, st));
   }
-  RUN("combine", 1, b200moe_combine(f.eo, w, f.slot_row, d.T, d.k, d.H, out, st));
+  RUN("combine", 1, combine_add(f.eo, ldh, d.kind == KIND_WEIGHTED ? nullptr : w, f.slot_row, nullptr, d.T, d.k, d.H, out, st));
   return 0;
 }
 
@@ -215,46 +212,42 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
                             const Backward& b, const Grads& g, int32_t* status, b200moe_stream_t st) {
   const int64_t rows = d.rows();
   const int32_t* total = f.poffs + d.E;
+  const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
   const bool weighted = d.kind == KIND_WEIGHTED;
   if (weighted)
-    RUN("gather_rows", 1, b200moe_gather_rows(grad_out, f.row_slot, total, d.k, d.H, rows, b.grad_eo, st));
+    RUN("gather_rows", 1, gather_rows(grad_out, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, st));
   else
-    RUN("combine_bwd", 1, b200moe_combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, rows, b.grad_eo, g.w != nullptr ? g.w : b.grad_w, st));
-  if (d.kind == KIND_TILES || weighted) {
-    if (weighted && (g.x != nullptr || g.gate_up != nullptr || g.w != nullptr)) {
-      RUN("expert_down_dgrad_glu", 1, expert_down_dgrad_weighted(b.grad_eo, down_proj, f.gate_up, codes, f.row_w, f.tile_expert, f.poffs, rows,
-                                                                 d.E, d.H, d.I, b.grad_gu, b.dots, status, st));
-      if (g.w != nullptr) RUN("row_dots", 1, row_dots(b.dots, (int)((d.I + 127) / 128), rows, f.row_slot, total, g.w, st));
+    RUN("combine_bwd", 1, combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, g.w != nullptr ? g.w : b.grad_w, st));
+  if (d.kind != KIND_ROWS) {
+    if (g.x != nullptr || g.gate_up != nullptr || (weighted && g.w != nullptr)) {
+      RUN("expert_down_dgrad_glu", 1, expert_down_dgrad(b.grad_eo, ldh, down_proj, f.gate_up, ld2, codes, f.row_w, f.tile_expert, f.poffs, rows, 0, 0,
+                                                        d.E, d.H, d.I, b.grad_gu, b.dots, status, st));
+      if (weighted && g.w != nullptr)
+        RUN("row_dots", 1, row_dots(b.dots, (int)((d.I + 127) / 128), rows, f.row_slot, total, g.w, st));
     }
-    if (g.x != nullptr || g.gate_up != nullptr) {
-      if (!weighted)
-        RUN("expert_down_dgrad_glu", 1,
-            b200moe_expert_down_dgrad_act(b.grad_eo, down_proj, f.gate_up, codes, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H,
-                                          d.I, b.grad_gu, status, st));
-      if (g.gate_up != nullptr)
-        RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_gu, f.x_s, f.poffs, f.counts, rows, d.E, 2 * d.I, d.H, g.gate_up, status, st));
-    }
+    if (g.gate_up != nullptr)
+      RUN("expert_wgrad", 1, expert_wgrad(b.grad_gu, ld2, f.x_s, ldh, f.poffs, f.counts, rows, d.E, 2 * d.I, d.H, g.gate_up, status, st));
     if (g.down != nullptr)
-      RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_eo, f.inter, f.poffs, f.counts, rows, d.E, d.H, d.I, g.down, status, st));
+      RUN("expert_wgrad", 1, expert_wgrad(b.grad_eo, ldh, f.inter, ldi, f.poffs, f.counts, rows, d.E, d.H, d.I, g.down, status, st));
     if (g.x != nullptr)
-      RUN("expert_gate_up_dgrad", 1, b200moe_expert_linear_t(b.grad_gu, gate_up_proj, f.tile_expert, f.poffs, rows, d.E, 2 * d.I,
-                                                             d.H, b.grad_x_s, status, st));
+      RUN("expert_gate_up_dgrad", 1, expert_linear_t(b.grad_gu, ld2, gate_up_proj, f.tile_expert, f.poffs, rows, d.E, 2 * d.I, d.H, 2 * d.I,
+                                                     b.grad_x_s, ldh, status, st));
     return 0;
   }
   const int n = d.n_glu;
-  RUN("expert_linear_t", 1, b200moe_expert_linear_t(b.grad_eo, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, b.grad_inter, status, st));
+  RUN("expert_linear_t", 1, expert_linear_t(b.grad_eo, ldh, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, d.H, b.grad_inter, ldi, status, st));
   float* da = g.params != nullptr ? b.row_da : nullptr;
   float* dg = g.params != nullptr ? b.row_dg : nullptr;
-  RUN("glu_bwd_rows", 1, b200moe_glu_bwd_rows(b.grad_inter, f.gate_up, f.tile_expert, codes, params, f.poffs + n, rows, d.I,
-                                              b.grad_gu, da, dg, st));
+  RUN("glu_bwd_rows", 1, glu_bwd_rows(b.grad_inter, ldi, f.gate_up, ld2, f.tile_expert, codes, params, f.poffs + n, rows, d.I, b.grad_gu, da, dg, st));
   if (g.down != nullptr)
-    RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_eo, f.inter, f.poffs, f.counts, rows, n, d.H, d.I, g.down, status, st));
+    RUN("expert_wgrad", 1, expert_wgrad(b.grad_eo, ldh, f.inter, ldi, f.poffs, f.counts, rows, n, d.H, d.I, g.down, status, st));
   if (g.gate_up != nullptr)
-    RUN("expert_wgrad", 1, b200moe_expert_wgrad(b.grad_gu, f.x_s, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, status, st));
+    RUN("expert_wgrad", 1, expert_wgrad(b.grad_gu, ld2, f.x_s, ldh, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, status, st));
   if (g.x != nullptr) {
-    RUN("expert_linear_t", 1, b200moe_expert_linear_t(b.grad_gu, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, b.grad_x_s, status, st));
+    RUN("expert_linear_t", 1, expert_linear_t(b.grad_gu, ld2, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, 2 * d.I, b.grad_x_s, ldh,
+                                              status, st));
     if (n < d.E)
-      RUN("special_rows", 1, b200moe_special_rows(b.grad_eo, f.tile_expert, codes, f.poffs, n, d.E, d.H, rows, b.grad_x_s, st));
+      RUN("special_rows", 1, special_rows(b.grad_eo, f.tile_expert, codes, f.poffs, n, d.E, d.H, ldh, rows, b.grad_x_s, st));
   }
   if (g.params != nullptr) {
     if (n < d.E)
@@ -474,7 +467,7 @@ int b200moe_moe_backward(const void* grad_out, const float* w, const void* gate_
   const Grads g{grad_x, grad_gate_up, grad_down, grad_w, grad_params};
   rc = experts_backward(d, grad_out, w, gate_up_proj, down_proj, act_codes, act_params, f, b, g, status, stream);
   if (rc) return rc;
-  if (grad_x != nullptr) RUN("combine", 1, b200moe_combine(b.grad_x_s, nullptr, f.slot_row, T, k, H, grad_x, stream));
+  if (grad_x != nullptr) RUN("combine", 1, combine_add(b.grad_x_s, d.ldh(), nullptr, f.slot_row, nullptr, T, k, H, grad_x, stream));
   return 0;
 }
 
@@ -528,7 +521,7 @@ int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate
     if (rc) return rc;
   }
   if (grad_x != nullptr)   // the experts' rows of a token and the router's share, added in fp32, one rounding
-    RUN("combine", 1, b200moe_combine_add(b.grad_x_s, nullptr, f.slot_row, b.grad_x_router, T, k, H, grad_x, stream));
+    RUN("combine", 1, combine_add(b.grad_x_s, d.ldh(), nullptr, f.slot_row, b.grad_x_router, T, k, H, grad_x, stream));
   return 0;
 }
 
@@ -548,7 +541,7 @@ int b200moe_newton_schulz(void* x, void* x_next, void* a, void* a2, const int32_
     const float ca = coeffs[3 * i], cb = coeffs[3 * i + 1], cc = coeffs[3 * i + 2];
     RUN("expert_gram", 1, expert_gram(x, tile_expert, poffs, rows, E, wide, 1, live, a, status, stream));
     RUN("expert_linear_axpby", 1, expert_linear_axpby(a, a, a, cc, cb, ca, 2, tile_expert, poffs, rows, E, Rp, Rp, live, live, a2, status, stream));
-    RUN("expert_linear_t", 1, expert_linear_t(a2, x, tile_expert, poffs, rows, E, Rp, wide, live, x_next, status, stream));
+    RUN("expert_linear_t", 1, expert_linear_t(a2, Rp, x, tile_expert, poffs, rows, E, Rp, wide, live, x_next, wide, status, stream));
     std::swap(x, x_next);
   }
   return 0;

@@ -25,7 +25,7 @@ constexpr int kVecBatch = 4;   // 16-byte vectors a lane keeps in flight per row
 // H 2048, top-8 223 -> 214 us.
 template <int TPR>
 __global__ void __launch_bounds__(256)
-combine_kernel(const uint4* rows, const float* w, const int* slot_row, const uint4* add, long long T, int k,
+combine_kernel(const uint4* rows, int pitch, const float* w, const int* slot_row, const uint4* add, long long T, int k,
                int vec_per_row, uint4* out) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
@@ -41,7 +41,7 @@ combine_kernel(const uint4* rows, const float* w, const int* slot_row, const uin
         for (int i = 0; i < 4; ++i) r[i] = j0 + i < k ? slots[j0 + i] : -1;
 #pragma unroll
         for (int i = 0; i < 4; ++i)   // a slot without a row (its expert index was out of range) adds nothing
-          if (r[i] >= 0) v[i] = rows[static_cast<long long>(r[i]) * vec_per_row + c];
+          if (r[i] >= 0) v[i] = rows[static_cast<long long>(r[i]) * pitch + c];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (r[i] >= 0) fma8(acc, v[i], w != nullptr ? w[t * k + j0 + i] : 1.0f);
@@ -62,21 +62,21 @@ combine_kernel(const uint4* rows, const float* w, const int* slot_row, const uin
 // reduced by shuffles in a fixed order.
 __global__ void __launch_bounds__(256)
 combine_bwd_kernel(const uint4* go, const uint4* eo, const float* w, const int* row_slot, const int* total_rows, int k,
-                   int vec_per_row, uint4* grad_eo, float* grad_w) {
+                   int vec_per_row, int pitch, uint4* grad_eo, float* grad_w) {
   grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const int total = *total_rows;
   for (long long r = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < total; r += warps) {
     const int slot = row_slot[r];
-    uint4* dst = grad_eo + r * vec_per_row;
+    uint4* dst = grad_eo + r * pitch;
     if (slot < 0) {
       for (int c = lane; c < vec_per_row; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
       continue;
     }
     const float wt = w[slot];
     const uint4* g = go + static_cast<long long>(slot / k) * vec_per_row;
-    const uint4* e = eo + r * vec_per_row;
+    const uint4* e = eo + r * pitch;
     float dot = 0.0f;
     for (int c0 = 0; c0 < vec_per_row; c0 += 32 * kVecBatch) {
       uint4 gv[kVecBatch], ev[kVecBatch];
@@ -116,7 +116,7 @@ combine_bwd_kernel(const uint4* go, const uint4* eo, const float* w, const int* 
 // faster one: 64 vectors 18 against 24 us, 256 vectors 200 against 248 us).
 __global__ void __launch_bounds__(256)
 combine_bwd_narrow_kernel(const uint4* go, const uint4* eo, const float* w, const int* row_slot, const int* total_rows,
-                          int k, int vec_per_row, uint4* grad_eo, float* grad_w) {
+                          int k, int vec_per_row, int pitch, uint4* grad_eo, float* grad_w) {
   grid_dep_begin();
   constexpr int RB = 4;
   const int lane = threadIdx.x & 31;
@@ -134,7 +134,7 @@ combine_bwd_narrow_kernel(const uint4* go, const uint4* eo, const float* w, cons
       const bool live = in && slot[q] >= 0;
       wt[q] = slot[q] >= 0 ? w[slot[q]] : 0.0f;
       g[q] = live ? go[static_cast<long long>(slot[q] / k) * vec_per_row + lane] : make_uint4(0u, 0u, 0u, 0u);
-      e[q] = live ? eo[(r0 + q) * vec_per_row + lane] : make_uint4(0u, 0u, 0u, 0u);
+      e[q] = live ? eo[(r0 + q) * pitch + lane] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
@@ -147,7 +147,7 @@ combine_bwd_narrow_kernel(const uint4* go, const uint4* eo, const float* w, cons
         dot += gf.x * ef.x + gf.y * ef.y;
         o[h] = slot[q] >= 0 ? pack_bf16x2(gf.x * wt[q], gf.y * wt[q]) : 0u;
       }
-      if (in && r0 + q < total) grad_eo[(r0 + q) * vec_per_row + lane] = make_uint4(o[0], o[1], o[2], o[3]);
+      if (in && r0 + q < total) grad_eo[(r0 + q) * pitch + lane] = make_uint4(o[0], o[1], o[2], o[3]);
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
       if (lane == 0 && slot[q] >= 0) grad_w[slot[q]] = dot;
@@ -182,19 +182,8 @@ int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, 
   return 0;
 }
 
-}  // namespace b200moe
-
-using namespace b200moe;
-
-extern "C" {
-
-int b200moe_combine(const void* rows, const float* w, const int32_t* slot_row, int64_t T, int k, int64_t H,
-                    void* out, b200moe_stream_t stream) {
-  return b200moe_combine_add(rows, w, slot_row, nullptr, T, k, H, out, stream);
-}
-
-int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k,
-                        int64_t H, void* out, b200moe_stream_t stream) {
+int combine_add(const void* rows, int64_t ldh, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k, int64_t H, void* out,
+                b200moe_stream_t stream) {
   B200_CHECK_ARG(rows && slot_row && out, B200MOE_E_NULL, "combine: null pointer");
   B200_CHECK_ARG(H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE, "combine: H = %lld must be a multiple of 8", (long long)H);
   B200_CHECK_ARG(k >= 1 && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "combine: k = %d", k);
@@ -205,16 +194,15 @@ int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_ro
     constexpr int G = 256 / tpr.value;
     const long long grid = std::min<long long>((T + G - 1) / G, static_cast<long long>(num_sms()) * 16);
     err = launch_chained(combine_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
-                         reinterpret_cast<const uint4*>(rows), w, slot_row, reinterpret_cast<const uint4*>(add), T, k,
+                         reinterpret_cast<const uint4*>(rows), static_cast<int>(ldh / 8), w, slot_row, reinterpret_cast<const uint4*>(add), T, k,
                          static_cast<int>(H / 8), reinterpret_cast<uint4*>(out));
   });
   B200_CUDA(err);
   return 0;
 }
 
-int b200moe_combine_bwd(const void* grad_out, const void* eo, const float* w, const int32_t* row_slot,
-                        const int32_t* total_rows, int k, int64_t H, int64_t rows_cap, void* grad_eo, float* grad_w,
-                        b200moe_stream_t stream) {
+int combine_bwd(const void* grad_out, const void* eo, const float* w, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,
+                int64_t ldh, int64_t rows_cap, void* grad_eo, float* grad_w, b200moe_stream_t stream) {
   B200_CHECK_ARG(grad_out && eo && w && row_slot && total_rows && grad_eo && grad_w, B200MOE_E_NULL,
                  "combine_bwd: null pointer");
   B200_CHECK_ARG(H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE, "combine_bwd: H = %lld must be a multiple of 8", (long long)H);
@@ -226,8 +214,30 @@ int b200moe_combine_bwd(const void* grad_out, const void* eo, const float* w, co
   const long long grid = std::min<long long>((rows_cap + 8 * rows_per_warp - 1) / (8 * rows_per_warp), static_cast<long long>(num_sms()) * 8);
   auto kernel = nvec <= 32 ? combine_bwd_narrow_kernel : combine_bwd_kernel;
   B200_LAUNCH(kernel, static_cast<int>(grid), 256, 0, stream, reinterpret_cast<const uint4*>(grad_out),
-              reinterpret_cast<const uint4*>(eo), w, row_slot, total_rows, k, nvec, reinterpret_cast<uint4*>(grad_eo), grad_w);
+              reinterpret_cast<const uint4*>(eo), w, row_slot, total_rows, k, nvec, static_cast<int>(ldh / 8), reinterpret_cast<uint4*>(grad_eo), grad_w);
   return 0;
+}
+
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" {
+
+int b200moe_combine(const void* rows, const float* w, const int32_t* slot_row, int64_t T, int k, int64_t H,
+                    void* out, b200moe_stream_t stream) {
+  return combine_add(rows, H, w, slot_row, nullptr, T, k, H, out, stream);
+}
+
+int b200moe_combine_add(const void* rows, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k,
+                        int64_t H, void* out, b200moe_stream_t stream) {
+  return combine_add(rows, H, w, slot_row, add, T, k, H, out, stream);
+}
+
+int b200moe_combine_bwd(const void* grad_out, const void* eo, const float* w, const int32_t* row_slot,
+                        const int32_t* total_rows, int k, int64_t H, int64_t rows_cap, void* grad_eo, float* grad_w,
+                        b200moe_stream_t stream) {
+  return combine_bwd(grad_out, eo, w, row_slot, total_rows, k, H, H, rows_cap, grad_eo, grad_w, stream);
 }
 
 }  // extern "C"

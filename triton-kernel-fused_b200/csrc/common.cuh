@@ -34,6 +34,39 @@ struct RowWeights {
   float* row_w;
   const float* slot_w;   // (T, k)
 };
+// Elements between rows of the block's own buffers.  A TMA box whose 128-byte rows start 16 bytes past a 32-byte sector moves at three
+// quarters of the rate (8.4 against 11.6 TB/s, all from L2; 32 bytes past a line: 10.9), and stores to such rows leave partial sectors: rows whose
+// length is no multiple of 64 bytes are padded to whole lines.  us a training pass, dense / padded: 3001 tokens, 32 experts of 1032 x 680, top-4
+// 370 / 350; 8192 tokens, 32 of 2056 x 1416 2426 / 2023, of 2040 x 1400 2237 / 1873; 8192 tokens, 16 of 1064 x 2088, top-2 880 / 783; 16 384
+// tokens, 64 of 520 x 264, top-6 776 / 722; 2000 tokens, 8 of 264 x 136, top-2 80 / 77.
+inline int64_t row_pitch(int64_t n) { return n % 32 == 0 ? n : (n + 63) / 64 * 64; }
+
+// The entry points of the block's steps with the distance between rows given (elements): of x_s, the experts' results and their gradients
+// (ldh), of inter (ldi), of gate_up and its gradient (ld2)
+int gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H, int64_t ldh, int64_t rows_cap, void* x_s,
+                b200moe_stream_t stream);
+int combine_add(const void* rows, int64_t ldh, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k, int64_t H, void* out,
+                b200moe_stream_t stream);
+int combine_bwd(const void* grad_out, const void* eo, const float* w, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,
+                int64_t ldh, int64_t rows_cap, void* grad_eo, float* grad_w, b200moe_stream_t stream);
+int glu_fwd_rows(const void* gate_up, int64_t ld2, const int32_t* tile_expert, const int32_t* act_codes, const float* act_params,
+                 const int32_t* total_rows, int64_t rows_cap, int64_t I, void* inter, int64_t ldi, b200moe_stream_t stream);
+int glu_bwd_rows(const void* grad_inter, int64_t ldi, const void* gate_up, int64_t ld2, const int32_t* tile_expert, const int32_t* act_codes,
+                 const float* act_params, const int32_t* total_rows, int64_t rows_cap, int64_t I, void* grad_gate_up, float* row_da, float* row_dg,
+                 b200moe_stream_t stream);
+int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special, int num_experts,
+                 int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream);
+int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+                   const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, int64_t ld2,
+                   void* inter, int64_t ldi, int32_t* status, b200moe_stream_t stream);
+int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, const void* gate_up, int64_t ld2, const int32_t* act_codes,
+                      const float* row_w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
+                      int64_t H, int64_t I, void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream);
+int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
+                  int64_t K, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream);
+int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
+                 int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream);
+
 // b200moe_permute_build; also stores the counts a second time (counts_out) and adds them to `load` (both nullable)
 int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs, int32_t* poffs,
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
@@ -42,14 +75,8 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
 // combine.cu: grad_w[slot] = sum over `parts` of dots[part][row], dots (parts, ld)
 int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, const int32_t* total_rows, float* grad_w, b200moe_stream_t stream);
 
-// gemm.cu: whether a block's rows are weighted by the epilogues of its GLU products, and those products
+// gemm.cu: whether a block's rows are weighted by the epilogues of its GLU products (their row_w, dots)
 bool weighted_rows(int64_t M, int E, int64_t H, int64_t I);
-int expert_gate_up_weighted(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
-                            const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I, void* gate_up, void* inter, int32_t* status,
-                            b200moe_stream_t stream);
-int expert_down_dgrad_weighted(const void* go_s, const void* down_proj, const void* gate_up, const int32_t* act_codes, const float* row_w,
-                               const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
-                               void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream);
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);
@@ -66,8 +93,8 @@ int expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs,
 int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha, float beta, float diag, int symmetric,
                         const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N, int64_t K,
                         int64_t n_live, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream);
-int expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
-                    int64_t K, int64_t N, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream);
+int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
+                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream);
 
 // Tells the observer set by b200moe_set_observer, if any, where an operation of a longer sequence begins and ends
 struct OpScope {

@@ -86,7 +86,7 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
-// WEIGHTED: the GLU epilogues of a block whose rows are weighted where their activations are made (expert_gate_up_weighted).
+// WEIGHTED: the GLU epilogues of a block whose rows are weighted where their activations are made (weighted_rows).
 template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -367,11 +367,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if constexpr (kGluRegs) {
           const int col0 = t.n0 + half * (BN / 2) + (step >> 1) * CW;
           const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.aux) +
-                                     static_cast<long long>(row0 + 16 * (step & 1)) * (2LL * p.I) + col0;
+                                     static_cast<long long>(row0 + 16 * (step & 1)) * p.ld2 + col0;
 #pragma unroll
           for (int s2 = 0; s2 < 2; ++s2) {
-            epi_pieces<NP>(src + 16LL * s2 * p.I, 2LL * p.I, p.I - col0, lane, gv[s2]);
-            epi_pieces<NP>(src + 16LL * s2 * p.I + p.I, 2LL * p.I, p.I - col0, lane, uv[s2]);
+            epi_pieces<NP>(src + 8LL * s2 * p.ld2, p.ld2, p.I - col0, lane, gv[s2]);
+            epi_pieces<NP>(src + 8LL * s2 * p.ld2 + p.I, p.ld2, p.I - col0, lane, uv[s2]);
           }
         }
       };
@@ -605,10 +605,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                   epi_pack(u[i], s2, uw[i]);
                   glu_fwd_pairs_by_code<POLY>(act_code, gw[i], uw[i], hw[i], 4);
                 }
-                __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(p.D) + r8 * (2LL * I) + col0;
-                epi_put<NP>(gu, 2LL * I, 8, I - col0, lane, gw);
-                epi_put<NP>(gu + I, 2LL * I, 8, I - col0, lane, uw);
-                epi_put<NP>(reinterpret_cast<__nv_bfloat16*>(p.aux) + r8 * I + col0, I, 8, I - col0, lane, hw);
+                __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(p.D) + r8 * p.ld2 + col0;
+                epi_put<NP>(gu, p.ld2, 8, I - col0, lane, gw);
+                epi_put<NP>(gu + I, p.ld2, 8, I - col0, lane, uw);
+                epi_put<NP>(reinterpret_cast<__nv_bfloat16*>(p.aux) + r8 * p.ldi + col0, p.ldi, 8, I - col0, lane, hw);
               }
             }
           }
@@ -636,9 +636,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 epi_pack(r[i], s2, iw);                         // rounded to bf16: the reference materialises grad_inter in bf16
                 glu_bwd_pairs<POLY>(act_code, iw, gw[s2][i], uw[s2][i]);      // now grad_gate, grad_up
               }
-              __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row0 + 16 * (step & 1) + 8 * s2) * (2LL * I) + col0;
-              epi_put<NP>(d, 2LL * I, 8, I - col0, lane, gw[s2]);
-              epi_put<NP>(d + I, 2LL * I, 8, I - col0, lane, uw[s2]);
+              __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row0 + 16 * (step & 1) + 8 * s2) * p.ld2 + col0;
+              epi_put<NP>(d, p.ld2, 8, I - col0, lane, gw[s2]);
+              epi_put<NP>(d + I, p.ld2, 8, I - col0, lane, uw[s2]);
             }
           }
         }
@@ -872,18 +872,18 @@ int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha
   return dispatch_bn<EPI_AXPBY>(256, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
-int expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
-                    int64_t K, int64_t N, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream) {
+int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
+                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_linear_t", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
   if (rc) return rc;
   B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear_t: null pointer");
   B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_linear_t: output not aligned");
-  Operand oa{a, 0, rows_cap, k_live, K, 1, rows_cap * K};
+  Operand oa{a, 0, rows_cap, k_live, lda, 1, rows_cap * lda};
   Operand ob{w, 1, N, k_live, N, E, K * N};   // W[e] stored (K, N): MN-major
   GemmParams p{};
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)k_live; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
-  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = ldo; p.status = status;
+  Operand d{out, 0, rows_cap, N, ldo, 1, rows_cap * ldo};
   return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
@@ -897,25 +897,26 @@ static int check_row_window(const char* who, int64_t rows_cap, int64_t row_lo, i
   return 0;
 }
 
-static int gate_up(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
-                   const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
-                   int32_t* status, b200moe_stream_t stream) {
+int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+                   const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, int64_t ld2,
+                   void* inter, int64_t ldi, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_gate_up_swiglu", x_s, gate_up_proj, gate_up, tile_expert, poffs, rows_cap, E, H, I);
   if (rc) return rc;
   rc = check_row_window("expert_gate_up_swiglu", rows_cap, row_lo, row_hi);
   if (rc) return rc;
   B200_CHECK_ARG(inter && tile_expert, B200MOE_E_NULL, "expert_gate_up_swiglu: null pointer");
   B200_CHECK_ARG(aligned16(gate_up) && aligned16(inter), B200MOE_E_ALIGN, "expert_gate_up_swiglu: outputs not aligned");
-  Operand a{x_s, 0, rows_cap, H, H, 1, rows_cap * H};
+  Operand a{x_s, 0, rows_cap, H, ldh, 1, rows_cap * ldh};
   // W_gu (E, 2I, H) seen as dims {H, I, 2E}: group 2e = gate rows of expert e, 2e+1 = up rows
   Operand b{gate_up_proj, 0, I, H, H, 2LL * E, I * H};
   GemmParams p{};
   p.sched = SCHED_GROUPED_M; p.N = (int)I; p.K = (int)H; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = gate_up; p.aux = inter; p.I = (int)I; p.status = status;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = gate_up; p.aux = inter; p.I = (int)I; p.ld2 = ld2; p.ldi = ldi;
+  p.status = status;
   p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
   const int bn = pick_bn_rows(I, rows_cap, E, 2);   // tile covers bn/2 intermediate columns
-  Operand d1{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // {I, rows, 2}: group 0 = gate half, 1 = up half
-  Operand d2{inter, 0, rows_cap, I, I, 1, rows_cap * I};
+  Operand d1{gate_up, 0, rows_cap, I, ld2, 2, I};         // {I, rows, 2}: group 0 = gate half, 1 = up half
+  Operand d2{inter, 0, rows_cap, I, ldi, 1, rows_cap * ldi};
   p.act_codes = act_codes;
   if (row_w != nullptr) {
     p.row_w = row_w;
@@ -926,25 +927,25 @@ static int gate_up(const void* x_s, const void* gate_up_proj, const int32_t* act
   return dispatch_bn<EPI_SWIGLU>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
 }
 
-static int down_dgrad(const void* grad_eo, const void* down_proj, const void* gate_up, const int32_t* act_codes, const float* row_w,
-                      const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I,
-                      void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
+int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, const void* gate_up, int64_t ld2, const int32_t* act_codes,
+                      const float* row_w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
+                      int64_t H, int64_t I, void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_down_dgrad_glu", grad_eo, down_proj, grad_gate_up, tile_expert, poffs, rows_cap, E, H, I);
   if (rc) return rc;
   rc = check_row_window("expert_down_dgrad_glu", rows_cap, row_lo, row_hi);
   if (rc) return rc;
   B200_CHECK_ARG(gate_up && tile_expert, B200MOE_E_NULL, "expert_down_dgrad_glu: null pointer");
   B200_CHECK_ARG(aligned16(grad_gate_up) && aligned16(gate_up), B200MOE_E_ALIGN, "expert_down_dgrad_glu: not aligned");
-  Operand a{grad_eo, 0, rows_cap, H, H, 1, rows_cap * H};
+  Operand a{grad_eo, 0, rows_cap, H, ldh, 1, rows_cap * ldh};
   Operand b{down_proj, 1, I, H, I, E, H * I};   // W_d[e] stored (K=H, N=I): MN-major
   GemmParams p{};
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)I; p.K = (int)H; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = grad_gate_up; p.aux = const_cast<void*>(gate_up);
-  p.I = (int)I; p.status = status;
+  p.I = (int)I; p.ld2 = ld2; p.status = status;
   p.row_lo = (int)row_lo; p.row_hi = (int)row_hi;
   const int bn = pick_bn_rows(I, rows_cap, E);
-  Operand d{grad_gate_up, 0, rows_cap, I, 2 * I, 2, I};   // {I, rows, 2}: grad_gate half, grad_up half
-  Operand d2{gate_up, 0, rows_cap, I, 2 * I, 2, I};       // the saved forward gate_up, same view (input)
+  Operand d{grad_gate_up, 0, rows_cap, I, ld2, 2, I};     // {I, rows, 2}: grad_gate half, grad_up half
+  Operand d2{gate_up, 0, rows_cap, I, ld2, 2, I};         // the saved forward gate_up, same view (input)
   p.act_codes = act_codes;
   if (row_w != nullptr) {
     p.row_w = row_w; p.dots = dots; p.dots_ld = rows_cap;
@@ -970,16 +971,39 @@ bool weighted_rows(int64_t M, int E, int64_t H, int64_t I) {
   return on_pairs(2 * I) && on_pairs(I);
 }
 
-int expert_gate_up_weighted(const void* x_s, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
-                            const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I, void* gate_up_out, void* inter, int32_t* status,
-                            b200moe_stream_t stream) {
-  return gate_up(x_s, gate_up_proj, act_codes, row_w, tile_expert, poffs, rows_cap, 0, 0, E, H, I, gate_up_out, inter, status, stream);
+int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
+                  int64_t K, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream) {
+  int rc = check_grouped("expert_linear", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
+  if (rc) return rc;
+  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear: null pointer");
+  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_linear: output not aligned");
+  Operand oa{a, 0, rows_cap, K, lda, 1, rows_cap * lda};
+  Operand ob{w, 0, N, K, K, E, N * K};   // W (E, N, K): rows = output columns
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_M; p.N = (int)N; p.K = (int)K; p.num_groups = E;
+  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = ldo; p.status = status;
+  Operand d{out, 0, rows_cap, N, ldo, 1, rows_cap * ldo};
+  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
-int expert_down_dgrad_weighted(const void* go_s, const void* down_proj, const void* gate_up_saved, const int32_t* act_codes, const float* row_w,
-                               const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t H, int64_t I,
-                               void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
-  return down_dgrad(go_s, down_proj, gate_up_saved, act_codes, row_w, tile_expert, poffs, rows_cap, 0, 0, E, H, I, grad_gate_up, dots, status, stream);
+int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
+                 int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
+  B200_CHECK_ARG(A && B && poffs && out, B200MOE_E_NULL, "expert_wgrad: null pointer");
+  B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_wgrad: E = %d", E);
+  B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
+                 "expert_wgrad: rows_cap = %lld must be a positive multiple of %d", (long long)rows_cap, B200MOE_TILE_M);
+  CHECK_DIM8(Na); CHECK_DIM8(Nb); CHECK_I32(Na); CHECK_I32(Nb);
+  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_wgrad: output not aligned");
+  Operand a{A, 1, Na, rows_cap, lda, 1, rows_cap * lda};
+  Operand b{B, 1, Nb, rows_cap, ldb, 1, rows_cap * ldb};
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)Na; p.N = (int)Nb; p.K = (int)rows_cap;
+  p.num_groups = E; p.poffs = poffs; p.counts = counts; p.D = out; p.ldd = Nb; p.d_group_stride = Na * Nb;
+  p.status = status;
+  const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
+  Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
+  return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn)),
+                                (cudaStream_t)stream);
 }
 
 }  // namespace b200moe
@@ -1146,23 +1170,14 @@ int b200moe_expert_gate_up_act(const void* x_s, const void* gate_up_proj, const 
                                const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo,
                                int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
                                int32_t* status, b200moe_stream_t stream) {
-  return ::b200moe::gate_up(x_s, gate_up_proj, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, gate_up, inter, status, stream);
+  return expert_gate_up(x_s, H, gate_up_proj, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, gate_up, 2 * I, inter, I, status,
+                        stream);
 }
 
 int b200moe_expert_linear(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
                           int64_t rows_cap, int E, int64_t N, int64_t K, void* out, int32_t* status,
                           b200moe_stream_t stream) {
-  int rc = check_grouped("expert_linear", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
-  if (rc) return rc;
-  B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear: null pointer");
-  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_linear: output not aligned");
-  Operand oa{a, 0, rows_cap, K, K, 1, rows_cap * K};
-  Operand ob{w, 0, N, K, K, E, N * K};   // W (E, N, K): rows = output columns
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_M; p.N = (int)N; p.K = (int)K; p.num_groups = E;
-  p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = N; p.status = status;
-  Operand d{out, 0, rows_cap, N, N, 1, rows_cap * N};
-  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return expert_linear(a, K, w, tile_expert, poffs, rows_cap, E, N, K, out, N, status, stream);
 }
 
 int b200moe_expert_gram(const void* x, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
@@ -1179,7 +1194,7 @@ int b200moe_expert_linear_axpby(const void* a, const void* w, const void* c, flo
 int b200moe_expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
                             int64_t rows_cap, int E, int64_t K, int64_t N, void* out, int32_t* status,
                             b200moe_stream_t stream) {
-  return expert_linear_t(a, w, tile_expert, poffs, rows_cap, E, K, N, K, out, status, stream);
+  return expert_linear_t(a, K, w, tile_expert, poffs, rows_cap, E, K, N, K, out, N, status, stream);
 }
 
 int b200moe_expert_linear_push(const void* a, const void* w, int w_kn, const int32_t* tile_expert, const int32_t* poffs,
@@ -1218,8 +1233,8 @@ int b200moe_expert_down_dgrad_act(const void* grad_eo, const void* down_proj, co
                                   const int32_t* act_codes, const int32_t* tile_expert, const int32_t* poffs,
                                   int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I,
                                   void* grad_gate_up, int32_t* status, b200moe_stream_t stream) {
-  return ::b200moe::down_dgrad(grad_eo, down_proj, gate_up, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, grad_gate_up,
-                               nullptr, status, stream);
+  return expert_down_dgrad(grad_eo, H, down_proj, gate_up, 2 * I, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, grad_gate_up,
+                           nullptr, status, stream);
 }
 
 int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_proj, const int32_t* tile_expert,
@@ -1231,22 +1246,7 @@ int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_p
 
 int b200moe_expert_wgrad(const void* A, const void* B, const int32_t* poffs, const int32_t* counts, int64_t rows_cap,
                          int E, int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
-  B200_CHECK_ARG(A && B && poffs && out, B200MOE_E_NULL, "expert_wgrad: null pointer");
-  B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_wgrad: E = %d", E);
-  B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
-                 "expert_wgrad: rows_cap = %lld must be a positive multiple of %d", (long long)rows_cap, B200MOE_TILE_M);
-  CHECK_DIM8(Na); CHECK_DIM8(Nb); CHECK_I32(Na); CHECK_I32(Nb);
-  B200_CHECK_ARG(aligned16(out), B200MOE_E_ALIGN, "expert_wgrad: output not aligned");
-  Operand a{A, 1, Na, rows_cap, Na, 1, rows_cap * Na};
-  Operand b{B, 1, Nb, rows_cap, Nb, 1, rows_cap * Nb};
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)Na; p.N = (int)Nb; p.K = (int)rows_cap;
-  p.num_groups = E; p.poffs = poffs; p.counts = counts; p.D = out; p.ldd = Nb; p.d_group_stride = Na * Nb;
-  p.status = status;
-  const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
-  Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
-  return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn)),
-                                (cudaStream_t)stream);
+  return expert_wgrad(A, Na, B, Nb, poffs, counts, rows_cap, E, Na, Nb, out, status, stream);
 }
 
 }  // extern "C"

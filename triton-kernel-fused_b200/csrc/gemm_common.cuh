@@ -34,6 +34,7 @@ struct GemmParams {
   long long d_group_stride;  // GROUPED_K: elements between D[e] and D[e+1]
   void* aux;                 // SwiGLU: inter (rows, I); GLU_BWD: saved gate_up (rows, 2I); AXPBY: C (rows, N)
   int I;
+  long long ld2, ldi;        // elements between rows of gate_up and its gradient (the up half I further), of inter
   // GROUPED_M with equal square groups (sym_rows rows and N = sym_rows columns each) whose result is symmetric:
   // only the tiles that reach the upper triangle of each group are computed (0 = all tiles); with sym_mirror the
   // epilogue also stores every chunk of a tile right of the diagonal tile a second time, transposed, so the

@@ -163,7 +163,7 @@ __device__ __forceinline__ void glu_fwd_row(const uint4 (&g)[VPT], const uint4 (
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 glu_fwd_vec_kernel(const uint4* gate_up, const int* tile_expert, const int* codes, const float* params,
-                   const int* total_rows, int nvec, uint4* inter) {
+                   const int* total_rows, int nvec, int pitch2, uint4* inter, int pitch) {
   grid_dep_begin();
   constexpr int RPB = kRowThreads / TPR;   // rows a CTA works on at a time; divides the 256-row tile
   __shared__ float red[kRowThreads / 32];
@@ -177,14 +177,14 @@ glu_fwd_vec_kernel(const uint4* gate_up, const int* tile_expert, const int* code
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c = t + TPR * i;
-      g[i] = c < n ? gate_up[r * (2LL * nvec) + c] : make_uint4(0u, 0u, 0u, 0u);
-      u[i] = c < n ? gate_up[r * (2LL * nvec) + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+      g[i] = c < n ? gate_up[r * pitch2 + c] : make_uint4(0u, 0u, 0u, 0u);
+      u[i] = c < n ? gate_up[r * pitch2 + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
     }
     const int e = tile_expert[r0 / B200MOE_TILE_M];
     const int code = codes[e];
     const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
     const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
-    uint4* dst = inter + r * nvec;
+    uint4* dst = inter + r * pitch;
     switch (code) {                        // uniform over the CTA
       case 1: glu_fwd_row<1, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
       case 2: glu_fwd_row<2, TPR, VPT>(g, u, dst, t, n, alpha, gamma, red); break;
@@ -251,7 +251,7 @@ __device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (
 
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(kRowThreads)
-glu_bwd_vec_kernel(const uint4* grad_inter, const uint4* gate_up, const int* tile_expert, const int* codes,
+glu_bwd_vec_kernel(const uint4* grad_inter, int pitch, const uint4* gate_up, int pitch2, const int* tile_expert, const int* codes,
                    const float* params, const int* total_rows, int nvec, uint4* grad_gate_up, float* row_da,
                    float* row_dg) {
   grid_dep_begin();
@@ -267,15 +267,15 @@ glu_bwd_vec_kernel(const uint4* grad_inter, const uint4* gate_up, const int* til
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int c = t + TPR * i;
-      g[i] = c < n ? gate_up[r * (2LL * nvec) + c] : make_uint4(0u, 0u, 0u, 0u);
-      u[i] = c < n ? gate_up[r * (2LL * nvec) + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
-      go[i] = c < n ? grad_inter[r * nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+      g[i] = c < n ? gate_up[r * pitch2 + c] : make_uint4(0u, 0u, 0u, 0u);
+      u[i] = c < n ? gate_up[r * pitch2 + nvec + c] : make_uint4(0u, 0u, 0u, 0u);
+      go[i] = c < n ? grad_inter[r * pitch + c] : make_uint4(0u, 0u, 0u, 0u);
     }
     const int e = tile_expert[r0 / B200MOE_TILE_M];
     const int code = codes[e];
     const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
     const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
-    uint4* gg = grad_gate_up + r * (2LL * nvec);
+    uint4* gg = grad_gate_up + r * pitch2;
     uint4* gu = gg + nvec;
     float da = 0.0f, dg = 0.0f;
     switch (code) {                        // uniform over the CTA
@@ -302,7 +302,7 @@ glu_bwd_vec_kernel(const uint4* grad_inter, const uint4* gate_up, const int* til
 // ---------------------------------------------------------------------------- one value per thread
 __global__ void __launch_bounds__(256)
 glu_fwd_rows_kernel(const __nv_bfloat16* gate_up, const int* tile_expert, const int* codes, const float* params,
-                    const int* total_rows, int I, __nv_bfloat16* inter) {
+                    const int* total_rows, int I, long long ld2, __nv_bfloat16* inter, long long ldi) {
   grid_dep_begin();
   __shared__ float red[8];
   const int total = *total_rows;
@@ -311,7 +311,7 @@ glu_fwd_rows_kernel(const __nv_bfloat16* gate_up, const int* tile_expert, const 
     const int code = codes[e];
     const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
     const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
-    const __nv_bfloat16* g = gate_up + r * (2LL * I);
+    const __nv_bfloat16* g = gate_up + r * ld2;
     const __nv_bfloat16* u = g + I;
     float inv_r = 1.0f;
     if (is_norm(code)) {
@@ -326,14 +326,14 @@ glu_fwd_rows_kernel(const __nv_bfloat16* gate_up, const int* tile_expert, const 
     for (int c = threadIdx.x; c < I; c += blockDim.x) {
       const float gate = __bfloat162float(g[c]);
       const float up = __bfloat162float(u[c]);
-      inter[r * static_cast<long long>(I) + c] = __float2bfloat16_rn(act_value(code, gate, gate * inv_r, alpha, gamma) * up);
+      inter[r * ldi + c] = __float2bfloat16_rn(act_value(code, gate, gate * inv_r, alpha, gamma) * up);
     }
   }
 }
 
 // grad_gate_up = [grad_gate | grad_up]; optional per-row d(alpha), d(gamma) for learnable SiTU.
 __global__ void __launch_bounds__(256)
-glu_bwd_rows_kernel(const __nv_bfloat16* grad_inter, const __nv_bfloat16* gate_up, const int* tile_expert,
+glu_bwd_rows_kernel(const __nv_bfloat16* grad_inter, long long ldi, const __nv_bfloat16* gate_up, long long ld2, const int* tile_expert,
                     const int* codes, const float* params, const int* total_rows, int I, __nv_bfloat16* grad_gate_up,
                     float* row_da, float* row_dg) {
   grid_dep_begin();
@@ -344,10 +344,10 @@ glu_bwd_rows_kernel(const __nv_bfloat16* grad_inter, const __nv_bfloat16* gate_u
     const int code = codes[e];
     const float alpha = (params != nullptr && code == 5) ? params[2 * e] : 1.0f;
     const float gamma = (params != nullptr && code == 5) ? params[2 * e + 1] : 1.0f;
-    const __nv_bfloat16* g = gate_up + r * (2LL * I);
+    const __nv_bfloat16* g = gate_up + r * ld2;
     const __nv_bfloat16* u = g + I;
-    const __nv_bfloat16* go = grad_inter + r * static_cast<long long>(I);
-    __nv_bfloat16* gg = grad_gate_up + r * (2LL * I);
+    const __nv_bfloat16* go = grad_inter + r * ldi;
+    __nv_bfloat16* gg = grad_gate_up + r * ld2;
     const bool norm = is_norm(code);
     float rr = 1.0f, S = 0.0f;
     if (norm) {
@@ -447,7 +447,7 @@ expert_row_sums_kernel(const float* row_da, const float* row_dg, const int* poff
 template <int TPR>
 __global__ void __launch_bounds__(256)
 special_rows_kernel(const uint4* src, const int* tile_expert, const int* codes, const int* poffs, int first_special,
-                    int num_experts, int vec_per_row, uint4* dst) {
+                    int num_experts, int vec_per_row, int pitch, uint4* dst) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int r0 = poffs[first_special], r1 = poffs[num_experts];
@@ -455,7 +455,7 @@ special_rows_kernel(const uint4* src, const int* tile_expert, const int* codes, 
        r += static_cast<long long>(gridDim.x) * G) {
     const bool copy = codes[tile_expert[r / B200MOE_TILE_M]] == 3;
     for (int c = threadIdx.x % TPR; c < vec_per_row; c += TPR)
-      dst[r * vec_per_row + c] = copy ? src[r * vec_per_row + c] : make_uint4(0u, 0u, 0u, 0u);
+      dst[r * pitch + c] = copy ? src[r * pitch + c] : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -487,15 +487,8 @@ static void by_row_width(int nvec, F f) {
   else f(std::integral_constant<int, 256>(), std::integral_constant<int, 4>());
 }
 
-}  // namespace b200moe
-
-using namespace b200moe;
-
-extern "C" {
-
-int b200moe_glu_fwd_rows(const void* gate_up, const int32_t* tile_expert, const int32_t* act_codes,
-                         const float* act_params, const int32_t* total_rows, int64_t rows_cap, int64_t I, void* inter,
-                         b200moe_stream_t stream) {
+int glu_fwd_rows(const void* gate_up, int64_t ld2, const int32_t* tile_expert, const int32_t* act_codes, const float* act_params,
+                 const int32_t* total_rows, int64_t rows_cap, int64_t I, void* inter, int64_t ldi, b200moe_stream_t stream) {
   B200_CHECK_ARG(gate_up && tile_expert && act_codes && total_rows && inter, B200MOE_E_NULL, "glu_fwd_rows: null pointer");
   B200_CHECK_ARG(I > 0, B200MOE_E_BAD_SHAPE, "glu_fwd_rows: I = %lld", (long long)I);
   if (rows_cap <= 0) return 0;
@@ -505,19 +498,20 @@ int b200moe_glu_fwd_rows(const void* gate_up, const int32_t* tile_expert, const 
     by_row_width(nvec, [&](auto tpr, auto vpt) {
       err = launch_chained(glu_fwd_vec_kernel<tpr.value, vpt.value>, rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)),
                            kRowThreads, 0, (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes,
-                           act_params, total_rows, nvec, reinterpret_cast<uint4*>(inter));
+                           act_params, total_rows, nvec, static_cast<int>(ld2 / 8), reinterpret_cast<uint4*>(inter), static_cast<int>(ldi / 8));
     });
     B200_CUDA(err);
     return 0;
   }
   B200_LAUNCH(glu_fwd_rows_kernel, rows_grid(rows_cap), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert,
-              act_codes, act_params, total_rows, static_cast<int>(I), reinterpret_cast<__nv_bfloat16*>(inter));
+              act_codes, act_params, total_rows, static_cast<int>(I), static_cast<long long>(ld2), reinterpret_cast<__nv_bfloat16*>(inter),
+              static_cast<long long>(ldi));
   return 0;
 }
 
-int b200moe_glu_bwd_rows(const void* grad_inter, const void* gate_up, const int32_t* tile_expert,
-                         const int32_t* act_codes, const float* act_params, const int32_t* total_rows, int64_t rows_cap,
-                         int64_t I, void* grad_gate_up, float* row_da, float* row_dg, b200moe_stream_t stream) {
+int glu_bwd_rows(const void* grad_inter, int64_t ldi, const void* gate_up, int64_t ld2, const int32_t* tile_expert, const int32_t* act_codes,
+                 const float* act_params, const int32_t* total_rows, int64_t rows_cap, int64_t I, void* grad_gate_up, float* row_da, float* row_dg,
+                 b200moe_stream_t stream) {
   B200_CHECK_ARG(grad_inter && gate_up && tile_expert && act_codes && total_rows && grad_gate_up, B200MOE_E_NULL,
                  "glu_bwd_rows: null pointer");
   B200_CHECK_ARG((row_da == nullptr) == (row_dg == nullptr), B200MOE_E_NULL, "glu_bwd_rows: row_da and row_dg go together");
@@ -529,16 +523,51 @@ int b200moe_glu_bwd_rows(const void* grad_inter, const void* gate_up, const int3
     by_row_width(nvec, [&](auto tpr, auto vpt) {
       err = launch_chained(glu_bwd_vec_kernel<tpr.value, vpt.value>, rows_grid(ceil_div64(rows_cap, kRowThreads / tpr.value)),
                            kRowThreads, 0, (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(grad_inter),
-                           reinterpret_cast<const uint4*>(gate_up), tile_expert, act_codes, act_params, total_rows, nvec,
+                           static_cast<int>(ldi / 8), reinterpret_cast<const uint4*>(gate_up), static_cast<int>(ld2 / 8), tile_expert, act_codes, act_params, total_rows, nvec,
                            reinterpret_cast<uint4*>(grad_gate_up), row_da, row_dg);
     });
     B200_CUDA(err);
     return 0;
   }
   B200_LAUNCH(glu_bwd_rows_kernel, rows_grid(rows_cap), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(grad_inter),
-              reinterpret_cast<const __nv_bfloat16*>(gate_up), tile_expert, act_codes, act_params, total_rows, static_cast<int>(I),
+              static_cast<long long>(ldi), reinterpret_cast<const __nv_bfloat16*>(gate_up), static_cast<long long>(ld2), tile_expert, act_codes, act_params, total_rows, static_cast<int>(I),
               reinterpret_cast<__nv_bfloat16*>(grad_gate_up), row_da, row_dg);
   return 0;
+}
+
+int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special, int num_experts,
+                 int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream) {
+  B200_CHECK_ARG(src && tile_expert && act_codes && poffs && dst, B200MOE_E_NULL, "special_rows: null pointer");
+  B200_CHECK_ARG(H > 0 && H % 8 == 0 && first_special >= 0 && first_special <= num_experts, B200MOE_E_BAD_SHAPE,
+                 "special_rows: H = %lld, first_special = %d, num_experts = %d", (long long)H, first_special, num_experts);
+  B200_CHECK_ARG(aligned16(src) && aligned16(dst), B200MOE_E_ALIGN, "special_rows: pointers must be 16-byte aligned");
+  if (rows_cap <= 0 || first_special == num_experts) return 0;
+  cudaError_t err = cudaSuccess;
+  by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
+    err = launch_chained(special_rows_kernel<tpr.value>, rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0,
+                         (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs,
+                         first_special, num_experts, static_cast<int>(H / 8), static_cast<int>(ldh / 8), reinterpret_cast<uint4*>(dst));
+  });
+  B200_CUDA(err);
+  return 0;
+}
+
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" {
+
+int b200moe_glu_fwd_rows(const void* gate_up, const int32_t* tile_expert, const int32_t* act_codes,
+                         const float* act_params, const int32_t* total_rows, int64_t rows_cap, int64_t I, void* inter,
+                         b200moe_stream_t stream) {
+  return glu_fwd_rows(gate_up, 2 * I, tile_expert, act_codes, act_params, total_rows, rows_cap, I, inter, I, stream);
+}
+
+int b200moe_glu_bwd_rows(const void* grad_inter, const void* gate_up, const int32_t* tile_expert,
+                         const int32_t* act_codes, const float* act_params, const int32_t* total_rows, int64_t rows_cap,
+                         int64_t I, void* grad_gate_up, float* row_da, float* row_dg, b200moe_stream_t stream) {
+  return glu_bwd_rows(grad_inter, I, gate_up, 2 * I, tile_expert, act_codes, act_params, total_rows, rows_cap, I, grad_gate_up, row_da, row_dg, stream);
 }
 
 int b200moe_expert_row_sums(const float* row_da, const float* row_dg, const int32_t* poffs, int E, float* out,
@@ -552,19 +581,7 @@ int b200moe_expert_row_sums(const float* row_da, const float* row_dg, const int3
 int b200moe_special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs,
                          int first_special, int num_experts, int64_t H, int64_t rows_cap, void* dst,
                          b200moe_stream_t stream) {
-  B200_CHECK_ARG(src && tile_expert && act_codes && poffs && dst, B200MOE_E_NULL, "special_rows: null pointer");
-  B200_CHECK_ARG(H > 0 && H % 8 == 0 && first_special >= 0 && first_special <= num_experts, B200MOE_E_BAD_SHAPE,
-                 "special_rows: H = %lld, first_special = %d, num_experts = %d", (long long)H, first_special, num_experts);
-  B200_CHECK_ARG(aligned16(src) && aligned16(dst), B200MOE_E_ALIGN, "special_rows: pointers must be 16-byte aligned");
-  if (rows_cap <= 0 || first_special == num_experts) return 0;
-  cudaError_t err = cudaSuccess;
-  by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
-    err = launch_chained(special_rows_kernel<tpr.value>, rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0,
-                         (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs,
-                         first_special, num_experts, static_cast<int>(H / 8), reinterpret_cast<uint4*>(dst));
-  });
-  B200_CUDA(err);
-  return 0;
+  return special_rows(src, tile_expert, act_codes, poffs, first_special, num_experts, H, H, rows_cap, dst, stream);
 }
 
 }  // extern "C"

@@ -218,14 +218,14 @@ static int launch_permute(const long long* idx, long long M, int E, int* hist, i
 // whole CTA a row 20 000 tokens of H 256, top-8 take 84 us (36 here), 16 384 of H 512, top-2 21 us (11 here).
 template <int TPR>
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const uint4* x, const int* row_slot, const int* total_rows, int k, int vec_per_row, uint4* x_s) {
+gather_rows_kernel(const uint4* x, const int* row_slot, const int* total_rows, int k, int vec_per_row, int pitch, uint4* x_s) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int total = *total_rows;
   for (long long r = static_cast<long long>(blockIdx.x) * G + threadIdx.x / TPR; r < total;
        r += static_cast<long long>(gridDim.x) * G) {
     const int slot = row_slot[r];
-    uint4* dst = x_s + r * vec_per_row;
+    uint4* dst = x_s + r * pitch;
     const uint4* src = x + static_cast<long long>(slot / k) * vec_per_row;
     for (int c = threadIdx.x % TPR; c < vec_per_row; c += TPR) dst[c] = slot < 0 ? make_uint4(0u, 0u, 0u, 0u) : src[c];
   }
@@ -255,6 +255,25 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
                 row_slot, tile_expert, order, slot_pos, counts_out, reinterpret_cast<long long*>(load), rows, status, (cudaStream_t)stream);
 }
 
+int gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H, int64_t ldh, int64_t rows_cap, void* x_s,
+                b200moe_stream_t stream) {
+  B200_CHECK_ARG(x && row_slot && total_rows && x_s, B200MOE_E_NULL, "gather_rows: null pointer");
+  B200_CHECK_ARG(H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE, "gather_rows: H = %lld must be a multiple of 8", (long long)H);
+  B200_CHECK_ARG(k >= 1, B200MOE_E_BAD_SHAPE, "gather_rows: k = %d", k);
+  B200_CHECK_ARG(aligned16(x) && aligned16(x_s), B200MOE_E_ALIGN, "gather_rows: pointers must be 16-byte aligned");
+  if (rows_cap <= 0) return 0;
+  cudaError_t err = cudaSuccess;
+  by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
+    constexpr int G = 256 / tpr.value;
+    const long long grid = std::min<long long>((rows_cap + G - 1) / G, static_cast<long long>(num_sms()) * 16);
+    err = launch_chained(gather_rows_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
+                         reinterpret_cast<const uint4*>(x), row_slot, total_rows, k, static_cast<int>(H / 8), static_cast<int>(ldh / 8),
+                         reinterpret_cast<uint4*>(x_s));
+  });
+  B200_CUDA(err);
+  return 0;
+}
+
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -282,21 +301,7 @@ int b200moe_permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* 
 
 int b200moe_gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,
                         int64_t rows_cap, void* x_s, b200moe_stream_t stream) {
-  B200_CHECK_ARG(x && row_slot && total_rows && x_s, B200MOE_E_NULL, "gather_rows: null pointer");
-  B200_CHECK_ARG(H > 0 && H % 8 == 0, B200MOE_E_BAD_SHAPE, "gather_rows: H = %lld must be a multiple of 8", (long long)H);
-  B200_CHECK_ARG(k >= 1, B200MOE_E_BAD_SHAPE, "gather_rows: k = %d", k);
-  B200_CHECK_ARG(aligned16(x) && aligned16(x_s), B200MOE_E_ALIGN, "gather_rows: pointers must be 16-byte aligned");
-  if (rows_cap <= 0) return 0;
-  cudaError_t err = cudaSuccess;
-  by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
-    constexpr int G = 256 / tpr.value;
-    const long long grid = std::min<long long>((rows_cap + G - 1) / G, static_cast<long long>(num_sms()) * 16);
-    err = launch_chained(gather_rows_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
-                         reinterpret_cast<const uint4*>(x), row_slot, total_rows, k, static_cast<int>(H / 8),
-                         reinterpret_cast<uint4*>(x_s));
-  });
-  B200_CUDA(err);
-  return 0;
+  return gather_rows(x, row_slot, total_rows, k, H, H, rows_cap, x_s, stream);
 }
 
 }  // extern "C"
