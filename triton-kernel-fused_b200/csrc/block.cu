@@ -375,7 +375,7 @@ int b200moe_conv_router_forward(const void* x, const void* weight, const float* 
   if (rc) return rc;
   const bool in_place = conv_in_place(B, S, H, E, taps);
   B200_CHECK_ARG(x && weight && weight_rows && logits && (ws || in_place), B200MOE_E_NULL, "conv_router_forward: null pointer");
-  RUN("conv_weight_rows", 1, b200moe_conv_weight_rows(weight, E, H, taps, 0, weight_rows, stream));
+  RUN("conv_weight_rows", 1, conv_weight_rows(weight, E, H, taps, 0, weight_rows, counts, stream));
   if (in_place) {
     RUN("conv_gemm_logits", 1, b200moe_conv_gemm_logits(x, weight_rows, logits, B, S, H, E, taps, status, stream));
   } else {
@@ -386,7 +386,7 @@ int b200moe_conv_router_forward(const void* x, const void* weight, const float* 
     RUN("conv_unfold", 1, b200moe_conv_unfold(x, B, S, H, taps, xu, stream));
     RUN("gemm_nt", 1, b200moe_gemm_nt(xu, wf, logits, B * S, E, taps * H, status, stream));
   }
-  RUN("router_topk_fwd", 1, b200moe_router_topk_fwd(logits, B200MOE_LOGITS_BF16, bias, B * S, E, k, norm_topk, scale, idx, w, counts, stream));
+  RUN("router_topk_fwd", 1, router_topk_fwd(logits, B200MOE_LOGITS_BF16, bias, B * S, E, k, norm_topk, scale, idx, w, counts, true, stream));
   return 0;
 }
 

@@ -72,6 +72,11 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
                   size_t ws_bytes, int32_t* counts_out, int64_t* load, const RowWeights& rows, int32_t* status, b200moe_stream_t stream);
 
+// router.cu.  counts (nullable): cleared by conv_weight_rows; counts_cleared: some kernel before has done so
+int conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, int32_t* counts, b200moe_stream_t stream);
+int router_topk_fwd(const void* input, int input_kind, const float* bias, int64_t T, int E, int k, int norm_topk, float scale, int64_t* idx,
+                    float* w, int32_t* counts, bool counts_cleared, b200moe_stream_t stream);
+
 // combine.cu: grad_w[slot] = sum over `parts` of dots[part][row], dots (parts, ld)
 int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, const int32_t* total_rows, float* grad_w, b200moe_stream_t stream);
 

@@ -13,8 +13,8 @@
 //             MMAs for both, each CTA's TMEM holds its 128 rows of the accumulator.  This halves
 //             the L2 -> shared-memory traffic per FLOP and leaves room for 6 stages instead of 4.
 //
-// Warp roles (320 threads): warp 0 = TMA producer and warp 1 = TMEM owner + MMA issuer (an elected
-// thread each), warps 2-9 = epilogue (TMEM lane quarter = warp_id % 4, two warps per quarter split the
+// Warp roles (320 threads, 352 with single-CTA tiles): warp 0 = TMA producer and warp 1 = TMEM owner + MMA issuer (an elected
+// thread each), warp 10 = TMA producer of B (single-CTA tiles only), warps 2-9 = epilogue (TMEM lane quarter = warp_id % 4, two warps per quarter split the
 // columns).
 #include <cuda.h>
 #include <stdlib.h>
@@ -87,8 +87,14 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
 // WEIGHTED: the GLU epilogues of a block whose rows are weighted where their activations are made (weighted_rows).
+// Single-CTA tiles have two loading warps, one for A and one for B: a k-block's MMAs take 256 cycles there, but one thread's wait, its two
+// boxes and a convolution's coordinates 480 (380 without those), whatever the batch.  Logits of 16 x 1024 positions of H 2048, 64 experts, 4
+// taps (us): one loading warp 35.7, two 29.8, the next stage's barrier asked for ahead 28.6, the convolution in a loop of its own 24.7; of
+// 1 x 1024 positions 34.2 -> 23.4.  Products of few k-blocks are as fast as before.
+__host__ __device__ constexpr int gemm_threads(int ctas) { return ctas == 1 ? kThreads + 32 : kThreads; }
+
 template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(gemm_threads(CTAS), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
             const GemmParams p) {
@@ -98,6 +104,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   constexpr int TM = C::TILE_ROWS;
   constexpr int NSTAGE = C::NSTAGE;
   constexpr int BNC = BN / CTAS;                          // B columns staged by one CTA
+  constexpr bool kPeek = CTAS == 1;                       // the next stage's barrier is asked for while this one's boxes / MMAs go out
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -158,12 +165,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int total = total_tiles(p, TN, TM, WINDOW);
   const int row_base = (WINDOW && p.row_hi > 0) ? p.row_lo : 0;
 
-  if (warp == 0) {
+  if (warp == 0 || warp >= 2 + kEpiWarps) {
     // ------------------------------------------------------------------ TMA producer (each CTA)
-    if (elect_one()) {
+    auto produce = [&](auto do_a, auto do_b) {
+      constexpr bool A = do_a.value, B = do_b.value;
       int s = 0;
       uint32_t ph = 0;
-      bool ok = true;
+      bool ok = true, ready = false;
       for (int tile = first_tile; tile < total && ok; tile += tile_step) {
         const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
         const int gB = (p.sched == SCHED_GROUPED_M) ? t.g : 0;
@@ -171,46 +179,75 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         // a narrower last pair tile: each CTA supplies half of its columns of B, the first ones of its (still
         // BN/2 wide) staging tile
         const int bstep = (CTAS == 2) ? pair_cols<BN, EPI>(p, t.n0) / 2 : BNC;
-        // coordinates of the A box (K-major case) and of the B boxes; a convolution operand (see GemmParams::conv_taps)
-        // replaces the flat row by (position + shift, batch).  Its divisions are done once per tile, the k-loop only counts
-        // (logits of x (16, 1024, 2048), 64 experts, 4 taps: 56 us with the divisions in the k-loop, 45 us without).
-        int a_c0 = t.k0, a_c1 = m0, a_c2 = 0, b_n0 = t.n0, b_k = t.k0, b_g = gB, b_c0 = t.k0;
-        if (CONV && p.conv_taps > 0) {
-          if (p.sched == SCHED_DENSE) {
-            a_c2 = t.g;                                            // batch
-            a_c1 = m0 - p.conv_sign * (p.conv_taps - 1);
-          } else {
-            const int tap = t.n0 / p.conv_C;
-            b_n0 = t.n0 - tap * p.conv_C;
-            b_g = t.k0 / p.conv_S;
-            b_k = t.k0 - b_g * p.conv_S + tap - (p.conv_taps - 1);
-          }
+        // coordinates of the B boxes; a convolution operand (see GemmParams::conv_taps) replaces the flat row by (position + shift,
+        // batch).  Its divisions are done once per tile, the k-loop only counts.
+        int b_n0 = t.n0, b_k = t.k0, b_g = gB;
+        if (CONV && p.conv_taps > 0 && p.sched != SCHED_DENSE) {
+          const int tap = t.n0 / p.conv_C;
+          b_n0 = t.n0 - tap * p.conv_C;
+          b_g = t.k0 / p.conv_S;
+          b_k = t.k0 - b_g * p.conv_S + tap - (p.conv_taps - 1);
         }
+        if constexpr (CONV && CTAS == 1)
+          if (p.conv_taps > 0 && p.sched == SCHED_DENSE) {       // tap by tap, with nothing in the loop but its box
+            const int pos0 = m0 - p.conv_sign * (p.conv_taps - 1);
+            for (int tap = 0; tap < p.conv_taps && ok; ++tap) {
+              for (int c0 = 0; c0 < p.conv_C; c0 += BK) {
+                if (!ready && !mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
+                  ok = false;
+                  break;
+                }
+                const uint32_t full = bar_full + 8 * s, sa = smem_u32(smem + s * C::STAGE_BYTES);
+                if (++s == NSTAGE) {
+                  s = 0;
+                  ph ^= 1;
+                }
+                ready = mbar_test_wait(bar_empty + 8 * s, ph ^ 1);
+                if constexpr (A) {
+                  mbar_arrive_expect_tx(full, C::STAGE_BYTES);
+                  tma_load_3d(sa, &tmA, full, c0, pos0 + p.conv_sign * tap, t.g);
+                }
+                if constexpr (B) {
+                  const uint32_t sb = sa + C::A_BYTES;
+                  if (!p.b_mn) {
+                    tma_load_3d(sb, &tmB, full, p.conv_b_taps ? c0 : tap * p.conv_C + c0, t.n0, p.conv_b_taps ? tap : 0);
+                  } else {
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) tma_load_3d(sb + j * (64 * BK * 2), &tmB, full, t.n0 + 64 * j, tap * p.conv_C + c0, 0);
+                  }
+                }
+              }
+            }
+            continue;
+          }
         for (int kb = 0; kb < t.nkb; ++kb) {
-          if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
+          if (!ready && !mbar_wait(bar_empty + 8 * s, ph ^ 1, abort_flag, ST_WAIT_PRODUCER)) {
             ok = false;
             break;
           }
+          if constexpr (kPeek) ready = mbar_test_wait(bar_empty + (s + 1 == NSTAGE ? 0 : 8 * (s + 1)), s + 1 == NSTAGE ? ph : ph ^ 1);
           const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
           const uint32_t sb = sa + C::A_BYTES;
           const int kk = t.k0 + kb * BK;
-          if (!CONV || p.conv_taps == 0) a_c0 = b_k = b_c0 = kk;
+          if (!CONV || p.conv_taps == 0) b_k = kk;
           if constexpr (CTAS == 1) {
             const uint32_t full = bar_full + 8 * s;
-            mbar_arrive_expect_tx(full, C::STAGE_BYTES);
-            if (!p.a_mn) {
-              tma_load_3d(sa, &tmA, full, a_c0, a_c1, a_c2);  // box {64 k, 128 rows}
+            if constexpr (A) mbar_arrive_expect_tx(full, C::STAGE_BYTES);
+            if (!A) {
+            } else if (!p.a_mn) {
+              tma_load_3d(sa, &tmA, full, kk, m0, 0);  // box {64 k, 128 rows}
             } else {
 #pragma unroll
               for (int j = 0; j < BM / 64; ++j)  // boxes {64 mn, 64 k-rows}
                 tma_load_3d(sa + j * (64 * BK * 2), &tmA, full, m0 + 64 * j, kk, 0);
             }
-            if constexpr (EPI == EPI_SWIGLU) {
+            if constexpr (!B) {
+            } else if constexpr (EPI == EPI_SWIGLU) {
               // gate rows [n0, n0+BN/2) of W[e] then up rows of the same range: dims {H, I, 2E}
               tma_load_3d(sb, &tmB, full, kk, t.n0, 2 * gB);
               tma_load_3d(sb + (BN / 2) * BK * 2, &tmB, full, kk, t.n0, 2 * gB + 1);
             } else if (!p.b_mn) {
-              tma_load_3d(sb, &tmB, full, b_c0, t.n0, b_g);  // box {64 k, BN rows}
+              tma_load_3d(sb, &tmB, full, kk, t.n0, b_g);  // box {64 k, BN rows}
             } else {
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
@@ -221,7 +258,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             const uint32_t full = mapa_shared(bar_full + 8 * s, 0);
             if (cta_rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2 * C::STAGE_BYTES);
             if (!p.a_mn) {
-              tma_load_3d_pair(sa, &tmA, full, a_c0, a_c1, a_c2);
+              tma_load_3d_pair(sa, &tmA, full, kk, m0, 0);
             } else {
 #pragma unroll
               for (int j = 0; j < BM / 64; ++j)
@@ -231,7 +268,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               // leader stages the gate rows, the peer the up rows of I-columns [n0, n0+128)
               tma_load_3d_pair(sb, &tmB, full, kk, t.n0, 2 * gB + static_cast<int>(cta_rank));
             } else if (!p.b_mn) {
-              tma_load_3d_pair(sb, &tmB, full, b_c0, t.n0 + bstep * static_cast<int>(cta_rank), b_g);
+              tma_load_3d_pair(sb, &tmB, full, kk, t.n0 + bstep * static_cast<int>(cta_rank), b_g);
             } else {
 #pragma unroll
               for (int j = 0; j < BNC / 64; ++j)
@@ -239,25 +276,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                                  b_n0 + bstep * static_cast<int>(cta_rank) + 64 * j, b_k, b_g);
             }
           }
-          if (CONV && p.conv_taps > 0) {       // the next k-block's coordinates
-            if (p.sched == SCHED_DENSE) {
-              a_c0 += BK;
-              b_c0 += BK;
-              b_k += BK;
-              if (a_c0 >= p.conv_C) {          // next tap
-                a_c0 = 0;
-                a_c1 += p.conv_sign;
-                if (p.conv_b_taps) {
-                  b_c0 = 0;
-                  ++b_g;
-                }
-              }
-            } else {
-              b_k += BK;
-              if (kk + BK - b_g * p.conv_S >= p.conv_S) {   // next batch
-                ++b_g;
-                b_k -= p.conv_S;
-              }
+          if (CONV && p.conv_taps > 0) {       // the next k-block's rows of B
+            b_k += BK;
+            if (kk + BK - b_g * p.conv_S >= p.conv_S) {   // next batch
+              ++b_g;
+              b_k -= p.conv_S;
             }
           }
           if (++s == NSTAGE) {
@@ -266,6 +289,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
+    };
+    if (elect_one()) {
+      if constexpr (CTAS == 2) produce(std::true_type(), std::true_type());
+      else if (warp == 0) produce(std::true_type(), std::false_type());
+      else produce(std::false_type(), std::true_type());
     }
     grid_dep_launch();   // the last loads are on their way
   } else if (warp == 1) {
@@ -278,7 +306,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t a_kstep = p.a_mn ? 2048 : 32, b_kstep = p.b_mn ? 2048 : 32;
       int s = 0, it = 0;
       uint32_t ph = 0;
-      bool ok = true;
+      bool ok = true, ready = false;
       for (int tile = first_tile; tile < total && ok; tile += tile_step, ++it) {
         const Tile t = get_tile(p, tile, TN, TM, 64, order, row_base, CONV);
         const int buf = it & 1;
@@ -287,10 +315,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const uint32_t d_tmem = tmem_base + buf * BN;
         const uint32_t idesc = umma_idesc_bf16(CTAS == 2 ? pair_cols<BN, EPI>(p, t.n0) : BN, p.a_mn, p.b_mn, TM);
         for (int kb = 0; kb < t.nkb; ++kb) {
-          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
+          if (!ready && !mbar_wait(bar_full + 8 * s, ph, abort_flag, ST_WAIT_MMA_FULL)) {
             ok = false;
             break;
           }
+          if constexpr (kPeek) ready = mbar_test_wait(bar_full + (s + 1 == NSTAGE ? 0 : 8 * (s + 1)), s + 1 == NSTAGE ? ph ^ 1 : ph);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
           const uint32_t sb = sa + C::A_BYTES;
@@ -686,7 +715,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensor
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, units * CTAS, kThreads, C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 

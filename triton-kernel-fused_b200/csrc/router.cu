@@ -149,10 +149,13 @@ router_topk_bwd_kernel(const void* logits, const long long* idx, const float* gr
   }
 }
 
-// w (E, H, taps) -> wt (taps, E, H), wt[j, e, h] = w[e, h, j] (the operand of the conv router's products), or (E, taps, H)
+// w (E, H, taps) -> wt (taps, E, H), wt[j, e, h] = w[e, h, j] (the operand of the conv router's products), or (E, taps, H).  counts (E,
+// nullable) are cleared for the top-k kernel further on: a memset between the two would end their chain of launches (5 us).
 __global__ void __launch_bounds__(256)
-conv_weight_rows_kernel(const __nv_bfloat16* w, int E, int H, int taps, int by_expert, __nv_bfloat16* wt) {
+conv_weight_rows_kernel(const __nv_bfloat16* w, int E, int H, int taps, int by_expert, __nv_bfloat16* wt, int* counts) {
   grid_dep_begin();
+  if (counts != nullptr && blockIdx.x == 0)
+    for (int e = threadIdx.x; e < E; e += 256) counts[e] = 0;
   const long long n = static_cast<long long>(E) * H;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
     const long long e = i / H, h = i - e * H;
@@ -252,15 +255,21 @@ static cudaError_t launch_topk_bwd(const void* logits, const long long* idx, con
   return err;
 }
 
-}  // namespace b200moe
+static int weight_grid(int64_t n) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(num_sms()) * 8)));
+}
 
-using namespace b200moe;
+int conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, int32_t* counts, b200moe_stream_t stream) {
+  B200_CHECK_ARG(w && wt, B200MOE_E_NULL, "conv_weight_rows: null pointer");
+  B200_CHECK_ARG(E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE, "conv_weight_rows: E = %d, H = %lld, taps = %d", E,
+                 (long long)H, taps);
+  B200_LAUNCH(conv_weight_rows_kernel, weight_grid(E * H), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(w), E,
+              static_cast<int>(H), taps, by_expert, reinterpret_cast<__nv_bfloat16*>(wt), counts);
+  return 0;
+}
 
-extern "C" {
-
-int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias, int64_t T, int E, int k,
-                            int norm_topk, float scale, int64_t* idx, float* w, int32_t* counts,
-                            b200moe_stream_t stream) {
+int router_topk_fwd(const void* input, int input_kind, const float* bias, int64_t T, int E, int k, int norm_topk, float scale, int64_t* idx,
+                    float* w, int32_t* counts, bool counts_cleared, b200moe_stream_t stream) {
   B200_CHECK_ARG(input && idx && w, B200MOE_E_NULL, "router_topk_fwd: null pointer");
   B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
                  "router_topk_fwd: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
@@ -268,7 +277,7 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
                  "router_topk_fwd: top_k = %d must be in 1..min(E=%d, %d)", k, E, B200MOE_MAX_TOPK);
   B200_CHECK_ARG(T >= 0, B200MOE_E_BAD_SHAPE, "router_topk_fwd: T = %lld", (long long)T);
   cudaStream_t st = (cudaStream_t)stream;
-  if (counts != nullptr) B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * E, st));
+  if (counts != nullptr && !counts_cleared) B200_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * E, st));
   if (T == 0) return 0;
   const int grid = grid_for_tokens(T);
   long long* idx_ll = reinterpret_cast<long long*>(idx);
@@ -289,6 +298,18 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
   }
   B200_CUDA(err);
   return 0;
+}
+
+}  // namespace b200moe
+
+using namespace b200moe;
+
+extern "C" {
+
+int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias, int64_t T, int E, int k,
+                            int norm_topk, float scale, int64_t* idx, float* w, int32_t* counts,
+                            b200moe_stream_t stream) {
+  return router_topk_fwd(input, input_kind, bias, T, E, k, norm_topk, scale, idx, w, counts, false, stream);
 }
 
 int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* idx, const float* grad_w, int64_t T,
@@ -329,17 +350,8 @@ int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* g
   return 0;
 }
 
-static int weight_grid(int64_t n) {
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(num_sms()) * 8)));
-}
-
 int b200moe_conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, b200moe_stream_t stream) {
-  B200_CHECK_ARG(w && wt, B200MOE_E_NULL, "conv_weight_rows: null pointer");
-  B200_CHECK_ARG(E >= 1 && H >= 1 && H < (1LL << 31) && taps >= 1, B200MOE_E_BAD_SHAPE, "conv_weight_rows: E = %d, H = %lld, taps = %d", E,
-                 (long long)H, taps);
-  B200_LAUNCH(conv_weight_rows_kernel, weight_grid(E * H), 256, 0, stream, reinterpret_cast<const __nv_bfloat16*>(w), E,
-              static_cast<int>(H), taps, by_expert, reinterpret_cast<__nv_bfloat16*>(wt));
-  return 0;
+  return conv_weight_rows(w, E, H, taps, by_expert, wt, nullptr, stream);
 }
 
 int b200moe_conv_weight_grad(const float* P, int64_t slices, int E, int64_t H, int taps, void* grad_w,
