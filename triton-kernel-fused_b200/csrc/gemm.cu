@@ -150,7 +150,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
-  grid_dep_wait();
+  if (p.early) grid_dep_early();
+  else grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
   __syncthreads();
@@ -178,7 +179,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int m0 = t.m0 + BM * static_cast<int>(cta_rank);
         // a narrower last pair tile: each CTA supplies half of its columns of B, the first ones of its (still
         // BN/2 wide) staging tile
-        const int bstep = (CTAS == 2) ? pair_cols<BN, EPI>(p, t.n0) / 2 : BNC;
+        [[maybe_unused]] const int bstep = (CTAS == 2) ? pair_cols<BN, EPI>(p, t.n0) / 2 : BNC;
         // coordinates of the B boxes; a convolution operand (see GemmParams::conv_taps) replaces the flat row by (position + shift,
         // batch).  Its divisions are done once per tile, the k-loop only counts.
         int b_n0 = t.n0, b_k = t.k0, b_g = gB;
@@ -685,6 +686,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   }
 
   // ------------------------------------------------------------------ tear-down
+  if (p.early) grid_dep_wait();      // so that this kernel's end is also that of the one before it
   tc_fence_before();
   __syncthreads();
   if constexpr (CTAS == 2) {   // nobody leaves while the peer may still touch it
@@ -902,7 +904,7 @@ int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha
 }
 
 int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
-                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream) {
+                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int early, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_linear_t", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
   if (rc) return rc;
   B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear_t: null pointer");
@@ -912,6 +914,7 @@ int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* ti
   GemmParams p{};
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)k_live; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = ldo; p.status = status;
+  p.early = early;
   Operand d{out, 0, rows_cap, N, ldo, 1, rows_cap * ldo};
   return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
@@ -1016,7 +1019,7 @@ int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile
 }
 
 int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
-                 int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
+                 int64_t Na, int64_t Nb, void* out, int early, int32_t* status, b200moe_stream_t stream) {
   B200_CHECK_ARG(A && B && poffs && out, B200MOE_E_NULL, "expert_wgrad: null pointer");
   B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_wgrad: E = %d", E);
   B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
@@ -1028,11 +1031,35 @@ int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const i
   GemmParams p{};
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)Na; p.N = (int)Nb; p.K = (int)rows_cap;
   p.num_groups = E; p.poffs = poffs; p.counts = counts; p.D = out; p.ldd = Nb; p.d_group_stride = Na * Nb;
-  p.status = status;
+  p.status = status; p.early = early;
   const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
   Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
   return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn)),
                                 (cudaStream_t)stream);
+}
+
+int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K, int64_t k_chunk, int early, int32_t* status,
+                   b200moe_stream_t stream) {
+  B200_CHECK_ARG(A && B && P, B200MOE_E_NULL, "gemm_tn_splitk: null pointer");
+  CHECK_DIM8(M); CHECK_DIM8(N); CHECK_I32(M); CHECK_I32(N); CHECK_I32(K);
+  B200_CHECK_ARG(k_chunk > 0 && k_chunk % 64 == 0, B200MOE_E_BAD_SHAPE,
+                 "gemm_tn_splitk: k_chunk = %lld must be a positive multiple of 64", (long long)k_chunk);
+  B200_CHECK_ARG(K > 0, B200MOE_E_BAD_SHAPE, "gemm_tn_splitk: K must be positive");
+  B200_CHECK_ARG(aligned16(P), B200MOE_E_ALIGN, "gemm_tn_splitk: P not 16-byte aligned");
+  const long long slices = ceil_div(K, k_chunk);
+  Operand a{A, 1, M, K, M, 1, M * K};   // stored (K, M)
+  Operand b{B, 1, N, K, N, 1, N * K};   // stored (K, N)
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
+  p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
+  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status; p.early = early;
+  // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
+  // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
+  // 1024 16.1 / 6.5.
+  const int bn = M <= BM ? std::min(pick_bn(N), 128)
+                         : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
+  return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
+                                    (cudaStream_t)stream);
 }
 
 }  // namespace b200moe
@@ -1075,26 +1102,7 @@ int b200moe_gemm_nn(const void* A, const void* B, void* D, int64_t M, int64_t N,
 
 int b200moe_gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K,
                            int64_t k_chunk, int32_t* status, b200moe_stream_t stream) {
-  B200_CHECK_ARG(A && B && P, B200MOE_E_NULL, "gemm_tn_splitk: null pointer");
-  CHECK_DIM8(M); CHECK_DIM8(N); CHECK_I32(M); CHECK_I32(N); CHECK_I32(K);
-  B200_CHECK_ARG(k_chunk > 0 && k_chunk % 64 == 0, B200MOE_E_BAD_SHAPE,
-                 "gemm_tn_splitk: k_chunk = %lld must be a positive multiple of 64", (long long)k_chunk);
-  B200_CHECK_ARG(K > 0, B200MOE_E_BAD_SHAPE, "gemm_tn_splitk: K must be positive");
-  B200_CHECK_ARG(aligned16(P), B200MOE_E_ALIGN, "gemm_tn_splitk: P not 16-byte aligned");
-  const long long slices = ceil_div(K, k_chunk);
-  Operand a{A, 1, M, K, M, 1, M * K};   // stored (K, M)
-  Operand b{B, 1, N, K, N, 1, N * K};   // stored (K, N)
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
-  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
-  // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
-  // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
-  // 1024 16.1 / 6.5.
-  const int bn = M <= BM ? std::min(pick_bn(N), 128)
-                         : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
-  return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
-                                    (cudaStream_t)stream);
+  return gemm_tn_splitk(A, B, P, M, N, K, k_chunk, 0, status, stream);
 }
 
 static int check_conv(const char* who, int64_t B, int64_t S, int64_t H, int64_t E, int taps, int64_t s_mult,
@@ -1223,7 +1231,7 @@ int b200moe_expert_linear_axpby(const void* a, const void* w, const void* c, flo
 int b200moe_expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
                             int64_t rows_cap, int E, int64_t K, int64_t N, void* out, int32_t* status,
                             b200moe_stream_t stream) {
-  return expert_linear_t(a, K, w, tile_expert, poffs, rows_cap, E, K, N, K, out, N, status, stream);
+  return expert_linear_t(a, K, w, tile_expert, poffs, rows_cap, E, K, N, K, out, N, 0, status, stream);
 }
 
 int b200moe_expert_linear_push(const void* a, const void* w, int w_kn, const int32_t* tile_expert, const int32_t* poffs,
@@ -1275,7 +1283,7 @@ int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_p
 
 int b200moe_expert_wgrad(const void* A, const void* B, const int32_t* poffs, const int32_t* counts, int64_t rows_cap,
                          int E, int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
-  return expert_wgrad(A, Na, B, Nb, poffs, counts, rows_cap, E, Na, Nb, out, status, stream);
+  return expert_wgrad(A, Na, B, Nb, poffs, counts, rows_cap, E, Na, Nb, out, 0, status, stream);
 }
 
 }  // extern "C"
