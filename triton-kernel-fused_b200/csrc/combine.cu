@@ -23,7 +23,9 @@ constexpr int kVecBatch = 4;   // 16-byte vectors a lane keeps in flight per row
 // idle; a thread reads its token's table entries itself (a broadcast) and keeps four rows' vectors in flight.
 // Against one CTA of 256 threads a token: 20 000 tokens of H 256, top-8 80 -> 29 us, 16 384 of H 512, top-2 21 -> 12 us, 32 768 of
 // H 2048, top-8 223 -> 214 us.
-template <int TPR>
+// PITCH: rows lie further apart than they are long.  As a launch parameter alone it made the rest slower: 4096 tokens of H 1024
+// 6.2 -> 6.5 us, 8192 of H 512 6.1 -> 6.6; with a kernel of each kind 6.2 and 6.1.
+template <int TPR, bool PITCH>
 __global__ void __launch_bounds__(256)
 combine_kernel(const uint4* rows, int pitch, const float* w, const int* slot_row, const uint4* add, long long T, int k,
                int vec_per_row, uint4* out) {
@@ -41,7 +43,7 @@ combine_kernel(const uint4* rows, int pitch, const float* w, const int* slot_row
         for (int i = 0; i < 4; ++i) r[i] = j0 + i < k ? slots[j0 + i] : -1;
 #pragma unroll
         for (int i = 0; i < 4; ++i)   // a slot without a row (its expert index was out of range) adds nothing
-          if (r[i] >= 0) v[i] = rows[static_cast<long long>(r[i]) * pitch + c];
+          if (r[i] >= 0) v[i] = rows[static_cast<long long>(r[i]) * (PITCH ? pitch : vec_per_row) + c];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           if (r[i] >= 0) fma8(acc, v[i], w != nullptr ? w[t * k + j0 + i] : 1.0f);
@@ -193,7 +195,8 @@ int combine_add(const void* rows, int64_t ldh, const float* w, const int32_t* sl
   by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
     constexpr int G = 256 / tpr.value;
     const long long grid = std::min<long long>((T + G - 1) / G, static_cast<long long>(num_sms()) * 16);
-    err = launch_chained(combine_kernel<tpr.value>, static_cast<int>(grid), 256, 0, (cudaStream_t)stream, 1,
+    err = launch_chained(ldh != H ? combine_kernel<tpr.value, true> : combine_kernel<tpr.value, false>, static_cast<int>(grid), 256, 0,
+                         (cudaStream_t)stream, 1,
                          reinterpret_cast<const uint4*>(rows), static_cast<int>(ldh / 8), w, slot_row, reinterpret_cast<const uint4*>(add), T, k,
                          static_cast<int>(H / 8), reinterpret_cast<uint4*>(out));
   });
