@@ -86,19 +86,22 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
-// WEIGHTED: the GLU epilogues of a block whose rows are weighted where their activations are made (weighted_rows).
+// ALT: GLU epilogues: of a block whose rows are weighted where their activations are made (weighted_rows); store epilogues: a kernel
+// that does not wait for the one before it (`early`, common.cuh; asked at run time it cost every launch 0.2 us: 15 products of 1 x
+// 1408 x 2048 236.8 -> 240.2 us, of 8 x 1024 x 1408 337.5 -> 341.7; compiled in 236.8 and 338.0).
 // Single-CTA tiles have two loading warps, one for A and one for B: a k-block's MMAs take 256 cycles there, but one thread's wait, its two
 // boxes and a convolution's coordinates 480 (380 without those), whatever the batch.  Logits of 16 x 1024 positions of H 2048, 64 experts, 4
 // taps (us): one loading warp 35.7, two 29.8, the next stage's barrier asked for ahead 28.6, the convolution in a loop of its own 24.7; of
 // 1 x 1024 positions 34.2 -> 23.4.  Products of few k-blocks are as fast as before.
 __host__ __device__ constexpr int gemm_threads(int ctas) { return ctas == 1 ? kThreads + 32 : kThreads; }
 
-template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
+template <int BN, int EPI, int CTAS, bool POLY = false, bool ALT = false>
 __global__ void __launch_bounds__(gemm_threads(CTAS), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
             const GemmParams p) {
   constexpr bool TMA_EPI = tma_epilogue<BN, EPI>();
+  constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD, WEIGHTED = ALT && GLU, EARLY = ALT && !GLU;
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   constexpr int TN = (EPI == EPI_SWIGLU) ? BN / 2 : BN;   // output columns one tile covers
   constexpr int TM = C::TILE_ROWS;
@@ -150,7 +153,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
-  if (p.early) grid_dep_early();
+  if constexpr (EARLY) grid_dep_early();
   else grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
@@ -686,7 +689,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   }
 
   // ------------------------------------------------------------------ tear-down
-  if (p.early) grid_dep_wait();      // so that this kernel's end is also that of the one before it
+  if constexpr (EARLY) grid_dep_wait();      // so that this kernel's end is also that of the one before it
   tc_fence_before();
   __syncthreads();
   if constexpr (CTAS == 2) {   // nobody leaves while the peer may still touch it
@@ -703,21 +706,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------------------- host side
-template <int BN, int EPI, int CTAS, bool POLY = false, bool WEIGHTED = false>
+template <int BN, int EPI, int CTAS, bool POLY = false, bool ALT = false>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD, const CUtensorMap& tmD2,
                   const GemmParams& p, int max_tiles, cudaStream_t stream) {
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, ALT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, WEIGHTED>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, ALT>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 
@@ -784,7 +787,7 @@ static int pick_bn_rows(long long n, long long rows_cap, int E, int cols_per_bn 
 
 // d1 / d2 describe the bf16 outputs as {columns, rows, groups} tensors for the TMA-store epilogue
 // (d2 = the SwiGLU `inter` output); they are ignored by the kernels that store directly.
-template <int EPI, bool POLY = false, bool WEIGHTED = false>
+template <int EPI, bool POLY = false, bool ALT = false>
 static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand* d1, const Operand* d2,
                        GemmParams& p, int max_tiles, cudaStream_t stream) {
   const bool pair = (bn == 256) && (p.sched != SCHED_DENSE) && pairs_enabled();
@@ -823,8 +826,8 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
       }
     }
   }
-  if (pair) return launch<256, EPI, 2, POLY, WEIGHTED>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
-  if constexpr (WEIGHTED) {
+  if (pair) return launch<256, EPI, 2, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
+  if constexpr (ALT && (EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD)) {
     set_error("internal: weighted epilogues are built for pair tiles");
     return B200MOE_E_UNSUPPORTED;
   } else if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
@@ -833,11 +836,11 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
     return B200MOE_E_UNSUPPORTED;
   } else
   switch (bn) {
-    case 256: return launch<256, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
-    case 128: return launch<128, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 256: return launch<256, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 128: return launch<128, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     default:
       if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32)
-        return launch<64, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+        return launch<64, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
       set_error("tile width %d not built for this epilogue", bn);
       return B200MOE_E_UNSUPPORTED;
   }
@@ -914,9 +917,10 @@ int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* ti
   GemmParams p{};
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)k_live; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = ldo; p.status = status;
-  p.early = early;
   Operand d{out, 0, rows_cap, N, ldo, 1, rows_cap * ldo};
-  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  const int bn = pick_bn_rows(N, rows_cap, E);
+  return early ? dispatch_bn<EPI_STORE, false, true>(bn, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream)
+               : dispatch_bn<EPI_STORE>(bn, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
 // row window of a grouped-M launch: (0, 0) = every row, else tile-aligned 0 <= row_lo < row_hi <= rows_cap
@@ -1031,11 +1035,12 @@ int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const i
   GemmParams p{};
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)Na; p.N = (int)Nb; p.K = (int)rows_cap;
   p.num_groups = E; p.poffs = poffs; p.counts = counts; p.D = out; p.ldd = Nb; p.d_group_stride = Na * Nb;
-  p.status = status; p.early = early;
+  p.status = status;
   const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
   Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
-  return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn)),
-                                (cudaStream_t)stream);
+  const int tiles = (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn));
+  return early ? dispatch_bn<EPI_STORE, false, true>(bn, a, b, &d, nullptr, p, tiles, (cudaStream_t)stream)
+               : dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, tiles, (cudaStream_t)stream);
 }
 
 int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K, int64_t k_chunk, int early, int32_t* status,
@@ -1052,14 +1057,15 @@ int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N,
   GemmParams p{};
   p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
-  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status; p.early = early;
+  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
   // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
   // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
   // 1024 16.1 / 6.5.
   const int bn = M <= BM ? std::min(pick_bn(N), 128)
                          : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
-  return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
-                                    (cudaStream_t)stream);
+  const int tiles = (int)(slices * ceil_div(M, BM) * ceil_div(N, bn));
+  return early ? dispatch_bn<EPI_STORE_F32, false, true>(bn, a, b, nullptr, nullptr, p, tiles, (cudaStream_t)stream)
+               : dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, tiles, (cudaStream_t)stream);
 }
 
 }  // namespace b200moe

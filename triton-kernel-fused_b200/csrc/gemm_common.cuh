@@ -69,7 +69,6 @@ struct GemmParams {
   const float* row_w;
   float* dots;
   long long dots_ld;
-  int early;                 // see common.cuh
 };
 
 struct Tile {
