@@ -530,7 +530,7 @@ int b200moe_conv_weight_grad(const float* P, int64_t slices, int E, int64_t H, i
 /* moe: the experts on given picks (idx (T,k), w (T,k) fp32).  E routed experts, the first n_glu with weights.
  * row_kernels: activations as row kernels (any code, act_params, Identity / Zero experts); 0: in the GEMM epilogues
  * (codes 0, 1, 5; act_codes NULL = SiLU).  keep = 0: no backward follows, which lets few rows per expert run over compact
- * rows.  grad_params (E,2), row_kernels only.  Gradients may be NULL: not wanted. */
+ * rows.  grad_params (E,2), row_kernels only. */
 size_t b200moe_moe_fwd_ws_bytes(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int row_kernels);
 int b200moe_moe_forward(const void* x, const int64_t* idx, const float* w, const void* gate_up_proj, const void* down_proj,
                         const int32_t* act_codes, const float* act_params, int64_t T, int64_t H, int64_t I, int E, int n_glu,

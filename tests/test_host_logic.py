@@ -238,6 +238,19 @@ def test_workspace_of_nothing_is_no_bytes():
     assert lib.b200moe_router_backward(16, 16, 16, 16, 16, 0, 256, 8, 2, 1, 1.0, 16, 16, 16, 16, None) != 0
 
 
+def test_backward_of_given_picks_needs_all_of_its_buffers():
+    """A moe backward without a place for the weights' gradient (or for any operand) is refused before anything is launched; the other gradients
+    may be left out."""
+    lib = importlib.import_module(PKG).lib()
+    args = [16, 16, 16, 16, None, None, 4, 256, 512, 8, 8, 2, 0, 16, 16, None, 16, None, None, None, 16, None]
+    null = lib.b200moe_layer_forward(None, 16, None, 16, 16, None, 4, 256, 512, 8, 2, 1, 1.0, 1, 16, 16, None, 16, 16, None)
+    assert null != 0
+    for i in (0, 1, 2, 3, 13, 14, 16):
+        bad = list(args)
+        bad[i] = None
+        assert lib.b200moe_moe_backward(*bad) == null, i
+
+
 def test_route_of_a_forward_without_backward():
     """Compact rows or row tiles: the workspace of the latter is that of a forward with a backward (it holds gate_up and the
     padded rows).  (experts, d_model, d_ff, picks, tokens, compact?): decoding; both sides of the limits on the mean rows of

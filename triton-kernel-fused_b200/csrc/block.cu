@@ -30,8 +30,7 @@ struct Carver {
   }
 };
 
-// KIND_WEIGHTED: row tiles weighted by the epilogues (weighted_rows)
-enum Kind { KIND_FEW = 0, KIND_TILES = 1, KIND_ROWS = 2, KIND_WEIGHTED = 3 };
+enum Kind { KIND_FEW = 0, KIND_TILES = 1, KIND_ROWS = 2 };
 
 struct Dims {
   int64_t T, H, I;
@@ -48,7 +47,6 @@ struct Dims {
 static Dims make_dims(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int rows_kernels) {
   Dims d{T, H, I, E, n_glu, k, KIND_TILES};
   if (rows_kernels) d.kind = KIND_ROWS;
-  else if (T > 0 && k > 0 && E > 0 && weighted_rows(T * k, E, H, I)) d.kind = KIND_WEIGHTED;
   else if (!keep && T > 0 && k > 0 && E > 0 && few_rows_forward(T * k, E, H, I)) d.kind = KIND_FEW;
   return d;
 }
@@ -63,7 +61,6 @@ static int check_dims(const char* who, const Dims& d) {
 
 struct Forward {
   int32_t *counts, *offs, *poffs, *slot_row, *row_slot, *tile_expert, *order, *slot_pos;
-  float* row_w;
   void* scratch;
   size_t scratch_bytes;
   bf16_t *x_s, *gate_up, *inter, *eo;
@@ -87,7 +84,6 @@ static Forward carve_forward(const Dims& d, bool router, void* ws, size_t* bytes
     f.order = c.take<int32_t>(M);
     f.slot_pos = c.take<int32_t>(M);
   }
-  if (d.kind == KIND_WEIGHTED) f.row_w = c.take<float>(cap);
   f.scratch_bytes = b200moe_permute_ws_bytes(M, d.E);
   f.scratch = c.take<char>(f.scratch_bytes);
   if (router) {
@@ -105,9 +101,8 @@ static Forward carve_forward(const Dims& d, bool router, void* ws, size_t* bytes
 
 struct Backward {
   bf16_t *grad_eo, *grad_gu, *grad_x_s, *grad_inter;
-  float* dots;
   float *row_da, *row_dg;
-  float* grad_w;                     // the router's backward reads it; else where its caller wants none
+  float* grad_w;                     // when the router's backward follows
   bf16_t *grad_logits, *grad_x_router;
   float* part;
 };
@@ -145,9 +140,8 @@ static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* byt
   } else {
     b.grad_x_s = b.grad_eo;                        // written after the last read of grad_eo
   }
-  if (d.kind == KIND_WEIGHTED) b.dots = c.take<float>((d.I + 127) / 128 * rows);
-  b.grad_w = c.take<float>(d.M());
   if (router) {
+    b.grad_w = c.take<float>(d.M());
     b.grad_logits = c.take<bf16_t>(d.T * d.E);
     b.grad_x_router = c.take<bf16_t>(d.T * d.H);
     b.part = c.take<float>(router_split(d.T, d.E, d.H, num_sms()).slices * d.E * d.H);
@@ -163,11 +157,11 @@ static Backward carve_backward(const Dims& d, bool router, void* ws, size_t* byt
     if (rc__) return rc__;            \
   } while (0)
 
-static int permute(const Dims& d, const int64_t* idx, const float* w, const Forward& f, int32_t* counts_out, int64_t* load,
-                   int32_t* status, b200moe_stream_t st) {
+static int permute(const Dims& d, const int64_t* idx, const Forward& f, int32_t* counts_out, int64_t* load, int32_t* status,
+                   b200moe_stream_t st) {
   RUN("permute_build", d.M() > 1024 ? 2 : 1,
       permute_build(idx, d.T, d.k, d.E, f.counts, f.offs, f.poffs, f.slot_row, f.row_slot, f.tile_expert, f.order,
-                    f.slot_pos, f.scratch, f.scratch_bytes, counts_out, load, RowWeights{f.row_w, w}, status, st));
+                    f.slot_pos, f.scratch, f.scratch_bytes, counts_out, load, status, st));
   return 0;
 }
 
@@ -186,8 +180,8 @@ static int experts_forward(const Dims& d, const void* x, const float* w, const v
   }
   const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
   RUN("gather_rows", 1, gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, ldh, rows, f.x_s, st));
-  if (d.kind != KIND_ROWS) {   // weighted rows carry their weights from the activations on
-    RUN("expert_gate_up_swiglu", 1, expert_gate_up(f.x_s, ldh, gate_up_proj, codes, f.row_w, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H, d.I,
+  if (d.kind == KIND_TILES) {
+    RUN("expert_gate_up_swiglu", 1, expert_gate_up(f.x_s, ldh, gate_up_proj, codes, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H, d.I,
                                                    f.gate_up, ld2, f.inter, ldi, status, st));
     RUN("expert_down", 1, expert_linear(f.inter, ldi, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, ldh, status, st));
   } else {   // the GEMMs and the activation kernels see the rows of the experts with weights only
@@ -197,11 +191,11 @@ static int experts_forward(const Dims& d, const void* x, const float* w, const v
     if (d.n_glu < d.E)
       RUN("special_rows", 1, special_rows(f.x_s, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, ldh, rows, f.eo, st));
   }
-  RUN("combine", 1, combine_add(f.eo, ldh, d.kind == KIND_WEIGHTED ? nullptr : w, f.slot_row, nullptr, d.T, d.k, d.H, out, st));
+  RUN("combine", 1, combine_add(f.eo, ldh, w, f.slot_row, nullptr, d.T, d.k, d.H, out, st));
   return 0;
 }
 
-// Gradients to compute (nullptr: not wanted, which lets a block leave out the products that only they need; x != nullptr: the rows b.grad_x_s, which the caller combines per token)
+// Gradients to compute (nullptr: not wanted; x != nullptr: the rows b.grad_x_s, which the caller combines per token)
 struct Grads {
   void *x, *gate_up, *down;
   float *w, *params;
@@ -213,21 +207,17 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
   const int64_t rows = d.rows();
   const int32_t* total = f.poffs + d.E;
   const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
-  const bool weighted = d.kind == KIND_WEIGHTED;
-  if (weighted)
-    RUN("gather_rows", 1, gather_rows(grad_out, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, st));
-  else
-    RUN("combine_bwd", 1, combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, g.w != nullptr ? g.w : b.grad_w, st));
+  RUN("combine_bwd", 1, combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, g.w, st));
   // The weight gradient of the down products needs nothing of the product in front of it, and the rows' gradient nothing of the other weight
   // gradient: each begins on the SMs that the kernel before has left (`early`), so their last waves overlap.  (b.grad_x_s may be
   // b.grad_eo: the last reader of that is complete when the second weight gradient has passed its wait.)
   const int n = d.n_glu;
-  bool beside = true;                                    // whether a kernel that waits stands between here and combine_bwd / the gather
-  if (d.kind != KIND_ROWS) {
-    beside = g.x != nullptr || g.gate_up != nullptr || (weighted && g.w != nullptr);
+  bool beside = true;                                    // whether a kernel that waits stands between here and combine_bwd
+  if (d.kind == KIND_TILES) {
+    beside = g.x != nullptr || g.gate_up != nullptr;
     if (beside)
-      RUN("expert_down_dgrad_glu", 1, expert_down_dgrad(b.grad_eo, ldh, down_proj, f.gate_up, ld2, codes, f.row_w, f.tile_expert, f.poffs, rows, 0, 0,
-                                                        d.E, d.H, d.I, b.grad_gu, b.dots, status, st));
+      RUN("expert_down_dgrad_glu", 1, expert_down_dgrad(b.grad_eo, ldh, down_proj, f.gate_up, ld2, codes, f.tile_expert, f.poffs, rows, 0, 0,
+                                                        d.E, d.H, d.I, b.grad_gu, status, st));
   } else {
     RUN("expert_linear_t", 1, expert_linear_t(b.grad_eo, ldh, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, d.H, b.grad_inter, ldi, 0, status, st));
   }
@@ -237,8 +227,6 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
   float* dg = g.params != nullptr ? b.row_dg : nullptr;
   if (d.kind == KIND_ROWS)
     RUN("glu_bwd_rows", 1, glu_bwd_rows(b.grad_inter, ldi, f.gate_up, ld2, f.tile_expert, codes, params, f.poffs + n, rows, d.I, b.grad_gu, da, dg, st));
-  else if (weighted && g.w != nullptr)
-    RUN("row_dots", 1, row_dots(b.dots, (int)((d.I + 127) / 128), rows, f.row_slot, total, g.w, st));
   if (g.gate_up != nullptr)
     RUN("expert_wgrad", 1, expert_wgrad(b.grad_gu, ld2, f.x_s, ldh, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, 0, status, st));
   if (g.x != nullptr) {
@@ -441,7 +429,7 @@ int b200moe_moe_forward(const void* x, const int64_t* idx, const float* w, const
   if (rc) return rc;
   B200_CHECK_ARG(x && idx && w && gate_up_proj && down_proj && ws && out, B200MOE_E_NULL, "moe_forward: null pointer");
   const Forward f = carve_forward(d, false, ws, nullptr);
-  rc = permute(d, idx, w, f, nullptr, nullptr, status, stream);
+  rc = permute(d, idx, f, nullptr, nullptr, status, stream);
   if (rc) return rc;
   return experts_forward(d, x, w, gate_up_proj, down_proj, act_codes, act_params, f, out, status, stream);
 }
@@ -460,7 +448,7 @@ int b200moe_moe_backward(const void* grad_out, const float* w, const void* gate_
   const Dims d = make_dims(T, H, I, E, n_glu, k, 1, row_kernels);
   int rc = check_dims("moe_backward", d);
   if (rc) return rc;
-  B200_CHECK_ARG(grad_out && w && gate_up_proj && down_proj && fwd_ws && ws, B200MOE_E_NULL, "moe_backward: null pointer");
+  B200_CHECK_ARG(grad_out && w && gate_up_proj && down_proj && fwd_ws && ws && grad_w, B200MOE_E_NULL, "moe_backward: null pointer");
   const Forward f = carve_forward(d, false, fwd_ws, nullptr);
   const Backward b = carve_backward(d, false, ws, nullptr);
   const Grads g{grad_x, grad_gate_up, grad_down, grad_w, grad_params};
@@ -489,7 +477,7 @@ int b200moe_layer_forward(const void* x, const void* gate_weight, const float* b
   const Forward f = carve_forward(d, true, ws, nullptr);
   rc = router_forward(x, gate_weight, bias, T, H, E, k, norm_topk, scale, f.logits, f.idx, f.w, nullptr, status, stream);
   if (rc) return rc;
-  rc = permute(d, f.idx, f.w, f, counts, load, status, stream);
+  rc = permute(d, f.idx, f, counts, load, status, stream);
   if (rc) return rc;
   return experts_forward(d, x, f.w, gate_up_proj, down_proj, act_codes, nullptr, f, out, status, stream);
 }
@@ -511,7 +499,7 @@ int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate
   B200_CHECK_ARG(grad_out && x && gate_weight && gate_up_proj && down_proj && fwd_ws && ws, B200MOE_E_NULL, "layer_backward: null pointer");
   const Forward f = carve_forward(d, true, fwd_ws, nullptr);
   const Backward b = carve_backward(d, true, ws, nullptr);
-  const Grads g{grad_x, grad_gate_up, grad_down, grad_x != nullptr || grad_gate_weight != nullptr ? b.grad_w : nullptr, nullptr};
+  const Grads g{grad_x, grad_gate_up, grad_down, b.grad_w, nullptr};
   rc = experts_backward(d, grad_out, f.w, gate_up_proj, down_proj, act_codes, nullptr, f, b, g, status, stream);
   if (rc) return rc;
   if (grad_x != nullptr || grad_gate_weight != nullptr) {

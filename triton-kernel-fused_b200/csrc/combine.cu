@@ -157,33 +157,6 @@ combine_bwd_narrow_kernel(const uint4* go, const uint4* eo, const float* w, cons
   }
 }
 
-// A routing weight's gradient from the sums that the GLU-backward product kept of its row, one per 128 columns, added in order.  Bound
-// by launch and load latency: 98 304 rows of 11 sums are 4 MB.
-__global__ void __launch_bounds__(256)
-row_dots_kernel(const float* dots, int parts, long long ld, const int* row_slot, const int* total_rows, float* grad_w) {
-  grid_dep_begin();
-  const int total = *total_rows;
-  for (int r = blockIdx.x * 256 + threadIdx.x; r < total; r += gridDim.x * 256) {
-    const int slot = row_slot[r];
-    if (slot < 0) continue;
-    float v = 0.0f;
-    for (int i0 = 0; i0 < parts; i0 += 8) {
-      float d[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) d[i] = i0 + i < parts ? dots[(i0 + i) * ld + r] : 0.0f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v += d[i];
-    }
-    grad_w[slot] = v;
-  }
-}
-
-int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, const int32_t* total_rows, float* grad_w, b200moe_stream_t stream) {
-  const long long grid = std::min<long long>((ld + 255) / 256, static_cast<long long>(num_sms()) * 8);
-  B200_LAUNCH(row_dots_kernel, static_cast<int>(grid), 256, 0, stream, dots, parts, static_cast<long long>(ld), row_slot, total_rows, grad_w);
-  return 0;
-}
-
 int combine_add(const void* rows, int64_t ldh, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k, int64_t H, void* out,
                 b200moe_stream_t stream) {
   B200_CHECK_ARG(rows && slot_row && out, B200MOE_E_NULL, "combine: null pointer");

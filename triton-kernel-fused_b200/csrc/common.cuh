@@ -29,11 +29,6 @@ int num_sms();
 int gemm_cta_budget();   // CTAs a persistent GEMM may occupy (num_sms() minus the reserved SMs)
 int exchange_sm_budget();   // SMs (= fat CTAs) the home-side pull kernel of the expert-parallel exchange may occupy
 
-// Routing weight of each padded row (pads: 0).  row_w == nullptr: not wanted
-struct RowWeights {
-  float* row_w;
-  const float* slot_w;   // (T, k)
-};
 // Elements between rows of the block's own buffers.  A TMA box whose 128-byte rows start 16 bytes past a 32-byte sector moves at three
 // quarters of the rate (8.4 against 11.6 TB/s, all from L2; 32 bytes past a line: 10.9), and stores to such rows leave partial sectors: rows whose
 // length is no multiple of 64 bytes are padded to whole lines.  us a training pass, dense / padded: 3001 tokens, 32 experts of 1032 x 680, top-4
@@ -60,12 +55,12 @@ int glu_bwd_rows(const void* grad_inter, int64_t ldi, const void* gate_up, int64
                  b200moe_stream_t stream);
 int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special, int num_experts,
                  int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream);
-int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const int32_t* tile_expert,
                    const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, int64_t ld2,
                    void* inter, int64_t ldi, int32_t* status, b200moe_stream_t stream);
 int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, const void* gate_up, int64_t ld2, const int32_t* act_codes,
-                      const float* row_w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
-                      int64_t H, int64_t I, void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream);
+                      const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
+                      int64_t H, int64_t I, void* grad_gate_up, int32_t* status, b200moe_stream_t stream);
 int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
                   int64_t K, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream);
 int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
@@ -74,7 +69,7 @@ int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const i
 // b200moe_permute_build; also stores the counts a second time (counts_out) and adds them to `load` (both nullable)
 int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs, int32_t* poffs,
                   int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert, int32_t* order, int32_t* slot_pos, void* ws,
-                  size_t ws_bytes, int32_t* counts_out, int64_t* load, const RowWeights& rows, int32_t* status, b200moe_stream_t stream);
+                  size_t ws_bytes, int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream);
 
 // router.cu.  counts (nullable): cleared by conv_weight_rows; counts_cleared: some kernel before has done so
 int conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, int32_t* counts, b200moe_stream_t stream);
@@ -85,12 +80,6 @@ int router_topk_bwd(const void* logits, int input_kind, const int64_t* idx, cons
                     float scale, int early, void* grad_logits, b200moe_stream_t stream);
 int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K, int64_t k_chunk, int early, int32_t* status,
                    b200moe_stream_t stream);
-
-// combine.cu: grad_w[slot] = sum over `parts` of dots[part][row], dots (parts, ld)
-int row_dots(const float* dots, int parts, int64_t ld, const int32_t* row_slot, const int32_t* total_rows, float* grad_w, b200moe_stream_t stream);
-
-// gemm.cu: whether a block's rows are weighted by the epilogues of its GLU products (their row_w, dots)
-bool weighted_rows(int64_t M, int E, int64_t H, int64_t I);
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);

@@ -178,15 +178,15 @@ struct Experts : torch::autograd::Function<Experts> {
     const int64_t T = w.size(0), k = w.size(1), H = ctx->saved_data["H"].toInt(), n = gate_up.size(0), I = down.size(2);
     const c10::cuda::CUDAGuard guard(ws.device());
     const Tensor go = grads[0].to(at::kBFloat16).contiguous();
-    const Tensor gw = ctx->needs_input_grad(1) ? at::empty_like(w) : Tensor();
+    const Tensor gw = at::empty_like(w);
     const Tensor gx = ctx->needs_input_grad(0) ? at::empty({T, H}, gate_up.options()) : Tensor();
     const Tensor ggu = grad_like(ctx->needs_input_grad(2), gate_up), gdn = grad_like(ctx->needs_input_grad(3), down);
     const Tensor gp = params.defined() && ctx->needs_input_grad(4) ? at::empty_like(params) : Tensor();
     Tensor tmp = bytes(b200moe_moe_bwd_ws_bytes(T, H, I, E, n, k, rows), ws);
     check(b200moe_moe_backward(ptr(go), w.data_ptr<float>(), ptr(gate_up), ptr(down), static_cast<const int32_t*>(ptr(codes)),
-                               static_cast<const float*>(ptr(params)), T, H, I, E, n, k, rows, ptr(ws), ptr(tmp), ptr(gx), static_cast<float*>(ptr(gw)),
+                               static_cast<const float*>(ptr(params)), T, H, I, E, n, k, rows, ptr(ws), ptr(tmp), ptr(gx), gw.data_ptr<float>(),
                                ptr(ggu), ptr(gdn), static_cast<float*>(ptr(gp)), status_ptr(status), stream_of(ws)));
-    return {gx, gw, ggu, gdn, gp, Tensor()};
+    return {gx, ctx->needs_input_grad(1) ? gw : Tensor(), ggu, gdn, gp, Tensor()};
   }
 };
 

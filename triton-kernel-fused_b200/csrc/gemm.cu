@@ -86,22 +86,20 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
-// ALT: GLU epilogues: of a block whose rows are weighted where their activations are made (weighted_rows); store epilogues: a kernel
-// that does not wait for the one before it (`early`, common.cuh; asked at run time it cost every launch 0.2 us: 15 products of 1 x
-// 1408 x 2048 236.8 -> 240.2 us, of 8 x 1024 x 1408 337.5 -> 341.7; compiled in 236.8 and 338.0).
+// EARLY: a kernel that does not wait for the one before it (`early`, common.cuh; asked at run time it cost every launch 0.2 us: 15
+// products of 1 x 1408 x 2048 236.8 -> 240.2 us, of 8 x 1024 x 1408 337.5 -> 341.7; compiled in 236.8 and 338.0).
 // Single-CTA tiles have two loading warps, one for A and one for B: a k-block's MMAs take 256 cycles there, but one thread's wait, its two
 // boxes and a convolution's coordinates 480 (380 without those), whatever the batch.  Logits of 16 x 1024 positions of H 2048, 64 experts, 4
 // taps (us): one loading warp 35.7, two 29.8, the next stage's barrier asked for ahead 28.6, the convolution in a loop of its own 24.7; of
 // 1 x 1024 positions 34.2 -> 23.4.  Products of few k-blocks are as fast as before.
 __host__ __device__ constexpr int gemm_threads(int ctas) { return ctas == 1 ? kThreads + 32 : kThreads; }
 
-template <int BN, int EPI, int CTAS, bool POLY = false, bool ALT = false>
+template <int BN, int EPI, int CTAS, bool POLY = false, bool EARLY = false>
 __global__ void __launch_bounds__(gemm_threads(CTAS), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
             const GemmParams p) {
   constexpr bool TMA_EPI = tma_epilogue<BN, EPI>();
-  constexpr bool GLU = EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD, WEIGHTED = ALT && GLU, EARLY = ALT && !GLU;
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   constexpr int TN = (EPI == EPI_SWIGLU) ? BN / 2 : BN;   // output columns one tile covers
   constexpr int TM = C::TILE_ROWS;
@@ -366,7 +364,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       if constexpr (POLY && (EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD)) act_code = p.act_codes[t.g];
       const int row0 = t.m0 + BM * static_cast<int>(cta_rank) + q * 32;   // first row of this warp
       const long long row = static_cast<long long>(row0) + lane;
-      const float row_w = WEIGHTED ? p.row_w[row] : 1.0f;
       // GLU backward works on four 32-column sub-chunks per warp with two sets of (gate, up) boxes of
       // 32 rows x 32 columns (2 KB, 64-byte swizzle): a set is loaded by TMA, overwritten in place with
       // grad_gate / grad_up and stored by TMA while the other set is loading or being computed on.  The saved
@@ -521,7 +518,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 og[16 * sub + i] = pack_bf16x2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
                 ou[16 * sub + i] = pack_bf16x2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
               }
-              glu_fwd_pairs_by_code<POLY>(act_code, og + 16 * sub, ou + 16 * sub, oh + 16 * sub, 16, row_w);
+              glu_fwd_pairs_by_code<POLY>(act_code, og + 16 * sub, ou + 16 * sub, oh + 16 * sub, 16);
             }
             staging_free(lane);
             stage_row(sbuf, lane, og);
@@ -535,7 +532,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         } else {  // EPI_GLU_BWD: accumulator = grad_inter columns [n0, n0+BN); this warp: 128 of them
           constexpr int W = BN / 2;
-          float dot = 0.0f;
 #pragma unroll 1
           for (int sub = 0; sub < W / 32; ++sub) {
             const int col = glu_col0 + 32 * sub;
@@ -556,7 +552,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
             tmem_ld_wait();
             uint32_t og[16], ou[16];
-            glu_bwd32<POLY>(r, g4, u4, og, ou, act_code, row_w, WEIGHTED ? &dot : nullptr);
+            glu_bwd32<POLY>(r, g4, u4, og, ou, act_code);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {              // results replace the inputs in place
               const int off = lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4);
@@ -577,8 +573,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               glu_load(sub + 2);
             }
           }
-          if constexpr (WEIGHTED)
-            if (glu_col0 < p.I) p.dots[(glu_col0 / W) * p.dots_ld + row] = dot;
         }
       } else {
         // Single-CTA tiles up to 128 wide, and fp32 partial sums: from tensor memory through registers.  16 rows x 64 (or 32) columns at a
@@ -706,21 +700,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------------------- host side
-template <int BN, int EPI, int CTAS, bool POLY = false, bool ALT = false>
+template <int BN, int EPI, int CTAS, bool POLY = false, bool EARLY = false>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD, const CUtensorMap& tmD2,
                   const GemmParams& p, int max_tiles, cudaStream_t stream) {
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, ALT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, ALT>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, EARLY>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 
@@ -787,7 +781,7 @@ static int pick_bn_rows(long long n, long long rows_cap, int E, int cols_per_bn 
 
 // d1 / d2 describe the bf16 outputs as {columns, rows, groups} tensors for the TMA-store epilogue
 // (d2 = the SwiGLU `inter` output); they are ignored by the kernels that store directly.
-template <int EPI, bool POLY = false, bool ALT = false>
+template <int EPI, bool POLY = false, bool EARLY = false>
 static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand* d1, const Operand* d2,
                        GemmParams& p, int max_tiles, cudaStream_t stream) {
   const bool pair = (bn == 256) && (p.sched != SCHED_DENSE) && pairs_enabled();
@@ -826,21 +820,18 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
       }
     }
   }
-  if (pair) return launch<256, EPI, 2, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
-  if constexpr (ALT && (EPI == EPI_SWIGLU || EPI == EPI_GLU_BWD)) {
-    set_error("internal: weighted epilogues are built for pair tiles");
-    return B200MOE_E_UNSUPPORTED;
-  } else if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
+  if (pair) return launch<256, EPI, 2, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
+  if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
     if (bn == 256) return launch<256, EPI, 1>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     set_error("tile width %d not built for this epilogue", bn);
     return B200MOE_E_UNSUPPORTED;
   } else
   switch (bn) {
-    case 256: return launch<256, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
-    case 128: return launch<128, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 256: return launch<256, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 128: return launch<128, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     default:
       if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32)
-        return launch<64, EPI, 1, POLY, ALT>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+        return launch<64, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
       set_error("tile width %d not built for this epilogue", bn);
       return B200MOE_E_UNSUPPORTED;
   }
@@ -933,7 +924,7 @@ static int check_row_window(const char* who, int64_t rows_cap, int64_t row_lo, i
   return 0;
 }
 
-int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const float* row_w, const int32_t* tile_expert,
+int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const int32_t* tile_expert,
                    const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, int64_t ld2,
                    void* inter, int64_t ldi, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_gate_up_swiglu", x_s, gate_up_proj, gate_up, tile_expert, poffs, rows_cap, E, H, I);
@@ -954,18 +945,13 @@ int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const
   Operand d1{gate_up, 0, rows_cap, I, ld2, 2, I};         // {I, rows, 2}: group 0 = gate half, 1 = up half
   Operand d2{inter, 0, rows_cap, I, ldi, 1, rows_cap * ldi};
   p.act_codes = act_codes;
-  if (row_w != nullptr) {
-    p.row_w = row_w;
-    return act_codes != nullptr ? dispatch_bn<EPI_SWIGLU, true, true>(256, a, b, &d1, &d2, p, 0, (cudaStream_t)stream)
-                                : dispatch_bn<EPI_SWIGLU, false, true>(256, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
-  }
   if (act_codes != nullptr) return dispatch_bn<EPI_SWIGLU, true>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
   return dispatch_bn<EPI_SWIGLU>(bn, a, b, &d1, &d2, p, 0, (cudaStream_t)stream);
 }
 
 int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, const void* gate_up, int64_t ld2, const int32_t* act_codes,
-                      const float* row_w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
-                      int64_t H, int64_t I, void* grad_gate_up, float* dots, int32_t* status, b200moe_stream_t stream) {
+                      const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E,
+                      int64_t H, int64_t I, void* grad_gate_up, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_down_dgrad_glu", grad_eo, down_proj, grad_gate_up, tile_expert, poffs, rows_cap, E, H, I);
   if (rc) return rc;
   rc = check_row_window("expert_down_dgrad_glu", rows_cap, row_lo, row_hi);
@@ -983,28 +969,8 @@ int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, c
   Operand d{grad_gate_up, 0, rows_cap, I, ld2, 2, I};     // {I, rows, 2}: grad_gate half, grad_up half
   Operand d2{gate_up, 0, rows_cap, I, ld2, 2, I};         // the saved forward gate_up, same view (input)
   p.act_codes = act_codes;
-  if (row_w != nullptr) {
-    p.row_w = row_w; p.dots = dots; p.dots_ld = rows_cap;
-    return act_codes != nullptr ? dispatch_bn<EPI_GLU_BWD, true, true>(256, a, b, &d, &d2, p, 0, (cudaStream_t)stream)
-                                : dispatch_bn<EPI_GLU_BWD, false, true>(256, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
-  }
   if (act_codes != nullptr) return dispatch_bn<EPI_GLU_BWD, true>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
   return dispatch_bn<EPI_GLU_BWD>(bn, a, b, &d, &d2, p, 0, (cudaStream_t)stream);
-}
-
-// ---- a routed row weighted where its activations are made, not where it is added up: inter = w act(gate) up, so the down product's rows
-// need no weight any more, the weight gradients no weighted copy of the upstream gradient, and grad_inter = w (go W_down) and the
-// weight's own gradient (go W_down) . (act(gate) up) both come out of one accumulator: the experts' results are not read a second time,
-// and go is rounded once less.  Pays where those results have left L2 by then (from about half of its 126 MB on).  us, go into expert order with its
-// weights and dots / without: 98 304 rows of H 2048 234 / 135 (a pass 4907 / 4772), 262 144 rows 655 / 410 (8422 / 8235), 32 768 rows of H 2056
-// 88 / 49 (2305 / 2281), of H 1024 36 / 21 (529 / 520), 16 384 rows of H 1024 16 / 11 but 307 / 306 a pass.
-bool weighted_rows(int64_t M, int E, int64_t H, int64_t I) {
-  // (Where a forward without a backward takes the few-rows kernels, which leave the weights to the combine, it would round elsewhere.)
-  if (M * H * 2 < (64LL << 20) || !pairs_enabled() || I <= 64 || few_rows_forward(M, E, H, I)) return false;
-  const int64_t tiles = std::max<int64_t>(1, ceil_div(M, B200MOE_TILE_M) + E / 2), pairs = num_sms() / 2;   // as pick_bn_rows
-  // both products on pair tiles by the rule of pick_bn_grouped
-  auto on_pairs = [&](int64_t n) { return 10 * ceil_div(tiles * ceil_div(n, 256), pairs) <= 8 * ceil_div(2 * tiles * ceil_div(n, 128), 2 * pairs); };
-  return on_pairs(2 * I) && on_pairs(I);
 }
 
 int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
@@ -1213,7 +1179,7 @@ int b200moe_expert_gate_up_act(const void* x_s, const void* gate_up_proj, const 
                                const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int64_t row_lo,
                                int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, void* inter,
                                int32_t* status, b200moe_stream_t stream) {
-  return expert_gate_up(x_s, H, gate_up_proj, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, gate_up, 2 * I, inter, I, status,
+  return expert_gate_up(x_s, H, gate_up_proj, act_codes, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, gate_up, 2 * I, inter, I, status,
                         stream);
 }
 
@@ -1276,8 +1242,8 @@ int b200moe_expert_down_dgrad_act(const void* grad_eo, const void* down_proj, co
                                   const int32_t* act_codes, const int32_t* tile_expert, const int32_t* poffs,
                                   int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I,
                                   void* grad_gate_up, int32_t* status, b200moe_stream_t stream) {
-  return expert_down_dgrad(grad_eo, H, down_proj, gate_up, 2 * I, act_codes, nullptr, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, grad_gate_up,
-                           nullptr, status, stream);
+  return expert_down_dgrad(grad_eo, H, down_proj, gate_up, 2 * I, act_codes, tile_expert, poffs, rows_cap, row_lo, row_hi, E, H, I, grad_gate_up,
+                           status, stream);
 }
 
 int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_proj, const int32_t* tile_expert,

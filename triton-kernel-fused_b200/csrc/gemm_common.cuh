@@ -64,11 +64,6 @@ struct GemmParams {
   // weight gradient): operand B, tap = tile column / conv_C, shift = tap - (conv_taps - 1); conv_S % 64 == 0.
   int conv_taps, conv_S, conv_C, conv_sign;
   int conv_b_taps;   // DENSE convolution: operand B is {conv_C channels, N, taps} (else {taps * conv_C, N})
-  // the WEIGHTED instantiations: weight of each padded row (0 for pads); GLU backward: inner products of a row's accumulators with its
-  // activations, one per 128 columns, as (columns / 128, dots_ld)
-  const float* row_w;
-  float* dots;
-  long long dots_ld;
 };
 
 struct Tile {
@@ -198,54 +193,52 @@ __device__ __forceinline__ float glu_fwd_val(float g, float u) {
 }
 // grad_gate = go * up * f'(g), grad_up = go * f(g)
 template <int CODE>
-__device__ __forceinline__ void glu_bwd_val(float g, float u, float go, float& grad_gate, float& grad_up, float& f) {
+__device__ __forceinline__ void glu_bwd_val(float g, float u, float go, float& grad_gate, float& grad_up) {
   if constexpr (CODE == 1) {
     const float r = fmaxf(g, 0.0f);
     grad_gate = go * u * (2.0f * r);
-    f = r * r;
+    grad_up = go * (r * r);
   } else {
     const float s = __fdividef(1.0f, 1.0f + __expf(-g));
     if constexpr (CODE == 5) {
       const float t = __fdividef(2.0f, 1.0f + __expf(-2.0f * g)) - 1.0f;
       const float d = (1.0f - t * t) * s + t * s * (1.0f - s);
       grad_gate = go * u * d;
-      f = t * s;
+      grad_up = go * (t * s);
     } else {
       const float d = s * (1.0f + g * (1.0f - s));
       grad_gate = go * u * d;
-      f = g * s;
+      grad_up = go * (g * s);
     }
   }
-  grad_up = go * f;
 }
 
 // Forward GLU on n packed pairs: pg / pu = bf16-rounded gate / up (the activation reads the rounded values, as the
-// reference's separate activation kernel does, kernels/sm75/moe.py:163-184); oh = act(gate) * up * w
+// reference's separate activation kernel does, kernels/sm75/moe.py:163-184); oh = act(gate) * up
 template <int CODE>
-__device__ __forceinline__ void glu_fwd_pairs(const uint32_t* pg, const uint32_t* pu, uint32_t* oh, int n, float w) {
+__device__ __forceinline__ void glu_fwd_pairs(const uint32_t* pg, const uint32_t* pu, uint32_t* oh, int n) {
 #pragma unroll
   for (int i = 0; i < n; ++i) {
     const float2 gf = unpack_bf16x2(pg[i]);
     const float2 uf = unpack_bf16x2(pu[i]);
-    oh[i] = pack_bf16x2(glu_fwd_val<CODE>(gf.x, uf.x) * w, glu_fwd_val<CODE>(gf.y, uf.y) * w);
+    oh[i] = pack_bf16x2(glu_fwd_val<CODE>(gf.x, uf.x), glu_fwd_val<CODE>(gf.y, uf.y));
   }
 }
 template <bool POLY>
 __device__ __forceinline__ void glu_fwd_pairs_by_code(int code, const uint32_t* pg, const uint32_t* pu, uint32_t* oh,
-                                                      int n, float w = 1.0f) {
+                                                      int n) {
   if constexpr (POLY) {
-    if (code == 1) return glu_fwd_pairs<1>(pg, pu, oh, n, w);
-    if (code == 5) return glu_fwd_pairs<5>(pg, pu, oh, n, w);
+    if (code == 1) return glu_fwd_pairs<1>(pg, pu, oh, n);
+    if (code == 5) return glu_fwd_pairs<5>(pg, pu, oh, n);
   }
-  glu_fwd_pairs<0>(pg, pu, oh, n, w);
+  glu_fwd_pairs<0>(pg, pu, oh, n);
 }
 
-// grad_gate = gi*up*f'(g), grad_up = gi*f(g) for 32 columns; gi (fp32 accumulator times w)
-// is rounded to bf16 first because the reference materialises grad_inter in bf16.  dot (not null): plus the accumulators' inner
-// product with f(g)*up
+// grad_gate = gi*up*f'(g), grad_up = gi*f(g) for 32 columns; gi (fp32 accumulator)
+// is rounded to bf16 first because the reference materialises grad_inter in bf16
 template <int CODE>
 __device__ __forceinline__ void glu_bwd32_code(const uint32_t (&r)[32], const uint4 (&g)[4], const uint4 (&u)[4],
-                                               uint32_t* og, uint32_t* ou, float w, float* dot) {
+                                               uint32_t* og, uint32_t* ou) {
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const uint32_t gw[4] = {g[v].x, g[v].y, g[v].z, g[v].w};
@@ -254,11 +247,11 @@ __device__ __forceinline__ void glu_bwd32_code(const uint32_t (&r)[32], const ui
     for (int h = 0; h < 4; ++h) {
       const float2 gf = unpack_bf16x2(gw[h]);
       const float2 uf = unpack_bf16x2(uw[h]);
-      const float acc0 = __uint_as_float(r[v * 8 + 2 * h]), acc1 = __uint_as_float(r[v * 8 + 2 * h + 1]);
-      float gg0, gu0, f0, gg1, gu1, f1;
-      glu_bwd_val<CODE>(gf.x, uf.x, bf16_round(acc0 * w), gg0, gu0, f0);
-      glu_bwd_val<CODE>(gf.y, uf.y, bf16_round(acc1 * w), gg1, gu1, f1);
-      if (dot != nullptr) *dot += acc0 * (f0 * uf.x) + acc1 * (f1 * uf.y);
+      const float go0 = bf16_round(__uint_as_float(r[v * 8 + 2 * h]));
+      const float go1 = bf16_round(__uint_as_float(r[v * 8 + 2 * h + 1]));
+      float gg0, gu0, gg1, gu1;
+      glu_bwd_val<CODE>(gf.x, uf.x, go0, gg0, gu0);
+      glu_bwd_val<CODE>(gf.y, uf.y, go1, gg1, gu1);
       og[4 * v + h] = pack_bf16x2(gg0, gg1);
       ou[4 * v + h] = pack_bf16x2(gu0, gu1);
     }
@@ -266,12 +259,12 @@ __device__ __forceinline__ void glu_bwd32_code(const uint32_t (&r)[32], const ui
 }
 template <bool POLY = false>
 __device__ __forceinline__ void glu_bwd32(const uint32_t (&r)[32], const uint4 (&g)[4], const uint4 (&u)[4],
-                                          uint32_t* og, uint32_t* ou, int code = 0, float w = 1.0f, float* dot = nullptr) {
+                                          uint32_t* og, uint32_t* ou, int code = 0) {
   if constexpr (POLY) {
-    if (code == 1) return glu_bwd32_code<1>(r, g, u, og, ou, w, dot);
-    if (code == 5) return glu_bwd32_code<5>(r, g, u, og, ou, w, dot);
+    if (code == 1) return glu_bwd32_code<1>(r, g, u, og, ou);
+    if (code == 5) return glu_bwd32_code<5>(r, g, u, og, ou);
   }
-  glu_bwd32_code<0>(r, g, u, og, ou, w, dot);
+  glu_bwd32_code<0>(r, g, u, og, ou);
 }
 
 // four packed pairs in place: gi = grad_inter, already rounded; g, u = gate, up -> grad_gate, grad_up
@@ -280,9 +273,9 @@ __device__ __forceinline__ void glu_bwd_pairs_code(const uint32_t (&gi)[4], uint
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const float2 gf = unpack_bf16x2(g[b]), uf = unpack_bf16x2(u[b]), go = unpack_bf16x2(gi[b]);
-    float gg0, gu0, gg1, gu1, f;
-    glu_bwd_val<CODE>(gf.x, uf.x, go.x, gg0, gu0, f);
-    glu_bwd_val<CODE>(gf.y, uf.y, go.y, gg1, gu1, f);
+    float gg0, gu0, gg1, gu1;
+    glu_bwd_val<CODE>(gf.x, uf.x, go.x, gg0, gu0);
+    glu_bwd_val<CODE>(gf.y, uf.y, go.y, gg1, gu1);
     g[b] = pack_bf16x2(gg0, gg1);
     u[b] = pack_bf16x2(gu0, gu1);
   }
@@ -447,6 +440,7 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t 
                  box_outer);
   return 0;
 }
+
 
 // A gate|up stack (E, 2I, K) as {K, 8, 2, I/8, E}: a box of {64, 8, 2, 8, 1} holds eight groups of 8 gate rows and the 8 up rows of
 // the same columns, so that a 16-lane block of an accumulator has gate and up of 8 columns in the same threads

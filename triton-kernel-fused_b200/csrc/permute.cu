@@ -56,7 +56,7 @@ template <int W, int PL>
 __global__ void __launch_bounds__(32 * W)
 permute_rank_kernel(const long long* idx, long long M, int E, const int* block_hist, int* counts, int* offs, int* poffs,
                     int* slot_row, int* row_slot, int* tile_expert, int* order, int* slot_pos, int* counts_out,
-                    long long* load, const RowWeights rows, int* status) {
+                    long long* load, int* status) {
   grid_dep_begin();
   constexpr int kPermWarps = W, kPermThreads = 32 * W;
   extern __shared__ int sh[];                          // [W][E]: ranks a warp's run starts at
@@ -173,10 +173,7 @@ permute_rank_kernel(const long long* idx, long long M, int E, const int* block_h
     }
   for (int e = blockIdx.x * kPermWarps + warp; e < E; e += gridDim.x * kPermWarps) {
     const int p0 = s_poff[e], p1 = s_poff[e + 1];
-    for (int r = p0 + s_cnt[e] + lane; r < p1; r += 32) {                          // pad rows of this expert
-      row_slot[r] = -1;
-      if (rows.row_w != nullptr) rows.row_w[r] = 0.0f;
-    }
+    for (int r = p0 + s_cnt[e] + lane; r < p1; r += 32) row_slot[r] = -1;          // pad rows of this expert
     for (int t = p0 / B200MOE_TILE_M + lane; t < p1 / B200MOE_TILE_M; t += 32) tile_expert[t] = e;
   }
 #pragma unroll
@@ -187,7 +184,6 @@ permute_rank_kernel(const long long* idx, long long M, int E, const int* block_h
       const int prow = s_poff[ex[i]] + r, pos = s_off[ex[i]] + r;
       slot_row[s] = prow;
       row_slot[prow] = static_cast<int>(s);
-      if (rows.row_w != nullptr) rows.row_w[prow] = rows.slot_w[s];
       if (order != nullptr) order[pos] = static_cast<int>(s);
       if (slot_pos != nullptr) slot_pos[s] = pos;
     } else if (s < M) {
@@ -202,14 +198,14 @@ permute_rank_kernel(const long long* idx, long long M, int E, const int* block_h
 template <int W, int PL>
 static int launch_permute(const long long* idx, long long M, int E, int* hist, int* counts, int* offs, int* poffs,
                           int* slot_row, int* row_slot, int* tile_expert, int* order, int* slot_pos, int* counts_out,
-                          long long* load, const RowWeights& rows, int* status, cudaStream_t st) {
+                          long long* load, int* status, cudaStream_t st) {
   constexpr int run = 32 * W * PL;
   const int blocks = M > run ? static_cast<int>((M + run - 1) / run) : 1;
   if (blocks > 1) {
     B200_LAUNCH((permute_hist_kernel<W, PL>), blocks, 32 * W, 0, st, idx, M, E, hist);
   }
   B200_LAUNCH((permute_rank_kernel<W, PL>), blocks, 32 * W, sizeof(int) * W * E, st, idx, M, E, hist, counts, offs, poffs,
-              slot_row, row_slot, tile_expert, order, slot_pos, counts_out, load, rows, status);
+              slot_row, row_slot, tile_expert, order, slot_pos, counts_out, load, status);
   return 0;
 }
 
@@ -234,7 +230,7 @@ gather_rows_kernel(const uint4* x, const int* row_slot, const int* total_rows, i
 int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs,
                   int32_t* poffs, int32_t* slot_row, int32_t* row_slot, int32_t* tile_expert,
                   int32_t* order, int32_t* slot_pos, void* ws, size_t ws_bytes,
-                  int32_t* counts_out, int64_t* load, const RowWeights& rows, int32_t* status, b200moe_stream_t stream) {
+                  int32_t* counts_out, int64_t* load, int32_t* status, b200moe_stream_t stream) {
   B200_CHECK_ARG(idx && counts && offs && poffs && slot_row && row_slot && tile_expert && ws && status,
                  B200MOE_E_NULL, "permute_build: null pointer");
   B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
@@ -252,7 +248,7 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
                 : split.warps == 16  ? launch_permute<16, 4>
                              : launch_permute<32, 4>;
   return launch(reinterpret_cast<const long long*>(idx), M, E, reinterpret_cast<int*>(ws), counts, offs, poffs, slot_row,
-                row_slot, tile_expert, order, slot_pos, counts_out, reinterpret_cast<long long*>(load), rows, status, (cudaStream_t)stream);
+                row_slot, tile_expert, order, slot_pos, counts_out, reinterpret_cast<long long*>(load), status, (cudaStream_t)stream);
 }
 
 int gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H, int64_t ldh, int64_t rows_cap, void* x_s,
@@ -296,7 +292,7 @@ int b200moe_permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* 
                           int32_t* order, int32_t* slot_pos, void* ws, size_t ws_bytes, int32_t* status,
                           b200moe_stream_t stream) {
   return permute_build(idx, T, k, E, counts, offs, poffs, slot_row, row_slot, tile_expert, order, slot_pos, ws, ws_bytes,
-                       nullptr, nullptr, RowWeights{}, status, stream);
+                       nullptr, nullptr, status, stream);
 }
 
 int b200moe_gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H,

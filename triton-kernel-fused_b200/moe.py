@@ -76,7 +76,7 @@ def _experts_backward(ctx, grad_out, need, want_params):
     dev = ws.device
     grad_out = grad_out.to(torch.bfloat16).contiguous()
     lib, bf16 = L.lib(), dict(dtype=torch.bfloat16, device=dev)
-    grad_w = torch.empty(N, k, dtype=torch.float32, device=dev) if need_w else None
+    grad_w = torch.empty(N, k, dtype=torch.float32, device=dev)
     grad_x = torch.empty(N, H, **bf16) if need_x else None
     grad_gu = torch.empty(n_glu, 2 * I, H, **bf16) if need_gu else None
     grad_dn = torch.empty(n_glu, H, I, **bf16) if need_dn else None
@@ -84,7 +84,7 @@ def _experts_backward(ctx, grad_out, need, want_params):
     tmp = L.workspace(lib.b200moe_moe_bwd_ws_bytes(N, H, I, E, n_glu, k, row_kernels), dev)
     L.check(lib.b200moe_moe_backward(grad_out.data_ptr(), w32.data_ptr(), gate_up_proj.data_ptr(), down_proj.data_ptr(),
                                      L.ptr(codes_dev), L.ptr(params), N, H, I, E, n_glu, k, row_kernels, ws.data_ptr(),
-                                     tmp.data_ptr(), L.ptr(grad_x), L.ptr(grad_w), L.ptr(grad_gu), L.ptr(grad_dn),
+                                     tmp.data_ptr(), L.ptr(grad_x), grad_w.data_ptr(), L.ptr(grad_gu), L.ptr(grad_dn),
                                      L.ptr(grad_ap), L.status_word(dev).data_ptr(), L.stream_of(ws)))
     return grad_x, (grad_w.to(ctx.wt_dtype) if need_w else None), grad_gu, grad_dn, grad_ap
 
