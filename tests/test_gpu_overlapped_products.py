@@ -1,4 +1,4 @@
-"""GPU: products of a backward that begin beside the end of the kernel before them (`early`, csrc/common.cuh) against plain launches."""
+"""GPU: a backward in chained launches, whose kernels are set up beside the end of the one before them (csrc/common.cuh), against plain launches."""
 import pytest
 import torch
 
@@ -7,7 +7,7 @@ DEV = "cuda"
 
 
 # single-CTA tiles, pair tiles of few and of several waves, row kernels with special experts; passes of other routings one after the other in the same
-# memory, so that a table or an operand read too early would be the one of the pass before; every subset of gradients that changes who runs beside whom
+# memory, so that a table or an operand read too early would be the one of the pass before; every subset of gradients that changes which kernels follow each other
 @pytest.mark.parametrize("T,H,I,E,k,codes", [(512, 256, 512, 8, 2, (0,)), (3001, 1032, 680, 16, 4, (0, 1, 5)), (1200, 520, 264, 9, 2, (2, 0, 7)),
                                              (20, 72, 40, 3, 1, (0,)), (8200, 1032, 200, 6, 4, (0,))])
 def test_overlapped_products_equal_plain_launches(pkg, T, H, I, E, k, codes):
@@ -43,7 +43,7 @@ def test_overlapped_products_equal_plain_launches(pkg, T, H, I, E, k, codes):
             assert all(torch.equal(s, t) for s, t in zip(a, b)), (want, p)
 
 
-# the router's backward: its top-k kernel beside the experts' last product, its weight gradient beside its dX
+# the router's backward behind the experts': its top-k kernel, dX and the weight gradient
 @pytest.mark.parametrize("T,H,E,k", [(512, 256, 8, 2), (3001, 1032, 32, 4), (2500, 264, 128, 8)])
 def test_overlapped_router_backward_equals_plain_launches(pkg, T, H, E, k):
     torch.manual_seed(T)

@@ -284,6 +284,30 @@ def test_chained_kernels_promise_no_constant_data():
         assert not re.search(r"__ldg\(|ld\.global\.nc", sources[shared]), shared
 
 
+def test_chained_kernels_wait_before_they_read():
+    """Every chained kernel waits for the one before it, in all of its threads, before it lets the next one begin and before it names what its
+    pointers point to.  The few-rows kernel's loads of weights ahead of its wait are the only exception."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), PKG, "csrc")
+    sources = {f: re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read()) for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))}
+    exceptions = []
+    for name, text in sources.items():
+        for kernel in re.split(r"(?=\b__global__\b)", text)[1:]:
+            head, body = kernel.split("{", 1)
+            calls = list(re.finditer(r"\bgrid_dep_(\w+)\(", body))
+            if not calls:
+                continue
+            title = re.search(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\(.*?\)\)?", "", head, flags=re.S)).group(1)
+            assert {c.group(1) for c in calls} <= {"wait", "begin", "launch"}, (name, title)
+            before = body[:calls[0].start()]
+            if re.search(r"(\)|\belse|[?:&|])\s*$", before):                        # the wait hangs on a condition
+                exceptions.append(title)
+                continue
+            assert before.count("{") == before.count("}") and calls[0].group(1) in ("wait", "begin"), (name, title)
+            for pointer in re.findall(r"\*\s*(?:const\s+)?(\w+)\s*[,)]", head):
+                assert not re.search(r"\b%s\b" % pointer, before), (name, title, pointer)
+    assert exceptions == ["few_rows_kernel"]
+
+
 def test_kept_copies_of_stacks_are_safe_on_other_streams(monkeypatch):
     """Quantised and bf16 copies that one stream made: a call on another stream waits for it before it reads them, until they are
     known to be complete, and records itself as a user of their memory; the stream that made them does neither (the default stream records its event when one is asked for)."""

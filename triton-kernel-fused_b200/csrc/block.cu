@@ -208,31 +208,23 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
   const int32_t* total = f.poffs + d.E;
   const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
   RUN("combine_bwd", 1, combine_bwd(grad_out, f.eo, w, f.row_slot, total, d.k, d.H, ldh, rows, b.grad_eo, g.w, st));
-  // The weight gradient of the down products needs nothing of the product in front of it, and the rows' gradient nothing of the other weight
-  // gradient: each begins on the SMs that the kernel before has left (`early`), so their last waves overlap.  (b.grad_x_s may be
-  // b.grad_eo: the last reader of that is complete when the second weight gradient has passed its wait.)
   const int n = d.n_glu;
-  bool beside = true;                                    // whether a kernel that waits stands between here and combine_bwd
-  if (d.kind == KIND_TILES) {
-    beside = g.x != nullptr || g.gate_up != nullptr;
-    if (beside)
-      RUN("expert_down_dgrad_glu", 1, expert_down_dgrad(b.grad_eo, ldh, down_proj, f.gate_up, ld2, codes, f.tile_expert, f.poffs, rows, 0, 0,
-                                                        d.E, d.H, d.I, b.grad_gu, status, st));
-  } else {
-    RUN("expert_linear_t", 1, expert_linear_t(b.grad_eo, ldh, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, d.H, b.grad_inter, ldi, 0, status, st));
-  }
-  if (g.down != nullptr)
-    RUN("expert_wgrad", 1, expert_wgrad(b.grad_eo, ldh, f.inter, ldi, f.poffs, f.counts, rows, n, d.H, d.I, g.down, beside, status, st));
   float* da = g.params != nullptr ? b.row_da : nullptr;
   float* dg = g.params != nullptr ? b.row_dg : nullptr;
-  if (d.kind == KIND_ROWS)
+  if (d.kind == KIND_ROWS) {
+    RUN("expert_linear_t", 1, expert_linear_t(b.grad_eo, ldh, down_proj, f.tile_expert, f.poffs, rows, n, d.H, d.I, d.H, b.grad_inter, ldi, status, st));
     RUN("glu_bwd_rows", 1, glu_bwd_rows(b.grad_inter, ldi, f.gate_up, ld2, f.tile_expert, codes, params, f.poffs + n, rows, d.I, b.grad_gu, da, dg, st));
+  } else if (g.x != nullptr || g.gate_up != nullptr) {
+    RUN("expert_down_dgrad_glu", 1, expert_down_dgrad(b.grad_eo, ldh, down_proj, f.gate_up, ld2, codes, f.tile_expert, f.poffs, rows, 0, 0,
+                                                      d.E, d.H, d.I, b.grad_gu, status, st));
+  }
+  if (g.down != nullptr)
+    RUN("expert_wgrad", 1, expert_wgrad(b.grad_eo, ldh, f.inter, ldi, f.poffs, f.counts, rows, n, d.H, d.I, g.down, status, st));
   if (g.gate_up != nullptr)
-    RUN("expert_wgrad", 1, expert_wgrad(b.grad_gu, ld2, f.x_s, ldh, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, 0, status, st));
+    RUN("expert_wgrad", 1, expert_wgrad(b.grad_gu, ld2, f.x_s, ldh, f.poffs, f.counts, rows, n, 2 * d.I, d.H, g.gate_up, status, st));
   if (g.x != nullptr) {
     RUN(d.kind == KIND_ROWS ? "expert_linear_t" : "expert_gate_up_dgrad", 1,
-        expert_linear_t(b.grad_gu, ld2, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, 2 * d.I, b.grad_x_s, ldh, g.gate_up != nullptr,
-                        status, st));
+        expert_linear_t(b.grad_gu, ld2, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, 2 * d.I, b.grad_x_s, ldh, status, st));
     if (d.kind == KIND_ROWS && n < d.E)
       RUN("special_rows", 1, special_rows(b.grad_eo, f.tile_expert, codes, f.poffs, n, d.E, d.H, ldh, rows, b.grad_x_s, st));
   }
@@ -262,15 +254,15 @@ static int router_forward(const void* x, const void* weight, const float* bias, 
 
 static int router_backward(const void* x, const void* weight, const void* logits, const int64_t* idx, const float* grad_w,
                            int64_t T, int64_t H, int E, int k, int norm, float scale, void* grad_logits, float* part,
-                           void* grad_x, void* grad_weight, int early, int32_t* status, b200moe_stream_t st) {
-  RUN("router_topk_bwd", 1, router_topk_bwd(logits, B200MOE_LOGITS_BF16, idx, grad_w, T, E, k, norm, scale, early, grad_logits, st));
+                           void* grad_x, void* grad_weight, int32_t* status, b200moe_stream_t st) {
+  RUN("router_topk_bwd", 1, b200moe_router_topk_bwd(logits, B200MOE_LOGITS_BF16, idx, grad_w, T, E, k, norm, scale, grad_logits, st));
   if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(grad_logits, weight, grad_x, T, H, E, status, st));
   if (grad_weight != nullptr) {
     OpScope scope("gemm_tn", 2);
     const Split sp = router_split(T, E, H, gemm_cta_budget());
     const bool tr = router_dw_transposed(E);
-    int rc = tr ? gemm_tn_splitk(x, grad_logits, part, H, E, T, sp.chunk, grad_x != nullptr, status, st)
-                : gemm_tn_splitk(grad_logits, x, part, E, H, T, sp.chunk, grad_x != nullptr, status, st);
+    int rc = tr ? b200moe_gemm_tn_splitk(x, grad_logits, part, H, E, T, sp.chunk, status, st)
+                : b200moe_gemm_tn_splitk(grad_logits, x, part, E, H, T, sp.chunk, status, st);
     if (rc) return rc;
     rc = tr ? b200moe_splitk_reduce_t(part, sp.slices, H, E, grad_weight, st)
             : b200moe_splitk_reduce(part, sp.slices, static_cast<int64_t>(E) * H, grad_weight, st);
@@ -319,7 +311,7 @@ int b200moe_router_backward(const void* x, const void* weight, const void* logit
   Carver c(ws);
   bf16_t* gl = c.take<bf16_t>(T * E);
   float* part = c.take<float>(router_split(T, E, H, num_sms()).slices * E * H);
-  return router_backward(x, weight, logits, idx, grad_w, T, H, E, k, norm_topk, scale, gl, part, grad_x, grad_weight, 0, status, stream);
+  return router_backward(x, weight, logits, idx, grad_w, T, H, E, k, norm_topk, scale, gl, part, grad_x, grad_weight, status, stream);
 }
 
 // ---------------------------------------------------------------------------- conv router
@@ -407,7 +399,7 @@ int b200moe_conv_router_backward(const void* x, const void* weight_rows, const v
   if (grad_x != nullptr) RUN("gemm_nn", 1, b200moe_gemm_nn(b.u, weight_rows, grad_x, T, H, rows, status, stream));
   if (grad_weight != nullptr) {
     const Split sp = conv_split(T, rows, H, gemm_cta_budget());
-    RUN("gemm_tn_splitk", 1, gemm_tn_splitk(b.u, x, b.part, rows, H, T, sp.chunk, grad_x != nullptr, status, stream));
+    RUN("gemm_tn_splitk", 1, b200moe_gemm_tn_splitk(b.u, x, b.part, rows, H, T, sp.chunk, status, stream));
     RUN("conv_weight_grad", 1, b200moe_conv_weight_grad(b.part, sp.slices, E, H, taps, grad_weight, stream));
   }
   return 0;
@@ -504,7 +496,7 @@ int b200moe_layer_backward(const void* grad_out, const void* x, const void* gate
   if (rc) return rc;
   if (grad_x != nullptr || grad_gate_weight != nullptr) {
     rc = router_backward(x, gate_weight, f.logits, f.idx, b.grad_w, T, H, E, k, norm_topk, scale, b.grad_logits, b.part,
-                         grad_x != nullptr ? b.grad_x_router : nullptr, grad_gate_weight, grad_x != nullptr, status, stream);
+                         grad_x != nullptr ? b.grad_x_router : nullptr, grad_gate_weight, status, stream);
     if (rc) return rc;
   }
   if (grad_x != nullptr)   // the experts' rows of a token and the router's share, added in fp32, one rounding
@@ -528,7 +520,7 @@ int b200moe_newton_schulz(void* x, void* x_next, void* a, void* a2, const int32_
     const float ca = coeffs[3 * i], cb = coeffs[3 * i + 1], cc = coeffs[3 * i + 2];
     RUN("expert_gram", 1, expert_gram(x, tile_expert, poffs, rows, E, wide, 1, live, a, status, stream));
     RUN("expert_linear_axpby", 1, expert_linear_axpby(a, a, a, cc, cb, ca, 2, tile_expert, poffs, rows, E, Rp, Rp, live, live, a2, status, stream));
-    RUN("expert_linear_t", 1, expert_linear_t(a2, Rp, x, tile_expert, poffs, rows, E, Rp, wide, live, x_next, wide, 0, status, stream));
+    RUN("expert_linear_t", 1, expert_linear_t(a2, Rp, x, tile_expert, poffs, rows, E, Rp, wide, live, x_next, wide, status, stream));
     std::swap(x, x_next);
   }
   return 0;

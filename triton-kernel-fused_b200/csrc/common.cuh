@@ -36,10 +36,6 @@ int exchange_sm_budget();   // SMs (= fat CTAs) the home-side pull kernel of the
 // tokens, 64 of 520 x 264, top-6 776 / 722; 2000 tokens, 8 of 264 x 136, top-2 80 / 77.
 inline int64_t row_pitch(int64_t n) { return n % 32 == 0 ? n : (n + 63) / 64 * 64; }
 
-// `early` in what follows: the kernel does not wait for the one in front of it, whose last wave it runs beside, but ends after it.  What it
-// reads, and whoever reads what it overwrites, was complete when some kernel before it in the stream had passed its wait: a kernel's CTAs are
-// placed once those of the one before have all called grid_dep_launch(), which a kernel that waits does after its wait.  us a training pass
-// without / with: 3001 tokens, 32 experts of 1032 x 680 350 / 338; 3000 tokens, 16 of 520 x 264 132 / 125; 512 tokens, 8 of 256 x 512 70 / 66.
 // The entry points of the block's steps with the distance between rows given (elements): of x_s, the experts' results and their gradients
 // (ldh), of inter (ldi), of gate_up and its gradient (ld2)
 int gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H, int64_t ldh, int64_t rows_cap, void* x_s,
@@ -64,7 +60,7 @@ int expert_down_dgrad(const void* grad_eo, int64_t ldh, const void* down_proj, c
 int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N,
                   int64_t K, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream);
 int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
-                 int64_t Na, int64_t Nb, void* out, int early, int32_t* status, b200moe_stream_t stream);
+                 int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream);
 
 // b200moe_permute_build; also stores the counts a second time (counts_out) and adds them to `load` (both nullable)
 int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, int32_t* offs, int32_t* poffs,
@@ -75,11 +71,6 @@ int permute_build(const int64_t* idx, int64_t T, int k, int E, int32_t* counts, 
 int conv_weight_rows(const void* w, int E, int64_t H, int taps, int by_expert, void* wt, int32_t* counts, b200moe_stream_t stream);
 int router_topk_fwd(const void* input, int input_kind, const float* bias, int64_t T, int E, int k, int norm_topk, float scale, int64_t* idx,
                     float* w, int32_t* counts, bool counts_cleared, b200moe_stream_t stream);
-
-int router_topk_bwd(const void* logits, int input_kind, const int64_t* idx, const float* grad_w, int64_t T, int E, int k, int norm_topk,
-                    float scale, int early, void* grad_logits, b200moe_stream_t stream);
-int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K, int64_t k_chunk, int early, int32_t* status,
-                   b200moe_stream_t stream);
 
 // gemm_few.cu: whether a forward that no backward follows runs M routed rows over compact rows or over row tiles
 bool few_rows_forward(int64_t M, int E, int64_t H, int64_t I);
@@ -97,7 +88,7 @@ int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha
                         const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E, int64_t N, int64_t K,
                         int64_t n_live, int64_t k_live, void* out, int32_t* status, b200moe_stream_t stream);
 int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
-                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int early, int32_t* status, b200moe_stream_t stream);
+                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream);
 
 // Tells the observer set by b200moe_set_observer, if any, where an operation of a longer sequence begins and ends
 struct OpScope {
@@ -133,7 +124,11 @@ inline void by_row_threads(int nvec, F f) {
 // Launch whose set-up may overlap the end of the kernel before it in the stream (programmatic stream serialisation).  Every
 // kernel launched this way calls grid_dep_wait() (ptx.cuh) in all of its threads before it reads or writes anything that
 // another kernel touches, and grid_dep_launch() only after that: when a kernel's first instruction runs, the kernel two
-// before it is complete, and past its wait the one before it too.  Its pointers are neither __restrict__ nor read by __ldg: both
+// before it is complete, and past its wait the one before it too.  What those wrote is visible past the wait only: nothing orders a
+// kernel's first reads behind writes that another kernel waited for.  (Products of a backward that neither wait for the one before them nor need
+// anything of it took 3 % off a pass of 3001 tokens, 32 experts of 1032 x 680; nothing that the programming model states made them correct.)  One
+// exception, FewParams::early in gemm_few.cu, says there what it rests on.
+// A kernel's pointers are neither __restrict__ nor read by __ldg: both
 // promise the compiler data that stays as it is for the kernel's whole life, which begins before the wait, so it could load ahead
 // of the wait or past the coherent cache.  (Taking the promises out cost next to nothing: combine of 98 304 rows of 2048 96.4 /
 // 96.3 us, both quantisers of them 186 / 184, GLU backward of 1408 columns 457 / 457, the conv router's pass 115.0 / 115.3.)  Why: between two plain launches the SMs idle for 1.5 to 4

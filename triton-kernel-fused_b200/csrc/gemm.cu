@@ -86,15 +86,13 @@ __device__ __forceinline__ int pair_cols(const GemmParams& p, int n0) {
 // POLY: the variant of the kernel.  GLU epilogues: per-expert activation codes 0 / 1 / 5 (p.act_codes); false =
 // SiLU for every expert.  Store epilogues (EPI_STORE, EPI_STORE_F32): a convolution operand (p.conv_taps), compiled
 // only into the instantiations the conv-router entry points launch, so that the expert GEMMs carry no code for it.
-// EARLY: a kernel that does not wait for the one before it (`early`, common.cuh; asked at run time it cost every launch 0.2 us: 15
-// products of 1 x 1408 x 2048 236.8 -> 240.2 us, of 8 x 1024 x 1408 337.5 -> 341.7; compiled in 236.8 and 338.0).
 // Single-CTA tiles have two loading warps, one for A and one for B: a k-block's MMAs take 256 cycles there, but one thread's wait, its two
 // boxes and a convolution's coordinates 480 (380 without those), whatever the batch.  Logits of 16 x 1024 positions of H 2048, 64 experts, 4
 // taps (us): one loading warp 35.7, two 29.8, the next stage's barrier asked for ahead 28.6, the convolution in a loop of its own 24.7; of
 // 1 x 1024 positions 34.2 -> 23.4.  Products of few k-blocks are as fast as before.
 __host__ __device__ constexpr int gemm_threads(int ctas) { return ctas == 1 ? kThreads + 32 : kThreads; }
 
-template <int BN, int EPI, int CTAS, bool POLY = false, bool EARLY = false>
+template <int BN, int EPI, int CTAS, bool POLY = false>
 __global__ void __launch_bounds__(gemm_threads(CTAS), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
@@ -151,8 +149,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   }
   __shared__ int s_order[B200MOE_MAX_EXPERTS];
-  if constexpr (EARLY) grid_dep_early();
-  else grid_dep_wait();
+  grid_dep_wait();
   const int* order = build_group_order(p, s_order);
   tc_fence_before();
   __syncthreads();
@@ -683,7 +680,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   }
 
   // ------------------------------------------------------------------ tear-down
-  if constexpr (EARLY) grid_dep_wait();      // so that this kernel's end is also that of the one before it
   tc_fence_before();
   __syncthreads();
   if constexpr (CTAS == 2) {   // nobody leaves while the peer may still touch it
@@ -700,21 +696,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------------------- host side
-template <int BN, int EPI, int CTAS, bool POLY = false, bool EARLY = false>
+template <int BN, int EPI, int CTAS, bool POLY = false>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD, const CUtensorMap& tmD2,
                   const GemmParams& p, int max_tiles, cudaStream_t stream) {
   using C = Cfg<BN, CTAS, epi_warp_bytes<BN, EPI>()>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(gemm_kernel<BN, EPI, CTAS, POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(max dynamic smem)");
   int units = gemm_cta_budget() / CTAS;  // CTAs, or CTA pairs
   if (max_tiles > 0 && max_tiles < units) units = max_tiles;
   if (units < 1) units = 1;
-  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY, EARLY>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
+  B200_CUDA(launch_chained(gemm_kernel<BN, EPI, CTAS, POLY>, units * CTAS, gemm_threads(CTAS), C::SMEM_BYTES, stream, CTAS, tmA, tmB, tmD, tmD2, p));
   return 0;
 }
 
@@ -781,7 +777,7 @@ static int pick_bn_rows(long long n, long long rows_cap, int E, int cols_per_bn 
 
 // d1 / d2 describe the bf16 outputs as {columns, rows, groups} tensors for the TMA-store epilogue
 // (d2 = the SwiGLU `inter` output); they are ignored by the kernels that store directly.
-template <int EPI, bool POLY = false, bool EARLY = false>
+template <int EPI, bool POLY = false>
 static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand* d1, const Operand* d2,
                        GemmParams& p, int max_tiles, cudaStream_t stream) {
   const bool pair = (bn == 256) && (p.sched != SCHED_DENSE) && pairs_enabled();
@@ -820,18 +816,18 @@ static int dispatch_bn(int bn, const Operand& A, const Operand& B, const Operand
       }
     }
   }
-  if (pair) return launch<256, EPI, 2, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
+  if (pair) return launch<256, EPI, 2, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles > 0 ? (max_tiles + 1) / 2 : 0, stream);
   if constexpr (EPI == EPI_AXPBY || EPI == EPI_STORE_SYM) {   // built for the 256-wide TMA-store epilogue only
     if (bn == 256) return launch<256, EPI, 1>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     set_error("tile width %d not built for this epilogue", bn);
     return B200MOE_E_UNSUPPORTED;
   } else
   switch (bn) {
-    case 256: return launch<256, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
-    case 128: return launch<128, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 256: return launch<256, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+    case 128: return launch<128, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
     default:
       if constexpr (EPI == EPI_STORE || EPI == EPI_STORE_F32)
-        return launch<64, EPI, 1, POLY, EARLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
+        return launch<64, EPI, 1, POLY>(tmA, tmB, tmD, tmD2, p, max_tiles, stream);
       set_error("tile width %d not built for this epilogue", bn);
       return B200MOE_E_UNSUPPORTED;
   }
@@ -898,7 +894,7 @@ int expert_linear_axpby(const void* a, const void* w, const void* c, float alpha
 }
 
 int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* tile_expert, const int32_t* poffs, int64_t rows_cap, int E,
-                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int early, int32_t* status, b200moe_stream_t stream) {
+                    int64_t K, int64_t N, int64_t k_live, void* out, int64_t ldo, int32_t* status, b200moe_stream_t stream) {
   int rc = check_grouped("expert_linear_t", a, w, out, tile_expert, poffs, rows_cap, E, N, K);
   if (rc) return rc;
   B200_CHECK_ARG(tile_expert, B200MOE_E_NULL, "expert_linear_t: null pointer");
@@ -909,9 +905,7 @@ int expert_linear_t(const void* a, int64_t lda, const void* w, const int32_t* ti
   p.sched = SCHED_GROUPED_M; p.b_mn = 1; p.N = (int)N; p.K = (int)k_live; p.num_groups = E;
   p.tile_expert = tile_expert; p.poffs = poffs; p.D = out; p.ldd = ldo; p.status = status;
   Operand d{out, 0, rows_cap, N, ldo, 1, rows_cap * ldo};
-  const int bn = pick_bn_rows(N, rows_cap, E);
-  return early ? dispatch_bn<EPI_STORE, false, true>(bn, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream)
-               : dispatch_bn<EPI_STORE>(bn, oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
+  return dispatch_bn<EPI_STORE>(pick_bn_rows(N, rows_cap, E), oa, ob, &d, nullptr, p, 0, (cudaStream_t)stream);
 }
 
 // row window of a grouped-M launch: (0, 0) = every row, else tile-aligned 0 <= row_lo < row_hi <= rows_cap
@@ -989,7 +983,7 @@ int expert_linear(const void* a, int64_t lda, const void* w, const int32_t* tile
 }
 
 int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const int32_t* poffs, const int32_t* counts, int64_t rows_cap, int E,
-                 int64_t Na, int64_t Nb, void* out, int early, int32_t* status, b200moe_stream_t stream) {
+                 int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
   B200_CHECK_ARG(A && B && poffs && out, B200MOE_E_NULL, "expert_wgrad: null pointer");
   B200_CHECK_ARG(E >= 1, B200MOE_E_BAD_SHAPE, "expert_wgrad: E = %d", E);
   B200_CHECK_ARG(rows_cap > 0 && rows_cap % B200MOE_TILE_M == 0 && rows_cap < (1LL << 31), B200MOE_E_BAD_SHAPE,
@@ -1005,33 +999,7 @@ int expert_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, const i
   const int bn = pick_bn_grouped(Nb, 64, E * ceil_div(Na, 256), E * ceil_div(Na, BM));
   Operand d{out, 0, Na, Nb, Nb, E, Na * Nb};
   const int tiles = (int)std::min<long long>(1 << 30, E * ceil_div(Na, BM) * ceil_div(Nb, bn));
-  return early ? dispatch_bn<EPI_STORE, false, true>(bn, a, b, &d, nullptr, p, tiles, (cudaStream_t)stream)
-               : dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, tiles, (cudaStream_t)stream);
-}
-
-int gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K, int64_t k_chunk, int early, int32_t* status,
-                   b200moe_stream_t stream) {
-  B200_CHECK_ARG(A && B && P, B200MOE_E_NULL, "gemm_tn_splitk: null pointer");
-  CHECK_DIM8(M); CHECK_DIM8(N); CHECK_I32(M); CHECK_I32(N); CHECK_I32(K);
-  B200_CHECK_ARG(k_chunk > 0 && k_chunk % 64 == 0, B200MOE_E_BAD_SHAPE,
-                 "gemm_tn_splitk: k_chunk = %lld must be a positive multiple of 64", (long long)k_chunk);
-  B200_CHECK_ARG(K > 0, B200MOE_E_BAD_SHAPE, "gemm_tn_splitk: K must be positive");
-  B200_CHECK_ARG(aligned16(P), B200MOE_E_ALIGN, "gemm_tn_splitk: P not 16-byte aligned");
-  const long long slices = ceil_div(K, k_chunk);
-  Operand a{A, 1, M, K, M, 1, M * K};   // stored (K, M)
-  Operand b{B, 1, N, K, N, 1, N * K};   // stored (K, N)
-  GemmParams p{};
-  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
-  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
-  // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
-  // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
-  // 1024 16.1 / 6.5.
-  const int bn = M <= BM ? std::min(pick_bn(N), 128)
-                         : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
-  const int tiles = (int)(slices * ceil_div(M, BM) * ceil_div(N, bn));
-  return early ? dispatch_bn<EPI_STORE_F32, false, true>(bn, a, b, nullptr, nullptr, p, tiles, (cudaStream_t)stream)
-               : dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, tiles, (cudaStream_t)stream);
+  return dispatch_bn<EPI_STORE>(bn, a, b, &d, nullptr, p, tiles, (cudaStream_t)stream);
 }
 
 }  // namespace b200moe
@@ -1074,7 +1042,26 @@ int b200moe_gemm_nn(const void* A, const void* B, void* D, int64_t M, int64_t N,
 
 int b200moe_gemm_tn_splitk(const void* A, const void* B, float* P, int64_t M, int64_t N, int64_t K,
                            int64_t k_chunk, int32_t* status, b200moe_stream_t stream) {
-  return gemm_tn_splitk(A, B, P, M, N, K, k_chunk, 0, status, stream);
+  B200_CHECK_ARG(A && B && P, B200MOE_E_NULL, "gemm_tn_splitk: null pointer");
+  CHECK_DIM8(M); CHECK_DIM8(N); CHECK_I32(M); CHECK_I32(N); CHECK_I32(K);
+  B200_CHECK_ARG(k_chunk > 0 && k_chunk % 64 == 0, B200MOE_E_BAD_SHAPE,
+                 "gemm_tn_splitk: k_chunk = %lld must be a positive multiple of 64", (long long)k_chunk);
+  B200_CHECK_ARG(K > 0, B200MOE_E_BAD_SHAPE, "gemm_tn_splitk: K must be positive");
+  B200_CHECK_ARG(aligned16(P), B200MOE_E_ALIGN, "gemm_tn_splitk: P not 16-byte aligned");
+  const long long slices = ceil_div(K, k_chunk);
+  Operand a{A, 1, M, K, M, 1, M * K};   // stored (K, M)
+  Operand b{B, 1, N, K, N, 1, N * K};   // stored (K, N)
+  GemmParams p{};
+  p.sched = SCHED_GROUPED_K; p.a_mn = 1; p.b_mn = 1; p.M = (int)M; p.N = (int)N; p.K = (int)K;
+  p.num_groups = (int)slices; p.k_chunk = (int)k_chunk; p.poffs = nullptr;
+  p.D = P; p.ldd = N; p.d_group_stride = M * N; p.status = status;
+  // Up to 128 rows the second half of a pair tile would multiply nothing but padding: single-CTA tiles.  us, 256-wide pair /
+  // 128-wide tiles, 16 384 tokens: 16 x 2048 22.8 / 14.0, 64 x 2048 24.7 / 15.1, 128 x 512 19.1 / 8.7; 1024 tokens, 128 x
+  // 1024 16.1 / 6.5.
+  const int bn = M <= BM ? std::min(pick_bn(N), 128)
+                         : pick_bn_grouped(N, 64, slices * ceil_div(M, 256), slices * ceil_div(M, BM));
+  return dispatch_bn<EPI_STORE_F32>(bn, a, b, nullptr, nullptr, p, (int)(slices * ceil_div(M, BM) * ceil_div(N, bn)),
+                                    (cudaStream_t)stream);
 }
 
 static int check_conv(const char* who, int64_t B, int64_t S, int64_t H, int64_t E, int taps, int64_t s_mult,
@@ -1203,7 +1190,7 @@ int b200moe_expert_linear_axpby(const void* a, const void* w, const void* c, flo
 int b200moe_expert_linear_t(const void* a, const void* w, const int32_t* tile_expert, const int32_t* poffs,
                             int64_t rows_cap, int E, int64_t K, int64_t N, void* out, int32_t* status,
                             b200moe_stream_t stream) {
-  return expert_linear_t(a, K, w, tile_expert, poffs, rows_cap, E, K, N, K, out, N, 0, status, stream);
+  return expert_linear_t(a, K, w, tile_expert, poffs, rows_cap, E, K, N, K, out, N, status, stream);
 }
 
 int b200moe_expert_linear_push(const void* a, const void* w, int w_kn, const int32_t* tile_expert, const int32_t* poffs,
@@ -1255,7 +1242,7 @@ int b200moe_expert_gate_up_dgrad(const void* grad_gate_up, const void* gate_up_p
 
 int b200moe_expert_wgrad(const void* A, const void* B, const int32_t* poffs, const int32_t* counts, int64_t rows_cap,
                          int E, int64_t Na, int64_t Nb, void* out, int32_t* status, b200moe_stream_t stream) {
-  return expert_wgrad(A, Na, B, Nb, poffs, counts, rows_cap, E, Na, Nb, out, 0, status, stream);
+  return expert_wgrad(A, Na, B, Nb, poffs, counts, rows_cap, E, Na, Nb, out, status, stream);
 }
 
 }  // extern "C"

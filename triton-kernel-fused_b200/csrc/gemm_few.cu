@@ -42,7 +42,9 @@ struct FewParams {
   int aligned;            // D is 16-byte aligned
   // Counts and weights were complete when the kernel in front had passed its own wait, so before this one began (its CTAs are
   // placed after that): the first blocks of weights are loaded before the wait for that kernel, so its end and this one's start
-  // cost no time on the memory bus.
+  // cost no time on the memory bus.  That they are visible here as well is an assumption: the programming model states it past the
+  // wait only.  It rests on a completed kernel's writes being in L2, where TMA reads the weights and few_tiles.cuh the counts.  Without it
+  // one token takes 36.5 us instead of 35.0, 48 tokens 187.8 instead of 184.7, 1500 tokens 263 instead of 258 (64 experts of 2048 x 1408).
   int early;
 };
 

@@ -157,12 +157,6 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the next kernel's CTAs may be placed once every CTA has got here (call it after grid_dep_wait only)
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// in place of the wait, in all threads, where a kernel ends after the one before it but does not begin after it (`early`, common.cuh): what it reads
-// is complete, but a line of it in L1 may be older
-__device__ __forceinline__ void grid_dep_early() {
-  if (threadIdx.x == 0) __threadfence();
-  __syncthreads();
-}
 __device__ __forceinline__ void grid_dep_begin() {
   grid_dep_wait();
   grid_dep_launch();

@@ -82,10 +82,8 @@ router_topk_fwd_kernel(const void* input, const float* bias, long long T, int E,
 template <int KIND, int VPL, bool PAIR>
 __global__ void __launch_bounds__(256)
 router_topk_bwd_kernel(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k,
-                       int norm, float scale, int S, int taps, int early, __nv_bfloat16* grad_logits) {
-  if (early) grid_dep_early();
-  else grid_dep_wait();
-  grid_dep_launch();
+                       int norm, float scale, int S, int taps, __nv_bfloat16* grad_logits) {
+  grid_dep_begin();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
@@ -149,7 +147,6 @@ router_topk_bwd_kernel(const void* logits, const long long* idx, const float* gr
       if (pos + back >= S) put(t * taps + j, zero);
     }
   }
-  if (early) grid_dep_wait();        // so that this kernel's end is also that of the one before it
 }
 
 // w (E, H, taps) -> wt (taps, E, H), wt[j, e, h] = w[e, h, j] (the operand of the conv router's products), or (E, taps, H).  counts (E,
@@ -246,14 +243,14 @@ static int grid_for_tokens(long long T) {
 
 template <int KIND>
 static cudaError_t launch_topk_bwd(const void* logits, const long long* idx, const float* grad_w, long long T, int E, int k, int norm,
-                            float scale, int S, int taps, int early, __nv_bfloat16* out, cudaStream_t st) {
+                            float scale, int S, int taps, __nv_bfloat16* out, cudaStream_t st) {
   const int grid = grid_for_tokens(T);
   cudaError_t err = cudaSuccess;
   by_experts(E, [&](auto v) {
     constexpr int VPL = v.value;
     const bool pair = VPL > 1 && E % 2 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0;
     err = launch_chained(pair ? router_topk_bwd_kernel<KIND, VPL, (VPL > 1)> : router_topk_bwd_kernel<KIND, VPL, false>, grid, 256, 0,
-                         st, 1, logits, idx, grad_w, T, E, k, norm, scale, S, taps, early, out);
+                         st, 1, logits, idx, grad_w, T, E, k, norm, scale, S, taps, out);
   });
   return err;
 }
@@ -303,30 +300,6 @@ int router_topk_fwd(const void* input, int input_kind, const float* bias, int64_
   return 0;
 }
 
-int router_topk_bwd(const void* logits, int input_kind, const int64_t* idx, const float* grad_w, int64_t T, int E, int k, int norm_topk,
-                    float scale, int early, void* grad_logits, b200moe_stream_t stream) {
-  B200_CHECK_ARG(logits && idx && grad_w && grad_logits, B200MOE_E_NULL, "router_topk_bwd: null pointer");
-  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
-                 "router_topk_bwd: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
-  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "router_topk_bwd: top_k = %d", k);
-  if (T <= 0) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  const long long* idx_ll = reinterpret_cast<const long long*>(idx);
-  __nv_bfloat16* gl = reinterpret_cast<__nv_bfloat16*>(grad_logits);
-  switch (input_kind) {
-    case B200MOE_LOGITS_BF16:
-      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, early, gl, st));
-      break;
-    case B200MOE_LOGITS_F32:
-      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_F32>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, early, gl, st));
-      break;
-    default:
-      set_error("router_topk_bwd: input_kind %d has no backward (logits are required)", input_kind);
-      return B200MOE_E_UNSUPPORTED;
-  }
-  return 0;
-}
-
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -341,7 +314,26 @@ int b200moe_router_topk_fwd(const void* input, int input_kind, const float* bias
 
 int b200moe_router_topk_bwd(const void* logits, int input_kind, const int64_t* idx, const float* grad_w, int64_t T,
                             int E, int k, int norm_topk, float scale, void* grad_logits, b200moe_stream_t stream) {
-  return router_topk_bwd(logits, input_kind, idx, grad_w, T, E, k, norm_topk, scale, 0, grad_logits, stream);
+  B200_CHECK_ARG(logits && idx && grad_w && grad_logits, B200MOE_E_NULL, "router_topk_bwd: null pointer");
+  B200_CHECK_ARG(E >= 1 && E <= B200MOE_MAX_EXPERTS, B200MOE_E_UNSUPPORTED,
+                 "router_topk_bwd: E = %d, supported 1..%d", E, B200MOE_MAX_EXPERTS);
+  B200_CHECK_ARG(k >= 1 && k <= E && k <= B200MOE_MAX_TOPK, B200MOE_E_BAD_SHAPE, "router_topk_bwd: top_k = %d", k);
+  if (T <= 0) return 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long* idx_ll = reinterpret_cast<const long long*>(idx);
+  __nv_bfloat16* gl = reinterpret_cast<__nv_bfloat16*>(grad_logits);
+  switch (input_kind) {
+    case B200MOE_LOGITS_BF16:
+      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st));
+      break;
+    case B200MOE_LOGITS_F32:
+      B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_F32>(logits, idx_ll, grad_w, T, E, k, norm_topk, scale, 1, 1, gl, st));
+      break;
+    default:
+      set_error("router_topk_bwd: input_kind %d has no backward (logits are required)", input_kind);
+      return B200MOE_E_UNSUPPORTED;
+  }
+  return 0;
 }
 
 int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* grad_w, int64_t B, int64_t S, int E, int taps,
@@ -353,7 +345,7 @@ int b200moe_conv_topk_bwd(const void* logits, const int64_t* idx, const float* g
   B200_CHECK_ARG(B >= 1 && S >= 1 && S < (1LL << 31) && taps >= 1 && taps <= 64, B200MOE_E_BAD_SHAPE,
                  "conv_topk_bwd: B = %lld, S = %lld, taps = %d (1..64)", (long long)B, (long long)S, taps);
   B200_CUDA(launch_topk_bwd<B200MOE_LOGITS_BF16>(logits, reinterpret_cast<const long long*>(idx), grad_w, B * S, E, k, norm_topk,
-                                                 scale, static_cast<int>(S), taps, 0, reinterpret_cast<__nv_bfloat16*>(u),
+                                                 scale, static_cast<int>(S), taps, reinterpret_cast<__nv_bfloat16*>(u),
                                                  (cudaStream_t)stream));
   return 0;
 }
