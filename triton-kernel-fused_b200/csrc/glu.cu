@@ -12,9 +12,10 @@
 // Rows of one CTA lie inside one 256-row tile and share its expert, so the activation code is uniform over the CTA and
 // the element loops are compiled per code.  The one-value-per-thread kernels below them read each value with a
 // 2-byte access, once per reduction; they remain for d_ff that is no multiple of 8 or above 8192 and for unaligned
-// buffers.  32 768 rows, codes 0 1 2 5 6 7 in turn, L2 flushed before, us (at copy rate): d_ff 768 forward 37 (25), backward 57 (41);
-// d_ff 1032 55 (33), 94 (55); 8192 rows of d_ff 4096 51 (31), 78 (52).  With divisions, rows of 64 x 2 and 128 x 2 vectors, and the
-// Norm codes' activations kept across the second reduction they took 53 / 98, 84 / 164 and 63 / 111.
+// buffers.  32 768 rows, codes 0 1 2 5 6 7 in turn, L2 flushed before, dense rows, us (at copy rate): d_ff 768 forward 37 (25), backward 59
+// (41); d_ff 1032 57 (33), 100 (55); 8192 rows of d_ff 4096 47 (31), 74 (52).  With divisions, rows of 64 x 2 and 128 x 2 vectors, and the
+// Norm codes' activations kept across the second reduction they took 51 / 96, 86 / 170 and 59 / 103.  1 - sigmoid and 1 - tanh^2 as differences: backward
+// 55, 107 and 72.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -74,22 +75,19 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
   return v;
 }
 
-// Reciprocal of 1 or more by the special-function unit, within one unit in the last place.  The correctly rounded division took more
-// instructions than the exponential beside it (forward 53 -> 44 us, backward 98 -> 80 of the rows above).
-__device__ __forceinline__ float rcp_above_1(float x) {
+// Reciprocal of a number from 0.5 to 2 by the special-function unit, within one unit in the last place.  The correctly rounded division took
+// more instructions than the exponential beside it (forward 53 -> 44 us, backward 98 -> 80 of 32 768 rows of d_ff 768, below).
+__device__ __forceinline__ float rcp_near_1(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// tanh(x) from e = exp(-2x): of the rounding errors only that of e is absolute (2 / (1 + e) - 1 has that of the quotient as well, next to
-// which a small tanh is lost).  An infinite e is -1, a NaN stays one.
-__device__ __forceinline__ float tanh_of_exp(float e) {
-  asm("min.NaN.f32 %0, %0, 0f7149F2CA;" : "+f"(e));     // 1e30
-  return (1.0f - e) * rcp_above_1(1.0f + e);
-}
 
 // activation value and its derivative with respect to gn (gn = gate, or gate / rms for the Norm codes).  Code 5:
 // dal = d(act)/d(alpha), t5s = act / gamma
+// Sigmoid and tanh from exponentials of -|x|, which lie in [0, 1]: sig and rest = 1 - sig are 1 / (1 + a) and a / (1 + a) or the other way
+// round, 1 - tanh^2 is 4 b / (1 + b)^2.  As differences from 1 nothing is left of the former from gates of 16 on, of the latter from 8 on; and
+// nothing overflows or is flushed.
 template <int CODE>
 __device__ __forceinline__ void act_eval(float gn, float alpha, float gamma, float& act, float& d, float& dal, float& t5s) {
   if constexpr (CODE == 1 || CODE == 6) {
@@ -97,20 +95,24 @@ __device__ __forceinline__ void act_eval(float gn, float alpha, float gamma, flo
     act = r * r;
     d = 2.0f * r;
   } else {
-    const float e = expf(-gn), sig = rcp_above_1(1.0f + e);
-    if constexpr (CODE == 5) {
-      const float t5 = tanh_of_exp(expf(-2.0f * (alpha * gn)));
-      t5s = t5 * sig;
-      act = gamma * t5s;
-      d = gamma * (alpha * (1.0f - t5 * t5) * sig + t5s * (1.0f - sig));
-      dal = gamma * gn * (1.0f - t5 * t5) * sig;
-    } else if constexpr (CODE == 7) {
-      const float tg = tanh_of_exp(e * e);
-      act = tg * sig;
-      d = (1.0f - tg * tg) * sig + tg * sig * (1.0f - sig);
+    const float a = expf(-fabsf(gn)), r = rcp_near_1(1.0f + a), ar = a * r;
+    const float sig = gn >= 0.0f ? r : ar;
+    if constexpr (CODE == 5 || CODE == 7) {
+      const float rest = gn >= 0.0f ? ar : r, x = CODE == 5 ? alpha * gn : gn;
+      const float b = CODE == 5 ? expf(-2.0f * fabsf(x)) : a * a, h = rcp_near_1(0.5f + 0.5f * b);       // h = 2 / (1 + b)
+      const float t = copysignf((0.5f - 0.5f * b) * h, x), dt = (b * h) * h;                          // tanh(x), 1 - tanh(x)^2
+      const float gs = CODE == 5 ? gamma * sig : sig;
+      act = gs * t;
+      if constexpr (CODE == 5) {
+        d = gs * (alpha * dt + t * rest);
+        dal = gs * gn * dt;
+        t5s = t * sig;
+      } else {
+        d = gs * (dt + t * rest);
+      }
     } else {
       act = gn * sig;
-      d = sig * (1.0f + gn * (1.0f - sig));
+      d = sig * (1.0f + gn * (1.0f - sig));        // (the difference is added to 1)
     }
   }
 }
@@ -249,8 +251,10 @@ __device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (
   }
 }
 
+// The register bounds hold three and two CTAs on an SM: left to itself the compiler took 87 registers for 32 x 2 vectors (32 768 rows of d_ff 256 36 -> 41
+// us) and scheduled three vectors a thread worse (d_ff 768 59 -> 64, 1032 100 -> 113); four are better left alone (4096 rows of d_ff 8192 88 -> 82).
 template <int TPR, int VPT>
-__global__ void __launch_bounds__(kRowThreads)
+__global__ void __launch_bounds__(kRowThreads, VPT == 2 ? 3 : VPT == 3 ? 2 : 0)
 glu_bwd_vec_kernel(const uint4* grad_inter, int pitch, const uint4* gate_up, int pitch2, const int* tile_expert, const int* codes,
                    const float* params, const int* total_rows, int nvec, uint4* grad_gate_up, float* row_da,
                    float* row_dg) {
