@@ -67,3 +67,22 @@ def test_saturated_gates_of_a_norm_code(pkg):
     for name, got, want in (("inter", inter, out.detach()), ("grad_gate", ggu[:, :I], G.grad), ("grad_up", ggu[:, I:], U.grad)):
         err = (got.double() - want).norm() / want.norm()
         assert err < 2.0 ** -9, (name, float(err))            # a rounding to bf16: at most that
+
+
+# 1024 values fill the lanes of a row, 776 and 72 do not, which must change nothing
+@pytest.mark.parametrize("I", [72, 776, 1024])
+@pytest.mark.parametrize("alpha,gamma", [(float("inf"), 1.5), (0.75, float("inf")), (float("-inf"), 1.0)])
+def test_infinite_parameters_reach_the_sums_through_values_only(pkg, I, alpha, gamma):
+    """An infinite alpha saturates tanh: its own gradient is 0 and that of gamma stays a number; an infinite gamma leaves its own gradient a number."""
+    R = 256
+    perm, cd, pr = _rows(R, 5, alpha, gamma)
+    g = torch.Generator(device=DEV).manual_seed(I)
+    gate = ((torch.rand(R, I, generator=g, device=DEV) + 0.5) * (1 - 2 * (torch.rand(R, I, generator=g, device=DEV) < 0.5).float())).bfloat16()
+    up, go = (torch.randn(R, I, generator=g, device=DEV).bfloat16() for _ in range(2))
+    _, da, dg = pkg.ops.glu_bwd_rows(go, torch.cat([gate, up], 1), cd, pr, perm, True)
+    G, w = gate.double(), go.double() * up.double()
+    want = w * torch.tanh(alpha * G) * torch.sigmoid(G)
+    # sums of I fp32 values, each off by a few roundings, in any order
+    assert ((dg.double() - want.sum(1)).abs() <= I * 2.0 ** -23 * want.abs().sum(1)).all()
+    if gamma != float("inf"):
+        assert (da == 0).all()

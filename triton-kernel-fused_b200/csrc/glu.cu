@@ -220,10 +220,11 @@ __device__ __forceinline__ void glu_bwd_row(const uint4 (&g)[VPT], const uint4 (
       float act, d, dal = 0.0f, t5s = 0.0f;
       act_eval<CODE>(gn, alpha, gamma, act, d, dal, t5s);
       const float w = of[j] * uf[j];
-      if constexpr (CODE == 5) {
-        da += w * dal;
-        dg += w * t5s;
-      }
+      if constexpr (CODE == 5)
+        if (c < nvec) {                    // an idle lane's zeros are NaN times an infinite parameter
+          da += w * dal;
+          dg += w * t5s;
+        }
       uf[j] = of[j] * act;
       if constexpr (NORM) {
         wd[i][j] = w * d;
