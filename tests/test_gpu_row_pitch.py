@@ -48,3 +48,23 @@ def test_block_equals_its_steps_over_dense_rows(pkg, T, H, I, E, k, codes):
     for name, a, b in zip(("out", "grad_x", "grad_w", "grad_gate_up", "grad_down"), got, want):
         assert torch.equal(a, b), name
     assert torch.equal(quiet, got[0])
+
+
+# x_s padded and the results dense, both dense, inter padded or dense, all padded; with Identity and Zero experts, whose rows go from one to the other
+@pytest.mark.parametrize("H,I", [(264, 520), (360, 256), (456, 200), (136, 72), (256, 456), (520, 264), (1288, 648)])
+@pytest.mark.parametrize("codes", [(0,), (0, 1, 5), (2, 7, 0, 3, 4)])
+def test_forward_without_backward_equals_the_one_with(pkg, H, I, codes):
+    T, k = 3000, 3
+    g = torch.Generator(device=DEV).manual_seed(H + I)
+    rand = lambda *s: (torch.randn(*s, generator=g, device=DEV) * 0.1).bfloat16()     # noqa: E731
+    E = 5 if 3 in codes else 8
+    n = E - 2 if 3 in codes else E
+    x, gu, dn = rand(T, H), rand(n, 2 * I, H), rand(n, H, I)
+    idx = torch.rand(T, E, generator=g, device=DEV).topk(k, 1).indices
+    w = torch.rand(T, k, generator=g, device=DEV)
+    cd = torch.tensor([codes[e % len(codes)] for e in range(E)], dtype=torch.int32, device=DEV)
+    kept = pkg.moe(x, idx, w, gu.clone().requires_grad_(), dn, cd).detach()
+    torch.full((256 << 20,), float("nan"), device=DEV)           # what the padding holds must not matter
+    with torch.no_grad():
+        assert torch.equal(pkg.moe(x, idx, w, gu, dn, cd), kept)
+    pkg.check_status()

@@ -264,6 +264,22 @@ def test_route_of_a_forward_without_backward():
         assert (quiet < kept) == compact, (E, H, I, k, T)
 
 
+def test_rows_of_a_forward_without_backward_are_padded_where_products_read_them():
+    """With a backward to follow, every buffer's rows lie at whole lines; without, those of x_s and inter where their product has more than 512 columns
+    or they are 448 wide, those of the others where they are 1280 wide.  Told from the workspaces' sizes (rows are multiples of 256, so each difference is exact)."""
+    lib = importlib.import_module(PKG).lib()
+    pitch = lambda n: n if n % 32 == 0 else (n + 63) // 64 * 64     # noqa: E731
+    read = lambda n, cols: pitch(n) if cols > 512 or n >= 448 else n     # noqa: E731
+    written = lambda n: pitch(n) if n >= 1280 else n     # noqa: E731
+    T, E, k = 9000, 16, 4
+    rows = lib.b200moe_padded_rows_cap(T * k, E)
+    for row_kernels in (0, 1):
+        for H, I in ((360, 256), (136, 72), (264, 520), (520, 264), (512, 200), (520, 200), (440, 256), (456, 256), (440, 264), (256, 440), (256, 456), (256, 256), (1288, 648), (1272, 632)):
+            kept, quiet = (lib.b200moe_moe_fwd_ws_bytes(T, H, I, E, E, k, keep, row_kernels) for keep in (1, 0))
+            less = 2 * pitch(H) + pitch(2 * I) + pitch(I) - (read(H, 2 * I) + written(H) + written(2 * I) + read(I, H))
+            assert kept - quiet == 2 * rows * less, (H, I, row_kernels)
+
+
 def test_chained_kernels_promise_no_constant_data():
     """A chained kernel (one with a grid_dep_wait) starts while the kernel before it still writes what it reads: none of its
     pointers may be __restrict__, nothing in its file read through the non-coherent path, and it waits."""

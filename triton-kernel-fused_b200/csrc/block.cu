@@ -35,17 +35,20 @@ enum Kind { KIND_FEW = 0, KIND_TILES = 1, KIND_ROWS = 2 };
 struct Dims {
   int64_t T, H, I;
   int E, n_glu, k;        // routed experts, those with weights, picks per token
+  int keep;               // whether a backward may follow
   Kind kind;
   int64_t M() const { return T * k; }
   int64_t rows() const { return kind == KIND_FEW ? M() : b200moe_padded_rows_cap(M(), E); }
-  // elements between rows of the workspace's buffers (row_pitch; the few-rows kernels take dense ones)
-  int64_t ldh() const { return kind == KIND_FEW ? H : row_pitch(H); }
-  int64_t ldi() const { return kind == KIND_FEW ? I : row_pitch(I); }
-  int64_t ld2() const { return row_pitch(2 * I); }
+  // elements between rows of x_s, of the experts' results and their gradient, of inter, of gate_up (row_pitch; the few-rows kernels take dense ones).
+  // Where no backward follows, a product reads x_s and inter only.
+  int64_t ldx() const { return keep ? row_pitch(H) : kind == KIND_FEW ? H : row_pitch_read(H, 2 * I); }
+  int64_t ldh() const { return keep ? row_pitch(H) : kind == KIND_FEW ? H : row_pitch_written(H); }
+  int64_t ldi() const { return keep ? row_pitch(I) : kind == KIND_FEW ? I : row_pitch_read(I, H); }
+  int64_t ld2() const { return keep ? row_pitch(2 * I) : row_pitch_written(2 * I); }
 };
 
 static Dims make_dims(int64_t T, int64_t H, int64_t I, int E, int n_glu, int k, int keep, int rows_kernels) {
-  Dims d{T, H, I, E, n_glu, k, KIND_TILES};
+  Dims d{T, H, I, E, n_glu, k, keep, KIND_TILES};
   if (rows_kernels) d.kind = KIND_ROWS;
   else if (!keep && T > 0 && k > 0 && E > 0 && few_rows_forward(T * k, E, H, I)) d.kind = KIND_FEW;
   return d;
@@ -91,7 +94,7 @@ static Forward carve_forward(const Dims& d, bool router, void* ws, size_t* bytes
     f.idx = c.take<int64_t>(M);
     f.w = c.take<float>(M);
   }
-  f.x_s = c.take<bf16_t>(rows * d.ldh());
+  f.x_s = c.take<bf16_t>(rows * d.ldx());
   if (!few) f.gate_up = c.take<bf16_t>(rows * d.ld2());
   f.inter = c.take<bf16_t>(rows * d.ldi());
   f.eo = c.take<bf16_t>(rows * d.ldh());
@@ -178,18 +181,18 @@ static int experts_forward(const Dims& d, const void* x, const float* w, const v
     RUN("combine", 1, b200moe_combine(f.eo, w, f.slot_pos, d.T, d.k, d.H, out, st));
     return 0;
   }
-  const int64_t ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
-  RUN("gather_rows", 1, gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, ldh, rows, f.x_s, st));
+  const int64_t ldx = d.ldx(), ldh = d.ldh(), ldi = d.ldi(), ld2 = d.ld2();
+  RUN("gather_rows", 1, gather_rows(x, f.row_slot, f.poffs + d.E, d.k, d.H, ldx, rows, f.x_s, st));
   if (d.kind == KIND_TILES) {
-    RUN("expert_gate_up_swiglu", 1, expert_gate_up(f.x_s, ldh, gate_up_proj, codes, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H, d.I,
+    RUN("expert_gate_up_swiglu", 1, expert_gate_up(f.x_s, ldx, gate_up_proj, codes, f.tile_expert, f.poffs, rows, 0, 0, d.E, d.H, d.I,
                                                    f.gate_up, ld2, f.inter, ldi, status, st));
     RUN("expert_down", 1, expert_linear(f.inter, ldi, down_proj, f.tile_expert, f.poffs, rows, d.E, d.H, d.I, f.eo, ldh, status, st));
   } else {   // the GEMMs and the activation kernels see the rows of the experts with weights only
-    RUN("expert_linear", 1, expert_linear(f.x_s, ldh, gate_up_proj, f.tile_expert, f.poffs, rows, d.n_glu, 2 * d.I, d.H, f.gate_up, ld2, status, st));
+    RUN("expert_linear", 1, expert_linear(f.x_s, ldx, gate_up_proj, f.tile_expert, f.poffs, rows, d.n_glu, 2 * d.I, d.H, f.gate_up, ld2, status, st));
     RUN("glu_fwd_rows", 1, glu_fwd_rows(f.gate_up, ld2, f.tile_expert, codes, params, f.poffs + d.n_glu, rows, d.I, f.inter, ldi, st));
     RUN("expert_linear", 1, expert_linear(f.inter, ldi, down_proj, f.tile_expert, f.poffs, rows, d.n_glu, d.H, d.I, f.eo, ldh, status, st));
     if (d.n_glu < d.E)
-      RUN("special_rows", 1, special_rows(f.x_s, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, ldh, rows, f.eo, st));
+      RUN("special_rows", 1, special_rows(f.x_s, ldx, f.tile_expert, codes, f.poffs, d.n_glu, d.E, d.H, ldh, rows, f.eo, st));
   }
   RUN("combine", 1, combine_add(f.eo, ldh, w, f.slot_row, nullptr, d.T, d.k, d.H, out, st));
   return 0;
@@ -226,7 +229,7 @@ static int experts_backward(const Dims& d, const void* grad_out, const float* w,
     RUN(d.kind == KIND_ROWS ? "expert_linear_t" : "expert_gate_up_dgrad", 1,
         expert_linear_t(b.grad_gu, ld2, gate_up_proj, f.tile_expert, f.poffs, rows, n, 2 * d.I, d.H, 2 * d.I, b.grad_x_s, ldh, status, st));
     if (d.kind == KIND_ROWS && n < d.E)
-      RUN("special_rows", 1, special_rows(b.grad_eo, f.tile_expert, codes, f.poffs, n, d.E, d.H, ldh, rows, b.grad_x_s, st));
+      RUN("special_rows", 1, special_rows(b.grad_eo, ldh, f.tile_expert, codes, f.poffs, n, d.E, d.H, ldh, rows, b.grad_x_s, st));
   }
   if (g.params != nullptr) {
     if (n < d.E)

@@ -33,11 +33,19 @@ int exchange_sm_budget();   // SMs (= fat CTAs) the home-side pull kernel of the
 // quarters of the rate (8.4 against 11.6 TB/s, all from L2; 32 bytes past a line: 10.9), and stores to such rows leave partial sectors: rows whose
 // length is no multiple of 64 bytes are padded to whole lines.  us a training pass, dense / padded: 3001 tokens, 32 experts of 1032 x 680, top-4
 // 370 / 350; 8192 tokens, 32 of 2056 x 1416 2426 / 2023, of 2040 x 1400 2237 / 1873; 8192 tokens, 16 of 1064 x 2088, top-2 880 / 783; 16 384
-// tokens, 64 of 520 x 264, top-6 776 / 722; 2000 tokens, 8 of 264 x 136, top-2 80 / 77.
+// tokens, 64 of 520 x 264, top-6 776 / 722; 2000 tokens, 8 of 264 x 136, top-2 80 / 77.  (Narrow rows grow most: 72 to 128, 8 to 64.)
 inline int64_t row_pitch(int64_t n) { return n % 32 == 0 ? n : (n + 63) / 64 * 64; }
+// The same where no backward follows, for rows of n that one product over `cols` output columns reads (x_s, inter).  Two tiles of 256 columns read them
+// twice only, which at widths below 448 does not pay for the longer rows.  us a forward, all buffers dense / all padded / by this rule: 2571 tokens, 128
+// experts of 360 x 256, top-8 81.7 / 83.2 / 81.6; 20 000 tokens, 16 of 136 x 72, top-4 81.5 / 87.4 / 81.4; 20 000, 64 of 392 x 200, top-6 231 / 240 / 231; 8192,
+// 32 of 1032 x 680, top-4 278 / 249 / 247; 8192, 128 of 264 x 520, top-8 227 / 211 / 212.
+inline int64_t row_pitch_read(int64_t n, int64_t cols) { return cols > 512 || n >= 448 ? row_pitch(n) : n; }
+// ... and for rows that no product reads (gate_up, the experts' results), where only their stores gain: dense / padded 8192 tokens, 32 experts of 1544 x 1032
+// 455 / 450, of 2056 x 1416 736 / 732, of 1032 x 680 257.6 / 259.2; 20 000 tokens, 16 of 520 x 512 263 / 264, 64 of 392 x 200 237 / 240 (the results alone).
+inline int64_t row_pitch_written(int64_t n) { return n >= 1280 ? row_pitch(n) : n; }
 
 // The entry points of the block's steps with the distance between rows given (elements): of x_s, the experts' results and their gradients
-// (ldh), of inter (ldi), of gate_up and its gradient (ld2)
+// (ldh), of inter (ldi), of gate_up and its gradient (ld2), of any other source (lds)
 int gather_rows(const void* x, const int32_t* row_slot, const int32_t* total_rows, int k, int64_t H, int64_t ldh, int64_t rows_cap, void* x_s,
                 b200moe_stream_t stream);
 int combine_add(const void* rows, int64_t ldh, const float* w, const int32_t* slot_row, const void* add, int64_t T, int k, int64_t H, void* out,
@@ -49,8 +57,8 @@ int glu_fwd_rows(const void* gate_up, int64_t ld2, const int32_t* tile_expert, c
 int glu_bwd_rows(const void* grad_inter, int64_t ldi, const void* gate_up, int64_t ld2, const int32_t* tile_expert, const int32_t* act_codes,
                  const float* act_params, const int32_t* total_rows, int64_t rows_cap, int64_t I, void* grad_gate_up, float* row_da, float* row_dg,
                  b200moe_stream_t stream);
-int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special, int num_experts,
-                 int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream);
+int special_rows(const void* src, int64_t lds, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special,
+                 int num_experts, int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream);
 int expert_gate_up(const void* x_s, int64_t ldh, const void* gate_up_proj, const int32_t* act_codes, const int32_t* tile_expert,
                    const int32_t* poffs, int64_t rows_cap, int64_t row_lo, int64_t row_hi, int E, int64_t H, int64_t I, void* gate_up, int64_t ld2,
                    void* inter, int64_t ldi, int32_t* status, b200moe_stream_t stream);

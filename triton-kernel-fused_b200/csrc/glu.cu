@@ -452,7 +452,7 @@ expert_row_sums_kernel(const float* row_da, const float* row_dg, const int* poff
 template <int TPR>
 __global__ void __launch_bounds__(256)
 special_rows_kernel(const uint4* src, const int* tile_expert, const int* codes, const int* poffs, int first_special,
-                    int num_experts, int vec_per_row, int pitch, uint4* dst) {
+                    int num_experts, int vec_per_row, int pitch_src, int pitch, uint4* dst) {
   grid_dep_begin();
   constexpr int G = 256 / TPR;
   const int r0 = poffs[first_special], r1 = poffs[num_experts];
@@ -460,7 +460,7 @@ special_rows_kernel(const uint4* src, const int* tile_expert, const int* codes, 
        r += static_cast<long long>(gridDim.x) * G) {
     const bool copy = codes[tile_expert[r / B200MOE_TILE_M]] == 3;
     for (int c = threadIdx.x % TPR; c < vec_per_row; c += TPR)
-      dst[r * pitch + c] = copy ? src[r * pitch + c] : make_uint4(0u, 0u, 0u, 0u);
+      dst[r * pitch + c] = copy ? src[r * pitch_src + c] : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -540,8 +540,8 @@ int glu_bwd_rows(const void* grad_inter, int64_t ldi, const void* gate_up, int64
   return 0;
 }
 
-int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special, int num_experts,
-                 int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream) {
+int special_rows(const void* src, int64_t lds, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs, int first_special,
+                 int num_experts, int64_t H, int64_t ldh, int64_t rows_cap, void* dst, b200moe_stream_t stream) {
   B200_CHECK_ARG(src && tile_expert && act_codes && poffs && dst, B200MOE_E_NULL, "special_rows: null pointer");
   B200_CHECK_ARG(H > 0 && H % 8 == 0 && first_special >= 0 && first_special <= num_experts, B200MOE_E_BAD_SHAPE,
                  "special_rows: H = %lld, first_special = %d, num_experts = %d", (long long)H, first_special, num_experts);
@@ -551,7 +551,7 @@ int special_rows(const void* src, const int32_t* tile_expert, const int32_t* act
   by_row_threads(static_cast<int>(H / 8), [&](auto tpr) {
     err = launch_chained(special_rows_kernel<tpr.value>, rows_grid(ceil_div64(rows_cap, 256 / tpr.value)), 256, 0,
                          (cudaStream_t)stream, 1, reinterpret_cast<const uint4*>(src), tile_expert, act_codes, poffs,
-                         first_special, num_experts, static_cast<int>(H / 8), static_cast<int>(ldh / 8), reinterpret_cast<uint4*>(dst));
+                         first_special, num_experts, static_cast<int>(H / 8), static_cast<int>(lds / 8), static_cast<int>(ldh / 8), reinterpret_cast<uint4*>(dst));
   });
   B200_CUDA(err);
   return 0;
@@ -586,7 +586,7 @@ int b200moe_expert_row_sums(const float* row_da, const float* row_dg, const int3
 int b200moe_special_rows(const void* src, const int32_t* tile_expert, const int32_t* act_codes, const int32_t* poffs,
                          int first_special, int num_experts, int64_t H, int64_t rows_cap, void* dst,
                          b200moe_stream_t stream) {
-  return special_rows(src, tile_expert, act_codes, poffs, first_special, num_experts, H, H, rows_cap, dst, stream);
+  return special_rows(src, H, tile_expert, act_codes, poffs, first_special, num_experts, H, H, rows_cap, dst, stream);
 }
 
 }  // extern "C"
