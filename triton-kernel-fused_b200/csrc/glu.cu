@@ -477,8 +477,9 @@ constexpr int64_t kMaxVecWidth = 8192;
 static bool rows_in_registers(int64_t I, const void* a, const void* b, const void* c) {
   return I % 8 == 0 && I <= kMaxVecWidth && aligned16(a) && aligned16(b) && aligned16(c);
 }
-// f(TPR, VPT): the narrowest row group that holds nvec vectors, of two or three vectors of each operand a thread, so that at most a
-// third of its lanes is idle (d_ff 768: 32 x 3, 1032: 64 x 3); beside more registers, fewer warps a row need fewer barriers
+// f(TPR, VPT): the narrowest row group that holds nvec vectors, of two or three vectors of each operand a thread: from d_ff 344 on at most
+// a third of its lanes is idle (d_ff 768: 32 x 3, 1032: 64 x 3; d_ff 256 uses half of 32 x 2); beside more registers, fewer warps a row need
+// fewer barriers
 template <class F>
 static void by_row_width(int nvec, F f) {
   auto width = [&](auto tpr) {
